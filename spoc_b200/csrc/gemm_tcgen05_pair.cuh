@@ -10,8 +10,8 @@
 // shared-memory ring holds 6 stages instead of 4 (TF32 mode; 3 instead of 2 in
 // 3xTF32 mode): less L2 bandwidth and 5/6 of 192 KiB in flight per SM.
 //
-// Roles per block: warp 0 lane 0 loads this block's A tile and B half with TMA
-// (completion counted on the leader's `full` barrier); warp 1 lane 0 of the
+// Roles per block: one lane of warp 0 loads this block's A tile and B half with TMA
+// (completion counted on the leader's `full` barrier); one lane of warp 1 of the
 // leader block (cluster rank 0) issues the 256x256x8 MMAs for both blocks and
 // commits to the `empty` and `tmem_full` barriers of both; warps 2-5 of both
 // blocks run the epilogue on their own accumulator rows and hand the
@@ -165,7 +165,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -258,7 +258,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------- MMA issuer (leader block)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = F16 ? umma_idesc_f16(PAIR_BM, BN) : umma_idesc_tf32(PAIR_BM, BN, DIRECT);
       int stage = 0;
       uint32_t phase = 0;
@@ -315,8 +315,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                 }
               }
             }
-            umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 0));
-            umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 1));
+            umma_commit_pair(smem_u32(&empty_bar[stage]));
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1u;
@@ -349,17 +348,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
             }
           }
           // the stage is free in both blocks once these MMAs retire
-          umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 0));
-          umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 1));
+          umma_commit_pair(smem_u32(&empty_bar[stage]));
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) {
-          umma_commit_pair(map_to_cta(smem_u32(&tmem_full_bar[acc]), 0));
-          umma_commit_pair(map_to_cta(smem_u32(&tmem_full_bar[acc]), 1));
-        }
+        if (ok) umma_commit_pair(smem_u32(&tmem_full_bar[acc]));
       }
     }
     __syncwarp();

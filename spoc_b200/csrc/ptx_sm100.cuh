@@ -54,18 +54,37 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s, far above any legitima
 
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                   uint64_t limit_ns = kWaitLimitNs) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_timer_ns();
+  // The clock is read for the first time after 64 attempts: reading %globaltimer after the first failed one put about
+  // 100 ns into every wait that was not already over, and a k-loop waits once per stage.
+  uint64_t t0 = 0;
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (global_timer_ns() - t0 > limit_ns) {
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > limit_ns) {
         *abort_flag = 1;
         return false;
       }
     }
   }
+}
+
+// True in exactly one lane of a converged warp, the same one every time.  The roles that a single thread plays (TMA
+// producer, MMA issuer) branch on this and not on `lane == 0`: the compiler then knows that one thread is active and keeps
+// descriptors and addresses in uniform registers, which tcgen05.mma and the bulk-tensor loads take them from.  With
+// `lane == 0` every MMA cost about 95 issue cycles whatever its size.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.b32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok));
+  return ok != 0;
 }
 
 // -------------------------------------------------------------------- TMA
@@ -271,10 +290,13 @@ __device__ __forceinline__ void umma_tf32_pair_scaled(uint32_t tmem_d, uint64_t 
 __device__ __forceinline__ void umma_f16_pair_scaled(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int scale) {
   SB200_UMMA_SCALED_BODY("f16")
 }
-// Arrive on one mbarrier (a shared::cluster address: this block's or the
-// peer's) once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
+// Arrive on the mbarriers at this shared-memory address in both blocks of the pair once every MMA issued so far by this
+// thread has completed: one instruction instead of a commit per block.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
 }
 
 // Shared-memory matrix descriptor for a K-major operand tile whose rows are
