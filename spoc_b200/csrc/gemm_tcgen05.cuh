@@ -42,8 +42,14 @@ constexpr uint32_t GEMM_A_BYTES = GEMM_BM * GEMM_BK * 4;  // 16 KiB
 constexpr uint32_t GEMM_B_BYTES = GEMM_BN * GEMM_BK * 4;  // 32 KiB
 constexpr uint32_t GEMM_TMEM_COLS = 512;                  // two 256-column accumulators
 constexpr int GEMM_EPI_LD = 36;                           // row stride (floats) of a warp's staging tile: 144 B, 16-byte aligned, conflict-free
-constexpr uint32_t GEMM_EPI_BUF_BYTES = 4 * 32 * GEMM_EPI_LD * 4;  // per-warp 32-row staging tiles
-constexpr uint32_t GEMM_CTRL_BYTES = 256;
+constexpr uint32_t GEMM_EPI_WARP_BYTES = 2 * 32 * 32 * 4;           // per epilogue warp: two 32 x 32 staging tiles
+constexpr uint32_t GEMM_EPI_BUF_BYTES = 4 * GEMM_EPI_WARP_BYTES;
+// control area: pipeline barriers and flags in the first 256 bytes, then per epilogue warp two barriers for tiles of C
+// and, from byte 512, 32 words of the bias and 32 column scales
+constexpr uint32_t GEMM_CTRL_BYTES = 2048;
+constexpr uint32_t GEMM_CTRL_CBAR = 256;
+constexpr uint32_t GEMM_CTRL_COLS = 512;
+static_assert(32 * GEMM_EPI_LD * 4 <= GEMM_EPI_WARP_BYTES, "the staging tile of the vector path fits the warp's buffer");
 
 template <int MODE>
 struct GemmCfg {
@@ -74,6 +80,9 @@ struct GemmParams {
   // Set by the host when D, C, bias and every replica are 16-byte aligned with leading dimensions and N that
   // are multiples of 4: the epilogue then moves 128-bit vectors (four rows of 128 bytes per warp instruction).
   int vec_epilogue;
+  // Set by the host when D (and C) can be addressed by TMA and there are no replicas: the epilogue then stores D, and
+  // fetches C, as 32 x 32 tiles with bulk-tensor copies (epilogue_tma).
+  int tma_epilogue;
   // L2 eviction policies, 2 bits each (0 normal, 1 evict first, 2 evict last): bits 0-1 loads of A (hi and lo),
   // bits 2-3 loads of B, bits 4-5 the epilogue's reads of C and writes of D.
   int l2_policy;
@@ -122,11 +131,140 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tn = within / band_m;
 }
 
-// Epilogue of one warp for its 32 rows x BN columns of a finished accumulator: tensor memory -> registers
-// (lane = row) -> the warp's staging tile in shared memory -> D = act(alpha*acc + beta*C + bias), and the same
-// values to every replica of D.  `taddr` addresses the warp's 32 tensor-memory lanes at the accumulator's
-// first column.  Both GEMM kernels use it; every element goes through the same operations in the same order
-// on either path, so the vector and scalar paths give the same bits.
+// Shared memory of one epilogue warp.
+struct EpiWarp {
+  float* buf;       // two 32 x 32 tiles, 1024-byte aligned (the other paths use it as one staging tile)
+  float* cols;      // 32 words of the bias, 32 column scales
+  uint64_t* c_bar;  // one barrier per tile for the loads of C
+  uint32_t c_phase; // bit b: parity of c_bar[b]
+  int next;         // tile of buf the next chunk uses (runs on from one accumulator to the next)
+};
+
+__device__ __forceinline__ EpiWarp epi_warp(uint8_t* epi_base, uint8_t* ctrl, int w) {
+  EpiWarp e;
+  e.buf = reinterpret_cast<float*>(epi_base + w * GEMM_EPI_WARP_BYTES);
+  e.cols = reinterpret_cast<float*>(ctrl + GEMM_CTRL_COLS + w * 256);
+  e.c_bar = reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + 2 * w;
+  e.c_phase = 0;
+  e.next = 0;
+  return e;
+}
+
+// Fetches one 32 x 32 tile of C into tile b of the warp's buffer, whose earlier store must have been read.
+__device__ __forceinline__ void epi_load_c(const CUtensorMap* map_c, const EpiWarp& e, int b, int col, int row, uint64_t pol) {
+  const uint32_t bar = smem_u32(&e.c_bar[b]);
+  mbar_arrive_expect_tx(bar, 32 * 32 * 4);
+  tma_load_2d_hint(smem_u32(e.buf + b * 1024), map_c, bar, col, row, pol);
+}
+
+// Before the accumulator is awaited: the first tile of C is on its way while the k-loop still runs.
+__device__ __forceinline__ void epilogue_tma_begin(const GemmParams& p, const CUtensorMap* map_c, const EpiWarp& e, int row0, int n0) {
+  if (p.C && row0 < p.M && elect_one()) {
+    bulk_wait_read<0>();
+    epi_load_c(map_c, e, e.next, n0, row0, l2_policy((p.l2_policy >> 4) & 3));
+  }
+  __syncwarp();
+}
+
+// Epilogue of one warp for its 32 rows x BN columns of a finished accumulator, D (and C) moved by TMA: tensor memory ->
+// registers (lane = row), D = act(alpha*acc + beta*C + bias) there, -> a 32 x 32 tile in shared memory in the 128-byte
+// swizzle (no bank conflicts: eight lanes of a phase hit eight 16-byte columns) -> one bulk store per tile, two tiles in
+// turn.  Bound by issue latency of the one warp a scheduler has: a 32-column chunk takes about 300 instructions without
+// any branch per row.  The path it replaced gave lanes quads of columns behind a branch per row and took 0.85 us a chunk
+// (6 us of 16 at 1024 x 1024 x 64 with 256-column tiles) whether it stored or not.
+// Returns false when a wait for C ran out (warp-uniform).
+template <int BN>
+__device__ __forceinline__ bool epilogue_tma(const GemmParams& p, const CUtensorMap* map_d, const CUtensorMap* map_c, uint32_t taddr,
+                                             EpiWarp& e, int lane, int row0, int n0, volatile int* abort_flag) {
+  if (row0 >= p.M) return true;
+  const uint64_t pol = l2_policy((p.l2_policy >> 4) & 3);
+  const int chunks = min(BN / 32, (p.N - n0 + 31) >> 5);
+  const bool scaled = p.row_scale != nullptr;
+  const float rs = scaled && row0 + lane < p.M ? p.row_scale[row0 + lane] : 1.0f;
+#pragma unroll 1
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int b = e.next, col0 = n0 + chunk * 32;
+    e.next ^= 1;
+    uint32_t v[32];
+    tmem_ld_32x32b_x32(taddr + chunk * 32, v);
+    const int col = col0 + lane;
+    float bias_v = 0.0f, scale_v = 1.0f;
+    if (p.bias && col < p.N) bias_v = p.bias[col];
+    if (scaled && col < p.N) scale_v = p.col_scale[col];
+    if (elect_one()) {
+      if (p.C) {
+        if (chunk + 1 < chunks) {
+          bulk_wait_read<0>();  // the store before this chunk read tile b ^ 1
+          epi_load_c(map_c, e, b ^ 1, col0 + 32, row0, pol);
+        }
+      } else {
+        bulk_wait_read<1>();  // the store two chunks ago read tile b
+      }
+    }
+    e.cols[lane] = bias_v;
+    if (scaled) e.cols[32 + lane] = scale_v;
+    __syncwarp();
+    tmem_ld_wait_x32(v);
+    float x[32];
+    if (scaled) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 cs = reinterpret_cast<const float4*>(e.cols + 32)[q];
+        x[4 * q] = __fmul_rn(p.alpha, (__uint_as_float(v[4 * q]) * rs) * cs.x);
+        x[4 * q + 1] = __fmul_rn(p.alpha, (__uint_as_float(v[4 * q + 1]) * rs) * cs.y);
+        x[4 * q + 2] = __fmul_rn(p.alpha, (__uint_as_float(v[4 * q + 2]) * rs) * cs.z);
+        x[4 * q + 3] = __fmul_rn(p.alpha, (__uint_as_float(v[4 * q + 3]) * rs) * cs.w);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = __fmul_rn(p.alpha, __uint_as_float(v[j]));
+    }
+    uint8_t* row = reinterpret_cast<uint8_t*>(e.buf + b * 1024) + lane * 128;
+    const int sw = lane & 7;
+    if (p.C) {
+      const bool landed = mbar_wait_bounded(smem_u32(&e.c_bar[b]), (e.c_phase >> b) & 1u, abort_flag);
+      e.c_phase ^= 1u << b;
+      if (!__all_sync(0xffffffffu, landed)) return false;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 c = *reinterpret_cast<const float4*>(row + ((q ^ sw) << 4));
+        x[4 * q] = fmaf(p.beta, c.x, x[4 * q]);
+        x[4 * q + 1] = fmaf(p.beta, c.y, x[4 * q + 1]);
+        x[4 * q + 2] = fmaf(p.beta, c.z, x[4 * q + 2]);
+        x[4 * q + 3] = fmaf(p.beta, c.w, x[4 * q + 3]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4 bv = reinterpret_cast<const float4*>(e.cols)[q];
+      x[4 * q] = __fadd_rn(x[4 * q], bv.x);
+      x[4 * q + 1] = __fadd_rn(x[4 * q + 1], bv.y);
+      x[4 * q + 2] = __fadd_rn(x[4 * q + 2], bv.z);
+      x[4 * q + 3] = __fadd_rn(x[4 * q + 3], bv.w);
+    }
+    if (p.act == 1) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = (x[j] > 0.0f) ? x[j] : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      *reinterpret_cast<float4*>(row + ((q ^ sw) << 4)) = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+    fence_async_shared();
+    __syncwarp();
+    if (elect_one()) {
+      tma_store_2d_hint(map_d, smem_u32(e.buf + b * 1024), col0, row0, pol);
+      bulk_commit();
+    }
+  }
+  __syncwarp();
+  return true;
+}
+
+// The same epilogue with ordinary loads and stores, for results with replicas (vector path) and for matrices TMA cannot
+// address (general path): tensor memory -> registers (lane = row) -> the warp's staging tile in shared memory ->
+// D = act(alpha*acc + beta*C + bias), and the same values to every replica of D.  `taddr` addresses the warp's 32
+// tensor-memory lanes at the accumulator's first column.  Every element goes through the same operations in the same
+// order on all paths, so they give the same bits.
 template <int BN>
 __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t taddr, float* tbuf, int lane, int row0, int n0) {
   const int rows_here = min(32, p.M - row0);  // may be <= 0 for a ragged last tile
@@ -217,36 +355,24 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t tadd
     if (col < p.N) {
       const float bias_v = p.bias ? p.bias[col] : 0.0f;
       const float cs = p.col_scale ? p.col_scale[col] : 1.0f;
-      if (rows_here >= 32) {
-        // full 32-row slab: issue all 32 loads of C before the first use so that
-        // their latencies overlap instead of adding up
-        float cv[32];
-        if (p.C) {
-          const float* cp = p.C + static_cast<long long>(row0) * p.ldc + col;
+      // all loads of C before the first use so that their latencies overlap instead of adding up
+      float cv[32];
+      if (p.C) {
+        const float* cp = p.C + static_cast<long long>(row0) * p.ldc + col;
 #pragma unroll
-          for (int rr = 0; rr < 32; ++rr) cv[rr] = cp[rr * p.ldc];
-        }
-        float* dp = p.D + static_cast<long long>(row0) * p.ldd + col;
+        for (int rr = 0; rr < 32; ++rr) cv[rr] = rr < rows_here ? cp[rr * p.ldc] : 0.0f;
+      }
+      float* dp = p.D + static_cast<long long>(row0) * p.ldd + col;
 #pragma unroll
-        for (int rr = 0; rr < 32; ++rr) {
-          const float rs = p.row_scale ? p.row_scale[row0 + rr] : 1.0f;
-          float x = p.alpha * ((tbuf[rr * 33 + lane] * rs) * cs);
-          if (p.C) x = fmaf(p.beta, cv[rr], x);
-          x += bias_v;
-          if (p.act == 1) x = (x > 0.0f) ? x : 0.0f;
+      for (int rr = 0; rr < 32; ++rr) {
+        const float rs = p.row_scale && rr < rows_here ? p.row_scale[row0 + rr] : 1.0f;
+        float x = p.alpha * ((tbuf[rr * 33 + lane] * rs) * cs);
+        if (p.C) x = fmaf(p.beta, cv[rr], x);
+        x += bias_v;
+        if (p.act == 1) x = (x > 0.0f) ? x : 0.0f;
+        if (rr < rows_here) {
           dp[rr * p.ldd] = x;
           if (p.n_replicas) store_replicas(p, static_cast<long long>(row0 + rr) * p.ldd + col, x);
-        }
-      } else {
-        for (int rr = 0; rr < rows_here; ++rr) {
-          const long long row = row0 + rr;
-          const float rs = p.row_scale ? p.row_scale[row] : 1.0f;
-          float x = p.alpha * ((tbuf[rr * 33 + lane] * rs) * cs);
-          if (p.C) x = fmaf(p.beta, p.C[row * p.ldc + col], x);
-          x += bias_v;
-          if (p.act == 1) x = (x > 0.0f) ? x : 0.0f;
-          p.D[row * p.ldd + col] = x;
-          if (p.n_replicas) store_replicas(p, row * p.ldd + col, x);
         }
       }
     }
@@ -258,15 +384,16 @@ template <int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_constant__ CUtensorMap map_b_hi,
                  const __grid_constant__ CUtensorMap map_a_lo, const __grid_constant__ CUtensorMap map_b_lo,
-                 const GemmParams p) {
+                 const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   using Cfg = GemmCfg<MODE>;
   constexpr int STAGES = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment is what the 128-byte swizzle pattern is anchored to
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stage_base = smem;
-  float* epi_buf = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes + GEMM_EPI_BUF_BYTES);
+  uint8_t* epi_base = smem + STAGES * Cfg::kStageBytes;
+  uint8_t* ctrl = epi_base + GEMM_EPI_BUF_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ctrl);
   // bars[0..STAGES) full, [STAGES..2*STAGES) empty, then tmem_full[2], tmem_empty[2]
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
@@ -288,10 +415,12 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       mbar_init(smem_u32(&tmem_full_bar[a]), 1);
       mbar_init(smem_u32(&tmem_empty_bar[a]), 4);  // one arrival per epilogue warp
     }
+    for (int i = 0; i < 8; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_a_hi);
     tma_prefetch_desc(&map_b_hi);
+    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
     if (MODE == 3) {
       tma_prefetch_desc(&map_a_lo);
       tma_prefetch_desc(&map_b_lo);
@@ -405,7 +534,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   } else {
     // --------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // tensor-memory lanes [32*quarter, 32*quarter+32)
-    float* tbuf = epi_buf + (warp - 2) * (32 * GEMM_EPI_LD);
+    EpiWarp epi = epi_warp(epi_base, ctrl, warp - 2);
     int local_tile = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
@@ -415,6 +544,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
       const int row0 = tm * GEMM_BM + quarter * 32;
       const int n0 = tn * GEMM_BN;
+      if (p.tma_epilogue) epilogue_tma_begin(p, &map_c, epi, row0, n0);
       // every lane waits; the warp then agrees on the outcome so that the
       // warp-collective tensor-memory loads below are never partly skipped
       const bool landed = mbar_wait_bounded(smem_u32(&tmem_full_bar[acc]), acc_phase, abort_flag);
@@ -424,11 +554,20 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
         break;
       }
       tc_fence_after_sync();
-      epilogue_rows<GEMM_BN>(p, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * GEMM_BN, tbuf, lane, row0, n0);
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * GEMM_BN;
+      if (!p.tma_epilogue) {
+        epilogue_rows<GEMM_BN>(p, taddr, epi.buf, lane, row0, n0);
+      } else if (!epilogue_tma<GEMM_BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, abort_flag)) {
+        if (lane == 0) atomicCAS(p.status, 0, 0x500 | acc);
+        ok = false;
+        break;
+      }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&tmem_empty_bar[acc]));
     }
+    __syncwarp();
+    if (elect_one()) bulk_wait_read<0>();  // the tiles must outlive the stores that read them
     __syncwarp();
   }
 

@@ -81,7 +81,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_constant__ CUtensorMap map_b_hi,
                  const __grid_constant__ CUtensorMap map_a_lo, const __grid_constant__ CUtensorMap map_b_lo,
                  const __grid_constant__ CUtensorMap map_a_x, const __grid_constant__ CUtensorMap map_b_x,
-                 const GemmParams p) {
+                 const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   using Cfg = PairCfg<MODE, BN>;
   constexpr bool MIXED = MODE == 5;
   static_assert(!MIXED || DIRECT, "the mixed mode reads the main term's operands where they lie");
@@ -99,8 +99,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stage_base = smem;
-  float* epi_buf = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes + GEMM_EPI_BUF_BYTES);
+  uint8_t* epi_base = smem + STAGES * Cfg::kStageBytes;
+  uint8_t* ctrl = epi_base + GEMM_EPI_BUF_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ctrl);
   uint64_t* full_bar = bars;                        // used in the leader only
   uint64_t* empty_bar = bars + STAGES;              // one set per block
   uint64_t* tmem_full_bar = bars + 2 * STAGES;      // one set per block
@@ -124,10 +125,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       mbar_init(smem_u32(&tmem_full_bar[a]), 1);
       mbar_init(smem_u32(&tmem_empty_bar[a]), 8);  // four epilogue warps in each of the two blocks
     }
+    for (int i = 0; i < 8; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_a_hi);
     tma_prefetch_desc(&map_b_hi);
+    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
     if (THREE || MIXED) {
       tma_prefetch_desc(&map_a_lo);
       tma_prefetch_desc(&map_b_lo);
@@ -361,7 +364,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   } else {
     // --------------------------------------------------------- epilogue
     const int quarter = warp & 3;
-    float* tbuf = epi_buf + (warp - 2) * (32 * GEMM_EPI_LD);
+    EpiWarp epi = epi_warp(epi_base, ctrl, warp - 2);
     int local_tile = 0;
     bool ok = true;
     for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
@@ -371,6 +374,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       pair_tile_coords(tile, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
       const int row0 = tm * PAIR_BM + static_cast<int>(rank) * 128 + quarter * 32;
       const int n0 = tn * BN;
+      if (p.tma_epilogue) epilogue_tma_begin(p, &map_c, epi, row0, n0);
       const bool landed = mbar_wait_bounded(smem_u32(&tmem_full_bar[acc]), acc_phase, abort_flag);
       if (!__all_sync(0xffffffffu, landed)) {
         if (lane == 0) atomicCAS(p.status, 0, 0x1400 | (rank << 4) | acc);
@@ -378,11 +382,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
         break;
       }
       tc_fence_after_sync();
-      epilogue_rows<BN>(p, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN, tbuf, lane, row0, n0);
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+      if (!p.tma_epilogue) {
+        epilogue_rows<BN>(p, taddr, epi.buf, lane, row0, n0);
+      } else if (!epilogue_tma<BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, abort_flag)) {
+        if (lane == 0) atomicCAS(p.status, 0, 0x1500 | (rank << 4) | acc);
+        ok = false;
+        break;
+      }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
     }
+    __syncwarp();
+    if (elect_one()) bulk_wait_read<0>();  // the tiles must outlive the stores that read them
     __syncwarp();
   }
 

@@ -359,6 +359,19 @@ void derive_params(GemmParams* gp) {
   gp->l2_policy = l2_policy_setting();
 }
 
+// Tensor maps of D and C for the epilogue that moves them by TMA; sets gp->tma_epilogue when it applies: 16-byte aligned
+// matrices and row strides, N a multiple of 4 (a store clips its columns at 16-byte granularity only), no replicas.  Otherwise the maps are left as `filler`.
+void epilogue_maps(GemmParams* gp, const CUtensorMap& filler, CUtensorMap* map_d, CUtensorMap* map_c) {
+  *map_d = filler;
+  *map_c = filler;
+  auto fits = [](const void* q, long long ld) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (ld & 3) == 0 && ld < (1ll << 36); };
+  gp->tma_epilogue = 0;
+  if (gp->n_replicas || (gp->N & 3) || !fits(gp->D, gp->ldd) || (gp->C && !fits(gp->C, gp->ldc))) return;
+  if (encode_map_2d(map_d, gp->D, gp->N, gp->M, gp->ldd, 32, 32, false)) return;
+  if (gp->C && encode_map_2d(map_c, gp->C, gp->N, gp->M, gp->ldc, 32, 32, false)) return;
+  gp->tma_epilogue = 1;
+}
+
 // The epoch counters for one launch of the CTA-pair kernel, zeroed on `st` — or null when the lockstep is off: k-loops
 // below 128 stages (K < 4096: two epochs at most, nothing to hold together), SAREK_B200_LOCKSTEP=0, or no memory for the
 // rings.  Measured in the sustained loop at 8192^3: 245 against 221-227 TFLOP/s in alternating runs on one box, the SM
@@ -499,8 +512,10 @@ int launch_pair(DeviceState& d, int dev_index, cudaStream_t st, const CUtensorMa
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
+  CUtensorMap map_d, map_c;
+  epilogue_maps(&gp, ma_hi, &map_d, &map_c);
   CU_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<MODE, DIRECT, BN>, ma_hi, mb_hi, ma_lo, mb_lo, ma_x ? *ma_x : ma_lo,
-                            mb_x ? *mb_x : mb_lo, gp));
+                            mb_x ? *mb_x : mb_lo, map_d, map_c, gp));
   return launch_check("gemm_pair_kernel");
 }
 
@@ -707,7 +722,9 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
                                   static_cast<int>(Cfg::kSmemBytes)));
       attr_set[dev_index].store(1);
     }
-    gemm_tf32_kernel<MODE><<<grid, GEMM_THREADS, Cfg::kSmemBytes, st>>>(ma_hi, mb_hi, ma_lo, mb_lo, gp);
+    CUtensorMap map_d, map_c;
+    epilogue_maps(&gp, ma_hi, &map_d, &map_c);
+    gemm_tf32_kernel<MODE><<<grid, GEMM_THREADS, Cfg::kSmemBytes, st>>>(ma_hi, mb_hi, ma_lo, mb_lo, map_d, map_c, gp);
     rc = launch_check("gemm_tf32_kernel");
   }
   if (prof) {
@@ -2576,7 +2593,9 @@ int launch_gemm_fixed_scratch(const NoAllocDevice& nd, cudaStream_t st, long lon
   derive_params(&gp);
   const long long tiles = static_cast<long long>(gp.tiles_m) * gp.tiles_n;
   const unsigned grid = static_cast<unsigned>(tiles < nd.sm_count ? tiles : nd.sm_count);
-  gemm_tf32_kernel<MODE><<<grid, GEMM_THREADS, Cfg::kSmemBytes, st>>>(ma_hi, mb_hi, ma_lo, mb_lo, gp);
+  CUtensorMap map_d, map_c;
+  epilogue_maps(&gp, ma_hi, &map_d, &map_c);
+  gemm_tf32_kernel<MODE><<<grid, GEMM_THREADS, Cfg::kSmemBytes, st>>>(ma_hi, mb_hi, ma_lo, mb_lo, map_d, map_c, gp);
   return launch_check("gemm_tf32_kernel");
 }
 
