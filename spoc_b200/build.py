@@ -1,4 +1,4 @@
-"""Build step: compiles libsarek_b200.so (CUDA, sm_100a only) in-tree.
+"""Build step: compiles libsarek_b200.so (CUDA, sm_100a only) and the extension _hostpath.so in-tree.
 
 Run as ``python -m spoc_b200.build``.  nvcc cross-compiles without a GPU.
 """
@@ -8,10 +8,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsarek_b200.so")
+HOSTPATH = os.path.join(HERE, "_hostpath.so")   # CPython extension: the marshalling half of run_vectors
 
 SOURCES = ["sb200_shim.cu", "sb200_group.cu", "ir.cc", "fusion.cc", "map_jit.cc", "transfer.cc"]
 HEADERS = ["gemm_tcgen05.cuh", "gemm_tcgen05_pair.cuh", "map_fused.cuh", "ptx_sm100.cuh", "ir.hpp", "map_jit.hpp", "transfer.hpp", "internal.hpp",
@@ -38,6 +40,7 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
+    build_hostpath(force)
     deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS] + [os.path.abspath(__file__)]
     if not force and not _stale(LIB, deps):
         return LIB
@@ -48,6 +51,17 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     if verbose:
         sys.stderr.write(res.stderr)
     return LIB
+
+
+def build_hostpath(force: bool = False) -> str:
+    src = os.path.join(CSRC, "hostpath.c")
+    if not force and not _stale(HOSTPATH, [src, os.path.join(HERE, "..", "include", "sb200.h"), os.path.abspath(__file__)]):
+        return HOSTPATH
+    cmd = ["gcc", "-std=gnu11", "-O2", "-Wall", "-Wextra", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], src, "-o", HOSTPATH]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("gcc failed:\n" + res.stdout + res.stderr)
+    return HOSTPATH
 
 
 if __name__ == "__main__":

@@ -77,7 +77,7 @@ bool debug_kernel() {
 
 struct DeviceState {
   std::mutex mu;
-  bool ready = false;
+  std::atomic<bool> ready{false};
   int sm_count = 0;
   int cc_major = 0;
   void* workspace = nullptr;
@@ -86,6 +86,7 @@ struct DeviceState {
   cudaEvent_t ws_event = nullptr;
   cudaStream_t ws_last_stream = nullptr;
   bool ws_in_use = false;
+  bool ws_event_due = false;  // the last user was stream 0: its event is recorded when another stream needs it
   // held by a call from the moment it sizes the scratch until its launches are enqueued and its event recorded, so
   // that another host thread cannot free and regrow the scratch under launches that already point into it
   std::mutex scratch_mu;
@@ -120,6 +121,11 @@ std::once_flag g_encode_once;
 
 int device_ready(int dev, DeviceState** out) {
   if (dev < 0 || dev >= kMaxDevices) return fail(SB200_ERR_INVALID_VALUE, "device index %d out of range", dev);
+  if (g_dev[dev].ready.load(std::memory_order_acquire)) {  // every call but a device's first
+    CU_TRY(cudaSetDevice(dev));
+    *out = &g_dev[dev];
+    return SB200_OK;
+  }
   int count = 0;
   cudaError_t e = cudaGetDeviceCount(&count);
   if (e != cudaSuccess || count == 0) {
@@ -140,7 +146,7 @@ int device_ready(int dev, DeviceState** out) {
     d.cc_major = prop.major;
     CU_TRY(cudaMalloc(&d.status, sizeof(int)));
     CU_TRY(cudaMemset(d.status, 0, sizeof(int)));
-    d.ready = true;
+    d.ready.store(true, std::memory_order_release);
   }
   *out = &d;
   return SB200_OK;
@@ -162,17 +168,24 @@ int check_status_word(DeviceState& d, bool device_wide = false) {
 
 // An operand that lies inside a buffer this library allocated must end inside it too; operands in memory from
 // elsewhere (another allocator's) are taken at the caller's word.  Turns a wrong size into an error instead of a fault.
-int check_extent(DeviceState& d, uint64_t ptr, uint64_t bytes, const char* what) {
-  if (!ptr || bytes == 0) return SB200_OK;
+// *left: bytes between ptr and the end of the buffer it lies in (when false is returned).
+bool extent_ok(DeviceState& d, uint64_t ptr, uint64_t bytes, uint64_t* left = nullptr) {
+  if (!ptr || bytes == 0) return true;
   std::lock_guard<std::mutex> lock(d.mu);
   auto it = d.allocs.upper_bound(ptr);
-  if (it == d.allocs.begin()) return SB200_OK;
+  if (it == d.allocs.begin()) return true;
   --it;
-  if (ptr >= it->first + it->second) return SB200_OK;  // not inside one of ours
-  if (ptr + bytes > it->first + it->second)
-    return fail(SB200_ERR_BOUNDS, "%s needs %llu bytes from its address but the buffer it lies in ends after %llu", what,
-                static_cast<unsigned long long>(bytes), static_cast<unsigned long long>(it->first + it->second - ptr));
-  return SB200_OK;
+  if (ptr >= it->first + it->second) return true;  // not inside one of ours
+  if (ptr + bytes <= it->first + it->second) return true;
+  if (left) *left = it->first + it->second - ptr;
+  return false;
+}
+
+int check_extent(DeviceState& d, uint64_t ptr, uint64_t bytes, const char* what) {
+  uint64_t left = 0;
+  if (extent_ok(d, ptr, bytes, &left)) return SB200_OK;
+  return fail(SB200_ERR_BOUNDS, "%s needs %llu bytes from its address but the buffer it lies in ends after %llu", what,
+              static_cast<unsigned long long>(bytes), static_cast<unsigned long long>(left));
 }
 
 inline cudaStream_t as_stream(uint64_t s) { return reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(s)); }
@@ -280,6 +293,32 @@ int ensure_workspace(DeviceState& d, size_t bytes) {
   }
   CU_TRY(cudaMalloc(&d.workspace, bytes));
   d.workspace_bytes = bytes;
+  return SB200_OK;
+}
+
+// Order of the calls that use the scratch, across streams: `st` waits for the last user when that was another stream.
+// Stream 0 exists as long as the process does, so the event behind its launches is only recorded when another stream asks
+// for it; a stream of the caller's may be destroyed at any time and records its event at once.
+int scratch_acquire(DeviceState& d, cudaStream_t st) {
+  std::lock_guard<std::mutex> lock(d.mu);
+  if (!d.ws_in_use || d.ws_last_stream == st) return SB200_OK;
+  if (d.ws_event_due) {
+    if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
+    CU_TRY(cudaEventRecord(d.ws_event, d.ws_last_stream));
+    d.ws_event_due = false;
+  }
+  CU_TRY(cudaStreamWaitEvent(st, d.ws_event, 0));
+  return SB200_OK;
+}
+
+int scratch_release(DeviceState& d, cudaStream_t st) {
+  std::lock_guard<std::mutex> lock(d.mu);
+  d.ws_last_stream = st;
+  d.ws_in_use = true;
+  d.ws_event_due = st == nullptr;
+  if (st == nullptr) return SB200_OK;
+  if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
+  CU_TRY(cudaEventRecord(d.ws_event, st));
   return SB200_OK;
 }
 
@@ -620,8 +659,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     }
     track_scratch = cap == cudaStreamCaptureStatusNone;
     if (track_scratch) {
-      std::lock_guard<std::mutex> lock(d.mu);
-      if (d.ws_in_use && d.ws_last_stream != st) CU_TRY(cudaStreamWaitEvent(st, d.ws_event, 0));
+      if ((rc = scratch_acquire(d, st))) return rc;
     }
   }
   unsigned int* epoch_ring = pair ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
@@ -733,11 +771,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     d.prof.push_back(rec);
   }
   if (track_scratch && rc == SB200_OK) {
-    std::lock_guard<std::mutex> lock(d.mu);
-    if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
-    CU_TRY(cudaEventRecord(d.ws_event, st));
-    d.ws_last_stream = st;
-    d.ws_in_use = true;
+    rc = scratch_release(d, st);
   }
   return rc;
 }
@@ -780,8 +814,7 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
   }
   const bool track_scratch = cap == cudaStreamCaptureStatusNone;
   if (track_scratch) {
-    std::lock_guard<std::mutex> lock(d.mu);
-    if (d.ws_in_use && d.ws_last_stream != st) CU_TRY(cudaStreamWaitEvent(st, d.ws_event, 0));
+    if ((rc = scratch_acquire(d, st))) return rc;
   }
   unsigned int* epoch_ring = next_epoch_ring(d, st, kp / 64);
   const bool prof = g_profiling.load() != 0;
@@ -864,11 +897,7 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
     d.prof.push_back(rec);
   }
   if (track_scratch && rc == SB200_OK) {
-    std::lock_guard<std::mutex> lock(d.mu);
-    if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
-    CU_TRY(cudaEventRecord(d.ws_event, st));
-    d.ws_last_stream = st;
-    d.ws_in_use = true;
+    rc = scratch_release(d, st);
   }
   return rc;
 }
@@ -910,8 +939,7 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
   }
   const bool track_scratch = cap == cudaStreamCaptureStatusNone;
   if (track_scratch) {
-    std::lock_guard<std::mutex> lock(d.mu);
-    if (d.ws_in_use && d.ws_last_stream != st) CU_TRY(cudaStreamWaitEvent(st, d.ws_event, 0));
+    if ((rc = scratch_acquire(d, st))) return rc;
   }
   unsigned int* epoch_ring = next_epoch_ring(d, st, 2 * (kp / 64) + 4);
   const bool prof = g_profiling.load() != 0;
@@ -997,11 +1025,7 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     d.prof.push_back(rec);
   }
   if (track_scratch && rc == SB200_OK) {
-    std::lock_guard<std::mutex> lock(d.mu);
-    if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
-    CU_TRY(cudaEventRecord(d.ws_event, st));
-    d.ws_last_stream = st;
-    d.ws_in_use = true;
+    rc = scratch_release(d, st);
   }
   return rc;
 }
@@ -1972,9 +1996,11 @@ static int kernel_launch_impl(uint64_t kernel, const sb200_arg* args, int nargs,
   // whatever length the caller passes with it
   for (size_t p = 0; p < slots.size(); ++p) {
     if (!slots[p].is_vec) continue;
+    const uint64_t bytes = static_cast<uint64_t>(slots[p].len) * 4;
+    if (extent_ok(*d, slots[p].ptr, bytes)) continue;
     const std::string what = "kernel '" + k->plan.name + "': vector " + k->plan.params[p].name + " of stated length " +
                              std::to_string(slots[p].len);
-    if ((rc = check_extent(*d, slots[p].ptr, static_cast<uint64_t>(slots[p].len) * 4, what.c_str()))) return rc;
+    if ((rc = check_extent(*d, slots[p].ptr, bytes, what.c_str()))) return rc;
   }
   if (debug_kernel())
     fprintf(stderr, "[sarek-b200] launch %s grid=(%u,%u,%u) block=(%u,%u,%u)\n", k->plan.description.c_str(), grid[0], grid[1],

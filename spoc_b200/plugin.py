@@ -556,10 +556,39 @@ class Vector:
                 self.location = Vector.CPU
 
 
+_hostpath_module = None
+
+
+def _hostpath():
+    """The native marshaller (csrc/hostpath.c), bound to the library on first use.  Like the library it has to be built."""
+    global _hostpath_module
+    if _hostpath_module is None:
+        lib = L.load()
+        try:
+            from . import _hostpath as m
+        except ImportError as e:
+            raise L.LibraryMissing(f"spoc_b200/_hostpath.so is missing or does not load ({e}): build it with "
+                                   "`python -m spoc_b200.build`") from e
+        m.bind(C.cast(lib.sb200_kernel_launch, C.c_void_p).value, Vector)
+        _hostpath_module = m
+    return _hostpath_module
+
+
 def run_vectors(backend: Backend, *, device: _Device.T, ir: str, args: Sequence, block: Dims, grid: Dims,
                 shared_mem: int = 0, kernel_name: str = "sarek_kern") -> None:
     """Sarek.Execute.run_vectors: args are Vector objects or ("int32"|"int64"|
     "float32"|"float64", value) pairs in the kernel's parameter order."""
+    # A kernel that has run before, on vectors that are on the device: marshalled natively.  Anything else (first launch,
+    # uploads, pinned vectors, results on their way back, a backend of another class) takes the path below.
+    if type(backend) is Backend:
+        k = backend.Kernel._cache.get((device.id, ir))
+        if k is not None:
+            rc = _hostpath().launch(k.handle, args, block, grid, shared_mem)
+            if rc is not None:
+                backend.Device._current = device.id
+                if rc:
+                    _check(rc)
+                return
     rs_args = []
     uploaded = []
     prefetch = os.environ.get("SAREK_B200_PREFETCH_RESULTS", "1") != "0"
