@@ -8,20 +8,11 @@
 // makes a round trip through HBM.
 //
 // Two stages:
-//  1. operand preparation (prep_a_kernel / prep_b_kernel): A and B are split
-//     into TF32-exact panels  hi = rn_tf32(x),  lo = rn_tf32(x - hi)  (lo only
-//     in 3xTF32 mode).  B is transposed on the way so both panels are K-major,
-//     and K is zero-padded to a multiple of 32 so every TMA box starts on a
-//     128-byte boundary whatever K is.
-//  2. gemm_tf32_kernel: a persistent, warp-specialised kernel, one block per
-//     SM.  Warp 0 streams 128x32 (A) and 256x32 (B) fp32 tiles into a ring of
-//     shared-memory stages with TMA (128-byte swizzle, no cluster forms);
-//     warp 1 issues tcgen05.mma kind::tf32 128x256x8 into one of two 256-column
-//     fp32 accumulators in tensor memory; warps 2-5 read the finished
-//     accumulator back with tcgen05.ld, apply the epilogue and store D while
-//     the MMA warp already works on the next tile.
-//     3xTF32 mode issues  lo*hi + hi*lo + hi*hi  per k-step into the same
-//     accumulator (the lo*lo term, ~2^-22 relative, is dropped).
+//  1. operand preparation, where it is needed: A and B split into TF32-exact panels  hi = rn_tf32(x),  lo = rn_tf32(x - hi)
+//     (prep_a_kernel / prep_b_kernel: K-major, B transposed on the way, K zero-padded to a multiple of 32), or the low parts
+//     alone (prep_lo_two_kernel), or fp16 panels.
+//  2. gemm_pair_kernel (gemm_tcgen05_pair.cuh).
+// This file has the preparation kernels, the parameters and the epilogue.
 //
 // Work per launch: 2*M*N*K useful flops (3x that in MMA flops in 3xTF32
 // mode); the bound is the tensor pipe.
@@ -33,13 +24,9 @@
 namespace sb200 {
 
 constexpr int GEMM_BM = 128;
-constexpr int GEMM_BN = 256;
 constexpr int GEMM_BK = 32;      // floats per k-block = one 128-byte swizzle row
 constexpr int GEMM_UMMA_K = 8;   // floats per tcgen05.mma kind::tf32 (32 bytes)
 constexpr int GEMM_THREADS = 192;
-constexpr int GEMM_GROUP_M = 16;  // tile rasterisation: bands of 16 row tiles
-constexpr uint32_t GEMM_A_BYTES = GEMM_BM * GEMM_BK * 4;  // 16 KiB
-constexpr uint32_t GEMM_B_BYTES = GEMM_BN * GEMM_BK * 4;  // 32 KiB
 constexpr uint32_t GEMM_TMEM_COLS = 512;                  // two 256-column accumulators
 constexpr int GEMM_EPI_LD = 36;                           // row stride (floats) of a warp's staging tile: 144 B, 16-byte aligned, conflict-free
 constexpr uint32_t GEMM_EPI_WARP_BYTES = 2 * 32 * 32 * 4;           // per epilogue warp: two 32 x 32 staging tiles
@@ -50,14 +37,6 @@ constexpr uint32_t GEMM_CTRL_BYTES = 2048;
 constexpr uint32_t GEMM_CTRL_CBAR = 256;
 constexpr uint32_t GEMM_CTRL_COLS = 512;
 static_assert(32 * GEMM_EPI_LD * 4 <= GEMM_EPI_WARP_BYTES, "the staging tile of the vector path fits the warp's buffer");
-
-template <int MODE>
-struct GemmCfg {
-  static constexpr int kOperands = (MODE == 3) ? 2 : 1;  // hi (+ lo)
-  static constexpr int kStages = (MODE == 3) ? 2 : 4;
-  static constexpr uint32_t kStageBytes = kOperands * (GEMM_A_BYTES + GEMM_B_BYTES);
-  static constexpr uint32_t kSmemBytes = kStages * kStageBytes + GEMM_EPI_BUF_BYTES + GEMM_CTRL_BYTES + 1024;
-};
 
 struct GemmParams {
   int M, N;
@@ -80,6 +59,8 @@ struct GemmParams {
   // Set by the host when D, C, bias and every replica are 16-byte aligned with leading dimensions and N that
   // are multiples of 4: the epilogue then moves 128-bit vectors (four rows of 128 bytes per warp instruction).
   int vec_epilogue;
+  // Work items a tile's k-loop is divided into (1: not divided), k-blocks of each, and rows of one partial result.
+  int splits, split_k_blocks, part_rows;
   // Set by the host when D (and C) can be addressed by TMA and there are no replicas: the epilogue then stores D, and
   // fetches C, as 32 x 32 tiles with bulk-tensor copies (epilogue_tma).
   int tma_epilogue;
@@ -119,16 +100,6 @@ struct MixCtl {
 __device__ __forceinline__ void store_replicas(const GemmParams& p, long long offset, float x) {
 #pragma unroll 1
   for (int r = 0; r < p.n_replicas; ++r) p.replicas[r][offset] = x;
-}
-
-__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  const int band_tiles = GEMM_GROUP_M * tiles_n;
-  const int band = tile / band_tiles;
-  const int within = tile - band * band_tiles;
-  const int first_m = band * GEMM_GROUP_M;
-  const int band_m = min(GEMM_GROUP_M, tiles_m - first_m);
-  tm = first_m + within % band_m;
-  tn = within / band_m;
 }
 
 // Shared memory of one epilogue warp.
@@ -172,10 +143,11 @@ __device__ __forceinline__ void epilogue_tma_begin(const GemmParams& p, const CU
 // turn.  Bound by issue latency of the one warp a scheduler has: a 32-column chunk takes about 300 instructions without
 // any branch per row.  The path it replaced gave lanes quads of columns behind a branch per row and took 0.85 us a chunk
 // (6 us of 16 at 1024 x 1024 x 64 with 256-column tiles) whether it stored or not.
+// row_shift: added to the row that is stored to (partial results of a divided k-loop lie below one another).
 // Returns false when a wait for C ran out (warp-uniform).
 template <int BN>
 __device__ __forceinline__ bool epilogue_tma(const GemmParams& p, const CUtensorMap* map_d, const CUtensorMap* map_c, uint32_t taddr,
-                                             EpiWarp& e, int lane, int row0, int n0, volatile int* abort_flag) {
+                                             EpiWarp& e, int lane, int row0, int n0, int row_shift, volatile int* abort_flag) {
   if (row0 >= p.M) return true;
   const uint64_t pol = l2_policy((p.l2_policy >> 4) & 3);
   const int chunks = min(BN / 32, (p.N - n0 + 31) >> 5);
@@ -252,7 +224,7 @@ __device__ __forceinline__ bool epilogue_tma(const GemmParams& p, const CUtensor
     fence_async_shared();
     __syncwarp();
     if (elect_one()) {
-      tma_store_2d_hint(map_d, smem_u32(e.buf + b * 1024), col0, row0, pol);
+      tma_store_2d_hint(map_d, smem_u32(e.buf + b * 1024), col0, row0 + row_shift, pol);
       bulk_commit();
     }
   }
@@ -341,241 +313,54 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t tadd
     }
     return;
   }
-  // general path: any alignment, any N; the tile is staged transposed so that lane = column
+  // general path: any alignment, any N; the tile is staged transposed so that lane = column.  No branch per row: rows past
+  // the end are predicated off, the row scale is applied by the row's lane on the way into the staging tile, and replicas are
+  // written in a loop of their own.
+  const float rs = p.row_scale && lane < rows_here ? p.row_scale[row0 + lane] : 1.0f;
 #pragma unroll 1
   for (int chunk = 0; chunk < BN / 32; ++chunk) {
     const int col = n0 + chunk * 32 + lane;
     if (n0 + chunk * 32 >= p.N) break;  // warp-uniform
     uint32_t v[32];
     tmem_ld_32x32b_x32(taddr + chunk * 32, v);
-    tmem_ld_wait();
+    tmem_ld_wait_x32(v);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) tbuf[lane * 33 + j] = __uint_as_float(v[j]);
+    for (int j = 0; j < 32; ++j) tbuf[lane * 33 + j] = __uint_as_float(v[j]) * rs;
     __syncwarp();
     if (col < p.N) {
       const float bias_v = p.bias ? p.bias[col] : 0.0f;
       const float cs = p.col_scale ? p.col_scale[col] : 1.0f;
-      // all loads of C before the first use so that their latencies overlap instead of adding up
-      float cv[32];
+      float x[32];
+#pragma unroll
+      for (int rr = 0; rr < 32; ++rr) x[rr] = __fmul_rn(p.alpha, tbuf[rr * 33 + lane] * cs);
       if (p.C) {
+        // all loads of C before the first use so that their latencies overlap instead of adding up
         const float* cp = p.C + static_cast<long long>(row0) * p.ldc + col;
+        float cv[32];
 #pragma unroll
         for (int rr = 0; rr < 32; ++rr) cv[rr] = rr < rows_here ? cp[rr * p.ldc] : 0.0f;
+#pragma unroll
+        for (int rr = 0; rr < 32; ++rr) x[rr] = fmaf(p.beta, cv[rr], x[rr]);
       }
-      float* dp = p.D + static_cast<long long>(row0) * p.ldd + col;
 #pragma unroll
       for (int rr = 0; rr < 32; ++rr) {
-        const float rs = p.row_scale && rr < rows_here ? p.row_scale[row0 + rr] : 1.0f;
-        float x = p.alpha * ((tbuf[rr * 33 + lane] * rs) * cs);
-        if (p.C) x = fmaf(p.beta, cv[rr], x);
-        x += bias_v;
-        if (p.act == 1) x = (x > 0.0f) ? x : 0.0f;
-        if (rr < rows_here) {
-          dp[rr * p.ldd] = x;
-          if (p.n_replicas) store_replicas(p, static_cast<long long>(row0 + rr) * p.ldd + col, x);
-        }
+        x[rr] = __fadd_rn(x[rr], bias_v);
+        if (p.act == 1) x[rr] = (x[rr] > 0.0f) ? x[rr] : 0.0f;
       }
-    }
-    __syncwarp();
-  }
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_constant__ CUtensorMap map_b_hi,
-                 const __grid_constant__ CUtensorMap map_a_lo, const __grid_constant__ CUtensorMap map_b_lo,
-                 const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
-  using Cfg = GemmCfg<MODE>;
-  constexpr int STAGES = Cfg::kStages;
-  extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment is what the 128-byte swizzle pattern is anchored to
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* stage_base = smem;
-  uint8_t* epi_base = smem + STAGES * Cfg::kStageBytes;
-  uint8_t* ctrl = epi_base + GEMM_EPI_BUF_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ctrl);
-  // bars[0..STAGES) full, [STAGES..2*STAGES) empty, then tmem_full[2], tmem_empty[2]
-  uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + STAGES;
-  uint64_t* tmem_full_bar = bars + 2 * STAGES;
-  uint64_t* tmem_empty_bar = bars + 2 * STAGES + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int num_tiles = p.tiles_m * p.tiles_n;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), 1);
-      mbar_init(smem_u32(&empty_bar[s]), 1);
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(smem_u32(&tmem_full_bar[a]), 1);
-      mbar_init(smem_u32(&tmem_empty_bar[a]), 4);  // one arrival per epilogue warp
-    }
-    for (int i = 0; i < 8; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
-    *abort_flag = 0;
-    mbar_fence_init();
-    tma_prefetch_desc(&map_a_hi);
-    tma_prefetch_desc(&map_b_hi);
-    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
-    if (MODE == 3) {
-      tma_prefetch_desc(&map_a_lo);
-      tma_prefetch_desc(&map_b_lo);
-    }
-  }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), GEMM_TMEM_COLS);
-    tmem_relinquish();
-    tc_fence_before_sync();
-  }
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == 0) {
-    // ------------------------------------------------------ TMA producer
-    if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int tm, tn;
-        tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
-        const int m0 = tm * GEMM_BM, n0 = tn * GEMM_BN;
-        for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!mbar_wait_bounded(smem_u32(&empty_bar[stage]), phase ^ 1u, abort_flag)) {
-            atomicCAS(p.status, 0, 0x100 | stage);
-            ok = false;
-            break;
-          }
-          const uint32_t bar = smem_u32(&full_bar[stage]);
-          uint8_t* sp = stage_base + stage * Cfg::kStageBytes;
-          mbar_arrive_expect_tx(bar, Cfg::kStageBytes);
-          tma_load_2d(smem_u32(sp), &map_a_hi, bar, kb * GEMM_BK, m0);
-          tma_load_2d(smem_u32(sp + GEMM_A_BYTES), &map_b_hi, bar, kb * GEMM_BK, n0);
-          if (MODE == 3) {
-            tma_load_2d(smem_u32(sp + GEMM_A_BYTES + GEMM_B_BYTES), &map_a_lo, bar, kb * GEMM_BK, m0);
-            tma_load_2d(smem_u32(sp + 2 * GEMM_A_BYTES + GEMM_B_BYTES), &map_b_lo, bar, kb * GEMM_BK, n0);
-          }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-      }
-      if (!ok) {
-        // Give loads that are still in flight a bounded chance to land before
-        // the block retires: a stage whose load was issued completes its
-        // full barrier regardless of the consumer.
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 2000000ull) {
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ------------------------------------------------------- MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_tf32(GEMM_BM, GEMM_BN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int local_tile = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
-        const int acc = local_tile & 1;
-        const uint32_t acc_phase = (local_tile >> 1) & 1;
-        if (!mbar_wait_bounded(smem_u32(&tmem_empty_bar[acc]), acc_phase ^ 1u, abort_flag)) {
-          atomicCAS(p.status, 0, 0x200 | acc);
-          ok = false;
-          break;
-        }
-        tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + acc * GEMM_BN;
-        for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), phase, abort_flag)) {
-            atomicCAS(p.status, 0, 0x300 | stage);
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          const uint32_t sa_hi = smem_u32(stage_base + stage * Cfg::kStageBytes);
-          const uint32_t sb_hi = sa_hi + GEMM_A_BYTES;
-          const uint32_t sa_lo = sb_hi + GEMM_B_BYTES;
-          const uint32_t sb_lo = sa_lo + GEMM_A_BYTES;
+      const long long off = static_cast<long long>(row0) * p.ldd + col;
+      float* dp = p.D + off;
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; ++k) {
-            const uint32_t koff = k * GEMM_UMMA_K * 4;  // 32 bytes along K inside the swizzle row
-            const uint64_t da_hi = umma_desc_k_sw128(sa_hi + koff);
-            const uint64_t db_hi = umma_desc_k_sw128(sb_hi + koff);
-            const uint32_t first = (kb | k) ? 1u : 0u;
-            if (MODE == 3) {
-              const uint64_t da_lo = umma_desc_k_sw128(sa_lo + koff);
-              const uint64_t db_lo = umma_desc_k_sw128(sb_lo + koff);
-              umma_tf32(tmem_d, da_lo, db_hi, idesc, first);
-              umma_tf32(tmem_d, da_hi, db_lo, idesc, 1u);
-              umma_tf32(tmem_d, da_hi, db_hi, idesc, 1u);
-            } else {
-              umma_tf32(tmem_d, da_hi, db_hi, idesc, first);
-            }
-          }
-          umma_commit(smem_u32(&empty_bar[stage]));  // stage is free once these MMAs retire
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-        if (ok) umma_commit(smem_u32(&tmem_full_bar[acc]));
+      for (int rr = 0; rr < 32; ++rr)
+        if (rr < rows_here) dp[rr * p.ldd] = x[rr];
+#pragma unroll 1
+      for (int rep = 0; rep < p.n_replicas; ++rep) {
+        float* rp = p.replicas[rep] + off;
+#pragma unroll
+        for (int rr = 0; rr < 32; ++rr)
+          if (rr < rows_here) rp[rr * p.ldd] = x[rr];
       }
     }
     __syncwarp();
-  } else {
-    // --------------------------------------------------------- epilogue
-    const int quarter = warp & 3;  // tensor-memory lanes [32*quarter, 32*quarter+32)
-    EpiWarp epi = epi_warp(epi_base, ctrl, warp - 2);
-    int local_tile = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
-      const int acc = local_tile & 1;
-      const uint32_t acc_phase = (local_tile >> 1) & 1;
-      int tm, tn;
-      tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn);
-      const int row0 = tm * GEMM_BM + quarter * 32;
-      const int n0 = tn * GEMM_BN;
-      if (p.tma_epilogue) epilogue_tma_begin(p, &map_c, epi, row0, n0);
-      // every lane waits; the warp then agrees on the outcome so that the
-      // warp-collective tensor-memory loads below are never partly skipped
-      const bool landed = mbar_wait_bounded(smem_u32(&tmem_full_bar[acc]), acc_phase, abort_flag);
-      if (!__all_sync(0xffffffffu, landed)) {
-        if (lane == 0) atomicCAS(p.status, 0, 0x400 | acc);
-        ok = false;
-        break;
-      }
-      tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * GEMM_BN;
-      if (!p.tma_epilogue) {
-        epilogue_rows<GEMM_BN>(p, taddr, epi.buf, lane, row0, n0);
-      } else if (!epilogue_tma<GEMM_BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, abort_flag)) {
-        if (lane == 0) atomicCAS(p.status, 0, 0x500 | acc);
-        ok = false;
-        break;
-      }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&tmem_empty_bar[acc]));
-    }
-    __syncwarp();
-    if (elect_one()) bulk_wait_read<0>();  // the tiles must outlive the stores that read them
-    __syncwarp();
-  }
-
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem_base, GEMM_TMEM_COLS);
   }
 }
 
@@ -591,6 +376,20 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
 // Elements that no non-finite operand reaches are unaffected; TF32 mode keeps fp32's Inf/NaN semantics.
 __device__ __forceinline__ float tf32_lo(float x, float hi) {
   return (fabsf(hi) <= 3.402823466e+38f) ? tf32_round(x - hi) : 0.0f;
+}
+
+// Rounding to TF32, nearest-even, in integer arithmetic: the same bits as tf32_round for finite x (its conversion instruction
+// issues at a quarter of the rate).
+__device__ __forceinline__ float tf32_round_int(float x) {
+  const uint32_t u = __float_as_uint(x);
+  return __uint_as_float((u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u);
+}
+
+// tf32_lo(x, tf32_round(x)) for the kernel that makes low parts on the fly: 12 instructions of full rate per element.  From
+// 0x7f7ff000 on (the upper half of FLT_MAX's last TF32 step, infinities, NaNs) the high part is not finite.
+__device__ __forceinline__ float tf32_lo_int(float x) {
+  const float lo = tf32_round_int(x - tf32_round_int(x));
+  return (__float_as_uint(x) & 0x7fffffffu) >= 0x7f7ff000u ? 0.0f : lo;
 }
 
 // A[M x K] (row stride lda) -> hi[M x Kp] (and lo[M x Kp]), Kp = K rounded up

@@ -12,4 +12,17 @@ inline bool valid_mode(int mode) {
          mode == SB200_MODE_3XMIXED;
 }
 
+// While one of these lives, the products its thread launches are row blocks of one of `rows` rows: a k-loop is then divided,
+// or not, as it would be for the whole, and the blocks have the bits of the whole.
+class RowBlocksOf {
+ public:
+  explicit RowBlocksOf(long long rows);
+  ~RowBlocksOf();
+  RowBlocksOf(const RowBlocksOf&) = delete;
+  RowBlocksOf& operator=(const RowBlocksOf&) = delete;
+
+ private:
+  long long before_;
+};
+
 }  // namespace sb200

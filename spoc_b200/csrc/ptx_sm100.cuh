@@ -333,6 +333,47 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
       : "memory");
 }
 
+// One block on its own, half-precision operands.
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same operations for a pair of blocks (CTAS = 2) or a block on its own (CTAS = 1).
+template <int CTAS>
+__device__ __forceinline__ void tmem_alloc_for(uint32_t dst_smem, uint32_t ncols) {
+  if constexpr (CTAS == 2) tmem_alloc_pair(dst_smem, ncols); else tmem_alloc(dst_smem, ncols);
+}
+template <int CTAS>
+__device__ __forceinline__ void tmem_relinquish_for() {
+  if constexpr (CTAS == 2) tmem_relinquish_pair(); else tmem_relinquish();
+}
+template <int CTAS>
+__device__ __forceinline__ void tmem_dealloc_for(uint32_t taddr, uint32_t ncols) {
+  if constexpr (CTAS == 2) tmem_dealloc_pair(taddr, ncols); else tmem_dealloc(taddr, ncols);
+}
+template <int CTAS>
+__device__ __forceinline__ void umma_commit_for(uint32_t bar) {
+  if constexpr (CTAS == 2) umma_commit_pair(bar); else umma_commit(bar);
+}
+template <bool F16, int CTAS>
+__device__ __forceinline__ void umma_for(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (F16 && CTAS == 2) umma_f16_pair(tmem_d, adesc, bdesc, idesc, accumulate);
+  else if constexpr (F16) umma_f16(tmem_d, adesc, bdesc, idesc, accumulate);
+  else if constexpr (CTAS == 2) umma_tf32_pair(tmem_d, adesc, bdesc, idesc, accumulate);
+  else umma_tf32(tmem_d, adesc, bdesc, idesc, accumulate);
+}
+template <int CTAS>
+__device__ __forceinline__ void tma_load_for(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar, int32_t x, int32_t y, uint64_t policy) {
+  if constexpr (CTAS == 2) tma_load_2d_pair_hint(dst_smem, map, bar, x, y, policy); else tma_load_2d_hint(dst_smem, map, bar, x, y, policy);
+}
+
 // Shared-memory matrix descriptor for a K-major operand tile whose rows are
 // 128 bytes (32 floats) long, stored with the 128-byte swizzle the TMA load
 // applies: 8-row groups of 1024 bytes.  Fields (64 bits): start address >> 4

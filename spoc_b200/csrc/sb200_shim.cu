@@ -462,12 +462,7 @@ size_t gemm_workspace_need(int mode, long long M, long long N, long long K) {
 
 std::atomic<int> g_tile_n{-1};  // -1 = not yet read from the environment; 0 automatic, else 64 / 128 / 256
 
-// Tile columns for the CTA-pair kernel.  256x256 tiles have the best ratio of tensor-core work to
-// shared-memory and L2 traffic, so they serve every problem that fills the GPU with them.  A problem
-// with fewer tiles than CTA pairs takes a narrower tile, which puts more SMs to work and shortens
-// the epilogue that nothing overlaps when a pair computes a single tile.  The estimate is in
-// MMA-cycle units per pair: waves * (k-blocks * cycles per k-block + fill and epilogue).
-int choose_tile_n(long long M, long long N, long long kblocks, int clusters, int mode) {
+int tile_n_setting() {
   int forced = g_tile_n.load();
   if (forced < 0) {
     const char* e = getenv("SAREK_B200_TILE_N");
@@ -475,107 +470,188 @@ int choose_tile_n(long long M, long long N, long long kblocks, int clusters, int
     if (forced != 64 && forced != 128 && forced != 256) forced = 0;
     g_tile_n.store(forced);
   }
-  if (forced) return forced;
-  const long long tiles_m = (M + PAIR_BM - 1) / PAIR_BM;
-  const double mmas = mode == 3 ? 3.0 : 1.0;
-  auto cost = [&](int bn) {
+  return forced;
+}
+
+// How a product is cut up: tile columns, and work items a tile's k-loop is divided into.
+struct TileShape {
+  int tile_n = 256, splits = 1;
+};
+
+constexpr int kMinSplitKBlocks = 16;  // a divided k-loop keeps at least this many k-blocks per work item
+constexpr int kMaxSplits = 32;
+
+// Estimates the time of each cut (in ns at 1.9 GHz) and takes the shortest.  Per k-block: measured on 1024 x 1024 x K, MMA-bound
+// at 256 columns (843 ns with three MMAs per k-step, 277 with one), near it at 192 and 128, bound by the operands' shared-memory
+// reads at 64 (340 ns) and by the latency around a stage in the one-MMA modes (165 ns).  256-column tiles have the best ratio of
+// tensor-core work to shared-memory, L2 and electric power, so a narrower tile is charged 10 % and has to win by 3 %: it does
+// when there are fewer 256-column tiles than pairs.  192 columns serve the three-MMA modes only.  Fixed: launch, set-up,
+// pipeline fill, and 400 ns per 32 columns of epilogue that nothing overlaps.
+// Dividing the k-loop pays when the tiles occupy a fraction of the SMs and k is long; it costs a second launch and the
+// partial results' way through L2 (about 4 TB/s), and is left to products that stay at 16 k-blocks per item or more.
+// fixed_splits > 0: the division is given (a row block of a larger product is divided as the whole is, so that it has the
+// same bits).
+TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0) {
+  TileShape best;
+  const int forced = tile_n_setting();
+  double best_cost = 0.0;
+  bool have = false;
+  const long long tiles_m = (M + 128 * ctas - 1) / (128 * ctas);
+  for (int bn : {256, 192, 128, 64}) {
+    if (ctas == 1 && bn > 128) continue;
+    if (bn == 192 && (!three || forced)) continue;
+    if (forced && bn != forced && !(ctas == 1 && forced == 256 && bn == 128)) continue;
+    const double per_kblock = three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0) : (bn == 256 ? 277.0 : 165.0);
     const long long tiles = tiles_m * ((N + bn - 1) / bn);
-    const long long waves = (tiles + clusters - 1) / clusters;
-    // cycles per k-block: 4 MMAs of bn/2 cycles each (x3 in 3xTF32 mode), or the time to fetch the stage at
-    // about 60 bytes per cycle and SM, whichever is longer.  That rate is the 192 KiB ring divided by the
-    // loaded TMA latency (measured); narrow tiles need more bytes per MMA cycle because A is re-read once
-    // per column of tiles, so they are fetch-bound where 256-column tiles are tensor-bound
-    const double mma_cycles = 4.0 * (bn / 2.0) * mmas;
-    const double fetch_cycles = (mode == 3 ? 2.0 : 1.0) * (16384.0 + bn * 64.0) / 60.0;
-    const double per_kblock = (mma_cycles > fetch_cycles ? mma_cycles : fetch_cycles) * (bn == 256 ? 1.0 : 1.1);
-    const double fixed = 6000.0 + 1000.0 * (bn / 32.0);
-    return static_cast<double>(waves) * (static_cast<double>(kblocks) * per_kblock + fixed);
-  };
-  int best = 256;
-  double best_cost = cost(256);
-  for (int bn : {128, 64}) {
-    const double c = cost(bn);
-    if (c < 0.97 * best_cost) {  // a narrower tile must win clearly
-      best = bn;
-      best_cost = c;
+    for (int sp = 1; sp <= kMaxSplits; ++sp) {
+      if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * kMinSplitKBlocks)) continue;
+      const long long per_item = (kblocks + sp - 1) / sp;
+      if (sp > 1 && per_item * (sp - 1) >= kblocks) continue;  // the last item would be empty
+      const long long waves = (tiles * sp + units - 1) / units;
+      double c = waves * per_item * per_kblock * (bn == 256 ? 1.0 : 1.1) + 5500.0 + 400.0 * (bn / 32) + 800.0 * (waves - 1);
+      if (sp > 1) c += 3000.0 + (sp + 1.0) * M * N * 4.0 / 4000.0;
+      if (!have || c < (sp > best.splits || bn < best.tile_n ? 0.97 : 1.0) * best_cost) {
+        best.tile_n = bn;
+        best.splits = sp;
+        best_cost = c;
+        have = true;
+      }
     }
   }
   return best;
 }
 
-// One instantiation of the CTA-pair kernel: shared-memory attribute and resident-cluster count are
-// looked up once per device, then the launch.
-template <int MODE, bool DIRECT, int BN>
-int launch_pair(DeviceState& d, int dev_index, cudaStream_t st, const CUtensorMap& ma_hi, const CUtensorMap& mb_hi,
-                const CUtensorMap& ma_lo, const CUtensorMap& mb_lo, GemmParams gp, long long M, long long N,
-                const CUtensorMap* ma_x = nullptr, const CUtensorMap* mb_x = nullptr) {
-  using PCfg = PairCfg<MODE, BN>;
-  static std::atomic<int> resident[kMaxDevices];  // 0 = not yet asked
-  int max_clusters = resident[dev_index].load();
-  if (max_clusters == 0) {
-    CU_TRY(cudaFuncSetAttribute(gemm_pair_kernel<MODE, DIRECT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(PCfg::kSmemBytes)));
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof cfg);
-    cfg.gridDim = dim3(static_cast<unsigned>(d.sm_count & ~1), 1, 1);
-    cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = PCfg::kSmemBytes;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&max_clusters, gemm_pair_kernel<MODE, DIRECT, BN>, &cfg) != cudaSuccess ||
-        max_clusters <= 0) {
-      cudaGetLastError();
-      max_clusters = d.sm_count / 2;
-    }
-    resident[dev_index].store(max_clusters);
-  }
-  gp.tiles_m = static_cast<int>((M + PAIR_BM - 1) / PAIR_BM);
-  gp.tiles_n = static_cast<int>((N + BN - 1) / BN);
-  gp.group_m = PAIR_GROUP_M;  // 8 measured best at 8192^3 against 2, 4, 16, 32 (both modes)
-  const long long tiles = static_cast<long long>(gp.tiles_m) * gp.tiles_n;
-  const long long pairs = tiles < max_clusters ? tiles : max_clusters;
-  // programmatic dependent launch: the kernel's set-up may overlap the preparation launch in front of it
+// Launches a kernel with programmatic stream serialization: it may set itself up while the kernel before it in the stream
+// still runs.  Every kernel launched this way passes griddepcontrol.wait before it touches global memory.  The launch call
+// itself is cheaper too (2.3 against 2.8 us).
+template <class... Params, class... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, Args&&... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs), 1, 1);
-  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = PCfg::kSmemBytes;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  CUtensorMap map_d, map_c;
-  epilogue_maps(&gp, ma_hi, &map_d, &map_c);
-  CU_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<MODE, DIRECT, BN>, ma_hi, mb_hi, ma_lo, mb_lo, ma_x ? *ma_x : ma_lo,
-                            mb_x ? *mb_x : mb_lo, map_d, map_c, gp));
-  return launch_check("gemm_pair_kernel");
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-template <int MODE, bool DIRECT>
-int launch_pair_bn(int bn, DeviceState& d, int dev_index, cudaStream_t st, const CUtensorMap& ma_hi, const CUtensorMap& mb_hi,
-                   const CUtensorMap& ma_lo, const CUtensorMap& mb_lo, const GemmParams& gp, long long M, long long N,
-                   const CUtensorMap* ma_x = nullptr, const CUtensorMap* mb_x = nullptr) {
-  if (bn == 64) return launch_pair<MODE, DIRECT, 64>(d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N, ma_x, mb_x);
-  if (bn == 128) return launch_pair<MODE, DIRECT, 128>(d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N, ma_x, mb_x);
-  return launch_pair<MODE, DIRECT, 256>(d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N, ma_x, mb_x);
+// The operand maps of one launch; x: the mixed mode's third pair (else unused).
+struct OperandMaps {
+  CUtensorMap a_hi, b_hi, a_lo, b_lo, a_x, b_x;
+};
+
+// One instantiation of the GEMM kernel: shared-memory attribute and resident blocks (pairs) are looked up once per device,
+// then the launch.  part: partial results of a divided k-loop ([gp.splits][gp.part_rows][part_ld] floats), added up by a
+// second launch.
+template <int MODE, int SRC, int BN, int CTAS>
+int launch_tiles(int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, GemmParams gp, float* part) {
+  using Cfg = TileCfg<MODE, SRC, BN, CTAS>;
+  auto kernel = gemm_pair_kernel<MODE, SRC, BN, CTAS>;
+  static std::atomic<int> resident[kMaxDevices];  // 0 = not yet asked
+  int units = resident[dev_index].load();
+  if (units == 0) {
+    CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
+    units = sm_count;
+    if (CTAS == 2) {
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof cfg);
+      cfg.gridDim = dim3(static_cast<unsigned>(sm_count & ~1), 1, 1);
+      cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
+      cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 2;
+      attr.val.clusterDim.y = 1;
+      attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&units, kernel, &cfg) != cudaSuccess || units <= 0) {
+        cudaGetLastError();
+        units = sm_count / 2;
+      }
+    }
+    resident[dev_index].store(units);
+  }
+  gp.tiles_m = static_cast<int>((gp.M + 128 * CTAS - 1) / (128 * CTAS));
+  gp.tiles_n = static_cast<int>((static_cast<long long>(gp.N) + BN - 1) / BN);
+  gp.group_m = PAIR_GROUP_M;  // 8 measured best at 8192^3 against 2, 4, 16, 32 (both modes)
+  if (gp.splits < 1) gp.splits = 1;
+  gp.split_k_blocks = (gp.num_k_blocks + gp.splits - 1) / gp.splits;
+  const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
+  const long long used = items < units ? items : units;
+  const dim3 grid(static_cast<unsigned>(CTAS * used)), block(Cfg::kThreads);
+  CUtensorMap map_d, map_c;
+  if (gp.splits == 1) {
+    gp.part_rows = 0;
+    epilogue_maps(&gp, m.a_hi, &map_d, &map_c);
+    CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_c, gp));
+    return launch_check("gemm_pair_kernel");
+  }
+  const long long ld = round_up(gp.N, 4);
+  gp.part_rows = static_cast<int>(round_up(gp.M, 32));
+  GemmParams pp = gp;  // the partial sums as they are
+  pp.C = pp.bias = pp.row_scale = pp.col_scale = nullptr;
+  pp.alpha = 1.0f;
+  pp.act = 0;
+  pp.n_replicas = 0;
+  pp.tma_epilogue = 1;
+  pp.epoch_ctr = nullptr;
+  if (int rc = encode_map_2d(&map_d, part, ld, static_cast<long long>(gp.part_rows) * gp.splits, ld, 32, 32, false)) return rc;
+  CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_d, pp));
+  if (int rc = launch_check("gemm_pair_kernel")) return rc;
+  const long long quads = static_cast<long long>(gp.M) * (ld >> 2);
+  long long blocks = (quads + 255) / 256;
+  if (blocks > static_cast<long long>(sm_count) * 8) blocks = static_cast<long long>(sm_count) * 8;
+  CU_TRY(launch_pdl(gemm_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, static_cast<const float*>(part), ld,
+                    gp.part_rows, gp.splits, gp));
+  return launch_check("gemm_reduce_kernel");
+}
+
+size_t partial_bytes(long long M, long long N, int splits) {
+  return splits > 1 ? static_cast<size_t>(round_up(M, 32)) * round_up(N, 4) * 4 * splits : 0;
+}
+
+template <int MODE, int SRC>
+int launch_tiles_for(int bn, int ctas, int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, const GemmParams& gp, float* part) {
+  constexpr bool kThree = MODE == 3 || MODE == 4 || MODE == 5;
+  if constexpr (MODE != 5 && !(MODE == 3 && SRC == SRC_DIRECT)) {
+    if (ctas == 1) {
+      if (bn == 64) return launch_tiles<MODE, SRC, 64, 1>(dev_index, sm_count, st, m, gp, part);
+      return launch_tiles<MODE, SRC, 128, 1>(dev_index, sm_count, st, m, gp, part);
+    }
+  }
+  if constexpr (!(MODE == 3 && SRC == SRC_DIRECT)) {
+    if (bn == 64) return launch_tiles<MODE, SRC, 64, 2>(dev_index, sm_count, st, m, gp, part);
+    if (bn == 128) return launch_tiles<MODE, SRC, 128, 2>(dev_index, sm_count, st, m, gp, part);
+  }
+  if constexpr (kThree) {
+    if (bn == 192) return launch_tiles<MODE, SRC, 192, 2>(dev_index, sm_count, st, m, gp, part);
+  }
+  if constexpr (SRC != SRC_SPLIT) {
+    return launch_tiles<MODE, SRC, 256, 2>(dev_index, sm_count, st, m, gp, part);
+  }
+  return fail(SB200_ERR_INVALID_VALUE, "no kernel for tiles of %d columns", bn);
 }
 
 // How sb200_gemm_f32 will run a product: which kernel, which tile, how much scratch.  One function decides, the
 // launch path and sb200_gemm_describe both ask it.
 struct GemmRoute {
-  bool pair = false;    // CTA-pair kernel (else the single-CTA kernel)
-  bool direct = false;  // operands read where they lie (else from prepared panels)
-  int tile_n = GEMM_BN;
+  int ctas = 2;         // blocks per tile: 2 a pair, 1 a block on its own
+  int src = SRC_PANELS; // where the operand tiles come from
+  int tile_n = 256, splits = 1;
   int stages = 0;
   long long tiles = 0, waves = 0;
-  size_t workspace = 0;  // bytes of library scratch
+  size_t operand_bytes = 0;  // scratch of the operand panels
+  size_t workspace = 0;      // bytes of library scratch, partial results included
 };
 
 int gemm_variant_setting() {
@@ -588,38 +664,55 @@ int gemm_variant_setting() {
   return variant;
 }
 
+// Products of at most this many rows are computed by blocks on their own: the second block of a pair would only see rows
+// past the end.
+constexpr long long kSingleRows = 64;
+
+int stages_of(bool three, int bn, int ctas) {
+  const long long stage = (three ? 2 : 1) * (16384ll + (bn / ctas) * 128ll);
+  const long long fit = 192 * 1024 / stage;
+  return static_cast<int>(fit > 8 ? 8 : fit);
+}
+
+// Set by RowBlocksOf (the host-operand calls, the launches that upload by blocks, partial launches, device groups).
+thread_local long long t_whole_rows = 0;
+
+TileShape shape_for(long long M, long long N, long long kblocks, int ctas, int sm_count, bool three, bool may_split) {
+  const int units = ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
+  if (!may_split || t_whole_rows <= M) return choose_tiles(M, N, kblocks, ctas, units, three, may_split);
+  const int whole_ctas = t_whole_rows <= kSingleRows ? 1 : 2;
+  const int whole_units = whole_ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
+  const int splits = choose_tiles(t_whole_rows, N, kblocks, whole_ctas, whole_units, three, true).splits;
+  return choose_tiles(M, N, kblocks, ctas, units, three, true, splits);
+}
+
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
   GemmRoute r;
   const int variant = gemm_variant_setting();
-  // CTA pairs work on 256-row tiles.  With at most 128 rows the second block of a pair computes nothing, and
-  // the pair kernel still wins when it can read the operands directly (measured 2x at 64..128 rows: no
-  // transposing pass over B); from prepared panels the single-CTA kernel serves such problems.
-  r.pair = variant >= 2 || (variant == 0 && (M > GEMM_BM || addressable));
-  // CTA pairs read the caller's matrices directly when TMA can address them: 16-byte aligned bases and
-  // row strides.  TMA rounds A and B to TF32 while loading and B is consumed N-major, so TF32 mode needs
-  // neither preparation kernels nor panel scratch, and 3xTF32 mode prepares only the low parts.
-  r.direct = r.pair && variant != 3 && addressable;
+  const bool three = mode == SB200_MODE_3XTF32;
+  // The caller's matrices are read where they lie when TMA can address them: 16-byte aligned bases and row strides.  TF32
+  // mode then needs no preparation and no scratch, and 3xTF32 mode none below 256 columns (SRC_SPLIT).
+  const bool direct = variant != 1 && variant != 3 && addressable;
+  // At most 128 rows: from panels a block on its own; read directly a pair wins from 65 rows on.
+  r.ctas = variant == 1 || (variant == 0 && M <= (direct ? kSingleRows : GEMM_BM)) ? 1 : 2;
   const long long kp = round_up(K, GEMM_BK);
-  const int clusters = sm_count / 2 > 0 ? sm_count / 2 : 1;
-  r.tile_n = r.pair ? choose_tile_n(M, N, kp / GEMM_BK, clusters, mode == SB200_MODE_3XTF32 ? 3 : 1) : GEMM_BN;
-  if (r.pair) {
-    const bool three = mode == SB200_MODE_3XTF32;
-    r.stages = r.tile_n == 256 ? (three ? PairCfg<3, 256>::kStages : PairCfg<1, 256>::kStages)
-             : r.tile_n == 128 ? (three ? PairCfg<3, 128>::kStages : PairCfg<1, 128>::kStages)
-                               : (three ? PairCfg<3, 64>::kStages : PairCfg<1, 64>::kStages);
-    r.tiles = ((M + PAIR_BM - 1) / PAIR_BM) * ((N + r.tile_n - 1) / r.tile_n);
-    r.waves = (r.tiles + clusters - 1) / clusters;
-  } else {
-    r.stages = mode == SB200_MODE_3XTF32 ? GemmCfg<3>::kStages : GemmCfg<1>::kStages;
-    r.tiles = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + GEMM_BN - 1) / GEMM_BN);
-    r.waves = (r.tiles + sm_count - 1) / (sm_count > 0 ? sm_count : 1);
-  }
+  const TileShape shape = shape_for(M, N, kp / GEMM_BK, r.ctas, sm_count, three, variant == 0);
+  r.tile_n = shape.tile_n;
+  r.splits = shape.splits;
+  // 3xTF32: at 256 columns the splitting warps' shared-memory traffic would come on top of MMAs that already keep it busy, so
+  // the low parts come from panels there
+  r.src = !direct ? SRC_PANELS : three && r.tile_n < 256 ? SRC_SPLIT : SRC_DIRECT;
+  const int units = r.ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
+  r.stages = stages_of(three, r.tile_n, r.ctas);
+  r.tiles = ((M + 128 * r.ctas - 1) / (128 * r.ctas)) * ((N + r.tile_n - 1) / r.tile_n);
+  r.waves = (r.tiles * r.splits + units - 1) / (units > 0 ? units : 1);
   if (panel_rows_a < M) panel_rows_a = M;
-  if (!r.direct) {
-    r.workspace = gemm_workspace_need(mode, panel_rows_a, N, K);
-  } else if (mode == SB200_MODE_3XTF32) {
-    r.workspace = round_up(K * round_up(N, 32) * 4, 1024) + round_up(panel_rows_a * kp * 4, 1024);
+  if (r.src == SRC_PANELS) {
+    r.operand_bytes = gemm_workspace_need(mode, panel_rows_a, N, K);
+  } else if (three && r.src == SRC_DIRECT) {
+    r.operand_bytes = round_up(K * round_up(N, 32) * 4, 1024) + round_up(panel_rows_a * kp * 4, 1024);
   }
+  r.workspace = r.operand_bytes + partial_bytes(M, N, r.splits);
   return r;
 }
 
@@ -630,12 +723,10 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   // panel_rows_a: rows the A panels are laid out for (>= M); callers that run several row blocks
   // against one prepared B pass the largest block so that the B panels keep their place.
   if (panel_rows_a < M) panel_rows_a = M;
-  using Cfg = GemmCfg<MODE>;
-
   const bool addressable = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0 &&
                            (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (ldb & 3) == 0;
   const GemmRoute route = route_gemm(MODE == 3 ? SB200_MODE_3XTF32 : SB200_MODE_TF32, M, N, K, addressable, d.sm_count, panel_rows_a);
-  const bool pair = route.pair, direct = route.direct;
+  const bool direct = route.src != SRC_PANELS;
   const int tile_n = route.tile_n;
 
   const long long kp = round_up(K, GEMM_BK);
@@ -662,7 +753,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
       if ((rc = scratch_acquire(d, st))) return rc;
     }
   }
-  unsigned int* epoch_ring = pair ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
+  unsigned int* epoch_ring =
+      route.ctas == 2 && route.splits == 1 ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
   const bool prof = g_profiling.load() != 0;
   DeviceState::ProfRec rec{nullptr, nullptr, nullptr};
   if (prof) {
@@ -677,7 +769,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     if ((rc = encode_map_2d(&mb_hi, B, N, K, ldb, 32, GEMM_BK, true, true))) return rc;
     ma_lo = ma_hi;
     mb_lo = mb_hi;
-    if constexpr (MODE == 3) {
+    if (MODE == 3 && route.src == SRC_DIRECT) {
       // low parts only: B's first (K x np, row-major like B), then A's (rows x kp)
       uint8_t* ws = static_cast<uint8_t*>(d.workspace);
       float* b_lo = reinterpret_cast<float*>(ws);
@@ -700,6 +792,9 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
       }
       if ((rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
       if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
+    } else if (MODE == 3) {  // SRC_SPLIT: the matrices themselves, as they are
+      if ((rc = encode_map_2d(&ma_lo, A, K, M, lda, GEMM_BK, GEMM_BM, false))) return rc;
+      if ((rc = encode_map_2d(&mb_lo, B, N, K, ldb, 32, GEMM_BK, false, true))) return rc;
     }
   } else {
     // workspace layout: B panels first (their size does not depend on M), then the A panels
@@ -730,7 +825,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
       rc = launch_check("prep_b_kernel");
       if (rc) return rc;
     }
-    const int b_box_rows = pair ? tile_n / 2 : GEMM_BN;
+    const int b_box_rows = tile_n / route.ctas;
     if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
     if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, b_box_rows))) return rc;
     if ((rc = encode_panel_map(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
@@ -744,26 +839,20 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   gp.epoch_ctr = epoch_ring;
   derive_params(&gp);
   if (prof) CU_TRY(cudaEventRecord(rec.e1, st));
-  if (pair) {
-    const int dev_index = static_cast<int>(&d - g_dev);
-    rc = direct ? launch_pair_bn<MODE, true>(tile_n, d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N)
-                : launch_pair_bn<MODE, false>(tile_n, d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N);
+  gp.splits = route.splits;
+  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
+  float* part = reinterpret_cast<float*>(static_cast<uint8_t*>(d.workspace) + route.operand_bytes);
+  const int dev_index = static_cast<int>(&d - g_dev);
+  if constexpr (MODE == 3) {
+    if (route.src == SRC_SPLIT)
+      rc = launch_tiles_for<3, SRC_SPLIT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
+    else if (route.src == SRC_DIRECT)
+      rc = launch_tiles_for<3, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
+    else
+      rc = launch_tiles_for<3, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
   } else {
-    gp.tiles_m = static_cast<int>((M + GEMM_BM - 1) / GEMM_BM);
-    gp.tiles_n = static_cast<int>((N + GEMM_BN - 1) / GEMM_BN);
-    const long long tiles = static_cast<long long>(gp.tiles_m) * gp.tiles_n;
-    const unsigned grid = static_cast<unsigned>(tiles < d.sm_count ? tiles : d.sm_count);
-    static std::atomic<int> attr_set[kMaxDevices];  // the shared-memory attribute is per device: set once on each
-    const int dev_index = static_cast<int>(&d - g_dev);
-    if (!attr_set[dev_index].load()) {
-      CU_TRY(cudaFuncSetAttribute(gemm_tf32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(Cfg::kSmemBytes)));
-      attr_set[dev_index].store(1);
-    }
-    CUtensorMap map_d, map_c;
-    epilogue_maps(&gp, ma_hi, &map_d, &map_c);
-    gemm_tf32_kernel<MODE><<<grid, GEMM_THREADS, Cfg::kSmemBytes, st>>>(ma_hi, mb_hi, ma_lo, mb_lo, map_d, map_c, gp);
-    rc = launch_check("gemm_tf32_kernel");
+    rc = direct ? launch_tiles_for<1, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
+                : launch_tiles_for<1, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
   }
   if (prof) {
     CU_TRY(cudaEventRecord(rec.e2, st));
@@ -803,9 +892,12 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
                     const float* B, long long ldb, const GemmParams& gp_in) {
   const long long kp = round_up(K, 64);
   const size_t a_bytes = round_up(M * kp * 2, 1024), b_bytes = round_up(N * kp * 2, 1024);
-  const size_t need = gemm_f16_workspace_need(M, N, K, THREE);
+  const int ctas = M <= GEMM_BM ? 1 : 2;  // from panels, as in the TF32 modes
+  const TileShape shape = shape_for(M, N, kp / 64, ctas, d.sm_count, THREE, true);
+  const int tile_n = shape.tile_n;
+  const size_t need = round_up(gemm_f16_workspace_need(M, N, K, THREE), 1024);
   std::unique_lock<std::mutex> scratch_lock(d.scratch_mu);
-  int rc = ensure_workspace(d, need);
+  int rc = ensure_workspace(d, need + partial_bytes(M, N, shape.splits));
   if (rc) return rc;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
@@ -816,7 +908,7 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
   if (track_scratch) {
     if ((rc = scratch_acquire(d, st))) return rc;
   }
-  unsigned int* epoch_ring = next_epoch_ring(d, st, kp / 64);
+  unsigned int* epoch_ring = ctas == 2 && shape.splits == 1 ? next_epoch_ring(d, st, kp / 64) : nullptr;
   const bool prof = g_profiling.load() != 0;
   DeviceState::ProfRec rec{nullptr, nullptr, nullptr};
   if (prof) {
@@ -868,16 +960,14 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
                                                                              static_cast<int>(kp));
     if ((rc = launch_check("prep_b_f16_kernel"))) return rc;
   }
-  const int clusters = d.sm_count / 2 > 0 ? d.sm_count / 2 : 1;
-  const int tile_n = choose_tile_n(M, N, kp / 64, clusters, THREE ? 3 : 1);
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
   if ((rc = encode_map_f16(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_map_f16(&mb_hi, b_hi, kp, N, tile_n / 2))) return rc;
+  if ((rc = encode_map_f16(&mb_hi, b_hi, kp, N, tile_n / ctas))) return rc;
   ma_lo = ma_hi;
   mb_lo = mb_hi;
   if (THREE) {
     if ((rc = encode_map_f16(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_map_f16(&mb_lo, b_lo, kp, N, tile_n / 2))) return rc;
+    if ((rc = encode_map_f16(&mb_lo, b_lo, kp, N, tile_n / ctas))) return rc;
   }
   GemmParams gp = gp_in;
   gp.num_k_blocks = static_cast<int>(kp / 64);
@@ -889,8 +979,10 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
   gp.col_scale = col_scale;
   if (prof) CU_TRY(cudaEventRecord(rec.e1, st));
   const int dev_index = static_cast<int>(&d - g_dev);
-  rc = THREE ? launch_pair_bn<4, false>(tile_n, d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N)
-             : launch_pair_bn<2, false>(tile_n, d, dev_index, st, ma_hi, mb_hi, ma_lo, mb_lo, gp, M, N);
+  gp.splits = shape.splits;
+  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
+  float* part = reinterpret_cast<float*>(ws + need);
+  rc = launch_tiles_for<THREE ? 4 : 2, SRC_PANELS>(tile_n, ctas, dev_index, d.sm_count, st, maps, gp, part);
   if (prof) {
     CU_TRY(cudaEventRecord(rec.e2, st));
     std::lock_guard<std::mutex> lock(d.mu);
@@ -980,7 +1072,7 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     if ((rc = launch_check("prep_mix_b_kernel"))) return rc;
   }
   const int clusters = d.sm_count / 2 > 0 ? d.sm_count / 2 : 1;
-  const int tile_n = choose_tile_n(M, N, kp32 / GEMM_BK, clusters, 3);
+  const int tile_n = choose_tiles(M, N, kp32 / GEMM_BK, 2, clusters, true, false).tile_n;
   CUtensorMap ma, mb, ma_hi16, mb_hi16, ma_lo16, mb_lo16;
   if ((rc = encode_map_2d(&ma, A, K, M, lda, GEMM_BK, GEMM_BM, true))) return rc;
   if ((rc = encode_map_2d(&mb, B, N, K, ldb, 32, GEMM_BK, true, true))) return rc;
@@ -999,7 +1091,8 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
   const int dev_index = static_cast<int>(&d - g_dev);
   gp.num_k_blocks = static_cast<int>(kp / 64);
   gp.gate_value = 1;
-  rc = launch_pair_bn<5, true>(tile_n, d, dev_index, st, ma, mb, ma_hi16, mb_hi16, gp, M, N, &ma_lo16, &mb_lo16);
+  const OperandMaps maps{ma, mb, ma_hi16, mb_hi16, ma_lo16, mb_lo16};
+  rc = launch_tiles_for<5, SRC_DIRECT>(tile_n, 2, dev_index, d.sm_count, st, maps, gp, nullptr);
   if (rc == SB200_OK) {
     // behind it, gated the other way: plain 3xTF32 on the same operands, its low-part panels in the same scratch
     float* pb_lo = reinterpret_cast<float*>(ws);
@@ -1017,7 +1110,8 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     gp.num_k_blocks = static_cast<int>(kp32 / GEMM_BK);
     gp.gate_value = 0;
     gp.epoch_ctr = nullptr;  // the ring belongs to the launch in front
-    rc = launch_pair_bn<3, true>(tile_n, d, dev_index, st, ma, mb, pma_lo, pmb_lo, gp, M, N);
+    const OperandMaps plain{ma, mb, pma_lo, pmb_lo, pma_lo, pmb_lo};
+    rc = launch_tiles_for<3, SRC_DIRECT>(256, 2, dev_index, d.sm_count, st, plain, gp, nullptr);
   }
   if (prof) {
     CU_TRY(cudaEventRecord(rec.e2, st));
@@ -1471,6 +1565,7 @@ int launch_gemm_kernel(DeviceState& d, const KernelPlan& plan, const std::vector
   }
   if (pipeline_uploads) return SB200_OK;  // partial launch: as above
   const long long full_rows = covered / N, rest = covered - full_rows * N;
+  const RowBlocksOf whole(M);
   rc = run_gemm(d, st, mode, full_rows, N, K, A, K, B, N, D, N, alpha, C, N, beta, bias, g.act);
   if (!rc && rest != 0) {
     const uint64_t off_a = static_cast<uint64_t>(full_rows) * K * 4, off_d = static_cast<uint64_t>(full_rows) * N * 4;
@@ -1488,6 +1583,7 @@ int launch_gemm_kernel(DeviceState& d, const KernelPlan& plan, const std::vector
 int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M, long long N, long long K, const Slot& a,
                          const Slot& b, const Slot* c, const Slot* bias, const Slot& dd, float alpha, float beta, int act, void* d_host) {
   std::lock_guard<std::mutex> host_call_lock(d.host_call_mu);  // the inbound stream is shared with the host-operand calls
+  const RowBlocksOf whole(M);
   int src = ensure_pipe_streams(d);
   if (src) return src;
   static const int nblocks = [] {  // row blocks per product (SAREK_B200_PIPE_BLOCKS, 2..64)
@@ -1588,6 +1684,9 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
 }  // namespace
 
 namespace sb200 {
+RowBlocksOf::RowBlocksOf(long long rows) : before_(t_whole_rows) { t_whole_rows = rows; }
+RowBlocksOf::~RowBlocksOf() { t_whole_rows = before_; }
+
 int set_error(int code, const char* fmt, ...) {
   char buf[1024];
   va_list ap;
@@ -2291,16 +2390,20 @@ int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64
   if (!bytes || M < 0 || N < 0 || K < 0) return fail(SB200_ERR_INVALID_VALUE, "bad argument");
   if (!sb200::valid_mode(mode))
     return fail(SB200_ERR_INVALID_VALUE, "unknown GEMM mode %d", mode);
+  *bytes = 0;
+  if (M == 0 || N == 0 || K == 0) return SB200_OK;
+  constexpr int kSms = 148;
   if (mode == SB200_MODE_3XF16 || mode == SB200_MODE_F16) {
-    *bytes = (M == 0 || N == 0 || K == 0) ? 0 : gemm_f16_workspace_need(M, N, K, mode == SB200_MODE_3XF16);
+    const bool three = mode == SB200_MODE_3XF16;
+    const TileShape shape = shape_for(M, N, round_up(K, 64) / 64, M <= GEMM_BM ? 1 : 2, kSms, three, true);
+    *bytes = gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape.splits);
     return SB200_OK;
   }
-  if (mode == SB200_MODE_3XMIXED) {  // upper bound: which of the two routes runs depends on the operands' addresses
-    const size_t plain = gemm_workspace_need(SB200_MODE_3XTF32, M, N, K), mixed = gemm_mix_workspace_need(M, N, K);
-    *bytes = (M == 0 || N == 0 || K == 0) ? 0 : (plain > mixed ? plain : mixed);
-    return SB200_OK;
-  }
-  *bytes = (M == 0 || N == 0 || K == 0) ? 0 : gemm_workspace_need(mode, M, N, K);
+  // upper bound: which route runs depends on the operands' addresses
+  const int plain = mode == SB200_MODE_TF32 ? SB200_MODE_TF32 : SB200_MODE_3XTF32;
+  uint64_t most = mode == SB200_MODE_3XMIXED ? gemm_mix_workspace_need(M, N, K) : 0;
+  for (bool addressable : {false, true}) most = std::max<uint64_t>(most, route_gemm(plain, M, N, K, addressable, kSms, M).workspace);
+  *bytes = most;
   return SB200_OK;
 }
 
@@ -2313,23 +2416,22 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   if (mode == SB200_MODE_3XF16 || mode == SB200_MODE_F16) {
     const bool three = mode == SB200_MODE_3XF16;
     const long long kp = round_up(K, 64);
-    const int clusters = sm_count / 2 > 0 ? sm_count / 2 : 1;
-    const int tn = choose_tile_n(M, N, kp / 64, clusters, three ? 3 : 1);
-    const long long tiles = ((M + PAIR_BM - 1) / PAIR_BM) * ((N + tn - 1) / tn);
-    const int stages = tn == 256 ? (three ? PairCfg<4, 256>::kStages : PairCfg<2, 256>::kStages)
-                     : tn == 128 ? (three ? PairCfg<4, 128>::kStages : PairCfg<2, 128>::kStages)
-                                 : (three ? PairCfg<4, 64>::kStages : PairCfg<2, 64>::kStages);
+    const int ctas = M <= GEMM_BM ? 1 : 2, units = ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
+    const TileShape shape = shape_for(M, N, kp / 64, ctas, sm_count, three, true);
+    const long long tiles = ((M + 128 * ctas - 1) / (128 * ctas)) * ((N + shape.tile_n - 1) / shape.tile_n);
     char fb[256];
-    snprintf(fb, sizeof fb, "pair fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu launches=4", PAIR_BM, tn, stages,
-             tiles, (tiles + clusters - 1) / clusters, gemm_f16_workspace_need(M, N, K, three));
+    snprintf(fb, sizeof fb, "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
+             ctas == 1 ? "single" : "pair", 128 * ctas, shape.tile_n, stages_of(three, shape.tile_n, ctas), tiles,
+             (tiles * shape.splits + units - 1) / units, shape.splits,
+             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape.splits), shape.splits > 1 ? 5 : 4);
     return copy_out(fb, out, outlen);
   }
   if (mode == SB200_MODE_3XMIXED) {
     if (gemm_mix_applies(M, N, K, addressable != 0)) {
       const int clusters = sm_count / 2 > 0 ? sm_count / 2 : 1;
-      const int tn = choose_tile_n(M, N, round_up(K, GEMM_BK) / GEMM_BK, clusters, 3);
+      const int tn = choose_tiles(M, N, round_up(K, GEMM_BK) / GEMM_BK, 2, clusters, true, false).tile_n;
       const long long tiles = ((M + PAIR_BM - 1) / PAIR_BM) * ((N + tn - 1) / tn);
-      const int stages = tn == 256 ? PairCfg<5, 256>::kStages : tn == 128 ? PairCfg<5, 128>::kStages : PairCfg<5, 64>::kStages;
+      const int stages = stages_of(true, tn, 2);
       char fb[256];
       snprintf(fb, sizeof fb, "pair mixed tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu launches=7", PAIR_BM, tn, stages,
                tiles, (tiles + clusters - 1) / clusters, gemm_mix_workspace_need(M, N, K));
@@ -2339,9 +2441,10 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   }
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
-  snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu launches=%d",
-           r.pair ? "pair" : "single", r.direct ? "direct" : "panels", r.pair ? PAIR_BM : GEMM_BM, r.tile_n, r.stages, r.tiles,
-           r.waves, r.workspace, r.direct ? (mode == SB200_MODE_3XTF32 ? 2 : 1) : 3);
+  const int launches = (r.src == SRC_PANELS ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + (r.splits > 1 ? 1 : 0);
+  snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
+           r.ctas == 2 ? "pair" : "single", r.src == SRC_PANELS ? "panels" : "direct", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
+           r.splits, r.workspace, launches);
   return copy_out(buf, out, outlen);
 }
 
@@ -2578,11 +2681,8 @@ int noalloc_setup(int dev, NoAllocDevice** out) {
 }
 
 template <int MODE>
-int launch_gemm_fixed_scratch(const NoAllocDevice& nd, cudaStream_t st, long long M, long long N, long long K, const float* A,
+int launch_gemm_fixed_scratch(const NoAllocDevice& nd, int dev, cudaStream_t st, long long M, long long N, long long K, const float* A,
                               long long lda, const float* B, long long ldb, GemmParams gp) {
-  using Cfg = GemmCfg<MODE>;
-  CU_TRY(cudaFuncSetAttribute(gemm_tf32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              static_cast<int>(Cfg::kSmemBytes)));
   const long long kp = round_up(K, GEMM_BK);
   const size_t a_bytes = round_up(M * kp * 4, 1024), b_bytes = round_up(N * kp * 4, 1024);
   float* a_hi = reinterpret_cast<float*>(nd.scratch);
@@ -2607,22 +2707,17 @@ int launch_gemm_fixed_scratch(const NoAllocDevice& nd, cudaStream_t st, long lon
                                                                                static_cast<int>(N), static_cast<int>(kp));
     if ((rc = launch_check("prep_b_kernel"))) return rc;
   }
+  const int tile_n = choose_tiles(M, N, kp / GEMM_BK, 1, nd.sm_count, MODE == 3, false).tile_n;
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
   if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, GEMM_BN))) return rc;
+  if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, tile_n))) return rc;
   if ((rc = encode_panel_map(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, GEMM_BN))) return rc;
+  if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, tile_n))) return rc;
   gp.num_k_blocks = static_cast<int>(kp / GEMM_BK);
-  gp.tiles_m = static_cast<int>((M + GEMM_BM - 1) / GEMM_BM);
-  gp.tiles_n = static_cast<int>((N + GEMM_BN - 1) / GEMM_BN);
   gp.status = nd.status;
   derive_params(&gp);
-  const long long tiles = static_cast<long long>(gp.tiles_m) * gp.tiles_n;
-  const unsigned grid = static_cast<unsigned>(tiles < nd.sm_count ? tiles : nd.sm_count);
-  CUtensorMap map_d, map_c;
-  epilogue_maps(&gp, ma_hi, &map_d, &map_c);
-  gemm_tf32_kernel<MODE><<<grid, GEMM_THREADS, Cfg::kSmemBytes, st>>>(ma_hi, mb_hi, ma_lo, mb_lo, map_d, map_c, gp);
-  return launch_check("gemm_tf32_kernel");
+  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
+  return launch_tiles_for<MODE, SRC_PANELS>(tile_n, 1, dev, nd.sm_count, st, maps, gp, nullptr);
 }
 
 }  // namespace
@@ -2685,9 +2780,9 @@ extern "C" int sb200_gemm_f32_noalloc(int dev, uint64_t stream, int mode, int64_
     gemm_k0_kernel<<<static_cast<unsigned>(grid), 256, 0, st>>>(gp);
     rc = launch_check("gemm_k0_kernel");
   } else if (mode == SB200_MODE_3XTF32) {
-    rc = launch_gemm_fixed_scratch<3>(*nd, st, M, N, K, as_ptr<const float>(A), lda, as_ptr<const float>(B), ldb, gp);
+    rc = launch_gemm_fixed_scratch<3>(*nd, dev, st, M, N, K, as_ptr<const float>(A), lda, as_ptr<const float>(B), ldb, gp);
   } else {
-    rc = launch_gemm_fixed_scratch<1>(*nd, st, M, N, K, as_ptr<const float>(A), lda, as_ptr<const float>(B), ldb, gp);
+    rc = launch_gemm_fixed_scratch<1>(*nd, dev, st, M, N, K, as_ptr<const float>(A), lda, as_ptr<const float>(B), ldb, gp);
   }
   if (rc) return rc;
   CU_TRY(cudaStreamSynchronize(st));
@@ -2726,6 +2821,7 @@ extern "C" int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int6
   int rc = device_ready(dev, &d);
   if (rc) return rc;
   std::lock_guard<std::mutex> host_call_lock(d->host_call_mu);
+  const RowBlocksOf whole(M);
   if ((rc = ensure_pipe_streams(*d))) return rc;
   // device mirrors, packed: A[M x K], B[K x N], C[M x N] (if any), D[M x N], bias[N]
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
