@@ -174,3 +174,164 @@ struct ConvTile {
     if (MODE == 3) *reinterpret_cast<float*>(dst + LO) = l;
   }
 };
+
+template <int MODE, int BN, bool VEC>
+__global__ void __launch_bounds__(CONV_THREADS, 1)
+gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c,
+                    const GemmParams p) {
+  using Cfg = ConvCfg<MODE, BN>;
+  constexpr int STAGES = Cfg::kStages;
+  constexpr uint32_t B_BYTES = Cfg::kBBytes;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ctrl = smem + STAGES * Cfg::kStageBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* done_bar = full_bar + 2 * STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full_bar + 2 * STAGES + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), CONV_WARPS);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(done_bar), 1);
+    for (int i = 0; i < 2 * CONV_WARPS; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
+  }
+  if (warp == CONV_WARPS) {
+    tmem_alloc(smem_u32(tmem_slot), BN);
+    tmem_relinquish();
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+  grid_dependency_wait();  // nothing above touched global memory
+  const int num_tiles = p.tiles_m * p.tiles_n, num_items = num_tiles * p.splits;
+
+  if (warp < CONV_WARPS) {
+    // ----------------------------------------- load, convert, store; then the epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CONV_REGS_CONVERT));
+    EpiWarp epi = epi_warp(smem, ctrl, warp);
+    const int quarter = warp & 3, half = warp >> 2;
+    int stage = 0, local = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++local) {
+      int tm, tn;
+      pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      const int m0 = tm * 128, n0 = tn * BN, split = item / num_tiles;
+      const int kb0 = split * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
+      ConvTile<BN, VEC> t[CONV_AHEAD + 1];
+#pragma unroll
+      for (int u = 0; u < CONV_AHEAD; ++u)
+        if (u < blocks) t[u].load(o, p.M, p.N, m0, n0, (kb0 + u) * GEMM_BK, threadIdx.x);
+      for (int kb = 0; kb < blocks && ok; kb += CONV_AHEAD + 1) {
+#pragma unroll
+        for (int u = 0; u <= CONV_AHEAD; ++u) {  // t[] is indexed by constants: it stays in registers
+          if (kb + u >= blocks) break;
+          if (kb + u + CONV_AHEAD < blocks)
+            t[(u + CONV_AHEAD) % (CONV_AHEAD + 1)].load(o, p.M, p.N, m0, n0, (kb0 + kb + u + CONV_AHEAD) * GEMM_BK, threadIdx.x);
+          const bool free = mbar_wait_bounded(smem_u32(&empty_bar[stage]), phase ^ 1u, abort_flag);
+          if (!__all_sync(0xffffffffu, free)) {
+            if (lane == 0) atomicCAS(p.status, 0, 0x2100 | stage);
+            ok = false;
+            break;
+          }
+          t[u].template store<MODE>(smem + stage * Cfg::kStageBytes, threadIdx.x);
+          fence_async_shared();  // before the tensor core reads what was written here
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&full_bar[stage]));
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      const bool landed = ok && mbar_wait_bounded(smem_u32(done_bar), local & 1, abort_flag);
+      if (!__all_sync(0xffffffffu, landed)) {
+        if (lane == 0) atomicCAS(p.status, 0, 0x2400);
+        ok = false;
+      }
+      if (ok) {
+        tc_fence_after_sync();
+        const int row0 = m0 + quarter * 32, c0 = n0 + half * (BN / 2);
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2);
+        if (c0 < p.N) {
+          if (!p.tma_epilogue) {
+            epilogue_rows<BN / 2>(p, taddr, epi.buf, lane, row0, c0);
+          } else {
+            epilogue_tma_begin(p, &map_c, epi, row0, c0);
+            if (!epilogue_tma<BN / 2>(p, &map_d, &map_c, taddr, epi, lane, row0, c0, split * p.part_rows, abort_flag)) {
+              if (lane == 0) atomicCAS(p.status, 0, 0x2500);
+              ok = false;
+            }
+          }
+        }
+        if (elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
+        tc_fence_before_sync();
+      }
+      // every warp is through with the accumulator and the tiles before the next item's operands arrive
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (*abort_flag) ok = false;  // a wait ran out in some warp: all leave together
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------- MMA issuer
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CONV_REGS_MMA));
+    if (warp == CONV_WARPS && elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_tf32(128, BN, true);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+        const int kb0 = (item / num_tiles) * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
+        for (int kb = 0; kb < blocks; ++kb) {
+          if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), phase, abort_flag)) {
+            atomicCAS(p.status, 0, 0x2300 | stage);
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t sa_hi = smem_u32(smem + stage * Cfg::kStageBytes), sb_hi = sa_hi + PAIR_A_BYTES;
+          const uint32_t sa_lo = sb_hi + B_BYTES, sb_lo = sa_lo + PAIR_A_BYTES;
+#pragma unroll
+          for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; ++k) {
+            const uint64_t da_hi = umma_desc_k_sw128(sa_hi + k * 32), db_hi = umma_desc_mn_sw128_32b(sb_hi + k * 1024, 4096);
+            const uint32_t accumulate = (kb | k) ? 1u : 0u;
+            if (MODE == 3) {
+              const uint64_t da_lo = umma_desc_k_sw128(sa_lo + k * 32), db_lo = umma_desc_mn_sw128_32b(sb_lo + k * 1024, 4096);
+              umma_tf32(tmem_base, da_lo, db_hi, idesc, accumulate);
+              umma_tf32(tmem_base, da_hi, db_lo, idesc, 1u);
+              umma_tf32(tmem_base, da_hi, db_hi, idesc, 1u);
+            } else {
+              umma_tf32(tmem_base, da_hi, db_hi, idesc, accumulate);
+            }
+          }
+          umma_commit(smem_u32(&empty_bar[stage]));
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        if (ok) umma_commit(smem_u32(done_bar));
+      }
+    }
+    __syncwarp();
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == CONV_WARPS) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, BN);
+  }
+}
+
+}  // namespace sb200

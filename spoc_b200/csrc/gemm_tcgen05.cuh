@@ -378,20 +378,6 @@ __device__ __forceinline__ float tf32_lo(float x, float hi) {
   return (fabsf(hi) <= 3.402823466e+38f) ? tf32_round(x - hi) : 0.0f;
 }
 
-// Rounding to TF32, nearest-even, in integer arithmetic: the same bits as tf32_round for finite x (its conversion instruction
-// issues at a quarter of the rate).
-__device__ __forceinline__ float tf32_round_int(float x) {
-  const uint32_t u = __float_as_uint(x);
-  return __uint_as_float((u + 0xfffu + ((u >> 13) & 1u)) & 0xffffe000u);
-}
-
-// tf32_lo(x, tf32_round(x)) for the kernel that makes low parts on the fly: 12 instructions of full rate per element.  From
-// 0x7f7ff000 on (the upper half of FLT_MAX's last TF32 step, infinities, NaNs) the high part is not finite.
-__device__ __forceinline__ float tf32_lo_int(float x) {
-  const float lo = tf32_round_int(x - tf32_round_int(x));
-  return (__float_as_uint(x) & 0x7fffffffu) >= 0x7f7ff000u ? 0.0f : lo;
-}
-
 // A[M x K] (row stride lda) -> hi[M x Kp] (and lo[M x Kp]), Kp = K rounded up
 // to 32, columns K..Kp zero.  One thread per 4 consecutive k.
 // LO_ONLY: store just the low parts (the high parts are then taken from the source matrix itself by a

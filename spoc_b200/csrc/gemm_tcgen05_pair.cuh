@@ -10,7 +10,7 @@
 // (completion counted on the leader's `full` barrier); one lane of warp 1 of the leader block (cluster rank 0) issues the
 // MMAs for both blocks and commits to the `empty` and `tmem_full` barriers of both; warps 2-5 run the epilogue on their own
 // accumulator rows and hand the accumulator back by arriving on the leader's `tmem_empty` barrier, while the MMA warp
-// already works on the next tile in the other accumulator; with SRC_SPLIT warps 6-9 make the low parts (below).
+// already works on the next tile in the other accumulator.
 // Every TMA load is issued by the block that consumes it (plain per-block loads).
 #pragma once
 #include "gemm_tcgen05.cuh"
@@ -26,10 +26,8 @@ constexpr uint32_t PAIR_A_BYTES = 128 * GEMM_BK * 4;  // this block's A rows: 16
 //   SRC_DIRECT  the caller's row-major A and B through TFLOAT32 tensor maps (TMA rounds to TF32 on the way in); B arrives as
 //               [32 k][32 n] slabs (swizzle 128B with 32-byte atoms) and is consumed through an MN-major descriptor.  The low
 //               parts of 3xTF32 come from prepared panels: A [M x Kp], B row-major [K x Np] read as slabs like B itself.
-//   SRC_SPLIT   3xTF32 without any preparation: the caller's tiles are loaded twice, once through the TFLOAT32 maps (the high
-//               parts) and once as they are into the low parts' place, where warps 6-9 replace every element x by
-//               rn_tf32(x - rn_tf32(x)) before the MMAs see the stage.  Elementwise and in place, so no layout is involved.
-enum { SRC_PANELS = 0, SRC_DIRECT = 1, SRC_SPLIT = 2 };
+//   SRC_CONVERT not this kernel: gemm_convert_kernel loads the caller's matrices itself (gemm_convert.cuh).
+enum { SRC_PANELS = 0, SRC_DIRECT = 1, SRC_CONVERT = 2 };
 
 template <int MODE, int SRC, int BN, int CTAS>
 struct TileCfg {
@@ -41,7 +39,7 @@ struct TileCfg {
   static constexpr int kStagesFit = (192 * 1024) / kStageBytes;
   static constexpr int kStages = kStagesFit > 8 ? 8 : kStagesFit;  // pairs, 256/192/128/64 columns: 6/6/8/8, 3xTF32 3/3/4/4
   static constexpr uint32_t kSmemBytes = kStages * kStageBytes + GEMM_EPI_BUF_BYTES + GEMM_CTRL_BYTES + 1024;
-  static constexpr int kThreads = GEMM_THREADS + (SRC == SRC_SPLIT ? 128 : 0);
+  static constexpr int kThreads = GEMM_THREADS;
 };
 
 constexpr int PAIR_EPOCH_RING = 64;    // epoch counters (a pair far ahead wraps onto an old counter: harmless, a hint)
@@ -90,10 +88,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   constexpr bool MIXED = MODE == 5;
   constexpr bool THREE = MODE == 3 || MODE == 4;
   constexpr bool F16 = MODE == 4 || MODE == 2;
-  constexpr bool DIRECT = SRC != SRC_PANELS, SPLIT = SRC == SRC_SPLIT;
+  constexpr bool DIRECT = SRC != SRC_PANELS;
   static_assert(!MIXED || SRC == SRC_DIRECT, "the mixed mode reads the main term's operands where they lie");
   static_assert(!(F16 && DIRECT), "fp16 panels are always prepared");
-  static_assert(!SPLIT || MODE == 3, "only 3xTF32 has low parts to make");
   constexpr int BK_ELEMS = F16 ? 2 * GEMM_BK : GEMM_BK;  // elements of K per k-block
   constexpr int STAGES = Cfg::kStages;
   constexpr uint32_t B_BYTES = Cfg::kBBytes;
@@ -113,8 +110,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   uint64_t* tmem_empty_bar = bars + 2 * STAGES + 2;  // used in the leader only
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* raw_bar = bars + 2 * STAGES + 5;         // SRC_SPLIT: the tiles to be split have landed (one set per block)
-  static_assert((3 * STAGES + 5) * 8 <= GEMM_CTRL_CBAR, "the barriers fit the control area");
+  static_assert((2 * STAGES + 5) * 8 <= GEMM_CTRL_CBAR, "the barriers fit the control area");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -124,9 +120,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), SPLIT ? 1 + CTAS : 1);  // the producer, and a splitting warp of each block
+      mbar_init(smem_u32(&full_bar[s]), 1);
       mbar_init(smem_u32(&empty_bar[s]), 1);
-      if (SPLIT) mbar_init(smem_u32(&raw_bar[s]), 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tmem_full_bar[a]), 1);
@@ -210,7 +205,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
             break;
           }
           // the leader arms its barrier with the bytes of both blocks
-          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), CTAS * (SPLIT ? Cfg::kStageBytes / 2 : Cfg::kStageBytes));
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), CTAS * Cfg::kStageBytes);
           const uint32_t bar = CTAS == 2 ? map_to_cta(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
           uint8_t* sp = stage_base + stage * Cfg::kStageBytes;
           auto load = [&](uint8_t* dst, const CUtensorMap& map, int x, int y, uint64_t pol) {
@@ -234,16 +229,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
               }
             }
           } else {
-            if (SPLIT) {
-              // the tiles the splitting warps of this block work on come first
-              const uint32_t raw = smem_u32(&raw_bar[stage]);
-              uint8_t* lp = sp + PAIR_A_BYTES + B_BYTES;
-              mbar_arrive_expect_tx(raw, Cfg::kStageBytes / 2);
-              tma_load_2d_hint(smem_u32(lp), &map_a_lo, raw, kb * BK_ELEMS, m0, pol_a);
-#pragma unroll
-              for (int sl = 0; sl < SLABS; ++sl)
-                tma_load_2d_hint(smem_u32(lp + PAIR_A_BYTES + sl * 4096), &map_b_lo, raw, n0 + 32 * sl, kb * BK_ELEMS, pol_b);
-            }
             load(sp, map_a_hi, kb * BK_ELEMS, m0, pol_a);
             if (DIRECT) {
               // B is K x N row-major: x = column, y = k; slabs of 32 columns cover this block's part
@@ -252,7 +237,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
             } else {
               load(sp + PAIR_A_BYTES, map_b_hi, kb * BK_ELEMS, n0, pol_b);
             }
-            if (THREE && !SPLIT) {
+            if (THREE) {
               uint8_t* lp = sp + PAIR_A_BYTES + B_BYTES;
               load(lp, map_a_lo, kb * BK_ELEMS, m0, pol_a);
               if (DIRECT) {
@@ -373,7 +358,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
+  } else {
     // --------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // tensor-memory lanes [32*quarter, 32*quarter+32)
     EpiWarp epi = epi_warp(epi_base, ctrl, warp - 2);
@@ -416,53 +401,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     __syncwarp();
     if (elect_one()) bulk_wait_read<0>();  // the tiles must outlive the stores that read them
     __syncwarp();
-  } else {
-    // -------------------------------------------------- low parts (SRC_SPLIT)
-    // Each warp has a stage of the ring of its own, so that the latencies of a stage — the wait, the loads, the fence, the
-    // arrival — overlap with those of the others; all four warps on one stage took 1 us a stage.  (One warp per stage also
-    // keeps every wait at most one phase behind its barrier, which is what waiting by parity needs.)
-    if constexpr (SPLIT) {
-      constexpr int QUADS = static_cast<int>(Cfg::kStageBytes / 2 / 16);  // float4 of the tiles to be split
-      constexpr int BATCH = 8;
-      static_assert(QUADS % (32 * BATCH) == 0, "every lane has the same work");
-      static_assert(STAGES <= 4, "a warp per stage");
-      const int w = warp - 6;
-      int n = 0;  // stages so far, over all work items
-      bool ok = true;
-      for (int item = pair_id; item < num_items && ok; item += num_pairs) {
-        int k0;
-        const int stages = item_stages(item, k0);
-        for (int it = (w + STAGES - n % STAGES) % STAGES; it < stages && w < STAGES; it += STAGES) {
-          const int stage = w;
-          const uint32_t phase = ((n + it) / STAGES) & 1;
-          const bool landed = mbar_wait_bounded(smem_u32(&raw_bar[stage]), phase, abort_flag);
-          if (!__all_sync(0xffffffffu, landed)) {
-            if (lane == 0) atomicCAS(p.status, 0, 0x1600 | (rank << 4) | stage);
-            ok = false;
-            break;
-          }
-          float4* lo = reinterpret_cast<float4*>(stage_base + stage * Cfg::kStageBytes + PAIR_A_BYTES + B_BYTES) + lane;
-#pragma unroll 1
-          for (int q = 0; q < QUADS / 32; q += BATCH) {
-            float4 x[BATCH];
-#pragma unroll
-            for (int j = 0; j < BATCH; ++j) x[j] = lo[(q + j) * 32];
-#pragma unroll
-            for (int j = 0; j < BATCH; ++j)
-              lo[(q + j) * 32] = make_float4(tf32_lo_int(x[j].x), tf32_lo_int(x[j].y), tf32_lo_int(x[j].z), tf32_lo_int(x[j].w));
-          }
-          fence_async_shared();  // before the tensor core reads what was written here
-          __syncwarp();
-          if (lane == 0) {
-            if (CTAS == 2)
-              mbar_arrive_cluster(map_to_cta(smem_u32(&full_bar[stage]), 0));
-            else
-              mbar_arrive(smem_u32(&full_bar[stage]));
-          }
-        }
-        n += stages;
-      }
-    }
   }
 
   // Neither block may retire, or free tensor memory, while its peer can still signal its barriers, read its shared memory or

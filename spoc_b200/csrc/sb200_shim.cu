@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/sb200.h"
+#include "gemm_convert.cuh"
 #include "gemm_tcgen05.cuh"
 #include "gemm_tcgen05_pair.cuh"
 #include "internal.hpp"
@@ -491,7 +492,9 @@ constexpr int kMaxSplits = 32;
 // partial results' way through L2 (about 4 TB/s), and is left to products that stay at 16 k-blocks per item or more.
 // fixed_splits > 0: the division is given (a row block of a larger product is divided as the whole is, so that it has the
 // same bits).
-TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0) {
+// convert: gemm_convert_kernel's rates (see there) instead of the pair kernel's.
+TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
+                       bool convert = false) {
   TileShape best;
   const int forced = tile_n_setting();
   double best_cost = 0.0;
@@ -501,7 +504,7 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
     if (ctas == 1 && bn > 128) continue;
     if (bn == 192 && (!three || forced)) continue;
     if (forced && bn != forced && !(ctas == 1 && forced == 256 && bn == 128)) continue;
-    const double per_kblock = three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0) : (bn == 256 ? 277.0 : 165.0);
+    const double per_kblock = convert ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0)) : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0) : (bn == 256 ? 277.0 : 165.0);
     const long long tiles = tiles_m * ((N + bn - 1) / bn);
     for (int sp = 1; sp <= kMaxSplits; ++sp) {
       if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * kMinSplitKBlocks)) continue;
@@ -549,6 +552,38 @@ struct OperandMaps {
   CUtensorMap a_hi, b_hi, a_lo, b_lo, a_x, b_x;
 };
 
+// The parameters and output maps a GEMM kernel is launched with: *kp is *gp with the epilogue as it is, or, when the k-loop is
+// divided, with one that stores plain partial sums to `part` ([splits][part_rows][roundup(N, 4)] floats).
+int output_maps(GemmParams* gp, GemmParams* kp, float* part, const CUtensorMap& filler, CUtensorMap* map_d, CUtensorMap* map_c) {
+  if (gp->splits == 1) {
+    gp->part_rows = 0;
+    epilogue_maps(gp, filler, map_d, map_c);
+    *kp = *gp;
+    return SB200_OK;
+  }
+  const long long ld = round_up(gp->N, 4);
+  gp->part_rows = static_cast<int>(round_up(gp->M, 32));
+  *kp = *gp;
+  kp->C = kp->bias = kp->row_scale = kp->col_scale = nullptr;
+  kp->alpha = 1.0f;
+  kp->act = 0;
+  kp->n_replicas = 0;
+  kp->tma_epilogue = 1;
+  kp->epoch_ctr = nullptr;
+  *map_c = filler;
+  return encode_map_2d(map_d, part, ld, static_cast<long long>(gp->part_rows) * gp->splits, ld, 32, 32, false);
+}
+
+// The launch that adds up the partial sums of a divided k-loop (none when it was not divided).
+int launch_reduce(int sm_count, cudaStream_t st, const GemmParams& gp, const float* part) {
+  if (gp.splits == 1) return SB200_OK;
+  const long long ld = round_up(gp.N, 4), quads = static_cast<long long>(gp.M) * (ld >> 2);
+  long long blocks = (quads + 255) / 256;
+  if (blocks > static_cast<long long>(sm_count) * 8) blocks = static_cast<long long>(sm_count) * 8;
+  CU_TRY(launch_pdl(gemm_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, part, ld, gp.part_rows, gp.splits, gp));
+  return launch_check("gemm_reduce_kernel");
+}
+
 // One instantiation of the GEMM kernel: shared-memory attribute and resident blocks (pairs) are looked up once per device,
 // then the launch.  part: partial results of a divided k-loop ([gp.splits][gp.part_rows][part_ld] floats), added up by a
 // second launch.
@@ -590,30 +625,45 @@ int launch_tiles(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   const long long used = items < units ? items : units;
   const dim3 grid(static_cast<unsigned>(CTAS * used)), block(Cfg::kThreads);
   CUtensorMap map_d, map_c;
-  if (gp.splits == 1) {
-    gp.part_rows = 0;
-    epilogue_maps(&gp, m.a_hi, &map_d, &map_c);
-    CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_c, gp));
-    return launch_check("gemm_pair_kernel");
-  }
-  const long long ld = round_up(gp.N, 4);
-  gp.part_rows = static_cast<int>(round_up(gp.M, 32));
-  GemmParams pp = gp;  // the partial sums as they are
-  pp.C = pp.bias = pp.row_scale = pp.col_scale = nullptr;
-  pp.alpha = 1.0f;
-  pp.act = 0;
-  pp.n_replicas = 0;
-  pp.tma_epilogue = 1;
-  pp.epoch_ctr = nullptr;
-  if (int rc = encode_map_2d(&map_d, part, ld, static_cast<long long>(gp.part_rows) * gp.splits, ld, 32, 32, false)) return rc;
-  CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_d, pp));
+  GemmParams kp;
+  if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
+  CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_c, kp));
   if (int rc = launch_check("gemm_pair_kernel")) return rc;
-  const long long quads = static_cast<long long>(gp.M) * (ld >> 2);
-  long long blocks = (quads + 255) / 256;
-  if (blocks > static_cast<long long>(sm_count) * 8) blocks = static_cast<long long>(sm_count) * 8;
-  CU_TRY(launch_pdl(gemm_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, static_cast<const float*>(part), ld,
-                    gp.part_rows, gp.splits, gp));
-  return launch_check("gemm_reduce_kernel");
+  return launch_reduce(sm_count, st, gp, part);
+}
+
+// gemm_convert_kernel, the same way.
+template <int MODE, int BN, bool VEC>
+int launch_convert(int dev_index, int sm_count, cudaStream_t st, const ConvOperands& o, GemmParams gp, float* part) {
+  using Cfg = ConvCfg<MODE, BN>;
+  auto kernel = gemm_convert_kernel<MODE, BN, VEC>;
+  static std::atomic<int> attr_set[kMaxDevices];
+  if (!attr_set[dev_index].load()) {
+    CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
+    attr_set[dev_index].store(1);
+  }
+  gp.tiles_m = (gp.M + 127) / 128;
+  gp.tiles_n = static_cast<int>((static_cast<long long>(gp.N) + BN - 1) / BN);
+  gp.group_m = PAIR_GROUP_M;
+  if (gp.splits < 1) gp.splits = 1;
+  gp.split_k_blocks = (gp.num_k_blocks + gp.splits - 1) / gp.splits;
+  const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
+  const dim3 grid(static_cast<unsigned>(items < sm_count ? items : sm_count));
+  CUtensorMap map_d, map_c;
+  memset(&map_d, 0, sizeof map_d);
+  GemmParams kp;
+  if (int rc = output_maps(&gp, &kp, part, map_d, &map_d, &map_c)) return rc;
+  CU_TRY(launch_pdl(kernel, grid, dim3(CONV_THREADS), Cfg::kSmemBytes, st, 1, o, map_d, map_c, kp));
+  if (int rc = launch_check("gemm_convert_kernel")) return rc;
+  return launch_reduce(sm_count, st, gp, part);
+}
+
+template <int MODE>
+int launch_convert_for(int bn, bool vec, int dev_index, int sm_count, cudaStream_t st, const ConvOperands& o, const GemmParams& gp,
+                       float* part) {
+  if (bn == 64)
+    return vec ? launch_convert<MODE, 64, true>(dev_index, sm_count, st, o, gp, part) : launch_convert<MODE, 64, false>(dev_index, sm_count, st, o, gp, part);
+  return vec ? launch_convert<MODE, 128, true>(dev_index, sm_count, st, o, gp, part) : launch_convert<MODE, 128, false>(dev_index, sm_count, st, o, gp, part);
 }
 
 size_t partial_bytes(long long M, long long N, int splits) {
@@ -629,17 +679,12 @@ int launch_tiles_for(int bn, int ctas, int dev_index, int sm_count, cudaStream_t
       return launch_tiles<MODE, SRC, 128, 1>(dev_index, sm_count, st, m, gp, part);
     }
   }
-  if constexpr (!(MODE == 3 && SRC == SRC_DIRECT)) {
-    if (bn == 64) return launch_tiles<MODE, SRC, 64, 2>(dev_index, sm_count, st, m, gp, part);
-    if (bn == 128) return launch_tiles<MODE, SRC, 128, 2>(dev_index, sm_count, st, m, gp, part);
-  }
+  if (bn == 64) return launch_tiles<MODE, SRC, 64, 2>(dev_index, sm_count, st, m, gp, part);
+  if (bn == 128) return launch_tiles<MODE, SRC, 128, 2>(dev_index, sm_count, st, m, gp, part);
   if constexpr (kThree) {
     if (bn == 192) return launch_tiles<MODE, SRC, 192, 2>(dev_index, sm_count, st, m, gp, part);
   }
-  if constexpr (SRC != SRC_SPLIT) {
-    return launch_tiles<MODE, SRC, 256, 2>(dev_index, sm_count, st, m, gp, part);
-  }
-  return fail(SB200_ERR_INVALID_VALUE, "no kernel for tiles of %d columns", bn);
+  return launch_tiles<MODE, SRC, 256, 2>(dev_index, sm_count, st, m, gp, part);
 }
 
 // How sb200_gemm_f32 will run a product: which kernel, which tile, how much scratch.  One function decides, the
@@ -667,6 +712,9 @@ int gemm_variant_setting() {
 // Products of at most this many rows are computed by blocks on their own: the second block of a pair would only see rows
 // past the end.
 constexpr long long kSingleRows = 64;
+// Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands.
+constexpr double kConvertMacs = 16777216.0;              // 2^24
+constexpr double kConvertMacsUnaligned = 536870912.0;    // 2^29
 
 int stages_of(bool three, int bn, int ctas) {
   const long long stage = (three ? 2 : 1) * (16384ll + (bn / ctas) * 128ll);
@@ -677,32 +725,48 @@ int stages_of(bool three, int bn, int ctas) {
 // Set by RowBlocksOf (the host-operand calls, the launches that upload by blocks, partial launches, device groups).
 thread_local long long t_whole_rows = 0;
 
-TileShape shape_for(long long M, long long N, long long kblocks, int ctas, int sm_count, bool three, bool may_split) {
-  const int units = ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
-  if (!may_split || t_whole_rows <= M) return choose_tiles(M, N, kblocks, ctas, units, three, may_split);
-  const int whole_ctas = t_whole_rows <= kSingleRows ? 1 : 2;
-  const int whole_units = whole_ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
-  const int splits = choose_tiles(t_whole_rows, N, kblocks, whole_ctas, whole_units, three, true).splits;
-  return choose_tiles(M, N, kblocks, ctas, units, three, true, splits);
+int units_of(int ctas, int sm_count) { return ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1); }
+
+// The fp16 modes: panels always, so a block on its own up to 128 rows.
+TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_count, int* ctas) {
+  auto cut = [&](long long rows, int fixed, int* c) {
+    *c = rows <= GEMM_BM ? 1 : 2;
+    return choose_tiles(rows, N, round_up(K, 64) / 64, *c, units_of(*c, sm_count), three, true, fixed);
+  };
+  int whole_ctas;
+  const int fixed_splits = t_whole_rows > M ? cut(t_whole_rows, 0, &whole_ctas).splits : 0;
+  return cut(M, fixed_splits, ctas);
 }
 
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
+  int fixed_splits = 0;
+  if (t_whole_rows > M) {
+    const long long whole = t_whole_rows;
+    t_whole_rows = 0;
+    fixed_splits = route_gemm(mode, whole, N, K, addressable, sm_count, whole).splits;
+    t_whole_rows = whole;
+  }
   GemmRoute r;
   const int variant = gemm_variant_setting();
   const bool three = mode == SB200_MODE_3XTF32;
   // The caller's matrices are read where they lie when TMA can address them: 16-byte aligned bases and row strides.  TF32
-  // mode then needs no preparation and no scratch, and 3xTF32 mode none below 256 columns (SRC_SPLIT).
+  // mode then needs no preparation and no scratch, 3xTF32 mode panels of the low parts.
   const bool direct = variant != 1 && variant != 3 && addressable;
-  // At most 128 rows: from panels a block on its own; read directly a pair wins from 65 rows on.
-  r.ctas = variant == 1 || (variant == 0 && M <= (direct ? kSingleRows : GEMM_BM)) ? 1 : 2;
   const long long kp = round_up(K, GEMM_BK);
-  const TileShape shape = shape_for(M, N, kp / GEMM_BK, r.ctas, sm_count, three, variant == 0);
+  // One launch that converts the operands on their way (gemm_convert_kernel): few rows in 3xTF32, where panels of B would
+  // triple the traffic, and any mode's few rows of matrices TMA cannot address; and products so small that the launches that
+  // would prepare panels weigh more than the pair kernel's faster tiles give (aligned: 256^3 is about even; transposing panels
+  // of unaligned matrices are two launches and serve from about 800^3).
+  const double macs = static_cast<double>(M) * N * K;
+  const bool convert = variant == 0 && tile_n_setting() != 256 &&
+                       (addressable ? three && (M <= kSingleRows || macs < kConvertMacs) : M <= kSingleRows || macs < kConvertMacsUnaligned);
+  // From panels at most 128 rows are served by a block on its own; read directly a pair wins from 65 rows on.
+  r.ctas = convert || variant == 1 || (variant == 0 && (direct ? !three && M <= kSingleRows : M <= GEMM_BM)) ? 1 : 2;
+  const int units = units_of(r.ctas, sm_count);
+  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, convert);
   r.tile_n = shape.tile_n;
   r.splits = shape.splits;
-  // 3xTF32: at 256 columns the splitting warps' shared-memory traffic would come on top of MMAs that already keep it busy, so
-  // the low parts come from panels there
-  r.src = !direct ? SRC_PANELS : three && r.tile_n < 256 ? SRC_SPLIT : SRC_DIRECT;
-  const int units = r.ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
+  r.src = convert ? SRC_CONVERT : direct ? SRC_DIRECT : SRC_PANELS;
   r.stages = stages_of(three, r.tile_n, r.ctas);
   r.tiles = ((M + 128 * r.ctas - 1) / (128 * r.ctas)) * ((N + r.tile_n - 1) / r.tile_n);
   r.waves = (r.tiles * r.splits + units - 1) / (units > 0 ? units : 1);
@@ -726,7 +790,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   const bool addressable = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0 &&
                            (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (ldb & 3) == 0;
   const GemmRoute route = route_gemm(MODE == 3 ? SB200_MODE_3XTF32 : SB200_MODE_TF32, M, N, K, addressable, d.sm_count, panel_rows_a);
-  const bool direct = route.src != SRC_PANELS;
+  const bool direct = route.src == SRC_DIRECT;
   const int tile_n = route.tile_n;
 
   const long long kp = round_up(K, GEMM_BK);
@@ -764,12 +828,14 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     CU_TRY(cudaEventRecord(rec.e0, st));
   }
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
-  if (direct) {
+  if (route.src == SRC_CONVERT) {
+    // no panels, no operand maps
+  } else if (direct) {
     if ((rc = encode_map_2d(&ma_hi, A, K, M, lda, GEMM_BK, GEMM_BM, true))) return rc;
     if ((rc = encode_map_2d(&mb_hi, B, N, K, ldb, 32, GEMM_BK, true, true))) return rc;
     ma_lo = ma_hi;
     mb_lo = mb_hi;
-    if (MODE == 3 && route.src == SRC_DIRECT) {
+    if (MODE == 3) {
       // low parts only: B's first (K x np, row-major like B), then A's (rows x kp)
       uint8_t* ws = static_cast<uint8_t*>(d.workspace);
       float* b_lo = reinterpret_cast<float*>(ws);
@@ -792,9 +858,6 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
       }
       if ((rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
       if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
-    } else if (MODE == 3) {  // SRC_SPLIT: the matrices themselves, as they are
-      if ((rc = encode_map_2d(&ma_lo, A, K, M, lda, GEMM_BK, GEMM_BM, false))) return rc;
-      if ((rc = encode_map_2d(&mb_lo, B, N, K, ldb, 32, GEMM_BK, false, true))) return rc;
     }
   } else {
     // workspace layout: B panels first (their size does not depend on M), then the A panels
@@ -840,19 +903,15 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   derive_params(&gp);
   if (prof) CU_TRY(cudaEventRecord(rec.e1, st));
   gp.splits = route.splits;
-  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
   float* part = reinterpret_cast<float*>(static_cast<uint8_t*>(d.workspace) + route.operand_bytes);
   const int dev_index = static_cast<int>(&d - g_dev);
-  if constexpr (MODE == 3) {
-    if (route.src == SRC_SPLIT)
-      rc = launch_tiles_for<3, SRC_SPLIT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
-    else if (route.src == SRC_DIRECT)
-      rc = launch_tiles_for<3, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
-    else
-      rc = launch_tiles_for<3, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
+  if (route.src == SRC_CONVERT) {
+    const ConvOperands o{A, B, lda, ldb, static_cast<int>(K)};
+    rc = launch_convert_for<MODE>(tile_n, addressable && (K & 3) == 0 && (N & 3) == 0, dev_index, d.sm_count, st, o, gp, part);
   } else {
-    rc = direct ? launch_tiles_for<1, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
-                : launch_tiles_for<1, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
+    const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
+    rc = direct ? launch_tiles_for<MODE, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
+                : launch_tiles_for<MODE, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
   }
   if (prof) {
     CU_TRY(cudaEventRecord(rec.e2, st));
@@ -892,8 +951,8 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
                     const float* B, long long ldb, const GemmParams& gp_in) {
   const long long kp = round_up(K, 64);
   const size_t a_bytes = round_up(M * kp * 2, 1024), b_bytes = round_up(N * kp * 2, 1024);
-  const int ctas = M <= GEMM_BM ? 1 : 2;  // from panels, as in the TF32 modes
-  const TileShape shape = shape_for(M, N, kp / 64, ctas, d.sm_count, THREE, true);
+  int ctas;
+  const TileShape shape = f16_shape(M, N, K, THREE, d.sm_count, &ctas);
   const int tile_n = shape.tile_n;
   const size_t need = round_up(gemm_f16_workspace_need(M, N, K, THREE), 1024);
   std::unique_lock<std::mutex> scratch_lock(d.scratch_mu);
@@ -2395,7 +2454,8 @@ int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64
   constexpr int kSms = 148;
   if (mode == SB200_MODE_3XF16 || mode == SB200_MODE_F16) {
     const bool three = mode == SB200_MODE_3XF16;
-    const TileShape shape = shape_for(M, N, round_up(K, 64) / 64, M <= GEMM_BM ? 1 : 2, kSms, three, true);
+    int ctas;
+    const TileShape shape = f16_shape(M, N, K, three, kSms, &ctas);
     *bytes = gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape.splits);
     return SB200_OK;
   }
@@ -2416,8 +2476,9 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   if (mode == SB200_MODE_3XF16 || mode == SB200_MODE_F16) {
     const bool three = mode == SB200_MODE_3XF16;
     const long long kp = round_up(K, 64);
-    const int ctas = M <= GEMM_BM ? 1 : 2, units = ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1);
-    const TileShape shape = shape_for(M, N, kp / 64, ctas, sm_count, three, true);
+    int ctas;
+    const TileShape shape = f16_shape(M, N, K, three, sm_count, &ctas);
+    const int units = units_of(ctas, sm_count);
     const long long tiles = ((M + 128 * ctas - 1) / (128 * ctas)) * ((N + shape.tile_n - 1) / shape.tile_n);
     char fb[256];
     snprintf(fb, sizeof fb, "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
@@ -2441,9 +2502,10 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   }
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
+  // "panels" for operands TMA cannot address also when they are converted on their way (launches=1, no scratch for operands)
   const int launches = (r.src == SRC_PANELS ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + (r.splits > 1 ? 1 : 0);
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
-           r.ctas == 2 ? "pair" : "single", r.src == SRC_PANELS ? "panels" : "direct", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
+           r.ctas == 2 ? "pair" : "single", r.src == SRC_DIRECT || (r.src == SRC_CONVERT && addressable) ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
            r.splits, r.workspace, launches);
   return copy_out(buf, out, outlen);
 }

@@ -1,0 +1,97 @@
+"""The routes the automatic variant of the GEMM takes for small, narrow and long-k products: blocks on their own, operands
+converted in registers, 192-column tiles, divided k-loops and their reduction — at the edges of tiles and divisions, with the
+epilogue, for operands TMA can and cannot address, against the oracle at the bounds of the numeric modes."""
+import ctypes as C
+import math
+
+import numpy as np
+import pytest
+
+from spoc_b200 import _lib as L
+from tests import oracle_lib as O
+from tests.gpu_util import CANARY, Dev, dev_from, gemm
+from tests.test_gpu_gemm import tol
+
+pytestmark = pytest.mark.gpu
+
+MODES = [L.MODE_3XTF32, L.MODE_TF32, L.MODE_3XF16, L.MODE_F16]
+
+
+def describe(mode, M, N, K, addressable):
+    out = C.create_string_buffer(256)
+    assert L.load().sb200_gemm_describe(mode, M, N, K, addressable, 148, out, 256) == 0
+    return out.value.decode()
+
+
+# (M, N, K): one row and the whole height of a block; k just at and beyond a division; ragged everything
+SHAPES = [(1, 8, 1024), (64, 256, 1028), (65, 132, 1000), (128, 64, 2080), (17, 33, 1025), (300, 100, 4100), (129, 700, 513),
+          (64, 64, 32), (63, 61, 31), (257, 191, 2049)]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("aligned", [True, False], ids=["aligned", "unaligned"])
+def test_automatic_routes_match_the_oracle(backend, device, mode, shape, aligned):
+    M, N, K = shape
+    lda, ldb, ldd = ((x + 3) // 4 * 4 + 4 if aligned else x + 1 - x % 2 for x in (K, N, N))
+    rng = np.random.default_rng(M + N + K)
+    a, b, c = (rng.uniform(-1, 1, (r, ld)).astype(np.float32) for r, ld in ((M, lda), (K, ldb), (M, ldd)))
+    bias = rng.uniform(-0.1, 0.1, N).astype(np.float32)
+    A, B, Cm, Bi = (dev_from(backend, device, x.ravel()) for x in (a, b, c, bias))
+    D = Dev(backend, device, M * ldd)
+    try:
+        gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=ldd, ldd=ldd)
+        got = D.download().reshape(M, ldd)
+        ref = O.gemm(np.ascontiguousarray(a[:, :K]).ravel(), np.ascontiguousarray(b[:, :N]).ravel(), M, N, K, 1.5, 0.5,
+                     np.ascontiguousarray(c[:, :N]).ravel(), bias, 1)
+        # the clamp halves the reference's mean square, alpha scales the error: as in the other epilogue tests
+        assert O.gemm_rel_error(got[:, :N], ref) <= tol(mode, K) * 1.5 * math.sqrt(2), describe(mode, M, N, K, int(aligned))
+        assert np.all(got[:, N:] == CANARY)
+    finally:
+        for x in (A, B, Cm, Bi, D):
+            x.free()
+
+
+@pytest.mark.parametrize("mode", [L.MODE_3XTF32, L.MODE_TF32])
+@pytest.mark.parametrize("shape", [(64, 64, 64), (33, 100, 200), (64, 512, 480)])
+def test_operands_converted_in_registers_give_the_bits_of_the_panels(backend, device, mode, shape):
+    """The same parts summed in the same order (no k-loop here is divided): aligned quads, single elements, prepared panels."""
+    M, N, K = shape
+    a, b = O.fill(M * K, 61, 1), O.fill(K * N, 61, 2)
+    a[5] = np.float32(3.4028234e38) if mode == L.MODE_TF32 else a[5]     # rounds to infinity: no low part may come of it
+    A, B, D = dev_from(backend, device, a), dev_from(backend, device, b), Dev(backend, device, M * N)
+    A1, B1 = dev_from(backend, device, a, offset=1), dev_from(backend, device, b, offset=1)
+    try:
+        backend.set_gemm_variant(3)
+        gemm(backend, device, mode, M, N, K, A, B, D)
+        want = D.download()
+        backend.set_gemm_variant(0)
+        assert "splits=1 " in describe(mode, M, N, K, 1) and "splits=1 " in describe(mode, M, N, K, 0)
+        for x, y in ((A, B), (A1, B1)):
+            D.clear()
+            gemm(backend, device, mode, M, N, K, x, y, D)
+            assert np.array_equal(D.download().view(np.uint32), want.view(np.uint32))
+    finally:
+        backend.set_gemm_variant(0)
+        for x in (A, B, A1, B1, D):
+            x.free()
+
+
+def test_192_column_tiles_match_the_256_column_ones(backend, device):
+    M, N, K = 1536, 2044, 256
+    assert "tile=256x192" in describe(L.MODE_3XTF32, M, N, K, 1)
+    a, b = O.fill(M * K, 62, 1), O.fill(K * N, 62, 2)
+    A, B, D = dev_from(backend, device, a), dev_from(backend, device, b), Dev(backend, device, M * N)
+    try:
+        for mode in (L.MODE_3XTF32, L.MODE_3XF16):
+            gemm(backend, device, mode, M, N, K, A, B, D)
+            got = D.download()
+            assert L.load().sb200_set_gemm_tile_n(256) == 0
+            D.clear()
+            gemm(backend, device, mode, M, N, K, A, B, D)
+            assert L.load().sb200_set_gemm_tile_n(0) == 0
+            assert np.array_equal(D.download(), got)
+    finally:
+        L.load().sb200_set_gemm_tile_n(0)
+        for x in (A, B, D):
+            x.free()
