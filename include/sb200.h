@@ -380,7 +380,8 @@ SB200_API int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int64
 /* bytes of library-owned scratch sb200_gemm_f32 needs for these sizes */
 SB200_API int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64_t *bytes);
 /* how sb200_gemm_f32 would run these sizes on a device with sm_count SMs, as text:
- * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L".
+ * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L"
+ * (L: kernels' passes, the preparation of A and of B counted apart although they may share a launch).
  * addressable = operands 16-byte aligned with row strides that are multiples of 4 floats.  Needs no GPU. */
 SB200_API int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressable, int sm_count,
                                   char *out, int outlen);

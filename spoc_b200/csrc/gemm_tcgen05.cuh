@@ -9,7 +9,7 @@
 //
 // Two stages:
 //  1. operand preparation, where it is needed: A and B split into TF32-exact panels  hi = rn_tf32(x),  lo = rn_tf32(x - hi)
-//     (prep_a_kernel / prep_b_kernel: K-major, B transposed on the way, K zero-padded to a multiple of 32), or the low parts
+//     (prep_panels_kernel: K-major, B transposed on the way, K zero-padded to a multiple of 32), or the low parts
 //     alone (prep_lo_two_kernel), or fp16 panels.
 //  2. gemm_pair_kernel (gemm_tcgen05_pair.cuh).
 // This file has the preparation kernels, the parameters and the epilogue.
@@ -378,36 +378,15 @@ __device__ __forceinline__ float tf32_lo(float x, float hi) {
   return (fabsf(hi) <= 3.402823466e+38f) ? tf32_round(x - hi) : 0.0f;
 }
 
-// A[M x K] (row stride lda) -> hi[M x Kp] (and lo[M x Kp]), Kp = K rounded up
-// to 32, columns K..Kp zero.  One thread per 4 consecutive k.
-// LO_ONLY: store just the low parts (the high parts are then taken from the source matrix itself by a
-// TFLOAT32 tensor map, which applies the same rounding).
-template <int MODE, bool LO_ONLY = false>
-__global__ void prep_a_kernel(const float* __restrict__ A, long long lda, float* __restrict__ hi,
-                              float* __restrict__ lo, int M, int K, int Kp, int vec_ok) {
-  const long long quads_per_row = Kp >> 2;
-  const long long total = static_cast<long long>(M) * quads_per_row;
-  for (long long q = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; q < total;
-       q += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long row = q / quads_per_row;
-    const int k = static_cast<int>(q - row * quads_per_row) << 2;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float* src = A + row * lda + k;
-    if (vec_ok && k + 3 < K) {
-      x = *reinterpret_cast<const float4*>(src);
-    } else {
-      if (k < K) x.x = src[0];
-      if (k + 1 < K) x.y = src[1];
-      if (k + 2 < K) x.z = src[2];
-      if (k + 3 < K) x.w = src[3];
-    }
-    float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
-    if (!LO_ONLY) *reinterpret_cast<float4*>(hi + row * Kp + k) = h;
-    if (MODE == 3) {
-      float4 l = make_float4(tf32_lo(x.x, h.x), tf32_lo(x.y, h.y), tf32_lo(x.z, h.z), tf32_lo(x.w, h.w));
-      *reinterpret_cast<float4*>(lo + row * Kp + k) = l;
-    }
-  }
+// Four elements of a row from column k on, zeros past the end.
+__device__ __forceinline__ float4 load_quad(const float* row, int k, int cols, int vec_ok) {
+  if (vec_ok && k + 3 < cols) return *reinterpret_cast<const float4*>(row + k);
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (k < cols) x.x = row[k];
+  if (k + 1 < cols) x.y = row[k + 1];
+  if (k + 2 < cols) x.z = row[k + 2];
+  if (k + 3 < cols) x.w = row[k + 3];
+  return x;
 }
 
 // The low parts of two row-major matrices in one launch (A and B of a 3xTF32 product whose high parts TMA
@@ -426,15 +405,7 @@ __device__ __forceinline__ void prep_lo_rows(const PrepLoJob& j, long long block
   for (long long q = block * blockDim.x + threadIdx.x; q < total; q += nblocks * blockDim.x) {
     const long long row = q / quads_per_row;
     const int k = static_cast<int>(q - row * quads_per_row) << 2;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float* src = j.src + row * j.ld + k;   // callers guarantee 16-byte aligned rows
-    if (k + 3 < j.cols) {
-      x = *reinterpret_cast<const float4*>(src);
-    } else {
-      if (k < j.cols) x.x = src[0];
-      if (k + 1 < j.cols) x.y = src[1];
-      if (k + 2 < j.cols) x.z = src[2];
-    }
+    const float4 x = load_quad(j.src + row * j.ld, k, j.cols, 1);  // callers guarantee 16-byte aligned rows
     const float4 l = make_float4(tf32_lo(x.x, tf32_round(x.x)), tf32_lo(x.y, tf32_round(x.y)),
                                  tf32_lo(x.z, tf32_round(x.z)), tf32_lo(x.w, tf32_round(x.w)));
     *reinterpret_cast<float4*>(j.lo + row * j.colsp + k) = l;
@@ -444,6 +415,7 @@ __device__ __forceinline__ void prep_lo_rows(const PrepLoJob& j, long long block
 // gate: when not null the kernel works only if *gate == 0 (the mixed mode declined the operands).
 __global__ void prep_lo_two_kernel(const PrepLoJob a, const PrepLoJob b, int blocks_a, const int* gate = nullptr) {
   grid_launch_dependents();  // the GEMM behind this launch may set itself up now; it waits before reading
+  grid_dependency_wait();    // launched the same way, so behind the last user of the panels' memory
   if (gate && *gate != 0) return;
   if (static_cast<int>(blockIdx.x) < blocks_a)
     prep_lo_rows(a, blockIdx.x, blocks_a);
@@ -451,35 +423,61 @@ __global__ void prep_lo_two_kernel(const PrepLoJob a, const PrepLoJob b, int blo
     prep_lo_rows(b, blockIdx.x - blocks_a, gridDim.x - blocks_a);
 }
 
-// B[K x N] (row stride ldb) -> hi[N x Kp] (and lo[N x Kp]): 32x32 tiles
-// transposed through shared memory; block (32, 8); 1-D grid over
-// (Kp/32) * ceil(N/32) tiles.
+// Panels for operands TMA cannot address, A and B in one launch (blocks [0, blocks_a) work on A).
+// A[M x K] (row stride lda) -> hi[M x Kp] (and lo[M x Kp]), Kp = K rounded up to 32, columns K..Kp zero: one thread per 4
+// consecutive k.  B[K x N] (row stride ldb) -> hi[N x Kp] (and lo[N x Kp]): 32x32 tiles transposed through shared memory.
+struct PanelJobA {
+  const float* src;
+  long long ld;
+  float *hi, *lo;
+  int rows, cols, colsp, vec_ok;
+};
+struct PanelJobB {
+  const float* src;
+  long long ld;
+  float *hi, *lo;
+  int K, N, Kp;
+};
+
 template <int MODE>
-__global__ void prep_b_kernel(const float* __restrict__ B, long long ldb, float* __restrict__ hi,
-                              float* __restrict__ lo, int K, int N, int Kp) {
+__global__ void __launch_bounds__(256) prep_panels_kernel(const PanelJobA a, const PanelJobB b, int blocks_a) {
   __shared__ float tile[32][33];
-  const long long k_tiles = Kp >> 5;
-  const long long n_tiles = (N + 31) >> 5;
-  const long long total = k_tiles * n_tiles;
-  for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (static_cast<int>(blockIdx.x) < blocks_a) {
+    const long long quads_per_row = a.colsp >> 2;
+    const long long total = a.rows * quads_per_row;
+    for (long long q = blockIdx.x * 256ll + threadIdx.x; q < total; q += blocks_a * 256ll) {
+      const long long row = q / quads_per_row;
+      const int k = static_cast<int>(q - row * quads_per_row) << 2;
+      const float4 x = load_quad(a.src + row * a.ld, k, a.cols, a.vec_ok);
+      const float4 h = make_float4(tf32_round(x.x), tf32_round(x.y), tf32_round(x.z), tf32_round(x.w));
+      *reinterpret_cast<float4*>(a.hi + row * a.colsp + k) = h;
+      if (MODE == 3)
+        *reinterpret_cast<float4*>(a.lo + row * a.colsp + k) =
+            make_float4(tf32_lo(x.x, h.x), tf32_lo(x.y, h.y), tf32_lo(x.z, h.z), tf32_lo(x.w, h.w));
+    }
+    return;
+  }
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long n_tiles = (b.N + 31) >> 5, total = (b.Kp >> 5) * n_tiles;
+  for (long long t = blockIdx.x - blocks_a; t < total; t += gridDim.x - blocks_a) {
     // n varies fastest so consecutive blocks read consecutive 128-byte runs of a B row
     const long long kt = t / n_tiles;
-    const int n0 = static_cast<int>(t - kt * n_tiles) << 5;
-    const int k0 = static_cast<int>(kt) << 5;
+    const int n0 = static_cast<int>(t - kt * n_tiles) << 5, k0 = static_cast<int>(kt) << 5;
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
-      const int k = k0 + threadIdx.y + j, n = n0 + threadIdx.x;
-      tile[threadIdx.y + j][threadIdx.x] = (k < K && n < N) ? B[static_cast<long long>(k) * ldb + n] : 0.0f;
+      const int k = k0 + ty + j, n = n0 + tx;
+      tile[ty + j][tx] = (k < b.K && n < b.N) ? b.src[static_cast<long long>(k) * b.ld + n] : 0.0f;
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
-      const int n = n0 + threadIdx.y + j, k = k0 + threadIdx.x;
-      if (n < N) {
-        const float x = tile[threadIdx.x][threadIdx.y + j];
-        const float h = tf32_round(x);
-        hi[static_cast<long long>(n) * Kp + k] = h;
-        if (MODE == 3) lo[static_cast<long long>(n) * Kp + k] = tf32_lo(x, h);
+      const int n = n0 + ty + j, k = k0 + tx;
+      if (n < b.N) {
+        const float x = tile[tx][ty + j], h = tf32_round(x);
+        b.hi[static_cast<long long>(n) * b.Kp + k] = h;
+        if (MODE == 3) b.lo[static_cast<long long>(n) * b.Kp + k] = tf32_lo(x, h);
       }
     }
     __syncthreads();
@@ -516,125 +514,193 @@ __device__ __forceinline__ void f16_split(float x, float s, __half& hi, __half& 
 }
 
 __device__ __forceinline__ unsigned int abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned int abs_bits_max(const float4& x) {
+  return max(max(abs_bits(x.x), abs_bits(x.y)), max(abs_bits(x.z), abs_bits(x.w)));
+}
 
 // A[M x K] -> hi, lo [M x Kp] halves (lo may be null: single-pass mode), Kp = K rounded up to 64, padding zero, and
-// row_scale[M].  One warp per row: a first sweep finds the row's largest magnitude (non-negative floats order like
-// unsigned integers), a second — the row comes from cache — scales, splits and stores 8 elements per lane and step
-// (two 128-bit loads when the rows allow it, one 128-bit store per panel).
-__global__ void prep_a_f16_kernel(const float* __restrict__ A, long long lda, __half* __restrict__ hi, __half* __restrict__ lo,
-                                  float* __restrict__ row_scale, int M, int K, int Kp, int vec_ok) {
-  const int lane = threadIdx.x & 31;
-  const int warps_per_block = blockDim.x >> 5;
-  for (long long row = blockIdx.x * static_cast<long long>(warps_per_block) + (threadIdx.x >> 5); row < M;
-       row += static_cast<long long>(gridDim.x) * warps_per_block) {
-    const float* src = A + row * lda;
+// inv_scale[M] = 2^-ea(i).
+struct F16PrepA {
+  const float* src;
+  long long ld;
+  __half *hi, *lo;
+  float* inv_scale;
+  int rows, cols, colsp, vec_ok;
+};
+// The largest magnitude (as float bits) of every column of B within each run of rows_per_part rows: part[runs][cols].
+struct F16ScanB {
+  const float* src;
+  long long ld;
+  unsigned int* part;
+  int rows, cols, rows_per_part, vec_ok;
+};
+
+__device__ __forceinline__ void f16_store_quad(const F16PrepA& j, long long row, int q, const float4& x, float s) {
+  __align__(8) __half h[4];
+  __align__(8) __half l[4];
+  f16_split(x.x, s, h[0], l[0]);
+  f16_split(x.y, s, h[1], l[1]);
+  f16_split(x.z, s, h[2], l[2]);
+  f16_split(x.w, s, h[3], l[3]);
+  *reinterpret_cast<uint2*>(j.hi + row * j.colsp + q * 4) = *reinterpret_cast<const uint2*>(h);
+  if (j.lo) *reinterpret_cast<uint2*>(j.lo + row * j.colsp + q * 4) = *reinterpret_cast<const uint2*>(l);
+}
+
+// TPR threads per row hold 32 elements each, so that a row of up to 32 * TPR elements is read once; what lies beyond is read a
+// second time, from cache.
+template <int TPR>
+__device__ __forceinline__ void prep_a_f16_rows(const F16PrepA& j, unsigned int block, unsigned int blocks, unsigned int* warp_max) {
+  constexpr int ROWS = 256 / TPR, HOLD = 8;
+  const int t = threadIdx.x % TPR, r = threadIdx.x / TPR, warp = threadIdx.x >> 5;
+  const int quads = j.colsp >> 2;
+  for (long long row0 = static_cast<long long>(block) * ROWS; row0 < j.rows; row0 += static_cast<long long>(blocks) * ROWS) {
+    const long long row = row0 + r;
+    const int cols = row < j.rows ? j.cols : 0;  // rows past the end: zeros, not stored
+    const float* src = j.src + row * j.ld;
+    float4 x[HOLD];
     unsigned int m = 0;
-    if (vec_ok) {
-      const float4* v = reinterpret_cast<const float4*>(src);
-      const int nq = K >> 2;
-      int q = lane;
-      for (; q + 96 < nq; q += 128) {  // four independent 128-bit loads in flight per lane
-        const float4 x0 = v[q], x1 = v[q + 32], x2 = v[q + 64], x3 = v[q + 96];
-        m = max(max(m, abs_bits(x0.x)), max(abs_bits(x0.y), max(abs_bits(x0.z), abs_bits(x0.w))));
-        m = max(max(m, abs_bits(x1.x)), max(abs_bits(x1.y), max(abs_bits(x1.z), abs_bits(x1.w))));
-        m = max(max(m, abs_bits(x2.x)), max(abs_bits(x2.y), max(abs_bits(x2.z), abs_bits(x2.w))));
-        m = max(max(m, abs_bits(x3.x)), max(abs_bits(x3.y), max(abs_bits(x3.z), abs_bits(x3.w))));
-      }
-      for (; q < nq; q += 32) {
-        const float4 x = v[q];
-        m = max(max(m, abs_bits(x.x)), max(abs_bits(x.y), max(abs_bits(x.z), abs_bits(x.w))));
-      }
-      for (int k = (K & ~3) + lane; k < K; k += 32) m = max(m, abs_bits(src[k]));
-    } else {
-      for (int k = lane; k < K; k += 32) m = max(m, abs_bits(src[k]));
-    }
+#pragma unroll
+    for (int u = 0; u < HOLD; ++u) x[u] = load_quad(src, (t + u * TPR) * 4, cols, j.vec_ok);
+#pragma unroll
+    for (int u = 0; u < HOLD; ++u) m = max(m, abs_bits_max(x[u]));
+#pragma unroll 4
+    for (int q = t + HOLD * TPR; q < quads; q += TPR) m = max(m, abs_bits_max(load_quad(src, q * 4, cols, j.vec_ok)));
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (TPR > 32) {
+      __syncthreads();  // the row before has been read from warp_max
+      if ((threadIdx.x & 31) == 0) warp_max[warp] = m;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < TPR / 32; ++w) m = max(m, warp_max[r * (TPR / 32) + w]);
+    }
+    if (row >= j.rows) continue;
     const float s = f16_panel_scale(m);
-    if (lane == 0) row_scale[row] = 1.0f / s;  // exact: s is a power of two
-    for (int k = lane * 8; k < Kp; k += 256) {
-      float x[8];
-      if (vec_ok && k + 7 < K) {
-        const float4 u = *reinterpret_cast<const float4*>(src + k), w = *reinterpret_cast<const float4*>(src + k + 4);
-        x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
-        x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
-      } else {
+    if (t == 0) j.inv_scale[row] = 1.0f / s;  // exact: s is a power of two
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = (k + j < K) ? src[k + j] : 0.0f;
-      }
-      __align__(16) __half h[8];
-      __align__(16) __half l[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f16_split(x[j], s, h[j], l[j]);
-      *reinterpret_cast<uint4*>(hi + row * Kp + k) = *reinterpret_cast<const uint4*>(h);
-      if (lo) *reinterpret_cast<uint4*>(lo + row * Kp + k) = *reinterpret_cast<const uint4*>(l);
-    }
+    for (int u = 0; u < HOLD; ++u)
+      if (t + u * TPR < quads) f16_store_quad(j, row, t + u * TPR, x[u], s);
+#pragma unroll 2
+    for (int q = t + HOLD * TPR; q < quads; q += TPR) f16_store_quad(j, row, q, load_quad(src, q * 4, cols, j.vec_ok), s);
   }
 }
 
-// Largest magnitude of every column of B[K x N] as float bits in col_bits[N] (zero before the launch).  Block
-// (x, y) scans rows [rows_per_block * y, ...) of a band of columns.  VEC: four columns per thread with 128-bit loads
-// (B 16-byte aligned, ldb and N multiples of 4), 1024 columns per block; else one column per thread, 256 per block.
-template <bool VEC>
-__global__ void colmax_kernel(const float* __restrict__ B, long long ldb, int K, int N, int rows_per_block,
-                              unsigned int* __restrict__ col_bits) {
-  const int k0 = blockIdx.y * rows_per_block, k1 = min(K, k0 + rows_per_block);
-  if (VEC) {
-    const int n = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (n >= N) return;
-    unsigned int m0 = 0, m1 = 0, m2 = 0, m3 = 0;
-    for (int k = k0; k < k1; ++k) {
-      const float4 x = *reinterpret_cast<const float4*>(B + static_cast<long long>(k) * ldb + n);
-      m0 = max(m0, abs_bits(x.x));
-      m1 = max(m1, abs_bits(x.y));
-      m2 = max(m2, abs_bits(x.z));
-      m3 = max(m3, abs_bits(x.w));
+// 128 columns by one run of rows per block: every warp takes each eighth row, eight rows in flight.
+__device__ __forceinline__ void scan_b_f16(const F16ScanB& j, unsigned int block, unsigned int* smem) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned int col_blocks = (j.cols + 127) / 128;
+  const int c0 = static_cast<int>(block % col_blocks) * 128, run = static_cast<int>(block / col_blocks);
+  const int k0 = run * j.rows_per_part, k1 = min(j.rows, k0 + j.rows_per_part);
+  const bool vec = j.vec_ok;
+  unsigned int m[4] = {0, 0, 0, 0};  // of columns c0 + 4 * lane + i, or c0 + lane + 32 * i
+#pragma unroll 8
+  for (int k = k0 + w; k < k1; k += 8) {
+    const float* row = j.src + static_cast<long long>(k) * j.ld;
+    if (vec) {
+      const float4 x = load_quad(row, c0 + lane * 4, j.cols, 1);
+      m[0] = max(m[0], abs_bits(x.x));
+      m[1] = max(m[1], abs_bits(x.y));
+      m[2] = max(m[2], abs_bits(x.z));
+      m[3] = max(m[3], abs_bits(x.w));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c0 + lane + 32 * i < j.cols) m[i] = max(m[i], abs_bits(row[c0 + lane + 32 * i]));
     }
-    if (m0) atomicMax(col_bits + n, m0);
-    if (m1) atomicMax(col_bits + n + 1, m1);
-    if (m2) atomicMax(col_bits + n + 2, m2);
-    if (m3) atomicMax(col_bits + n + 3, m3);
-  } else {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    unsigned int m = 0;
-    for (int k = k0; k < k1; ++k) m = max(m, abs_bits(B[static_cast<long long>(k) * ldb + n]));
-    if (m) atomicMax(col_bits + n, m);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) smem[w * 128 + (vec ? lane * 4 + i : lane + 32 * i)] = m[i];
+  __syncthreads();
+  if (threadIdx.x < 128 && c0 + static_cast<int>(threadIdx.x) < j.cols) {
+    unsigned int v = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v = max(v, smem[i * 128 + threadIdx.x]);
+    j.part[static_cast<long long>(run) * j.cols + c0 + threadIdx.x] = v;
   }
 }
 
-// B[K x N] -> hi, lo [N x Kp] halves and col_scale[N], transposed through shared memory in tiles of 64 k x 32 n so
-// that every warp store writes one 128-byte run of a panel row (64 halves of k); block (32, 8); Kp is a multiple
-// of 64; column j is scaled by the power of two its largest magnitude (col_bits) asks for.
-__global__ void prep_b_f16_kernel(const float* __restrict__ B, long long ldb, __half* __restrict__ hi, __half* __restrict__ lo,
-                                  float* __restrict__ col_scale, const unsigned int* __restrict__ col_bits, int K, int N, int Kp) {
-  __shared__ float tile[64][33];
-  const long long k_tiles = Kp >> 6;
-  const long long n_tiles = (N + 31) >> 5;
-  const long long total = k_tiles * n_tiles;
+// First preparation launch of the fp16 modes: A's panels, and the column maxima of B by runs of rows.  Blocks [0, blocks_a) work
+// on A.  (Two launches and a memset fewer than a pass each; the maxima need no atomics.  The column scan alone took 21 us of
+// the 50 a 2048^3 product's preparation took, on 64 blocks.)
+template <int TPR>
+__global__ void __launch_bounds__(256) prep_f16_first_kernel(const F16PrepA a, const F16ScanB b, int blocks_a) {
+  __shared__ unsigned int smem[8 * 128];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (static_cast<int>(blockIdx.x) < blocks_a)
+    prep_a_f16_rows<TPR>(a, blockIdx.x, blocks_a, smem);
+  else
+    scan_b_f16(b, blockIdx.x - blocks_a, smem);
+}
+
+// B[K x N] -> hi, lo [N x Kp] halves and col_scale[N], transposed through shared memory in tiles of 64 k x 64 n: 128-bit loads
+// when B allows them, and every thread stores 8 halves of k, so that eight lanes write a 128-byte run of a panel row.  Column j
+// is scaled by the power of two its largest magnitude (over the `parts` runs in part) asks for.
+__global__ void __launch_bounds__(256) prep_b_f16_kernel(const float* B, long long ldb, __half* hi, __half* lo, float* col_scale,
+                                                         const unsigned int* part, int parts, int K, int N, int Kp,
+                                                         int vec_ok) {
+  __shared__ float tile[64][65];
+  __shared__ float scale[64];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int tid = threadIdx.x;
+  const long long n_tiles = (N + 63) >> 6, total = (Kp >> 6) * n_tiles;
   for (long long t = blockIdx.x; t < total; t += gridDim.x) {
-    // n varies fastest so consecutive blocks read consecutive 128-byte runs of a B row
+    // n varies fastest so that consecutive blocks read consecutive runs of a B row
     const long long kt = t / n_tiles;
-    const int n0 = static_cast<int>(t - kt * n_tiles) << 5;
-    const int k0 = static_cast<int>(kt) << 6;
+    const int n0 = static_cast<int>(t - kt * n_tiles) << 6, k0 = static_cast<int>(kt) << 6;
+    if (vec_ok) {
+      const int n = (tid & 15) * 4;
+      float4 x[4];
 #pragma unroll
-    for (int j = 0; j < 64; j += 8) {
-      const int k = k0 + threadIdx.y + j, n = n0 + threadIdx.x;
-      tile[threadIdx.y + j][threadIdx.x] = (k < K && n < N) ? B[static_cast<long long>(k) * ldb + n] : 0.0f;
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 + (tid >> 4) + 16 * i;
+        x[i] = k < K ? load_quad(B + static_cast<long long>(k) * ldb, n0 + n, N, 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float* dst = &tile[(tid >> 4) + 16 * i][n];
+        dst[0] = x[i].x;
+        dst[1] = x[i].y;
+        dst[2] = x[i].z;
+        dst[3] = x[i].w;
+      }
+    } else {
+      const int n = tid & 63;
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int k = k0 + (tid >> 6) + 4 * i;
+        x[i] = k < K && n0 + n < N ? B[static_cast<long long>(k) * ldb + n0 + n] : 0.0f;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) tile[(tid >> 6) + 4 * i][n] = x[i];
+    }
+    {
+      const int n = n0 + (tid >> 2);
+      unsigned int m = 0;
+      if (n < N)
+        for (int p = tid & 3; p < parts; p += 4) m = max(m, part[static_cast<long long>(p) * N + n]);
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      const float s = f16_panel_scale(m);
+      if ((tid & 3) == 0) {
+        scale[tid >> 2] = s;
+        if (kt == 0 && n < N) col_scale[n] = 1.0f / s;
+      }
     }
     __syncthreads();
-    // lane l of a warp takes k = k0 + 2l and 2l + 1 of panel row n: one 4-byte store per lane, 128 bytes per warp
 #pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-      const int nl = threadIdx.y + j, n = n0 + nl;
-      if (n < N) {
-        const float s = f16_panel_scale(col_bits[n]);
-        if (kt == 0 && threadIdx.x == 0) col_scale[n] = 1.0f / s;
-        __half h0, l0, h1, l1;
-        f16_split(tile[2 * threadIdx.x][nl], s, h0, l0);
-        f16_split(tile[2 * threadIdx.x + 1][nl], s, h1, l1);
-        const long long off = static_cast<long long>(n) * Kp + k0 + 2 * threadIdx.x;
-        *reinterpret_cast<__half2*>(hi + off) = __halves2half2(h0, h1);
-        if (lo) *reinterpret_cast<__half2*>(lo + off) = __halves2half2(l0, l1);
+    for (int i = 0; i < 2; ++i) {
+      const int nl = (tid >> 3) + 32 * i, kq = (tid & 7) * 8;
+      if (n0 + nl < N) {
+        __align__(16) __half h[8];
+        __align__(16) __half l[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f16_split(tile[kq + j][nl], scale[nl], h[j], l[j]);
+        const long long off = static_cast<long long>(n0 + nl) * Kp + k0 + kq;
+        *reinterpret_cast<uint4*>(hi + off) = *reinterpret_cast<const uint4*>(h);
+        if (lo) *reinterpret_cast<uint4*>(lo + off) = *reinterpret_cast<const uint4*>(l);
       }
     }
     __syncthreads();

@@ -420,7 +420,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
 // The second half of a product whose k-loop was divided (p.splits > 1): D = act(alpha*sum + beta*C + bias), the partial sums
 // added in order of k, so that the result does not depend on which block finished first.  part: [splits][part_rows][ld]
 // floats, ld a multiple of 4; one thread per four columns.  Bound by L2 (the partials were just written).
-__global__ void __launch_bounds__(256) gemm_reduce_kernel(const float* __restrict__ part, long long ld, int part_rows, int splits,
+__global__ void __launch_bounds__(256) gemm_reduce_kernel(const float* part, long long ld, int part_rows, int splits,
                                                           const GemmParams p) {
   grid_launch_dependents();
   grid_dependency_wait();

@@ -780,6 +780,33 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   return r;
 }
 
+int grid_for(long long work, long long per_block, long long cap) {
+  const long long g = (work + per_block - 1) / per_block;
+  return static_cast<int>(g < cap ? g : cap);
+}
+
+int launch_prep_lo(int sm_count, cudaStream_t st, const PrepLoJob& a, const PrepLoJob& b, bool b_ready, const int* gate) {
+  const long long cap = static_cast<long long>(sm_count) * 16;
+  const int grid_a = grid_for(static_cast<long long>(a.rows) * (a.colsp >> 2), 256, cap);
+  const int grid_b = b_ready ? 0 : grid_for(static_cast<long long>(b.rows) * (b.colsp >> 2), 256, cap);
+  CU_TRY(launch_pdl(prep_lo_two_kernel, dim3(static_cast<unsigned>(grid_a + grid_b)), dim3(256), 0, st, 1, a, b, grid_a, gate));
+  return launch_check("prep_lo_two_kernel");
+}
+
+// High (and low) panels of both operands, or of A alone.
+template <int MODE>
+int launch_prep_panels(int sm_count, cudaStream_t st, const float* A, long long lda, float* a_hi, float* a_lo, const float* B,
+                       long long ldb, float* b_hi, float* b_lo, long long M, long long N, long long K, bool b_ready) {
+  const int kp = static_cast<int>(round_up(K, GEMM_BK));
+  const int vec_ok = ((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0) ? 1 : 0;
+  const PanelJobA ja{A, lda, a_hi, a_lo, static_cast<int>(M), static_cast<int>(K), kp, vec_ok};
+  const PanelJobB jb{B, ldb, b_hi, b_lo, static_cast<int>(K), static_cast<int>(N), kp};
+  const int grid_a = grid_for(M * (kp >> 2), 256, static_cast<long long>(sm_count) * 16);
+  const int grid_b = b_ready ? 0 : grid_for((kp >> 5) * ((N + 31) >> 5), 1, static_cast<long long>(sm_count) * 32);
+  CU_TRY(launch_pdl(prep_panels_kernel<MODE>, dim3(static_cast<unsigned>(grid_a + grid_b)), dim3(256), 0, st, 1, ja, jb, grid_a));
+  return launch_check("prep_panels_kernel");
+}
+
 template <int MODE>
 int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, long long K, const float* A,
                      long long lda, const float* B, long long ldb, const GemmParams& gp_in, long long panel_rows_a = 0,
@@ -840,22 +867,10 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
       uint8_t* ws = static_cast<uint8_t*>(d.workspace);
       float* b_lo = reinterpret_cast<float*>(ws);
       float* a_lo = reinterpret_cast<float*>(ws + blo_bytes);
-      const long long cap = static_cast<long long>(d.sm_count) * 16;
-      long long grid_a = (M * (kp >> 2) + 255) / 256;
-      if (grid_a > cap) grid_a = cap;
-      if (b_panels_ready) {
-        prep_a_kernel<3, true><<<static_cast<unsigned>(grid_a), 256, 0, st>>>(A, lda, nullptr, a_lo, static_cast<int>(M),
-                                                                               static_cast<int>(K), static_cast<int>(kp), 1);
-        if ((rc = launch_check("prep_a_kernel(lo)"))) return rc;
-      } else {
-        // both low-part panels in one launch
-        long long grid_b = (K * (np >> 2) + 255) / 256;
-        if (grid_b > cap) grid_b = cap;
-        const PrepLoJob ja{A, lda, a_lo, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp)};
-        const PrepLoJob jb{B, ldb, b_lo, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np)};
-        prep_lo_two_kernel<<<static_cast<unsigned>(grid_a + grid_b), 256, 0, st>>>(ja, jb, static_cast<int>(grid_a));
-        if ((rc = launch_check("prep_lo_two_kernel"))) return rc;
-      }
+      // both in one launch (B's are not made again for the row blocks after the first)
+      const PrepLoJob ja{A, lda, a_lo, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp)};
+      const PrepLoJob jb{B, ldb, b_lo, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np)};
+      if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, b_panels_ready, nullptr))) return rc;
       if ((rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
       if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     }
@@ -867,27 +882,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     float* b_lo = MODE == 3 ? reinterpret_cast<float*>(ws + b_bytes) : b_hi;
     float* a_hi = reinterpret_cast<float*>(ws + kOps * b_bytes);
     float* a_lo = MODE == 3 ? reinterpret_cast<float*>(ws + kOps * b_bytes + a_bytes) : a_hi;
-    {
-      const long long quads = M * (kp >> 2);
-      long long grid = (quads + 255) / 256;
-      const long long cap = static_cast<long long>(d.sm_count) * 16;
-      if (grid > cap) grid = cap;
-      const int vec_ok = ((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0) ? 1 : 0;
-      prep_a_kernel<MODE><<<static_cast<unsigned>(grid), 256, 0, st>>>(A, lda, a_hi, a_lo, static_cast<int>(M),
-                                                                        static_cast<int>(K), static_cast<int>(kp), vec_ok);
-      rc = launch_check("prep_a_kernel");
-      if (rc) return rc;
-    }
-    if (!b_panels_ready) {
-      const long long tiles = (kp >> 5) * ((N + 31) >> 5);
-      long long grid = tiles;
-      const long long cap = static_cast<long long>(d.sm_count) * 32;
-      if (grid > cap) grid = cap;
-      prep_b_kernel<MODE><<<static_cast<unsigned>(grid), dim3(32, 8), 0, st>>>(B, ldb, b_hi, b_lo, static_cast<int>(K),
-                                                                                 static_cast<int>(N), static_cast<int>(kp));
-      rc = launch_check("prep_b_kernel");
-      if (rc) return rc;
-    }
+    if ((rc = launch_prep_panels<MODE>(d.sm_count, st, A, lda, a_hi, a_lo, B, ldb, b_hi, b_lo, M, N, K, b_panels_ready))) return rc;
     const int b_box_rows = tile_n / route.ctas;
     if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
     if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, b_box_rows))) return rc;
@@ -939,9 +934,19 @@ int encode_map_f16(CUtensorMap* map, const __half* base, long long kp, long long
   return SB200_OK;
 }
 
+// Rows of B per run of the column scan: enough runs to occupy the GPU (about four blocks of 128 columns an SM), at most 64,
+// because every block of the pass that follows goes over the runs' maxima, and at least 32 rows each.
+long long f16_scan_rows(long long N, long long K) {
+  const long long col_blocks = (N + 127) / 128;
+  long long runs = (592 + col_blocks - 1) / col_blocks;
+  if (runs > 64) runs = 64;
+  const long long rows = round_up((K + runs - 1) / runs, 8);
+  return rows < 32 ? 32 : rows;
+}
+
 size_t gemm_f16_workspace_need(long long M, long long N, long long K, bool three) {
-  const long long kp = round_up(K, 64);
-  return 2 * round_up(N * 4, 1024) + round_up(M * 4, 1024) +
+  const long long kp = round_up(K, 64), per = f16_scan_rows(N, K), runs = (K + per - 1) / per;
+  return round_up(runs * N * 4, 1024) + round_up(N * 4, 1024) + round_up(M * 4, 1024) +
          (three ? 2 : 1) * (round_up(M * kp * 2, 1024) + round_up(N * kp * 2, 1024));
 }
 
@@ -976,47 +981,36 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
     CU_TRY(cudaEventCreate(&rec.e2));
     CU_TRY(cudaEventRecord(rec.e0, st));
   }
-  // scratch: [column maxima of B, N words][1/scale per column, N floats][1/scale per row of A, M floats]
+  // scratch: [column maxima of B by runs of rows, runs x N words][1/scale per column, N floats][1/scale per row of A, M floats]
   //          [A_hi][B_hi]([A_lo][B_lo]), every part rounded up to 1 KiB
   uint8_t* ws = static_cast<uint8_t*>(d.workspace);
-  const size_t col_bytes = round_up(N * 4, 1024), row_bytes = round_up(M * 4, 1024);
-  unsigned int* col_bits = reinterpret_cast<unsigned int*>(ws);
-  float* col_scale = reinterpret_cast<float*>(ws + col_bytes);
-  float* row_scale = reinterpret_cast<float*>(ws + 2 * col_bytes);
-  uint8_t* panels = ws + 2 * col_bytes + row_bytes;
+  const long long scan_rows = f16_scan_rows(N, K), runs = (K + scan_rows - 1) / scan_rows;
+  const size_t part_bytes = round_up(runs * N * 4, 1024), col_bytes = round_up(N * 4, 1024), row_bytes = round_up(M * 4, 1024);
+  unsigned int* col_max = reinterpret_cast<unsigned int*>(ws);
+  float* col_scale = reinterpret_cast<float*>(ws + part_bytes);
+  float* row_scale = reinterpret_cast<float*>(ws + part_bytes + col_bytes);
+  uint8_t* panels = ws + part_bytes + col_bytes + row_bytes;
   __half* a_hi = reinterpret_cast<__half*>(panels);
   __half* b_hi = reinterpret_cast<__half*>(panels + a_bytes);
   __half* a_lo = THREE ? reinterpret_cast<__half*>(panels + a_bytes + b_bytes) : nullptr;
   __half* b_lo = THREE ? reinterpret_cast<__half*>(panels + 2 * a_bytes + b_bytes) : nullptr;
-  CU_TRY(cudaMemsetAsync(col_bits, 0, static_cast<size_t>(N) * 4, st));
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   {
-    // A: one warp per row finds the row's scale and writes its panels
-    long long grid = (M + 7) / 8;
-    const long long cap = static_cast<long long>(d.sm_count) * 8;  // fewer rows in flight (to keep them in L2) measured slower
-    if (grid > cap) grid = cap;
-    const int vec_ok = (al16(A) && (lda & 3) == 0) ? 1 : 0;
-    prep_a_f16_kernel<<<static_cast<unsigned>(grid), 256, 0, st>>>(A, lda, a_hi, a_lo, row_scale, static_cast<int>(M),
-                                                                    static_cast<int>(K), static_cast<int>(kp), vec_ok);
-    if ((rc = launch_check("prep_a_f16_kernel"))) return rc;
-    // B: column maxima, then the transposing split
-    const int rows_per_block = 64;
-    const bool vec_b = al16(B) && (ldb & 3) == 0 && (N & 3) == 0;
-    const long long cols_per_block = vec_b ? 1024 : 256;
-    const dim3 cgrid(static_cast<unsigned>((N + cols_per_block - 1) / cols_per_block),
-                     static_cast<unsigned>((K + rows_per_block - 1) / rows_per_block));
-    if (cgrid.y > 65535u) return fail(SB200_ERR_TOO_LARGE, "K beyond the fp16 modes' column scan (K=%lld)", K);
-    if (vec_b)
-      colmax_kernel<true><<<cgrid, 256, 0, st>>>(B, ldb, static_cast<int>(K), static_cast<int>(N), rows_per_block, col_bits);
-    else
-      colmax_kernel<false><<<cgrid, 256, 0, st>>>(B, ldb, static_cast<int>(K), static_cast<int>(N), rows_per_block, col_bits);
-    if ((rc = launch_check("colmax_kernel"))) return rc;
-    long long tiles = (kp >> 6) * ((N + 31) >> 5);
-    const long long cap32 = static_cast<long long>(d.sm_count) * 32;
-    if (tiles > cap32) tiles = cap32;
-    prep_b_f16_kernel<<<static_cast<unsigned>(tiles), dim3(32, 8), 0, st>>>(B, ldb, b_hi, b_lo, col_scale, col_bits,
-                                                                             static_cast<int>(K), static_cast<int>(N),
-                                                                             static_cast<int>(kp));
+    const F16PrepA ja{A, lda, a_hi, a_lo, row_scale, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp),
+                      al16(A) && (lda & 3) == 0 ? 1 : 0};
+    const int vec_b = al16(B) && (ldb & 3) == 0 ? 1 : 0;
+    const F16ScanB jb{B, ldb, col_max, static_cast<int>(K), static_cast<int>(N), static_cast<int>(scan_rows), vec_b};
+    // threads per row of A: as few as hold a row in their registers
+    const int tpr = kp <= 1024 ? 32 : kp <= 4096 ? 128 : 256;
+    const int grid_a = grid_for(M, 256 / tpr, static_cast<long long>(d.sm_count) * 8);
+    const dim3 grid(static_cast<unsigned>(grid_a + ((N + 127) / 128) * runs));
+    auto first = tpr == 32 ? prep_f16_first_kernel<32> : tpr == 128 ? prep_f16_first_kernel<128> : prep_f16_first_kernel<256>;
+    CU_TRY(launch_pdl(first, grid, dim3(256), 0, st, 1, ja, jb, grid_a));
+    if ((rc = launch_check("prep_f16_first_kernel"))) return rc;
+    const int tiles = grid_for((kp >> 6) * ((N + 63) >> 6), 1, static_cast<long long>(d.sm_count) * 16);
+    CU_TRY(launch_pdl(prep_b_f16_kernel, dim3(static_cast<unsigned>(tiles)), dim3(256), 0, st, 1, B, ldb, b_hi, b_lo, col_scale,
+                      static_cast<const unsigned int*>(col_max), static_cast<int>(runs), static_cast<int>(K), static_cast<int>(N),
+                      static_cast<int>(kp), vec_b));
     if ((rc = launch_check("prep_b_f16_kernel"))) return rc;
   }
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
@@ -1156,13 +1150,9 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     // behind it, gated the other way: plain 3xTF32 on the same operands, its low-part panels in the same scratch
     float* pb_lo = reinterpret_cast<float*>(ws);
     float* pa_lo = reinterpret_cast<float*>(ws + round_up(K * np * 4, 1024));
-    long long grid_a = (M * (kp32 >> 2) + 255) / 256, grid_b = (K * (np >> 2) + 255) / 256;
-    if (grid_a > cap16) grid_a = cap16;
-    if (grid_b > cap16) grid_b = cap16;
     const PrepLoJob ja{A, lda, pa_lo, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp32)};
     const PrepLoJob jb{B, ldb, pb_lo, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np)};
-    prep_lo_two_kernel<<<static_cast<unsigned>(grid_a + grid_b), 256, 0, st>>>(ja, jb, static_cast<int>(grid_a), gp.gate);
-    if ((rc = launch_check("prep_lo_two_kernel(gated)"))) return rc;
+    if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, false, gp.gate))) return rc;
     CUtensorMap pma_lo, pmb_lo;
     if ((rc = encode_map_2d(&pma_lo, pa_lo, kp32, M, kp32, GEMM_BK, GEMM_BM, false))) return rc;
     if ((rc = encode_map_2d(&pmb_lo, pb_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
@@ -2502,7 +2492,8 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   }
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
-  // "panels" for operands TMA cannot address also when they are converted on their way (launches=1, no scratch for operands)
+  // "panels" for operands TMA cannot address also when they are converted on their way (launches=1, no scratch for operands);
+  // the passes over A and B are counted apart although one launch makes both
   const int launches = (r.src == SRC_PANELS ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + (r.splits > 1 ? 1 : 0);
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
            r.ctas == 2 ? "pair" : "single", r.src == SRC_DIRECT || (r.src == SRC_CONVERT && addressable) ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
@@ -2751,24 +2742,8 @@ int launch_gemm_fixed_scratch(const NoAllocDevice& nd, int dev, cudaStream_t st,
   float* b_hi = reinterpret_cast<float*>(nd.scratch + a_bytes);
   float* a_lo = MODE == 3 ? reinterpret_cast<float*>(nd.scratch + a_bytes + b_bytes) : a_hi;
   float* b_lo = MODE == 3 ? reinterpret_cast<float*>(nd.scratch + 2 * a_bytes + b_bytes) : b_hi;
-  int rc;
-  {
-    long long grid = (M * (kp >> 2) + 255) / 256;
-    const long long cap = static_cast<long long>(nd.sm_count) * 16;
-    if (grid > cap) grid = cap;
-    const int vec_ok = ((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0) ? 1 : 0;
-    prep_a_kernel<MODE><<<static_cast<unsigned>(grid), 256, 0, st>>>(A, lda, a_hi, a_lo, static_cast<int>(M),
-                                                                      static_cast<int>(K), static_cast<int>(kp), vec_ok);
-    if ((rc = launch_check("prep_a_kernel"))) return rc;
-  }
-  {
-    long long grid = (kp >> 5) * ((N + 31) >> 5);
-    const long long cap = static_cast<long long>(nd.sm_count) * 32;
-    if (grid > cap) grid = cap;
-    prep_b_kernel<MODE><<<static_cast<unsigned>(grid), dim3(32, 8), 0, st>>>(B, ldb, b_hi, b_lo, static_cast<int>(K),
-                                                                               static_cast<int>(N), static_cast<int>(kp));
-    if ((rc = launch_check("prep_b_kernel"))) return rc;
-  }
+  int rc = launch_prep_panels<MODE>(nd.sm_count, st, A, lda, a_hi, a_lo, B, ldb, b_hi, b_lo, M, N, K, false);
+  if (rc) return rc;
   const int tile_n = choose_tiles(M, N, kp / GEMM_BK, 1, nd.sm_count, MODE == 3, false).tile_n;
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
   if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
