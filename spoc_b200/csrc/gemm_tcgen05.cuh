@@ -546,11 +546,11 @@ __device__ __forceinline__ void f16_store_quad(const F16PrepA& j, long long row,
   if (j.lo) *reinterpret_cast<uint2*>(j.lo + row * j.colsp + q * 4) = *reinterpret_cast<const uint2*>(l);
 }
 
-// TPR threads per row hold 32 elements each, so that a row of up to 32 * TPR elements is read once; what lies beyond is read a
-// second time, from cache.
-template <int TPR>
+// TPR threads per row hold HOLD quads each, so that a row of up to 4 * HOLD * TPR elements is read once; what lies beyond is
+// read a second time, from cache.
+template <int TPR, int HOLD>
 __device__ __forceinline__ void prep_a_f16_rows(const F16PrepA& j, unsigned int block, unsigned int blocks, unsigned int* warp_max) {
-  constexpr int ROWS = 256 / TPR, HOLD = 8;
+  constexpr int ROWS = 256 / TPR;
   const int t = threadIdx.x % TPR, r = threadIdx.x / TPR, warp = threadIdx.x >> 5;
   const int quads = j.colsp >> 2;
   for (long long row0 = static_cast<long long>(block) * ROWS; row0 < j.rows; row0 += static_cast<long long>(blocks) * ROWS) {
@@ -622,13 +622,13 @@ __device__ __forceinline__ void scan_b_f16(const F16ScanB& j, unsigned int block
 // First preparation launch of the fp16 modes: A's panels, and the column maxima of B by runs of rows.  Blocks [0, blocks_a) work
 // on A.  (Two launches and a memset fewer than a pass each; the maxima need no atomics.  The column scan alone took 21 us of
 // the 50 a 2048^3 product's preparation took, on 64 blocks.)
-template <int TPR>
-__global__ void __launch_bounds__(256) prep_f16_first_kernel(const F16PrepA a, const F16ScanB b, int blocks_a) {
+template <int TPR, int HOLD>
+__global__ void __launch_bounds__(256, HOLD == 4 ? 4 : 2) prep_f16_first_kernel(const F16PrepA a, const F16ScanB b, int blocks_a) {
   __shared__ unsigned int smem[8 * 128];
   grid_launch_dependents();
   grid_dependency_wait();
   if (static_cast<int>(blockIdx.x) < blocks_a)
-    prep_a_f16_rows<TPR>(a, blockIdx.x, blocks_a, smem);
+    prep_a_f16_rows<TPR, HOLD>(a, blockIdx.x, blocks_a, smem);
   else
     scan_b_f16(b, blockIdx.x - blocks_a, smem);
 }

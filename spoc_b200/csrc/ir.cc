@@ -691,6 +691,12 @@ bool gen_int(GenCtx& g, const Sx& e, std::string* out) {
   return false;
 }
 
+// Every generated kernel is launched with programmatic stream serialization and calls this before it touches memory.
+const char* const kPdlSource =
+    "__device__ __forceinline__ void sb200_begin() {\n"
+    "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
+    "  asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n}\n";
+
 std::string generic_map_source(const KernelPlan& plan, const GenericMap& gm, const std::vector<std::string>& store_exprs) {
   const size_t ni = gm.inputs.size(), no = gm.outputs.size(), ns = gm.scalars.size();
   auto scalar_type = [&](size_t i) {
@@ -698,7 +704,10 @@ std::string generic_map_source(const KernelPlan& plan, const GenericMap& gm, con
     return (elt == "f32" || elt == "f64") ? "double" : "long long";
   };
   std::ostringstream o;
-  o << "// generated for kernel '" << plan.name << "'\n";
+  o << "// generated for kernel '" << plan.name << "'\n" << kPdlSource;
+  o << "__device__ __forceinline__ float4 sb200_ld(const float4* p) {\n  float4 v;\n"
+       "  asm volatile(\"ld.global.L1::no_allocate.L2::256B.v4.f32 {%0,%1,%2,%3}, [%4];\" : \"=f\"(v.x), \"=f\"(v.y), \"=f\"(v.z), "
+       "\"=f\"(v.w) : \"l\"(p));\n  return v;\n}\n";
   o << "__device__ __forceinline__ void sb200_elem(";
   for (size_t i = 0; i < ni; ++i) o << "float x" << i << ", ";
   for (size_t i = 0; i < ns; ++i) o << scalar_type(i) << " s" << i << ", ";
@@ -711,10 +720,10 @@ std::string generic_map_source(const KernelPlan& plan, const GenericMap& gm, con
   // nvec whole vectors follow; the ragged ends (head, and up to 3 elements after the vectors) are taken by the
   // first threads of block 0
   o << "extern \"C\" __global__ void __launch_bounds__(256) sb200_map_vec(";
-  for (size_t i = 0; i < ni; ++i) o << "const float* __restrict__ sin" << i << ", ";
-  for (size_t i = 0; i < no; ++i) o << "float* __restrict__ sout" << i << ", ";
+  for (size_t i = 0; i < ni; ++i) o << "const float* sin" << i << ", ";
+  for (size_t i = 0; i < no; ++i) o << "float* sout" << i << ", ";
   for (size_t i = 0; i < ns; ++i) o << scalar_type(i) << " s" << i << ", ";
-  o << "int head, long long nvec, long long n) {\n";
+  o << "int head, long long nvec, long long n) {\n  sb200_begin();\n";
   o << "  if (blockIdx.x == 0) {\n";
   o << "    const long long body_end = head + nvec * 4;\n";
   o << "    const int ragged = head + (int)(n - body_end);\n";
@@ -728,25 +737,43 @@ std::string generic_map_source(const KernelPlan& plan, const GenericMap& gm, con
   o << ");\n";
   for (size_t i = 0; i < no; ++i) o << "      sout" << i << "[e] = r" << i << ";\n";
   o << "    }\n  }\n";
-  for (size_t i = 0; i < ni; ++i) o << "  const float4* __restrict__ in" << i << " = reinterpret_cast<const float4*>(sin" << i << " + head);\n";
-  for (size_t i = 0; i < no; ++i) o << "  float4* __restrict__ out" << i << " = reinterpret_cast<float4*>(sout" << i << " + head);\n";
-  o << "  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvec; v += (long long)gridDim.x * blockDim.x) {\n";
-  for (size_t i = 0; i < ni; ++i) o << "    const float4 a" << i << " = in" << i << "[v];\n";
-  for (size_t i = 0; i < no; ++i) o << "    float4 r" << i << ";\n";
-  for (const char* c : {"x", "y", "z", "w"}) {
-    o << "    sb200_elem(";
-    for (size_t i = 0; i < ni; ++i) o << "a" << i << "." << c << ", ";
-    for (size_t i = 0; i < ns; ++i) o << "s" << i << ", ";
-    for (size_t i = 0; i < no; ++i) o << "r" << i << "." << c << (i + 1 < no ? ", " : "");
-    o << ");\n";
-  }
-  for (size_t i = 0; i < no; ++i) o << "    out" << i << "[v] = r" << i << ";\n";
-  o << "  }\n}\n";
+  // body: `unroll` vectors of every input are loaded before the first is used, so that a thread keeps about eight 128-bit
+  // loads in flight; chunks of 256 * unroll vectors, ragged last chunk vector by vector
+  for (size_t i = 0; i < ni; ++i) o << "  const float4* in" << i << " = reinterpret_cast<const float4*>(sin" << i << " + head);\n";
+  for (size_t i = 0; i < no; ++i) o << "  float4* out" << i << " = reinterpret_cast<float4*>(sout" << i << " + head);\n";
+  auto one_vector = [&](const char* indent, const std::string& at, const std::string& u) {
+    o << indent << "{\n";
+    for (size_t i = 0; i < no; ++i) o << indent << "  float4 r" << i << ";\n";
+    for (const char* c : {"x", "y", "z", "w"}) {
+      o << indent << "  sb200_elem(";
+      for (size_t i = 0; i < ni; ++i) o << "a" << i << u << "." << c << ", ";
+      for (size_t i = 0; i < ns; ++i) o << "s" << i << ", ";
+      for (size_t i = 0; i < no; ++i) o << "r" << i << "." << c << (i + 1 < no ? ", " : "");
+      o << ");\n";
+    }
+    for (size_t i = 0; i < no; ++i) o << indent << "  __stcs(out" << i << " + " << at << ", r" << i << ");\n";
+    o << indent << "}\n";
+  };
+  o << "  constexpr int U = " << gm.unroll << ";\n";
+  o << "  const long long nchunks = (nvec + 256 * U - 1) / (256 * U);\n";
+  o << "  for (long long c = blockIdx.x; c < nchunks; c += gridDim.x) {\n";
+  o << "    const long long v = c * (256 * U) + threadIdx.x;\n";
+  o << "    if (v + (U - 1) * 256 < nvec) {\n";
+  for (size_t i = 0; i < ni; ++i) o << "      float4 a" << i << "[U];\n";
+  for (size_t i = 0; i < ni; ++i)
+    o << "#pragma unroll\n      for (int u = 0; u < U; ++u) a" << i << "[u] = sb200_ld(in" << i << " + v + u * 256);\n";
+  o << "#pragma unroll\n      for (int u = 0; u < U; ++u)\n";
+  one_vector("      ", "v + u * 256", "[u]");
+  o << "    } else {\n";
+  o << "#pragma unroll 1\n      for (int u = 0; u < U; ++u) {\n        const long long w = v + u * 256;\n        if (w >= nvec) break;\n";
+  for (size_t i = 0; i < ni; ++i) o << "        const float4 a" << i << " = sb200_ld(in" << i << " + w);\n";
+  one_vector("        ", "w", "");
+  o << "      }\n    }\n  }\n}\n";
   o << "extern \"C\" __global__ void __launch_bounds__(256) sb200_map_scalar(";
-  for (size_t i = 0; i < ni; ++i) o << "const float* __restrict__ in" << i << ", ";
-  for (size_t i = 0; i < no; ++i) o << "float* __restrict__ out" << i << ", ";
+  for (size_t i = 0; i < ni; ++i) o << "const float* in" << i << ", ";
+  for (size_t i = 0; i < no; ++i) o << "float* out" << i << ", ";
   for (size_t i = 0; i < ns; ++i) o << scalar_type(i) << " s" << i << ", ";
-  o << "long long first, long long n) {\n";
+  o << "long long first, long long n) {\n  sb200_begin();\n";
   o << "  for (long long e = first + blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {\n";
   for (size_t i = 0; i < no; ++i) o << "    float r" << i << ";\n";
   o << "    sb200_elem(";
@@ -833,6 +860,7 @@ bool match_map_generic(Ctx& cx, const Sx& body) {
     gm.outputs.push_back(out);
   }
   // an input that is also an output is read before it is written by the same thread: allowed
+  gm.unroll = gm.inputs.size() <= 2 ? 4 : gm.inputs.size() <= 4 ? 2 : 1;
   gm.source = generic_map_source(plan, gm, exprs);
   mp.op = OP_GENERIC;
   mp.out0 = gm.outputs[0];
@@ -859,7 +887,7 @@ std::string block_reduce_source(const KernelPlan& plan, const GenericMap& gm, co
     return (elt == "f32" || elt == "f64") ? "double" : "long long";
   };
   std::ostringstream o;
-  o << "// generated for kernel '" << plan.name << "' (block tree reduction, block = " << block << ")\n";
+  o << "// generated for kernel '" << plan.name << "' (block tree reduction, block = " << block << ")\n" << kPdlSource;
   o << "__device__ __forceinline__ double sb200_elem(";
   for (size_t i = 0; i < ni; ++i) o << "float x" << i << (i + 1 < ni || ns ? ", " : "");
   for (size_t i = 0; i < ns; ++i) o << scalar_type(i) << " s" << i << (i + 1 < ns ? ", " : "");
@@ -867,10 +895,10 @@ std::string block_reduce_source(const KernelPlan& plan, const GenericMap& gm, co
   for (size_t i = 0; i < ni; ++i) o << "  const double X" << i << " = (double)x" << i << ";\n";
   o << "  return " << expr << ";\n}\n";
   o << "extern \"C\" __global__ void __launch_bounds__(256) sb200_reduce(";
-  for (size_t i = 0; i < ni; ++i) o << "const float* __restrict__ in" << i << ", ";
-  o << "float* __restrict__ out, ";
+  for (size_t i = 0; i < ni; ++i) o << "const float* in" << i << ", ";
+  o << "float* out, ";
   for (size_t i = 0; i < ns; ++i) o << scalar_type(i) << " s" << i << ", ";
-  o << "long long n, long long nseg) {\n";
+  o << "long long n, long long nseg) {\n  sb200_begin();\n";
   o << "  constexpr int B = " << block << ", PER = B / 32;\n";
   o << "  const int lane = threadIdx.x & 31;\n";
   o << "  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;\n";

@@ -77,6 +77,7 @@ struct GenericMap {
   std::vector<int> inputs;   // float32 vector params read at the element index
   std::vector<int> outputs;  // float32 vector params stored, in store order
   std::vector<int> scalars;  // scalar params used by the expression (passed as double / long long)
+  int unroll = 1;            // 128-bit vectors of each operand a thread of the vector kernel moves per step
   std::string source;        // complete CUDA translation unit (kernels sb200_map_vec, sb200_map_scalar)
 };
 

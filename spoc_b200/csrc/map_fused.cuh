@@ -22,6 +22,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
+
 namespace sb200 {
 
 constexpr int MAP_THREADS = 256;
@@ -78,8 +80,10 @@ __device__ __forceinline__ void apply4(const float4& x0, const float4& x1, float
 // of MAP_THREADS*MAP_UNROLL vectors so a warp's accesses are 512-byte runs.
 template <class Op>
 __global__ void __launch_bounds__(MAP_THREADS)
-map2_vec_kernel(const float* __restrict__ sin0, const float* __restrict__ sin1, float* __restrict__ sout0,
-                float* __restrict__ sout1, float s, int head, long long nvec, long long n) {
+map2_vec_kernel(const float* sin0, const float* sin1, float* sout0, float* sout1, float s, int head, long long nvec, long long n) {
+  // launched with programmatic stream serialization: the next kernel may be set up, and wait, while this one runs
+  grid_launch_dependents();
+  grid_dependency_wait();
   if (blockIdx.x == 0) {
     const long long body_end = head + nvec * 4;
     const int ragged = head + static_cast<int>(n - body_end);  // at most 6
@@ -91,10 +95,10 @@ map2_vec_kernel(const float* __restrict__ sin0, const float* __restrict__ sin1, 
       if (Op::kOutputs == 2) sout1[i] = y1;
     }
   }
-  const float4* __restrict__ in0 = reinterpret_cast<const float4*>(sin0 + head);
-  const float4* __restrict__ in1 = reinterpret_cast<const float4*>(sin1 + head);
-  float4* __restrict__ out0 = reinterpret_cast<float4*>(sout0 + head);
-  float4* __restrict__ out1 = Op::kOutputs == 2 ? reinterpret_cast<float4*>(sout1 + head) : nullptr;
+  const float4* in0 = reinterpret_cast<const float4*>(sin0 + head);
+  const float4* in1 = reinterpret_cast<const float4*>(sin1 + head);
+  float4* out0 = reinterpret_cast<float4*>(sout0 + head);
+  float4* out1 = Op::kOutputs == 2 ? reinterpret_cast<float4*>(sout1 + head) : nullptr;
   constexpr long long kChunk = static_cast<long long>(MAP_THREADS) * MAP_UNROLL;
   const long long nchunks = (nvec + kChunk - 1) / kChunk;
   for (long long c = blockIdx.x; c < nchunks; c += gridDim.x) {
@@ -131,8 +135,9 @@ map2_vec_kernel(const float* __restrict__ sin0, const float* __restrict__ sin1, 
 // and for operands whose addresses differ in their 16-byte misalignment (4-byte accesses stay coalesced).
 template <class Op>
 __global__ void __launch_bounds__(MAP_THREADS)
-map2_scalar_kernel(const float* __restrict__ in0, const float* __restrict__ in1, float* __restrict__ out0,
-                   float* __restrict__ out1, float s, long long first, long long n) {
+map2_scalar_kernel(const float* in0, const float* in1, float* out0, float* out1, float s, long long first, long long n) {
+  grid_launch_dependents();
+  grid_dependency_wait();
   for (long long i = first + blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     float y0, y1;

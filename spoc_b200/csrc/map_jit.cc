@@ -67,8 +67,7 @@ struct Driver {
   CUresult (*ModuleLoadData)(CUmodule*, const void*) = nullptr;
   CUresult (*ModuleGetFunction)(CUfunction*, CUmodule, const char*) = nullptr;
   CUresult (*ModuleUnload)(CUmodule) = nullptr;
-  CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream, void**,
-                           void**) = nullptr;
+  CUresult (*LaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
   bool ok = false;
 };
 Driver g_drv;
@@ -87,8 +86,8 @@ void load_driver() {
   g_drv.ModuleLoadData = reinterpret_cast<decltype(g_drv.ModuleLoadData)>(get("cuModuleLoadData"));
   g_drv.ModuleGetFunction = reinterpret_cast<decltype(g_drv.ModuleGetFunction)>(get("cuModuleGetFunction"));
   g_drv.ModuleUnload = reinterpret_cast<decltype(g_drv.ModuleUnload)>(get("cuModuleUnload"));
-  g_drv.LaunchKernel = reinterpret_cast<decltype(g_drv.LaunchKernel)>(get("cuLaunchKernel"));
-  g_drv.ok = g_drv.ModuleLoadData && g_drv.ModuleGetFunction && g_drv.ModuleUnload && g_drv.LaunchKernel;
+  g_drv.LaunchKernelEx = reinterpret_cast<decltype(g_drv.LaunchKernelEx)>(get("cuLaunchKernelEx"));
+  g_drv.ok = g_drv.ModuleLoadData && g_drv.ModuleGetFunction && g_drv.ModuleUnload && g_drv.LaunchKernelEx;
 }
 
 }  // namespace
@@ -167,9 +166,21 @@ void jit_unload(JitModule* m) {
 }
 
 int jit_launch(void* fn, unsigned grid, unsigned block, void* stream, void** args, std::string* err) {
-  CUresult r = g_drv.LaunchKernel(static_cast<CUfunction>(fn), grid, 1, 1, block, 1, 1, 0, static_cast<CUstream>(stream), args, nullptr);
+  // programmatic stream serialization: the kernel is set up while the one before it still runs (sb200_begin waits)
+  CUlaunchAttribute attr;
+  attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig cfg = {};
+  cfg.gridDimX = grid;
+  cfg.gridDimY = cfg.gridDimZ = 1;
+  cfg.blockDimX = block;
+  cfg.blockDimY = cfg.blockDimZ = 1;
+  cfg.hStream = static_cast<CUstream>(stream);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  CUresult r = g_drv.LaunchKernelEx(&cfg, static_cast<CUfunction>(fn), args, nullptr);
   if (r != CUDA_SUCCESS) {
-    *err = "cuLaunchKernel failed with CUresult " + std::to_string(static_cast<int>(r));
+    *err = "cuLaunchKernelEx failed with CUresult " + std::to_string(static_cast<int>(r));
     return static_cast<int>(r);
   }
   return SB200_OK;

@@ -218,6 +218,29 @@ int current_mode() {
   return m;
 }
 
+// Launches a kernel with programmatic stream serialization: it may set itself up while the kernel before it in the stream
+// still runs.  Every kernel launched this way passes griddepcontrol.wait before it touches global memory.  The launch call
+// itself is cheaper too (2.3 against 2.8 us).
+template <class... Params, class... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 // --------------------------------------------------------------- map host
 template <class Op>
 int launch_map2(DeviceState& d, cudaStream_t st, const float* in0, const float* in1, float* out0, float* out1, float s,
@@ -241,15 +264,15 @@ int launch_map2(DeviceState& d, cudaStream_t st, const float* in0, const float* 
     long long grid = nchunks;
     const long long cap = static_cast<long long>(d.sm_count) * 32;
     if (grid > cap) grid = cap;
-    map2_vec_kernel<Op><<<static_cast<unsigned>(grid), MAP_THREADS, 0, st>>>(in0, in1, out0, Op::kOutputs == 2 ? out1 : nullptr, s,
-                                                                             static_cast<int>(head), nvec, n);
+    CU_TRY(launch_pdl(map2_vec_kernel<Op>, dim3(static_cast<unsigned>(grid)), dim3(MAP_THREADS), 0, st, 1, in0, in1, out0,
+                      Op::kOutputs == 2 ? out1 : static_cast<float*>(nullptr), s, static_cast<int>(head), nvec, n));
     return launch_check("map body");
   }
   {
     long long grid = (n + MAP_THREADS - 1) / MAP_THREADS;
     const long long cap = static_cast<long long>(d.sm_count) * 16;
     if (grid > cap) grid = cap;
-    map2_scalar_kernel<Op><<<static_cast<unsigned>(grid), MAP_THREADS, 0, st>>>(in0, in1, out0, out1, s, 0, n);
+    CU_TRY(launch_pdl(map2_scalar_kernel<Op>, dim3(static_cast<unsigned>(grid)), dim3(MAP_THREADS), 0, st, 1, in0, in1, out0, out1, s, 0ll, n));
     int rc = launch_check("map scalar");
     if (rc) return rc;
   }
@@ -522,29 +545,6 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
     }
   }
   return best;
-}
-
-// Launches a kernel with programmatic stream serialization: it may set itself up while the kernel before it in the stream
-// still runs.  Every kernel launched this way passes griddepcontrol.wait before it touches global memory.  The launch call
-// itself is cheaper too (2.3 against 2.8 us).
-template <class... Params, class... Args>
-cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, Args&&... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // The operand maps of one launch; x: the mixed mode's third pair (else unused).
@@ -1000,11 +1000,15 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
                       al16(A) && (lda & 3) == 0 ? 1 : 0};
     const int vec_b = al16(B) && (ldb & 3) == 0 ? 1 : 0;
     const F16ScanB jb{B, ldb, col_max, static_cast<int>(K), static_cast<int>(N), static_cast<int>(scan_rows), vec_b};
-    // threads per row of A: as few as hold a row in their registers
-    const int tpr = kp <= 1024 ? 32 : kp <= 4096 ? 128 : 256;
+    // threads per row of A: as few as hold a row in four quads each, which lets four blocks share an SM
+    const int tpr = kp <= 512 ? 32 : kp <= 1024 ? 64 : kp <= 2048 ? 128 : 256;
     const int grid_a = grid_for(M, 256 / tpr, static_cast<long long>(d.sm_count) * 8);
     const dim3 grid(static_cast<unsigned>(grid_a + ((N + 127) / 128) * runs));
-    auto first = tpr == 32 ? prep_f16_first_kernel<32> : tpr == 128 ? prep_f16_first_kernel<128> : prep_f16_first_kernel<256>;
+    auto first = tpr == 32   ? prep_f16_first_kernel<32, 4>
+                 : tpr == 64  ? prep_f16_first_kernel<64, 4>
+                 : tpr == 128 ? prep_f16_first_kernel<128, 4>
+                 : kp <= 4096 ? prep_f16_first_kernel<256, 4>
+                              : prep_f16_first_kernel<256, 8>;
     CU_TRY(launch_pdl(first, grid, dim3(256), 0, st, 1, ja, jb, grid_a));
     if ((rc = launch_check("prep_f16_first_kernel"))) return rc;
     const int tiles = grid_for((kp >> 6) * ((N + 63) >> 6), 1, static_cast<long long>(d.sm_count) * 16);
@@ -1370,8 +1374,9 @@ int launch_generic_map(DeviceState& d, KernelObj& k, const std::vector<Slot>& s,
     args.push_back(&head_i);
     args.push_back(&nvec);
     args.push_back(&n);
-    long long grid = (nvec + 255) / 256;
-    const long long cap = static_cast<long long>(d.sm_count) * 8;
+    const long long per_block = 256ll * gm.unroll;
+    long long grid = (nvec + per_block - 1) / per_block;
+    const long long cap = static_cast<long long>(d.sm_count) * 32;
     if (grid > cap) grid = cap;
     int rc = jit_launch(jm->vec_fn, static_cast<unsigned>(grid), 256, st, args.data(), &err);
     if (rc) return fail(rc, "kernel '%s': %s", k.plan.name.c_str(), err.c_str());
