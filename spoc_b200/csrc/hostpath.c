@@ -3,7 +3,7 @@
  * A launch of a short kernel spends most of its time above the C ABI: walking the arguments, expanding every vector to
  * (buffer, int32 length) as the reference does (sarek/sarek/Execute.ml:197-216), filling the argument table.  Interpreted,
  * that took 12 us of a 17 us launch; here it takes under 1 us.  Only the case a running program meets every time is
- * handled: all vectors already on the device, nothing pinned or on its way back, plain Python scalars.  Everything else
+ * handled: all vectors already on the device, nothing on its way back or to be sent back behind the launch, plain Python scalars.  Everything else
  * returns None and takes the interpreted path, which also raises the errors.
  *
  * The library is not linked: bind() receives the address of sb200_kernel_launch from the ctypes binding. */
@@ -16,6 +16,7 @@
 typedef int (*launch_fn)(uint64_t, const sb200_arg *, int, const uint32_t *, const uint32_t *, uint32_t, uint64_t);
 
 #define MAX_ARGS 64
+#define SEND_BACK_BYTES (16u << 20) /* Vector.PIN_MIN_BYTES */
 
 static launch_fn g_launch;
 static PyObject *g_vector_type;              /* plugin.Vector */
@@ -54,13 +55,17 @@ static int push_vector(PyObject *v, sb200_arg *args, int *n, int *both) {
   PyObject *buffer = NULL, *location = NULL, *pinned = NULL, *prefetch = NULL, *host = NULL;
   if (!(buffer = PyObject_GetAttr(v, s_buffer)) || buffer == Py_None) goto out;
   if (!(location = PyObject_GetAttr(v, s_location)) || same_text(location, g_cpu)) goto out;
-  if (!(pinned = PyObject_GetAttr(v, s_pinned)) || pinned != Py_False) goto out;
+  if (!(pinned = PyObject_GetAttr(v, s_pinned)) || (pinned != Py_False && pinned != Py_True)) goto out;
   if (!(prefetch = PyObject_GetAttr(v, s_prefetch)) || prefetch != Py_None) goto out;
   if (!(host = PyObject_GetAttr(v, s_host))) goto out;
   {
     PyObject *ptr = PyObject_GetAttr(buffer, s_ptr);
     const Py_ssize_t len = PyObject_Size(host);
     if (!ptr) goto out;
+    if (pinned == Py_True && (uint64_t)len * 4 >= SEND_BACK_BYTES) { /* its result would follow the launch to the host */
+      Py_DECREF(ptr);
+      goto out;
+    }
     const unsigned long long address = PyLong_CheckExact(ptr) ? PyLong_AsUnsignedLongLong(ptr) : 0;
     Py_DECREF(ptr);
     if (PyErr_Occurred() || address == 0 || len < 0 || len > INT32_MAX) goto out;

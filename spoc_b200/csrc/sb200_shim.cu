@@ -1645,7 +1645,10 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
     const int v = e ? atoi(e) : 0;
     return v >= 2 && v <= 64 ? v : 8;
   }();
+  // A copy costs about 4 us beside its bytes, 12 us while copies run both ways, so a block brings at least 4 MiB.
+  const long long row_bytes = 4 * ((a.host ? K : 0) + (c && c->host ? N : 0));
   long long block_rows = (M + nblocks - 1) / nblocks;
+  if (row_bytes > 0 && block_rows * row_bytes < (4 << 20)) block_rows = ((4 << 20) + row_bytes - 1) / row_bytes;
   block_rows = (block_rows + 255) / 256 * 256;
   if (block_rows > M) block_rows = M;
   std::vector<cudaEvent_t> events;
@@ -1706,7 +1709,7 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
       const char* e = getenv("SAREK_B200_PIPE_TAPER");
       return !(e && e[0] == '0');
     }();
-    for (int split = 0; split < 2 && taper && M - r >= 512; ++split) {
+    for (int split = 0; split < 2 && taper && M - r >= 512 && (M - r) * row_bytes >= (2 << 20); ++split) {
       cuts.push_back(r);
       r += ((M - r) / 2 + 255) / 256 * 256;
     }
@@ -1974,7 +1977,10 @@ int sb200_host_register(void* ptr, uint64_t bytes) {
   cudaError_t e = cudaHostRegister(ptr, bytes, cudaHostRegisterPortable);
   if (e == cudaErrorHostMemoryAlreadyRegistered) {
     cudaGetLastError();
-    return SB200_OK;
+    // registered before as it is; or else the range only shares a page with somebody's registration and is not pinned
+    const char* c = static_cast<const char*>(ptr);
+    if (!host_memory_is_pageable(c) && !host_memory_is_pageable(c + bytes / 2) && !host_memory_is_pageable(c + bytes - 1)) return SB200_OK;
+    return cuda_fail(e, "cudaHostRegister");
   }
   if (e != cudaSuccess) return cuda_fail(e, "cudaHostRegister");
   return SB200_OK;

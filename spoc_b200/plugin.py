@@ -459,6 +459,11 @@ class Vector:
     CPU, BOTH, STALE_CPU = "CPU", "Both", "Stale_CPU"
 
     PIN_MIN_BYTES = 16 << 20   # vectors at least this large are pinned in place on their second transfer
+    # Smaller vectors are pinned once this many bytes of them have been moved: registering and releasing 0.25 to 12 MiB takes
+    # 1.1 to 5.5 ms, as much as pinning saves in about that traffic (a pageable MiB takes 70-220 us up and 170 down, a pinned
+    # one 35 and 29).  Below PIN_LEAST_BYTES a pageable copy is as quick.
+    PIN_TRAFFIC_BYTES = 64 << 20
+    PIN_LEAST_BYTES = 256 << 10
 
     def __init__(self, backend: Backend, host: np.ndarray):
         assert host.dtype == np.float32 and host.ndim == 1 and host.flags["C_CONTIGUOUS"]
@@ -467,6 +472,9 @@ class Vector:
         self.buffer: _Memory.Buffer | None = None
         self.location = Vector.CPU
         self._transfers = 0
+        nbytes = host.nbytes             # the transfer before which the array is pinned
+        self._pin_at = (2 if nbytes >= Vector.PIN_MIN_BYTES else
+                        Vector.PIN_TRAFFIC_BYTES // nbytes if nbytes >= Vector.PIN_LEAST_BYTES else -1)
         self._pinned = False
         self._prefetch_dev = None    # device whose outbound stream is bringing the result back to self.host
 
@@ -474,10 +482,10 @@ class Vector:
         """A vector owns its host array for its whole life (as Spoc_core.Vector owns its Bigarray), so the array can be
         pinned in place: the first large transfer goes through the staged pageable copier, and a vector that is moved a
         second time is registered with the driver (sb200_host_register) so that this and every later transfer run at the
-        pinned rate.  SAREK_B200_PIN_VECTORS=0 switches this off; free() unregisters."""
+        pinned rate; smaller vectors follow when they keep being moved.  SAREK_B200_PIN_VECTORS=0 switches this off; free()
+        unregisters."""
         self._transfers += 1
-        if (self._transfers == 2 and not self._pinned and self.host.nbytes >= Vector.PIN_MIN_BYTES
-                and os.environ.get("SAREK_B200_PIN_VECTORS", "1") != "0"):
+        if self._transfers == self._pin_at and not self._pinned and os.environ.get("SAREK_B200_PIN_VECTORS", "1") != "0":
             if L.load().sb200_host_register(self.host.ctypes.data_as(C.c_void_p), self.host.nbytes) == 0:
                 self._pinned = True
 
@@ -590,6 +598,7 @@ def run_vectors(backend: Backend, *, device: _Device.T, ir: str, args: Sequence,
                     _check(rc)
                 return
     rs_args = []
+    pinned = []
     uploaded = []
     prefetch = os.environ.get("SAREK_B200_PREFETCH_RESULTS", "1") != "0"
     for a in args:
@@ -598,12 +607,18 @@ def run_vectors(backend: Backend, *, device: _Device.T, ir: str, args: Sequence,
             host = a.pending_upload(device)
             if host is not None:
                 uploaded.append(a)
-            # a page-locked host array can take the kernel's result back while later row blocks are still computing
-            rs_args.append(RSA_Buffer(a.buffer, a.length, host, a.host if (a._pinned and prefetch) else None))
+            # a page-locked host array can take the kernel's result back while later row blocks are still computing; a small
+            # one only in a launch that moves data anyway, so that launches on resident vectors stay launches
+            rs_args.append(RSA_Buffer(a.buffer, a.length, host))
+            if a._pinned and prefetch:
+                pinned.append((a, rs_args[-1]))
             rs_args.append(RSA_Int32(a.length))
         else:
             kind, v = a
             rs_args.append({"int32": RSA_Int32, "int64": RSA_Int64, "float32": RSA_Float32, "float64": RSA_Float64}[kind](v))
+    for a, arg in pinned:
+        if uploaded or a.host.nbytes >= Vector.PIN_MIN_BYTES:
+            arg.host_copy = a.host
     backend.Device.set_current(device)
     source = backend.generate_source(ir, block)
     coming_back = backend.run_source(source=source, lang=backend.supported_source_langs[0], kernel_name=kernel_name,

@@ -53,6 +53,16 @@ def test_vectors_on_the_device_are_expanded_and_marked_stale(calls):
     assert a.location == Vector.STALE_CPU and b.location == Vector.STALE_CPU
 
 
+def test_a_small_pinned_vector_is_launched_on(calls):
+    v = _vector(Vector.PIN_MIN_BYTES // 4 - 1, Vector.STALE_CPU)
+    v._pinned = True
+    try:
+        assert plugin._hostpath().launch(9, [v], dims1d(1), dims1d(1), 0) == 0
+        assert len(calls.seen) == 1
+    finally:
+        v._pinned, v.buffer = False, None
+
+
 def test_a_failed_launch_leaves_the_locations(calls):
     calls.rc = L.ERR_BOUNDS
     a = _vector(5, Vector.BOTH)
@@ -61,7 +71,7 @@ def test_a_failed_launch_leaves_the_locations(calls):
 
 
 def _pinned():
-    v = _vector(4, Vector.BOTH)
+    v = _vector(Vector.PIN_MIN_BYTES // 4, Vector.BOTH)     # its result would be sent back behind the launch
     v._pinned = True
     return v
 
