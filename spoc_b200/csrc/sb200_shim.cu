@@ -1499,6 +1499,17 @@ int download_behind(DeviceState& d, cudaStream_t st, void* host, uint64_t dev_pt
   return ce == cudaSuccess ? SB200_OK : cuda_fail(ce, "download of a result behind its kernel");
 }
 
+// The same on `st` itself; the outbound stream, which a reader waits for, follows it.
+int download_on(DeviceState& d, cudaStream_t st, void* host, uint64_t dev_ptr, size_t bytes) {
+  cudaEvent_t e = nullptr;
+  CU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  cudaError_t ce = cudaMemcpyAsync(host, as_ptr<void>(dev_ptr), bytes, cudaMemcpyDeviceToHost, st);
+  if (ce == cudaSuccess) ce = cudaEventRecord(e, st);
+  if (ce == cudaSuccess) ce = cudaStreamWaitEvent(d.pipe_out, e, 0);
+  cudaEventDestroy(e);
+  return ce == cudaSuccess ? SB200_OK : cuda_fail(ce, "download of a result behind its kernel");
+}
+
 // The element-wise operators by chunks: the inputs of a chunk come over on the inbound stream, the kernel of the chunk
 // follows them on `st`, and the outputs of the chunk go back on the outbound stream to the page-locked arrays the caller
 // named for them (out_host[0], out_host[1]; null: stay on the device).  Every element depends on its own index only, so
@@ -1651,14 +1662,24 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
   if (row_bytes > 0 && block_rows * row_bytes < (4 << 20)) block_rows = ((4 << 20) + row_bytes - 1) / row_bytes;
   block_rows = (block_rows + 255) / 256 * 256;
   if (block_rows > M) block_rows = M;
+  // A product of one block has nothing to overlap: everything goes through `st` itself, without the events between streams
+  // (several microseconds each on the way from copy to kernel to copy).
+  const bool one_block = block_rows == M;
+  const cudaStream_t in = one_block ? st : d.pipe_in;
   std::vector<cudaEvent_t> events;
+  cudaEvent_t uploaded = nullptr;  // one_block: recorded behind the last upload
   auto done = [&](int rc) {
-    cudaStreamSynchronize(d.pipe_in);  // every upload has landed (or failed) before the host arrays are given back
+    // every upload has landed (or failed) before the host arrays are given back
+    if (uploaded)
+      cudaEventSynchronize(uploaded);
+    else
+      cudaStreamSynchronize(in);
     for (auto e : events) cudaEventDestroy(e);
     cudaGetLastError();
     return rc;
   };
   auto mark = [&]() -> int {  // `st` continues only after what the inbound stream has been given so far
+    if (one_block) return SB200_OK;
     cudaEvent_t e = nullptr;
     cudaError_t ce = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     if (ce == cudaSuccess) {
@@ -1669,7 +1690,7 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
     return ce == cudaSuccess ? SB200_OK : cuda_fail(ce, "ordering a row block behind its upload");
   };
   // the inbound stream must not overtake work that still reads or writes these buffers on `st`
-  {
+  if (!one_block) {
     cudaEvent_t e = nullptr;
     CU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     events.push_back(e);
@@ -1684,16 +1705,16 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
   auto upload_from = [&](const Slot* v, long long first) -> bool {
     if (!v || !v->host || v->len <= first) return true;
     return cudaMemcpyAsync(as_ptr<float>(v->ptr) + first, static_cast<const float*>(v->host) + first,
-                           static_cast<size_t>(v->len - first) * 4, cudaMemcpyHostToDevice, d.pipe_in) == cudaSuccess;
+                           static_cast<size_t>(v->len - first) * 4, cudaMemcpyHostToDevice, in) == cudaSuccess;
   };
   if (!upload_from(&a, M * K) || !upload_from(&b, K * N) || !upload_from(c, M * N) || !upload_from(bias, N) ||
       !upload_from(&dd, c && c->ptr == dd.ptr ? dd.len : M * N))
     return done(cuda_fail(cudaGetLastError(), "upload of a vector's tail"));
   if (b.host && K > 0)
-    if (cudaMemcpyAsync(as_ptr<void>(b.ptr), b.host, static_cast<size_t>(K) * N * 4, cudaMemcpyHostToDevice, d.pipe_in) != cudaSuccess)
+    if (cudaMemcpyAsync(as_ptr<void>(b.ptr), b.host, static_cast<size_t>(K) * N * 4, cudaMemcpyHostToDevice, in) != cudaSuccess)
       return done(cuda_fail(cudaGetLastError(), "upload of B"));
   if (bias && bias->host)
-    if (cudaMemcpyAsync(as_ptr<void>(bias->ptr), bias->host, static_cast<size_t>(N) * 4, cudaMemcpyHostToDevice, d.pipe_in) != cudaSuccess)
+    if (cudaMemcpyAsync(as_ptr<void>(bias->ptr), bias->host, static_cast<size_t>(N) * 4, cudaMemcpyHostToDevice, in) != cudaSuccess)
       return done(cuda_fail(cudaGetLastError(), "upload of the bias"));
   if ((rc = mark())) return done(rc);
   // The last block's GEMM and download cannot hide behind any upload, so the final stretch is cut finer: whole blocks
@@ -1701,7 +1722,7 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
   std::vector<long long> cuts;  // first row of every block, then M
   {
     long long r = 0;
-    while (M - r > block_rows) {
+    while (!one_block && M - r > block_rows) {
       cuts.push_back(r);
       r += block_rows;
     }
@@ -1709,7 +1730,7 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
       const char* e = getenv("SAREK_B200_PIPE_TAPER");
       return !(e && e[0] == '0');
     }();
-    for (int split = 0; split < 2 && taper && M - r >= 512 && (M - r) * row_bytes >= (2 << 20); ++split) {
+    for (int split = 0; split < 2 && taper && !one_block && M - r >= 512 && (M - r) * row_bytes >= (2 << 20); ++split) {
       cuts.push_back(r);
       r += ((M - r) / 2 + 255) / 256 * 256;
     }
@@ -1720,20 +1741,33 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
     const long long r0 = cuts[bi], rows = cuts[bi + 1] - r0;
     if (a.host && K > 0 &&
         cudaMemcpyAsync(as_ptr<float>(a.ptr) + r0 * K, static_cast<const float*>(a.host) + r0 * K, static_cast<size_t>(rows) * K * 4,
-                        cudaMemcpyHostToDevice, d.pipe_in) != cudaSuccess)
+                        cudaMemcpyHostToDevice, in) != cudaSuccess)
       return done(cuda_fail(cudaGetLastError(), "upload of a block of A"));
     if (c && c->host &&
         cudaMemcpyAsync(as_ptr<float>(c->ptr) + r0 * N, static_cast<const float*>(c->host) + r0 * N, static_cast<size_t>(rows) * N * 4,
-                        cudaMemcpyHostToDevice, d.pipe_in) != cudaSuccess)
+                        cudaMemcpyHostToDevice, in) != cudaSuccess)
       return done(cuda_fail(cudaGetLastError(), "upload of a block of C"));
     if ((rc = mark())) break;
+    if (one_block) {
+      cudaError_t ce = cudaEventCreateWithFlags(&uploaded, cudaEventDisableTiming);
+      if (ce == cudaSuccess) {
+        events.push_back(uploaded);
+        ce = cudaEventRecord(uploaded, st);
+      }
+      if (ce != cudaSuccess) {
+        uploaded = nullptr;
+        return done(cuda_fail(ce, "event behind the uploads"));
+      }
+    }
     rc = run_gemm(d, st, mode, rows, N, K, a.ptr + static_cast<uint64_t>(r0) * K * 4, K, b.ptr, N, D + static_cast<uint64_t>(r0) * N * 4, N,
                   alpha, c ? c->ptr + static_cast<uint64_t>(r0) * N * 4 : 0, N, beta, bias ? bias->ptr : 0, act);
-    if (!rc && d_host)
+    if (!rc && d_host && one_block) {
+      rc = download_on(d, st, d_host, D, static_cast<size_t>(dd.len) * 4);
+    } else if (!rc && d_host)
       rc = download_behind(d, st, static_cast<float*>(d_host) + r0 * N, D + static_cast<uint64_t>(r0) * N * 4, static_cast<size_t>(rows) * N * 4);
   }
   // what D's vector holds beyond the product goes back too: the caller is told that the whole host copy is current
-  if (!rc && d_host && dd.len > M * N)
+  if (!rc && d_host && !one_block && dd.len > M * N)
     rc = download_behind(d, st, static_cast<float*>(d_host) + M * N, D + static_cast<uint64_t>(M) * N * 4, static_cast<size_t>(dd.len - M * N) * 4);
   return done(rc);
 }
