@@ -619,18 +619,19 @@ __device__ __forceinline__ void scan_b_f16(const F16ScanB& j, unsigned int block
   }
 }
 
-// First preparation launch of the fp16 modes: A's panels, and the column maxima of B by runs of rows.  Blocks [0, blocks_a) work
-// on A.  (Two launches and a memset fewer than a pass each; the maxima need no atomics.  The column scan alone took 21 us of
+// First preparation launch of the fp16 modes: the column maxima of B by runs of rows (blocks [0, blocks_b), in front because they
+// take longest), and A's panels.  A block loads its rows, reduces and stores, so half of the blocks of an SM are loading at a
+// time: three to five of them keep the loads in flight that HBM needs (two: 3 TB/s at 8192^2).  (Two launches and a memset fewer than a pass each; the maxima need no atomics.  The column scan alone took 21 us of
 // the 50 a 2048^3 product's preparation took, on 64 blocks.)
 template <int TPR, int HOLD>
-__global__ void __launch_bounds__(256, HOLD == 4 ? 4 : 2) prep_f16_first_kernel(const F16PrepA a, const F16ScanB b, int blocks_a) {
+__global__ void __launch_bounds__(256, HOLD == 4 ? 5 : 3) prep_f16_first_kernel(const F16PrepA a, const F16ScanB b, int blocks_b) {
   __shared__ unsigned int smem[8 * 128];
   grid_launch_dependents();
   grid_dependency_wait();
-  if (static_cast<int>(blockIdx.x) < blocks_a)
-    prep_a_f16_rows<TPR, HOLD>(a, blockIdx.x, blocks_a, smem);
+  if (static_cast<int>(blockIdx.x) >= blocks_b)
+    prep_a_f16_rows<TPR, HOLD>(a, blockIdx.x - blocks_b, gridDim.x - blocks_b, smem);
   else
-    scan_b_f16(b, blockIdx.x - blocks_a, smem);
+    scan_b_f16(b, blockIdx.x, smem);
 }
 
 // B[K x N] -> hi, lo [N x Kp] halves and col_scale[N], transposed through shared memory in tiles of 64 k x 64 n: 128-bit loads

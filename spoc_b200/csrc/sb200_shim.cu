@@ -502,17 +502,21 @@ struct TileShape {
   int tile_n = 256, splits = 1;
 };
 
-constexpr int kMinSplitKBlocks = 16;  // a divided k-loop keeps at least this many k-blocks per work item
+// a divided k-loop keeps at least this many k-blocks per work item: 16 in the three-MMA pairs, whose k-blocks take longest, else 8
+constexpr int kMinSplitKBlocks = 8, kMinSplitKBlocksThree = 16;
 constexpr int kMaxSplits = 32;
 
 // Estimates the time of each cut (in ns at 1.9 GHz) and takes the shortest.  Per k-block: measured on 1024 x 1024 x K, MMA-bound
 // at 256 columns (843 ns with three MMAs per k-step, 277 with one), near it at 192 and 128, bound by the operands' shared-memory
 // reads at 64 (340 ns) and by the latency around a stage in the one-MMA modes (165 ns).  256-column tiles have the best ratio of
-// tensor-core work to shared-memory, L2 and electric power, so a narrower tile is charged 10 % and has to win by 3 %: it does
-// when there are fewer 256-column tiles than pairs.  192 columns serve the three-MMA modes only.  Fixed: launch, set-up,
-// pipeline fill, and 400 ns per 32 columns of epilogue that nothing overlaps.
+// tensor-core work to shared-memory, L2 and electric power, so a narrower tile has to win by 3 % after a charge: 10 % in the
+// one-MMA modes, which wait for operands, and for k-loops of 128 blocks and more, whose operands outgrow L2; 2 % otherwise.  It
+// does when there are fewer 256-column tiles than pairs, or when its last wave is fuller (4096 x 4096 x 1024 in 3xTF32: 3.5
+// waves of 256 columns 154 us, 6.9 waves of 128 columns 143 us).  192 columns serve the three-MMA modes only.  Fixed: launch,
+// set-up, pipeline fill, and 500 ns per 32 columns of epilogue that nothing overlaps.
 // Dividing the k-loop pays when the tiles occupy a fraction of the SMs and k is long; it costs a second launch and the
-// partial results' way through L2 (about 4 TB/s), and is left to products that stay at 16 k-blocks per item or more.
+// partial results' way through L2 (about 4 TB/s), and has to win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one
+// of 32 takes 11.1; 40 x 300 x 1200 unaligned 18.7 against 28.8).
 // fixed_splits > 0: the division is given (a row block of a larger product is divided as the whole is, so that it has the
 // same bits).
 // convert: gemm_convert_kernel's rates (see there) instead of the pair kernel's.
@@ -523,20 +527,24 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
   double best_cost = 0.0;
   bool have = false;
   const long long tiles_m = (M + 128 * ctas - 1) / (128 * ctas);
-  for (int bn : {256, 192, 128, 64}) {
-    if (ctas == 1 && bn > 128) continue;
-    if (bn == 192 && (!three || forced)) continue;
-    if (forced && bn != forced && !(ctas == 1 && forced == 256 && bn == 128)) continue;
-    const double per_kblock = convert ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0)) : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0) : (bn == 256 ? 277.0 : 165.0);
-    const long long tiles = tiles_m * ((N + bn - 1) / bn);
-    for (int sp = 1; sp <= kMaxSplits; ++sp) {
-      if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * kMinSplitKBlocks)) continue;
-      const long long per_item = (kblocks + sp - 1) / sp;
-      if (sp > 1 && per_item * (sp - 1) >= kblocks) continue;  // the last item would be empty
+  const int min_blocks = three && ctas == 2 ? kMinSplitKBlocksThree : kMinSplitKBlocks;
+  for (int sp = 1; sp <= kMaxSplits; ++sp) {
+    if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * min_blocks)) continue;
+    const long long per_item = (kblocks + sp - 1) / sp;
+    if (sp > 1 && per_item * (sp - 1) >= kblocks) continue;  // the last item would be empty
+    for (int bn : {256, 192, 128, 64}) {
+      if (ctas == 1 && bn > 128) continue;
+      if (bn == 192 && (!three || forced)) continue;
+      if (forced && bn != forced && !(ctas == 1 && forced == 256 && bn == 128)) continue;
+      const double per_kblock = convert ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0))
+                                : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0)
+                                        : (bn == 256 ? 277.0 : 165.0);
+      const double charge = bn == 256 ? 1.0 : three && kblocks < 128 ? 1.02 : 1.1;
+      const long long tiles = tiles_m * ((N + bn - 1) / bn);
       const long long waves = (tiles * sp + units - 1) / units;
-      double c = waves * per_item * per_kblock * (bn == 256 ? 1.0 : 1.1) + 5500.0 + 400.0 * (bn / 32) + 800.0 * (waves - 1);
-      if (sp > 1) c += 3000.0 + (sp + 1.0) * M * N * 4.0 / 4000.0;
-      if (!have || c < (sp > best.splits || bn < best.tile_n ? 0.97 : 1.0) * best_cost) {
+      double c = waves * per_item * per_kblock * charge + 5500.0 + 500.0 * (bn / 32) + 800.0 * (waves - 1);
+      if (sp > 1) c += 2500.0 + (sp + 1.0) * M * N * 4.0 / 4000.0;
+      if (!have || c < (sp == best.splits ? 0.97 : best.splits == 1 ? 0.92 : 0.97) * best_cost) {
         best.tile_n = bn;
         best.splits = sp;
         best_cost = c;
@@ -1002,14 +1010,15 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
     const F16ScanB jb{B, ldb, col_max, static_cast<int>(K), static_cast<int>(N), static_cast<int>(scan_rows), vec_b};
     // threads per row of A: as few as hold a row in four quads each, which lets four blocks share an SM
     const int tpr = kp <= 512 ? 32 : kp <= 1024 ? 64 : kp <= 2048 ? 128 : 256;
-    const int grid_a = grid_for(M, 256 / tpr, static_cast<long long>(d.sm_count) * 8);
-    const dim3 grid(static_cast<unsigned>(grid_a + ((N + 127) / 128) * runs));
+    const int grid_a = grid_for(M, 256 / tpr, static_cast<long long>(d.sm_count) * 64);
+    const int grid_b = static_cast<int>(((N + 127) / 128) * runs);
+    const dim3 grid(static_cast<unsigned>(grid_a + grid_b));
     auto first = tpr == 32   ? prep_f16_first_kernel<32, 4>
                  : tpr == 64  ? prep_f16_first_kernel<64, 4>
                  : tpr == 128 ? prep_f16_first_kernel<128, 4>
                  : kp <= 4096 ? prep_f16_first_kernel<256, 4>
                               : prep_f16_first_kernel<256, 8>;
-    CU_TRY(launch_pdl(first, grid, dim3(256), 0, st, 1, ja, jb, grid_a));
+    CU_TRY(launch_pdl(first, grid, dim3(256), 0, st, 1, ja, jb, grid_b));
     if ((rc = launch_check("prep_f16_first_kernel"))) return rc;
     const int tiles = grid_for((kp >> 6) * ((N + 63) >> 6), 1, static_cast<long long>(d.sm_count) * 16);
     CU_TRY(launch_pdl(prep_b_f16_kernel, dim3(static_cast<unsigned>(tiles)), dim3(256), 0, st, 1, B, ldb, b_hi, b_lo, col_scale,
