@@ -267,7 +267,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
           if (!p.tma_epilogue) {
             epilogue_rows<BN / 2>(p, taddr, epi.buf, lane, row0, c0);
           } else {
-            epilogue_tma_begin(p, &map_c, epi, row0, c0);
+            epilogue_tma_begin(p, &map_c, epi, lane, row0, c0);
             if (!epilogue_tma<BN / 2>(p, &map_d, &map_c, taddr, epi, lane, row0, c0, split * p.part_rows, abort_flag)) {
               if (lane == 0) atomicCAS(p.status, 0, 0x2500);
               ok = false;

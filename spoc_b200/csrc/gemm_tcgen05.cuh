@@ -108,6 +108,7 @@ struct EpiWarp {
   float* cols;      // 32 words of the bias, 32 column scales
   uint64_t* c_bar;  // one barrier per tile for the loads of C
   uint32_t c_phase; // bit b: parity of c_bar[b]
+  float bias, scale; // this lane's column of the next chunk: loaded a chunk ahead, or before the accumulator is awaited
   int next;         // tile of buf the next chunk uses (runs on from one accumulator to the next)
 };
 
@@ -117,6 +118,8 @@ __device__ __forceinline__ EpiWarp epi_warp(uint8_t* epi_base, uint8_t* ctrl, in
   e.cols = reinterpret_cast<float*>(ctrl + GEMM_CTRL_COLS + w * 256);
   e.c_bar = reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + 2 * w;
   e.c_phase = 0;
+  e.bias = 0.0f;
+  e.scale = 1.0f;
   e.next = 0;
   return e;
 }
@@ -128,8 +131,14 @@ __device__ __forceinline__ void epi_load_c(const CUtensorMap* map_c, const EpiWa
   tma_load_2d_hint(smem_u32(e.buf + b * 1024), map_c, bar, col, row, pol);
 }
 
-// Before the accumulator is awaited: the first tile of C is on its way while the k-loop still runs.
-__device__ __forceinline__ void epilogue_tma_begin(const GemmParams& p, const CUtensorMap* map_c, const EpiWarp& e, int row0, int n0) {
+__device__ __forceinline__ void epi_load_cols(const GemmParams& p, EpiWarp& e, int col) {
+  if (p.bias) e.bias = col < p.N ? p.bias[col] : 0.0f;
+  if (p.col_scale) e.scale = col < p.N ? p.col_scale[col] : 1.0f;
+}
+
+// Before the accumulator is awaited: the first tile of C, the bias and the scales are on their way while the k-loop still runs.
+__device__ __forceinline__ void epilogue_tma_begin(const GemmParams& p, const CUtensorMap* map_c, EpiWarp& e, int lane, int row0, int n0) {
+  epi_load_cols(p, e, n0 + lane);
   if (p.C && row0 < p.M && elect_one()) {
     bulk_wait_read<0>();
     epi_load_c(map_c, e, e.next, n0, row0, l2_policy((p.l2_policy >> 4) & 3));
@@ -159,10 +168,8 @@ __device__ __forceinline__ bool epilogue_tma(const GemmParams& p, const CUtensor
     e.next ^= 1;
     uint32_t v[32];
     tmem_ld_32x32b_x32(taddr + chunk * 32, v);
-    const int col = col0 + lane;
-    float bias_v = 0.0f, scale_v = 1.0f;
-    if (p.bias && col < p.N) bias_v = p.bias[col];
-    if (scaled && col < p.N) scale_v = p.col_scale[col];
+    const float bias_v = e.bias, scale_v = e.scale;
+    epi_load_cols(p, e, col0 + 32 + lane);  // of the next chunk: the latency of a global load is about a chunk's time
     if (elect_one()) {
       if (p.C) {
         if (chunk + 1 < chunks) {

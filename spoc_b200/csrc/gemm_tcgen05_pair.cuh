@@ -371,7 +371,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
       const int row0 = tm * BM + static_cast<int>(rank) * 128 + quarter * 32;
       const int n0 = tn * BN;
-      if (p.tma_epilogue) epilogue_tma_begin(p, &map_c, epi, row0, n0);
+      if (p.tma_epilogue) epilogue_tma_begin(p, &map_c, epi, lane, row0, n0);
       // every lane waits; the warp then agrees on the outcome so that the warp-collective tensor-memory loads below are
       // never partly skipped
       const bool landed = mbar_wait_bounded(smem_u32(&tmem_full_bar[acc]), acc_phase, abort_flag);
