@@ -520,6 +520,7 @@ struct GenCtx {
 };
 
 bool gen_int(GenCtx& g, const Sx& e, std::string* out);
+bool gen_cond(GenCtx& g, const Sx& e, std::string* out);
 
 bool gen_float(GenCtx& g, const Sx& e, std::string* out) {
   const Ctx& cx = *g.cx;
@@ -583,38 +584,7 @@ bool gen_float(GenCtx& g, const Sx& e, std::string* out) {
   }
   if (e.is("if") && e.size() == 4) {
     std::string c, a, b;
-    std::function<bool(const Sx&, std::string*)> cond = [&](const Sx& x, std::string* o) -> bool {
-      if (x.is("const") && x.size() == 3 && x[1].s == "bool") {
-        *o = x[2].s == "true" ? "true" : "false";
-        return true;
-      }
-      if (x.is("unop") && x.size() == 3 && x[1].s == "not") {
-        std::string i;
-        if (!cond(x[2], &i)) return false;
-        *o = "(!" + i + ")";
-        return true;
-      }
-      if (x.is("binop") && x.size() == 4) {
-        static const std::map<std::string, const char*> cmp = {{"lt", "<"}, {"le", "<="}, {"gt", ">"}, {"ge", ">="}, {"eq", "=="}, {"ne", "!="}};
-        auto it = cmp.find(x[1].s);
-        std::string l, r;
-        if (it != cmp.end()) {
-          if (gen_float(g, x[2], &l) && gen_float(g, x[3], &r)) {
-            *o = "(" + l + " " + it->second + " " + r + ")";
-            return true;
-          }
-          return false;
-        }
-        if (x[1].s == "and" || x[1].s == "or") {
-          if (!cond(x[2], &l) || !cond(x[3], &r)) return false;
-          *o = "(" + l + (x[1].s == "and" ? " && " : " || ") + r + ")";
-          return true;
-        }
-      }
-      g.why = "unsupported condition";
-      return false;
-    };
-    if (!cond(e[1], &c) || !gen_float(g, e[2], &a) || !gen_float(g, e[3], &b)) return false;
+    if (!gen_cond(g, e[1], &c) || !gen_float(g, e[2], &a) || !gen_float(g, e[3], &b)) return false;
     *out = "(" + c + " ? " + a + " : " + b + ")";
     return true;
   }
@@ -668,6 +638,106 @@ bool gen_float(GenCtx& g, const Sx& e, std::string* out) {
   return false;
 }
 
+// Emits e as a float32 expression when its value is a float32 for certain (elements, values stored before, literals that are
+// one, and what negation, absolute value and choice make of them); nothing is recorded when it is not.
+bool gen_exact(GenCtx& g, const Sx& e, std::string* out) {
+  if (e.is("const") && e.size() == 3 && (e[1].s == "f32" || e[1].s == "f64")) {
+    const double v = strtod(e[2].s.c_str(), nullptr);
+    if (!(v == static_cast<double>(static_cast<float>(v)))) return false;
+    std::string t;
+    if (!gen_float(g, e, &t)) return false;
+    *out = "((float)" + t + ")";
+    return true;
+  }
+  if (e.is("read") && e.size() == 3 && e[1].atom && sx_equal(e[2], *g.idx)) {
+    auto it = g.stored.find(e[1].s);
+    if (it != g.stored.end()) {
+      *out = it->second;
+      return true;
+    }
+    std::string t;
+    if (!gen_float(g, e, &t)) return false;
+    *out = "x" + t.substr(1);  // X3, the element as a double, was made from x3
+    return true;
+  }
+  std::string a, b, c;
+  if (e.is("unop") && e.size() == 3 && e[1].s == "neg" && gen_exact(g, e[2], &a)) {
+    *out = "(-" + a + ")";
+    return true;
+  }
+  if (e.is("intrinsic") && e.size() == 4 && e[2].s == "abs_float" && gen_exact(g, e[3], &a)) {
+    *out = "fabsf(" + a + ")";
+    return true;
+  }
+  if (e.is("if") && e.size() == 4 && gen_exact(g, e[2], &a) && gen_exact(g, e[3], &b) && gen_cond(g, e[1], &c)) {
+    *out = "(" + c + " ? " + a + " : " + b + ")";
+    return true;
+  }
+  return false;
+}
+
+// Emits e rounded to float32, as a store rounds it.  One operation on float32 values needs no double arithmetic: rounding the
+// exact result to 53 bits and then to 24 gives what rounding it to 24 at once gives for +, -, *, / and the square root, since
+// 53 >= 2 * 24 + 2 (S. Figueroa, "When is double rounding innocuous?", 1995), subnormal results included (a quotient of two
+// 24-bit significands that is no midpoint is at least 2^-48 of itself away from one).  The two conversions per operand and one
+// per result that this saves run at a quarter of the rate of the arithmetic.
+bool gen_rounded(GenCtx& g, const Sx& e, std::string* out) {
+  if (gen_exact(g, e, out)) return true;
+  std::string a, b, c;
+  if (e.is("binop") && e.size() == 4) {
+    static const std::map<std::string, const char*> ar = {{"add", "__fadd_rn"}, {"sub", "__fsub_rn"}, {"mul", "__fmul_rn"}, {"div", "__fdiv_rn"}};
+    auto it = ar.find(e[1].s);
+    if (it != ar.end() && gen_exact(g, e[2], &a) && gen_exact(g, e[3], &b)) {
+      *out = std::string(it->second) + "(" + a + ", " + b + ")";
+      return true;
+    }
+  }
+  if (e.is("intrinsic") && e.size() == 4 && e[2].s == "sqrt" && gen_exact(g, e[3], &a)) {
+    *out = "__fsqrt_rn(" + a + ")";
+    return true;
+  }
+  if (e.is("if") && e.size() == 4) {
+    if (!gen_cond(g, e[1], &c) || !gen_rounded(g, e[2], &a) || !gen_rounded(g, e[3], &b)) return false;
+    *out = "(" + c + " ? " + a + " : " + b + ")";
+    return true;
+  }
+  if (!gen_float(g, e, &a)) return false;
+  *out = "(float)(" + a + ")";
+  return true;
+}
+
+bool gen_cond(GenCtx& g, const Sx& x, std::string* o) {
+  if (x.is("const") && x.size() == 3 && x[1].s == "bool") {
+    *o = x[2].s == "true" ? "true" : "false";
+    return true;
+  }
+  if (x.is("unop") && x.size() == 3 && x[1].s == "not") {
+    std::string i;
+    if (!gen_cond(g, x[2], &i)) return false;
+    *o = "(!" + i + ")";
+    return true;
+  }
+  if (x.is("binop") && x.size() == 4) {
+    static const std::map<std::string, const char*> cmp = {{"lt", "<"}, {"le", "<="}, {"gt", ">"}, {"ge", ">="}, {"eq", "=="}, {"ne", "!="}};
+    auto it = cmp.find(x[1].s);
+    std::string l, r;
+    if (it != cmp.end()) {
+      if ((gen_exact(g, x[2], &l) && gen_exact(g, x[3], &r)) || (gen_float(g, x[2], &l) && gen_float(g, x[3], &r))) {
+        *o = "(" + l + " " + it->second + " " + r + ")";
+        return true;
+      }
+      return false;
+    }
+    if (x[1].s == "and" || x[1].s == "or") {
+      if (!gen_cond(g, x[2], &l) || !gen_cond(g, x[3], &r)) return false;
+      *o = "(" + l + (x[1].s == "and" ? " && " : " || ") + r + ")";
+      return true;
+    }
+  }
+  g.why = "unsupported condition";
+  return false;
+}
+
 bool gen_int(GenCtx& g, const Sx& e, std::string* out) {
   if (e.is("const") && e.size() == 3 && (e[1].s == "i32" || e[1].s == "i64")) {
     *out = "((long long)" + std::to_string(atoll(e[2].s.c_str())) + "ll)";
@@ -714,7 +784,7 @@ std::string generic_map_source(const KernelPlan& plan, const GenericMap& gm, con
   for (size_t i = 0; i < no; ++i) o << "float& y" << i << (i + 1 < no ? ", " : "");
   o << ") {\n";
   for (size_t i = 0; i < ni; ++i) o << "  const double X" << i << " = (double)x" << i << ";\n";
-  for (size_t i = 0; i < no; ++i) o << "  const float t" << i << " = (float)(" << store_exprs[i] << ");\n  y" << i << " = t" << i << ";\n";
+  for (size_t i = 0; i < no; ++i) o << "  const float t" << i << " = " << store_exprs[i] << ";\n  y" << i << " = t" << i << ";\n";
   o << "}\n";
   // vector kernel, one launch for any n: after `head` (0..3) single elements every operand is 16-byte aligned and
   // nvec whole vectors follow; the ragged ends (head, and up to 3 elements after the vectors) are taken by the
@@ -851,7 +921,7 @@ bool match_map_generic(Ctx& cx, const Sx& body) {
         return false;
       }
     std::string code;
-    if (!gen_float(g, inline_expr((*it)[2], pl.env), &code)) {
+    if (!gen_rounded(g, inline_expr((*it)[2], pl.env), &code)) {
       cx.why = g.why;
       return false;
     }

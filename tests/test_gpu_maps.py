@@ -422,3 +422,42 @@ def test_block_reduction_with_wrong_block_size_is_rejected(backend, device):
     assert e.value.code == L.ERR_ARGS
     va.free()
     vo.free()
+
+
+@pytest.mark.parametrize("op", ["add", "sub", "mul", "div", "sqrt", "choice"])
+def test_single_operations_on_elements_round_as_the_double_path_does(backend, device, op):
+    """One operation on float32 elements is emitted in float32: the same bits as float64 arithmetic rounded once, over the
+    whole range of magnitudes, subnormal operands and results, zeros of both signs, infinities and ragged lengths."""
+    rng = np.random.default_rng(11)
+    n = 50021
+    bits = rng.integers(0, 1 << 32, (2, n), dtype=np.uint64).astype(np.uint32)
+    bits[:, :4000] &= np.uint32(0x80ffffff)          # the smallest normal numbers and subnormals
+    x, y = bits.view(np.float32)
+    special = np.array([0.0, -0.0, np.inf, -np.inf, 1.0, -1.0, 1e-45, -1e-45, 3.4028235e38, 1.1754944e-38], np.float32)
+    x[-100:], y[-100:] = np.repeat(special, 10), np.tile(special, 10)
+    x, y = (np.where(np.isnan(v), np.float32(0.5), v) for v in (x, y))
+    b = sarek_ir.Builder()
+    p = b.params([("vec", "o", "f32"), ("vec", "x", "f32"), ("vec", "y", "f32"), ("scalar", "n", "i32")])
+
+    def body():
+        i = b.evar("i")
+        ex, ey = b.read("x", i), b.read("y", i)
+        f32 = ("Float32",)
+        e = {"sqrt": ("intrinsic", f32, "sqrt", ("intrinsic", f32, "abs_float", ex)),
+             "choice": ("if", b.binop("gt", ("unop", "neg", ex), ey), b.binop("mul", ex, ex), ("unop", "neg", ey))}.get(op) or b.binop(op, ex, ey)
+        return ("sif", b.binop("lt", i, b.evar("n")), ("assign", ("elem", "o", i), e))
+
+    ir = sarek_ir.sx(("kernel", "single", p, ("body", b.let("i", "i32", b.intr("global_thread_id"), body))))
+    vo, vx, vy = Vector.create(backend, n), Vector(backend, x.copy()), Vector(backend, y.copy())
+    run_vectors(backend, device=device, ir=ir, args=[vo, vx, vy, ("int32", n)], block=dims1d(256), grid=dims1d((n + 255) // 256),
+                kernel_name="single")
+    X, Y = x.astype(np.float64), y.astype(np.float64)
+    with np.errstate(all="ignore"):
+        ref = {"add": lambda: X + Y, "sub": lambda: X - Y, "mul": lambda: X * Y, "div": lambda: X / Y, "sqrt": lambda: np.sqrt(np.abs(X)),
+               "choice": lambda: np.where(-X > Y, X * X, -Y)}[op]().astype(np.float32)
+    got = vo.to_array()
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    keep = ~np.isnan(ref)
+    assert np.array_equal(got[keep].view(np.uint32), ref[keep].view(np.uint32))
+    for v in (vo, vx, vy):
+        v.free()
