@@ -423,14 +423,15 @@ __device__ __forceinline__ float4 load_quad(const float* row, int k, int cols, i
   return x;
 }
 
-// The low parts of two row-major matrices in one launch (A and B of a 3xTF32 product whose high parts TMA
-// takes from the caller's matrices): lo[r][c] = rn_tf32(x - rn_tf32(x)), row length padded to colsp with
-// zeros.  Blocks [0, blocks_a) work on job a, the rest on job b.
+// What the direct kernel needs of two row-major matrices beside the matrices themselves, in one launch: the low parts of a
+// 3xTF32 product (lo[r][c] = rn_tf32(x - rn_tf32(x))), and for matrices TMA cannot address copies of their elements; row length
+// padded to colsp with zeros, either may be null.  Elementwise and row by row: the transposing panels it replaced for unaligned
+// operands went through shared memory and took half as long again.  Blocks [0, blocks_a) work on job a, the rest on job b.
 struct PrepLoJob {
   const float* src;
   long long ld;
-  float* lo;
-  int rows, cols, colsp;
+  float *lo, *copy;
+  int rows, cols, colsp, vec_ok;
 };
 
 __device__ __forceinline__ void prep_lo_rows(const PrepLoJob& j, long long block, long long nblocks) {
@@ -439,10 +440,12 @@ __device__ __forceinline__ void prep_lo_rows(const PrepLoJob& j, long long block
   for (long long q = block * blockDim.x + threadIdx.x; q < total; q += nblocks * blockDim.x) {
     const long long row = q / quads_per_row;
     const int k = static_cast<int>(q - row * quads_per_row) << 2;
-    const float4 x = load_quad(j.src + row * j.ld, k, j.cols, 1);  // callers guarantee 16-byte aligned rows
-    const float4 l = make_float4(tf32_lo(x.x, tf32_round(x.x)), tf32_lo(x.y, tf32_round(x.y)),
-                                 tf32_lo(x.z, tf32_round(x.z)), tf32_lo(x.w, tf32_round(x.w)));
-    *reinterpret_cast<float4*>(j.lo + row * j.colsp + k) = l;
+    const float4 x = load_quad(j.src + row * j.ld, k, j.cols, j.vec_ok);
+    if (j.copy) *reinterpret_cast<float4*>(j.copy + row * j.colsp + k) = x;
+    if (j.lo)
+      *reinterpret_cast<float4*>(j.lo + row * j.colsp + k) =
+          make_float4(tf32_lo(x.x, tf32_round(x.x)), tf32_lo(x.y, tf32_round(x.y)), tf32_lo(x.z, tf32_round(x.z)),
+                      tf32_lo(x.w, tf32_round(x.w)));
   }
 }
 

@@ -722,7 +722,7 @@ int gemm_variant_setting() {
 constexpr long long kSingleRows = 64;
 // Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands.
 constexpr double kConvertMacs = 16777216.0;              // 2^24
-constexpr double kConvertMacsUnaligned = 536870912.0;    // 2^29
+constexpr double kConvertMacsUnaligned = 134217728.0;    // 2^27
 
 int stages_of(bool three, int bn, int ctas) {
   const long long stage = (three ? 2 : 1) * (16384ll + (bn / ctas) * 128ll);
@@ -746,6 +746,9 @@ TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_co
   return cut(M, fixed_splits, ctas);
 }
 
+// Row length of the parts of B the direct kernel reads from the scratch.
+long long route_b_pitch(long long N, bool addressable) { return round_up(N, addressable ? 32 : 4); }
+
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
   int fixed_splits = 0;
   if (t_whole_rows > M) {
@@ -758,18 +761,18 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   const int variant = gemm_variant_setting();
   const bool three = mode == SB200_MODE_3XTF32;
   // The caller's matrices are read where they lie when TMA can address them: 16-byte aligned bases and row strides.  TF32
-  // mode then needs no preparation and no scratch, 3xTF32 mode panels of the low parts.
-  const bool direct = variant != 1 && variant != 3 && addressable;
+  // mode then needs no preparation and no scratch, 3xTF32 mode panels of the low parts.  Matrices TMA cannot address are copied
+  // row by row into the scratch first (elementwise, beside the low parts) and read there.
+  const bool direct = variant == 0 || (variant == 2 && addressable);
   const long long kp = round_up(K, GEMM_BK);
   // One launch that converts the operands on their way (gemm_convert_kernel): few rows in 3xTF32, where panels of B would
   // triple the traffic, and any mode's few rows of matrices TMA cannot address; and products so small that the launches that
-  // would prepare panels weigh more than the pair kernel's faster tiles give (aligned: 256^3 is about even; transposing panels
-  // of unaligned matrices are two launches and serve from about 800^3).
+  // would prepare panels weigh more than the pair kernel's faster tiles give (aligned: 256^3 is about even; unaligned: 512^3).
   const double macs = static_cast<double>(M) * N * K;
   const bool convert = variant == 0 && tile_n_setting() != 256 &&
                        (addressable ? three && (M <= kSingleRows || macs < kConvertMacs) : M <= kSingleRows || macs < kConvertMacsUnaligned);
-  // From panels at most 128 rows are served by a block on its own; read directly a pair wins from 65 rows on.
-  r.ctas = convert || variant == 1 || (variant == 0 && (direct ? !three && M <= kSingleRows : M <= GEMM_BM)) ? 1 : 2;
+  // Read directly a pair wins from 65 rows on; from panels a block on its own serves up to 128 rows when a single block is asked for.
+  r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
   const int units = units_of(r.ctas, sm_count);
   const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, convert);
   r.tile_n = shape.tile_n;
@@ -781,8 +784,9 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   if (panel_rows_a < M) panel_rows_a = M;
   if (r.src == SRC_PANELS) {
     r.operand_bytes = gemm_workspace_need(mode, panel_rows_a, N, K);
-  } else if (three && r.src == SRC_DIRECT) {
-    r.operand_bytes = round_up(K * round_up(N, 32) * 4, 1024) + round_up(panel_rows_a * kp * 4, 1024);
+  } else if (r.src == SRC_DIRECT && (three || !addressable)) {
+    const size_t parts = round_up(K * route_b_pitch(N, addressable) * 4, 1024) + round_up(panel_rows_a * kp * 4, 1024);
+    r.operand_bytes = addressable ? parts : std::max<size_t>((three ? 2 : 1) * parts, gemm_workspace_need(mode, panel_rows_a, N, K));
   }
   r.workspace = r.operand_bytes + partial_bytes(M, N, r.splits);
   return r;
@@ -795,8 +799,9 @@ int grid_for(long long work, long long per_block, long long cap) {
 
 int launch_prep_lo(int sm_count, cudaStream_t st, const PrepLoJob& a, const PrepLoJob& b, bool b_ready, const int* gate) {
   const long long cap = static_cast<long long>(sm_count) * 16;
-  const int grid_a = grid_for(static_cast<long long>(a.rows) * (a.colsp >> 2), 256, cap);
-  const int grid_b = b_ready ? 0 : grid_for(static_cast<long long>(b.rows) * (b.colsp >> 2), 256, cap);
+  const int grid_a = a.lo || a.copy ? grid_for(static_cast<long long>(a.rows) * (a.colsp >> 2), 256, cap) : 0;
+  const int grid_b = !b_ready && (b.lo || b.copy) ? grid_for(static_cast<long long>(b.rows) * (b.colsp >> 2), 256, cap) : 0;
+  if (grid_a + grid_b == 0) return SB200_OK;
   CU_TRY(launch_pdl(prep_lo_two_kernel, dim3(static_cast<unsigned>(grid_a + grid_b)), dim3(256), 0, st, 1, a, b, grid_a, gate));
   return launch_check("prep_lo_two_kernel");
 }
@@ -822,8 +827,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   // panel_rows_a: rows the A panels are laid out for (>= M); callers that run several row blocks
   // against one prepared B pass the largest block so that the B panels keep their place.
   if (panel_rows_a < M) panel_rows_a = M;
-  const bool addressable = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0 &&
-                           (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (ldb & 3) == 0;
+  const bool addressable_a = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0,
+             addressable_b = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (ldb & 3) == 0, addressable = addressable_a && addressable_b;
   const GemmRoute route = route_gemm(MODE == 3 ? SB200_MODE_3XTF32 : SB200_MODE_TF32, M, N, K, addressable, d.sm_count, panel_rows_a);
   const bool direct = route.src == SRC_DIRECT;
   const int tile_n = route.tile_n;
@@ -831,8 +836,6 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   const long long kp = round_up(K, GEMM_BK);
   const size_t a_bytes = round_up(panel_rows_a * kp * 4, 1024), b_bytes = round_up(N * kp * 4, 1024);
   int rc = SB200_OK;
-  const long long np = round_up(N, 32);  // row length of the low-part panel of B in the direct layout
-  const size_t blo_bytes = round_up(K * np * 4, 1024);
   // Calls that use the device's scratch are ordered across streams: two streams would otherwise write their
   // operand panels into the same memory at once.  Not while the stream is being captured into a graph (an
   // event of the capture cannot order work outside it): a captured sequence is ordered by its own stream.
@@ -866,19 +869,30 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   if (route.src == SRC_CONVERT) {
     // no panels, no operand maps
   } else if (direct) {
-    if ((rc = encode_map_2d(&ma_hi, A, K, M, lda, GEMM_BK, GEMM_BM, true))) return rc;
-    if ((rc = encode_map_2d(&mb_hi, B, N, K, ldb, 32, GEMM_BK, true, true))) return rc;
+    // Workspace, B's parts first (their place does not depend on M): [B copy][B lo][A copy][A lo], each only when it is needed;
+    // B's as K rows of np, A's as rows of kp.  The copies stand in for matrices TMA cannot address.
+    const bool copy_a = !addressable_a, copy_b = !addressable_b;
+    const long long np = route_b_pitch(N, addressable);
+    const size_t b_part = round_up(K * np * 4, 1024), a_part = round_up(panel_rows_a * kp * 4, 1024);
+    uint8_t* at = static_cast<uint8_t*>(d.workspace);
+    auto take = [&](bool wanted, size_t bytes) {
+      float* q = wanted ? reinterpret_cast<float*>(at) : nullptr;
+      at += wanted ? bytes : 0;
+      return q;
+    };
+    float* b_copy = take(copy_b, b_part);
+    float* b_lo = take(MODE == 3, b_part);
+    float* a_copy = take(copy_a, a_part);
+    float* a_lo = take(MODE == 3, a_part);
+    // one launch (B's are not made again for the row blocks after the first)
+    const PrepLoJob ja{A, lda, a_lo, a_copy, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp), addressable_a ? 1 : 0};
+    const PrepLoJob jb{B, ldb, b_lo, b_copy, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), addressable_b ? 1 : 0};
+    if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, b_panels_ready, nullptr))) return rc;
+    if ((rc = encode_map_2d(&ma_hi, copy_a ? a_copy : A, K, M, copy_a ? kp : lda, GEMM_BK, GEMM_BM, true))) return rc;
+    if ((rc = encode_map_2d(&mb_hi, copy_b ? b_copy : B, N, K, copy_b ? np : ldb, 32, GEMM_BK, true, true))) return rc;
     ma_lo = ma_hi;
     mb_lo = mb_hi;
     if (MODE == 3) {
-      // low parts only: B's first (K x np, row-major like B), then A's (rows x kp)
-      uint8_t* ws = static_cast<uint8_t*>(d.workspace);
-      float* b_lo = reinterpret_cast<float*>(ws);
-      float* a_lo = reinterpret_cast<float*>(ws + blo_bytes);
-      // both in one launch (B's are not made again for the row blocks after the first)
-      const PrepLoJob ja{A, lda, a_lo, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp)};
-      const PrepLoJob jb{B, ldb, b_lo, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np)};
-      if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, b_panels_ready, nullptr))) return rc;
       if ((rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
       if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     }
@@ -1163,8 +1177,8 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     // behind it, gated the other way: plain 3xTF32 on the same operands, its low-part panels in the same scratch
     float* pb_lo = reinterpret_cast<float*>(ws);
     float* pa_lo = reinterpret_cast<float*>(ws + round_up(K * np * 4, 1024));
-    const PrepLoJob ja{A, lda, pa_lo, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp32)};
-    const PrepLoJob jb{B, ldb, pb_lo, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np)};
+    const PrepLoJob ja{A, lda, pa_lo, nullptr, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp32), 1};
+    const PrepLoJob jb{B, ldb, pb_lo, nullptr, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), 1};
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, false, gp.gate))) return rc;
     CUtensorMap pma_lo, pmb_lo;
     if ((rc = encode_map_2d(&pma_lo, pa_lo, kp32, M, kp32, GEMM_BK, GEMM_BM, false))) return rc;
@@ -2546,11 +2560,12 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   }
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
-  // "panels" for operands TMA cannot address also when they are converted on their way (launches=1, no scratch for operands);
-  // the passes over A and B are counted apart although one launch makes both
-  const int launches = (r.src == SRC_PANELS ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + (r.splits > 1 ? 1 : 0);
+  // "panels" for operands TMA cannot address also when they are copied or converted on their way (converted: launches=1, no
+  // scratch for operands); the passes over A and B are counted apart although one launch makes both
+  const bool apart = r.src == SRC_PANELS || (r.src == SRC_DIRECT && !addressable);
+  const int launches = (apart ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + (r.splits > 1 ? 1 : 0);
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
-           r.ctas == 2 ? "pair" : "single", r.src == SRC_DIRECT || (r.src == SRC_CONVERT && addressable) ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
+           r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
            r.splits, r.workspace, launches);
   return copy_out(buf, out, outlen);
 }
