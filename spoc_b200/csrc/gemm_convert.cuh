@@ -191,6 +191,9 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full_bar + 2 * STAGES + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // a k-loop divided within a cluster: item `split * num_tiles + tile` is this block's only one
+  const bool in_cluster = p.cluster_splits > 1;
+  const int split_rank = in_cluster ? static_cast<int>(cluster_ctarank()) : 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -214,6 +217,8 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   grid_launch_dependents();
   grid_dependency_wait();  // nothing above touched global memory
   const int num_tiles = p.tiles_m * p.tiles_n, num_items = num_tiles * p.splits;
+  const int first_item = in_cluster ? static_cast<int>(blockIdx.x) / p.cluster_splits + split_rank * num_tiles : static_cast<int>(blockIdx.x);
+  const int item_step = in_cluster ? 1 << 30 : static_cast<int>(gridDim.x);
 
   if (warp < CONV_WARPS) {
     // ----------------------------------------- load, convert, store; then the epilogue
@@ -223,7 +228,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     int stage = 0, local = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++local) {
+    for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn;
       pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
       const int m0 = tm * 128, n0 = tn * BN, split = item / num_tiles;
@@ -264,7 +269,10 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
         const int row0 = m0 + quarter * 32, c0 = n0 + half * (BN / 2);
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2);
         if (c0 < p.N) {
-          if (!p.tma_epilogue) {
+          if (in_cluster) {
+            static_assert(ClusterPart<BN>::kBytes <= STAGES * Cfg::kStageBytes, "partial sums fit the ring");
+            cluster_part_store<BN>(reinterpret_cast<float*>(smem), taddr, quarter * 32 + lane, half * (BN / 2), BN / 2);
+          } else if (!p.tma_epilogue) {
             epilogue_rows<BN / 2>(p, taddr, epi.buf, lane, row0, c0);
           } else {
             epilogue_tma_begin(p, &map_c, epi, lane, row0, c0);
@@ -282,6 +290,16 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       if (*abort_flag) ok = false;  // a wait ran out in some warp: all leave together
     }
     __syncwarp();
+    if (in_cluster) {
+      cluster_arrive();
+      cluster_wait();
+      int tm, tn;
+      pair_tile_coords(first_item - split_rank * num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      if (p.vec_epilogue)
+        cluster_part_finish<BN, 1, CONV_WARPS * 32, true>(p, smem, split_rank, 0, tm * 128, tn * BN, threadIdx.x);
+      else
+        cluster_part_finish<BN, 1, CONV_WARPS * 32, false>(p, smem, split_rank, 0, tm * 128, tn * BN, threadIdx.x);
+    }
   } else {
     // ------------------------------------------------------- MMA issuer
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CONV_REGS_MMA));
@@ -290,7 +308,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      for (int item = first_item; item < num_items && ok; item += item_step) {
         const int kb0 = (item / num_tiles) * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
         for (int kb = 0; kb < blocks; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), phase, abort_flag)) {
@@ -324,10 +342,18 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       }
     }
     __syncwarp();
+    if (in_cluster) {
+      cluster_arrive();
+      cluster_wait();
+    }
   }
 
   tc_fence_before_sync();
   __syncthreads();
+  if (in_cluster) {  // no block retires while others read its partial sums
+    cluster_arrive();
+    cluster_wait();
+  }
   if (warp == CONV_WARPS) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, BN);

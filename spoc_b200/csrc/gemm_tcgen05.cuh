@@ -61,6 +61,9 @@ struct GemmParams {
   int vec_epilogue;
   // Work items a tile's k-loop is divided into (1: not divided), k-blocks of each, and rows of one partial result.
   int splits, split_k_blocks, part_rows;
+  // > 1: the items of a tile are the blocks (pairs) of one cluster, which add up their partial sums through distributed shared
+  // memory; else 1, and a divided k-loop goes through partial results in global memory.
+  int cluster_splits;
   // Set by the host when D (and C) can be addressed by TMA and there are no replicas: the epilogue then stores D, and
   // fetches C, as 32 x 32 tiles with bulk-tensor copies (epilogue_tma).
   int tma_epilogue;

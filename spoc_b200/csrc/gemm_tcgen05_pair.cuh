@@ -13,6 +13,8 @@
 // already works on the next tile in the other accumulator.
 // Every TMA load is issued by the block that consumes it (plain per-block loads).
 #pragma once
+#include <type_traits>
+
 #include "gemm_tcgen05.cuh"
 
 namespace sb200 {
@@ -42,6 +44,7 @@ struct TileCfg {
   static constexpr int kThreads = GEMM_THREADS;
 };
 
+constexpr int REDUCE_THREADS = 64;     // gemm_reduce_kernel: small blocks, so that small results are spread over the SMs
 constexpr int PAIR_EPOCH_RING = 64;    // epoch counters (a pair far ahead wraps onto an old counter: harmless, a hint)
 
 // Count this pair into epoch e and wait, for wait_ns at most, until all `pairs` pairs of the launch have reached it.
@@ -64,6 +67,154 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tile
   tn = within / band_m;
 }
 
+// Four columns of a row of D = act(alpha*sum + beta*C + bias): the operations of the other epilogues in the same order.  VEC: 128-bit
+// accesses (p.vec_epilogue).  Columns from N on are left out.
+struct QuadColumns {  // what the rows of a column quad share
+  float bias[4], scale[4];
+};
+template <bool VEC>
+__device__ __forceinline__ QuadColumns quad_columns(const GemmParams& p, int col) {
+  QuadColumns q;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const bool in = col + j < p.N;
+    q.bias[j] = in && p.bias ? p.bias[col + j] : 0.0f;
+    q.scale[j] = in && p.col_scale ? p.col_scale[col + j] : 1.0f;
+  }
+  return q;
+}
+template <bool VEC>
+__device__ __forceinline__ float4 quad_of_c(const GemmParams& p, long long row, int col) {
+  float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!p.C || col >= p.N) return c;
+  const float* src = p.C + row * p.ldc + col;
+  if (VEC) return *reinterpret_cast<const float4*>(src);
+  c.x = src[0];
+  if (col + 1 < p.N) c.y = src[1];
+  if (col + 2 < p.N) c.z = src[2];
+  if (col + 3 < p.N) c.w = src[3];
+  return c;
+}
+template <bool VEC>
+__device__ __forceinline__ void finish_quad(const GemmParams& p, long long row, int col, const float4& sum, const float4& c4,
+                                            const QuadColumns& q) {
+  float x[4] = {sum.x, sum.y, sum.z, sum.w};
+  const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+  const float rs = p.row_scale ? p.row_scale[row] : 1.0f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float y = __fmul_rn(p.alpha, (x[j] * rs) * q.scale[j]);
+    if (p.C) y = fmaf(p.beta, c[j], y);
+    y = __fadd_rn(y, q.bias[j]);
+    if (p.act == 1) y = (y > 0.0f) ? y : 0.0f;
+    x[j] = y;
+  }
+  const long long off = row * p.ldd + col;
+  if (VEC) {
+    *reinterpret_cast<float4*>(p.D + off) = make_float4(x[0], x[1], x[2], x[3]);
+    for (int r = 0; r < p.n_replicas; ++r) *reinterpret_cast<float4*>(p.replicas[r] + off) = make_float4(x[0], x[1], x[2], x[3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (col + j >= p.N) break;
+      p.D[off + j] = x[j];
+      if (p.n_replicas) store_replicas(p, off + j, x[j]);
+    }
+  }
+}
+__device__ __forceinline__ void add_to(float4& s, const float4& v) {
+  s.x += v.x;
+  s.y += v.y;
+  s.z += v.z;
+  s.w += v.w;
+}
+
+// A k-loop divided among the blocks (pairs) of one cluster (p.cluster_splits > 1).  Each block leaves the partial sums of its
+// 128 rows and BN columns in its operand ring, which is idle once the accumulator is complete; behind a cluster barrier every
+// block adds up a share of the rows' quads from all of them, in order of k, and finishes it.  Bound by the peers' shared memory,
+// which delivers about 14 bytes a cycle and SM with the loads of several quads in flight (2 ns a quad).  Against partial results in
+// global memory and a second launch: 64 x 4096 x 4096 TF32 20.4 -> 17.5 us, 256 x 512 x 1024 3xTF32 15.2 -> 12.3 us, TF32 10.0 -> 8.0.
+template <int BN>
+struct ClusterPart {
+  static constexpr int kPitch = BN + 4;  // floats per row: consecutive rows start four banks apart
+  static constexpr uint32_t kBytes = 128 * kPitch * 4;
+};
+// One warp's 32 rows (tensor-memory lanes from `row` of the block's 128) and `cols` columns from `col` on.
+template <int BN>
+__device__ __forceinline__ void cluster_part_store(float* part, uint32_t taddr, int row, int col, int cols) {
+#pragma unroll 1
+  for (int c = 0; c < cols; c += 32) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(taddr + c, r);
+    tmem_ld_wait_x32(r);
+    uint4* dst = reinterpret_cast<uint4*>(part + row * ClusterPart<BN>::kPitch + col + c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dst[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+  }
+}
+// share: this block's split; rank: its rank in its pair; row0, n0: the first row and column of its part of the tile.
+template <int BN, int CTAS, int THREADS, bool VEC>
+__device__ __forceinline__ void cluster_part_finish(const GemmParams& p, const void* part, int share, int rank, int row0, int n0, int tid) {
+  constexpr int QUADS = BN / 4;
+  static_assert(THREADS % QUADS == 0, "a thread stays in its column quad");
+  constexpr int BATCH = 4, AHEAD = 4;    // quads, and partial sums of each, that a thread has in flight
+  constexpr int STEP = THREADS / QUADS;  // rows between a thread's quads
+  const int rows = min(128, p.M - row0);
+  if (rows <= 0) return;
+  const int total = rows * QUADS, splits = p.cluster_splits;
+  const int begin = total * share / splits + tid, end = total * (share + 1) / splits;
+  const int first_row = begin / QUADS, quad = begin - first_row * QUADS, col = n0 + quad * 4;
+  if (col >= p.N) return;
+  const QuadColumns columns = quad_columns<VEC>(p, col);
+  const uint8_t* own = static_cast<const uint8_t*>(part) + quad * 16;
+  constexpr int PITCH = ClusterPart<BN>::kPitch * 4;
+  for (int at = begin, row = first_row; at < end; at += BATCH * THREADS, row += BATCH * STEP) {
+    const int count = (end - at + THREADS - 1) / THREADS;  // quads left to this thread
+    auto batch = [&](auto whole) {
+      constexpr int N = decltype(whole)::value;
+      float4 s[N], c[N];
+#pragma unroll
+      for (int u = 0; u < N; ++u) c[u] = quad_of_c<VEC>(p, row0 + row + u * STEP, col);
+#pragma unroll 1
+      for (int k0 = 0; k0 < splits; k0 += AHEAD) {
+        float4 v[AHEAD][N];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+          if (k0 + j >= splits) break;
+          if (k0 + j == share) {
+#pragma unroll
+            for (int u = 0; u < N; ++u) v[j][u] = *reinterpret_cast<const float4*>(own + (row + u * STEP) * PITCH);
+          } else {
+            const uint32_t peer = map_to_cta(smem_u32(own), (k0 + j) * CTAS + rank) + row * PITCH;
+#pragma unroll
+            for (int u = 0; u < N; ++u) v[j][u] = ld_cluster_v4(peer + u * STEP * PITCH);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+          if (k0 + j >= splits) break;
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            if (k0 + j == 0)
+              s[u] = v[j][u];
+            else
+              add_to(s[u], v[j][u]);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < N; ++u) finish_quad<VEC>(p, row0 + row + u * STEP, col, s[u], c[u], columns);
+    };
+    if (count >= BATCH) {
+      batch(std::integral_constant<int, BATCH>());
+    } else {
+      if (count & 2) batch(std::integral_constant<int, 2>());
+      if (count & 2) row += 2 * STEP;
+      if (count & 1) batch(std::integral_constant<int, 1>());
+    }
+  }
+}
+
 // MODE 1: TF32, one MMA per k-step.  MODE 3: 3xTF32, lo*hi + hi*lo + hi*hi per k-step into one accumulator (the lo*lo term,
 // 2^-22 relative, is dropped).  MODE 4: the same three-term split on fp16 panels (kind::f16): a 128-byte operand row holds 64
 // halves instead of 32 floats, so a k-block spans 64 k and a k-step 16, in the same bytes, descriptors and cycles as the TF32
@@ -77,7 +228,8 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tile
 // the accumulator by 2^-first_scale).
 //
 // p.splits > 1: the k-blocks of a tile are divided among `splits` work items, each of which stores its partial sums to rows
-// [s * p.part_rows, ...) of a partial matrix (map_d); gemm_reduce_kernel adds them up in order and runs the epilogue.
+// [s * p.part_rows, ...) of a partial matrix (map_d); gemm_reduce_kernel adds them up in order and runs the epilogue.  With
+// p.cluster_splits > 1 the items of a tile are the pairs of one cluster instead, one tile per cluster, and the sums stay on chip.
 template <int MODE, int SRC, int BN, int CTAS>
 __global__ void __launch_bounds__(TileCfg<MODE, SRC, BN, CTAS>::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_constant__ CUtensorMap map_b_hi,
@@ -114,9 +266,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;  // 0 = leader
-  const int pair_id = static_cast<int>(blockIdx.x) / CTAS;
-  const int num_pairs = static_cast<int>(gridDim.x) / CTAS;
+  const bool in_cluster = MODE != 5 && p.cluster_splits > 1;
+  const uint32_t cta = CTAS == 2 || in_cluster ? cluster_ctarank() : 0u;
+  const uint32_t rank = cta & (CTAS - 1u), leader = cta - rank;  // rank 0 = leader of its pair
+  // in_cluster: item `split * num_tiles + tile` is this pair's only one
+  const int split_rank = in_cluster ? static_cast<int>(cta) / CTAS : 0;
+  const int pair_id = in_cluster ? static_cast<int>(blockIdx.x) / (CTAS * p.cluster_splits) + split_rank * p.tiles_m * p.tiles_n
+                                 : static_cast<int>(blockIdx.x) / CTAS;
+  const int num_pairs = in_cluster ? 1 << 30 : static_cast<int>(gridDim.x) / CTAS;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -149,7 +306,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   }
   __syncthreads();
   if (CTAS == 2) {
-    // both blocks' barriers exist before any signal crosses between them
+    // the blocks' barriers exist before any signal crosses between them
     cluster_arrive();
     cluster_wait();
   }
@@ -206,7 +363,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
           }
           // the leader arms its barrier with the bytes of both blocks
           if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), CTAS * Cfg::kStageBytes);
-          const uint32_t bar = CTAS == 2 ? map_to_cta(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
+          const uint32_t bar = CTAS == 2 ? map_to_cta(smem_u32(&full_bar[stage]), leader) : smem_u32(&full_bar[stage]);
           uint8_t* sp = stage_base + stage * Cfg::kStageBytes;
           auto load = [&](uint8_t* dst, const CUtensorMap& map, int x, int y, uint64_t pol) {
             tma_load_for<CTAS>(smem_u32(dst), &map, bar, x, y, pol);
@@ -348,13 +505,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
               }
             }
           }
-          umma_commit_for<CTAS>(smem_u32(&empty_bar[stage]));  // the stage is free (in both blocks) once these MMAs retire
+          umma_commit_for<CTAS>(smem_u32(&empty_bar[stage]), leader);  // the stage is free (in both blocks) once these MMAs retire
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) umma_commit_for<CTAS>(smem_u32(&tmem_full_bar[acc]));
+        if (ok) umma_commit_for<CTAS>(smem_u32(&tmem_full_bar[acc]), leader);
       }
     }
     __syncwarp();
@@ -382,7 +539,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       }
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * 256;
-      if (!p.tma_epilogue) {
+      if (in_cluster) {
+        static_assert(ClusterPart<BN>::kBytes <= STAGES * Cfg::kStageBytes, "partial sums fit the ring");
+        cluster_part_store<BN>(reinterpret_cast<float*>(stage_base), taddr, quarter * 32 + lane, 0, BN);
+      } else if (!p.tma_epilogue) {
         epilogue_rows<BN>(p, taddr, epi.buf, lane, row0, n0);
       } else if (!epilogue_tma<BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, (item / num_tiles) * p.part_rows, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, 0x1500 | (rank << 4) | acc);
@@ -393,7 +553,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       __syncwarp();
       if (lane == 0) {
         if (CTAS == 2)
-          mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
+          mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), leader));
         else
           mbar_arrive(smem_u32(&tmem_empty_bar[acc]));
       }
@@ -403,11 +563,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     __syncwarp();
   }
 
+  if (in_cluster) {
+    cluster_arrive();
+    cluster_wait();
+    int tm, tn;
+    pair_tile_coords(pair_id - split_rank * num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+    const int row0 = tm * BM + static_cast<int>(rank) * 128;
+    if (p.vec_epilogue)
+      cluster_part_finish<BN, CTAS, Cfg::kThreads, true>(p, stage_base, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
+    else
+      cluster_part_finish<BN, CTAS, Cfg::kThreads, false>(p, stage_base, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
+  }
+
   // Neither block may retire, or free tensor memory, while its peer can still signal its barriers, read its shared memory or
   // write its accumulators.
   tc_fence_before_sync();
   __syncthreads();
-  if (CTAS == 2) {
+  if (CTAS == 2 || in_cluster) {
     cluster_arrive();
     cluster_wait();
   }
@@ -417,51 +589,44 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   }
 }
 
-// The second half of a product whose k-loop was divided (p.splits > 1): D = act(alpha*sum + beta*C + bias), the partial sums
-// added in order of k, so that the result does not depend on which block finished first.  part: [splits][part_rows][ld]
-// floats, ld a multiple of 4; one thread per four columns.  Bound by L2 (the partials were just written).
-__global__ void __launch_bounds__(256) gemm_reduce_kernel(const float* part, long long ld, int part_rows, int splits,
-                                                          const GemmParams p) {
-  grid_launch_dependents();
-  grid_dependency_wait();
+// The second half of a product whose k-loop was divided (p.splits > 1, p.cluster_splits == 1): the partial sums added in order
+// of k, so that the result does not depend on which block finished first.  part: [splits][part_rows][ld]
+// floats, ld a multiple of 4; one thread per four columns, which keeps eight partial sums in flight.  Bound by latency and L2 (the
+// partials were just written): 32 partials of 128 x 96, 6.2 us with a row of dependent loads a thread, 4.4 so.
+template <bool VEC>
+__device__ __forceinline__ void reduce_quads(const float* part, long long ld, int part_rows, int splits, const GemmParams& p) {
+  constexpr int AHEAD = 8;
   const long long quads = (p.N + 3) >> 2, total = quads * p.M;
+  const long long step = static_cast<long long>(part_rows) * ld >> 2;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long row = i / quads;
     const int col = static_cast<int>(i - row * quads) << 2;
     const float4* src = reinterpret_cast<const float4*>(part + row * ld + col);
-    const long long step = static_cast<long long>(part_rows) * ld >> 2;
-    float4 s = src[0];
-#pragma unroll 4
-    for (int k = 1; k < splits; ++k) {
-      const float4 v = src[k * step];
-      s.x += v.x;
-      s.y += v.y;
-      s.z += v.z;
-      s.w += v.w;
-    }
-    float x[4] = {s.x, s.y, s.z, s.w};
-    const float rs = p.row_scale ? p.row_scale[row] : 1.0f;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f), c, v[AHEAD];
+    QuadColumns columns;
+    for (int k = 0; k < splits; k += AHEAD) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (col + j >= p.N) break;
-      float y = __fmul_rn(p.alpha, (x[j] * rs) * (p.col_scale ? p.col_scale[col + j] : 1.0f));
-      if (p.C) y = fmaf(p.beta, p.C[row * p.ldc + col + j], y);
-      y = __fadd_rn(y, p.bias ? p.bias[col + j] : 0.0f);
-      if (p.act == 1) y = (y > 0.0f) ? y : 0.0f;
-      x[j] = y;
-    }
-    const long long off = row * p.ldd + col;
-    if (p.vec_epilogue) {
-      *reinterpret_cast<float4*>(p.D + off) = make_float4(x[0], x[1], x[2], x[3]);
-      for (int r = 0; r < p.n_replicas; ++r) *reinterpret_cast<float4*>(p.replicas[r] + off) = make_float4(x[0], x[1], x[2], x[3]);
-    } else {
-      for (int j = 0; j < 4 && col + j < p.N; ++j) {
-        p.D[off + j] = x[j];
-        if (p.n_replicas) store_replicas(p, off + j, x[j]);
+      for (int u = 0; u < AHEAD; ++u) v[u] = src[min(k + u, splits - 1) * step];
+      if (k == 0) {
+        c = quad_of_c<VEC>(p, row, col);
+        columns = quad_columns<VEC>(p, col);
+        s = v[0];
       }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+        if (k + u > 0 && k + u < splits) add_to(s, v[u]);
     }
+    finish_quad<VEC>(p, row, col, s, c, columns);
   }
+}
+__global__ void __launch_bounds__(REDUCE_THREADS) gemm_reduce_kernel(const float* part, long long ld, int part_rows, int splits, const GemmParams p) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (p.vec_epilogue)
+    reduce_quads<true>(part, ld, part_rows, splits, p);
+  else
+    reduce_quads<false>(part, ld, part_rows, splits, p);
 }
 
 }  // namespace sb200

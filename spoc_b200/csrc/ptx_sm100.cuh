@@ -215,6 +215,12 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
+// 128-bit load from the shared memory of a block of the cluster (address from map_to_cta)
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
+  return v;
+}
 // arrive on an mbarrier that may live in the peer block (address from map_to_cta)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -324,12 +330,12 @@ __device__ __forceinline__ void umma_tf32_pair_scaled(uint32_t tmem_d, uint64_t 
 __device__ __forceinline__ void umma_f16_pair_scaled(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int scale) {
   SB200_UMMA_SCALED_BODY("f16")
 }
-// Arrive on the mbarriers at this shared-memory address in both blocks of the pair once every MMA issued so far by this
-// thread has completed: one instruction instead of a commit per block.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+// Arrive on the mbarriers at this shared-memory address in both blocks of the pair (the leader's rank in the cluster and the
+// next) once every MMA issued so far by this thread has completed: one instruction instead of a commit per block.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t leader) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"(static_cast<uint16_t>(3))
+      "h"(static_cast<uint16_t>(3u << leader))
       : "memory");
 }
 
@@ -359,8 +365,8 @@ __device__ __forceinline__ void tmem_dealloc_for(uint32_t taddr, uint32_t ncols)
   if constexpr (CTAS == 2) tmem_dealloc_pair(taddr, ncols); else tmem_dealloc(taddr, ncols);
 }
 template <int CTAS>
-__device__ __forceinline__ void umma_commit_for(uint32_t bar) {
-  if constexpr (CTAS == 2) umma_commit_pair(bar); else umma_commit(bar);
+__device__ __forceinline__ void umma_commit_for(uint32_t bar, uint32_t leader) {
+  if constexpr (CTAS == 2) umma_commit_pair(bar, leader); else umma_commit(bar);
 }
 template <bool F16, int CTAS>
 __device__ __forceinline__ void umma_for(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {

@@ -502,6 +502,20 @@ struct TileShape {
   int tile_n = 256, splits = 1;
 };
 
+// Clusters of `blocks` (at most 8) blocks that are resident at once when every block has an SM to itself.  A cluster lies within a
+// GPC, whose SMs it may not divide evenly: the runtime counts 148, 74, 45, 33, 26, 22, 15 and 15 on a 148-SM B200.  One less from
+// three blocks on, because chips differ in the SMs that are switched off and one cluster too many is a second wave.
+long long cluster_capacity(int blocks, int sm_count) {
+  static const int resident[9] = {0, 148, 74, 44, 32, 25, 21, 14, 14};
+  return static_cast<long long>(resident[blocks]) * sm_count / 148;
+}
+// Whether the items of a divided k-loop are the blocks (pairs) of one cluster: at most eight blocks, the portable size, and
+// all tiles at once, because a cluster works on one tile and ends.
+bool split_in_cluster(long long tiles, int splits, int ctas, int sm_count) {
+  return splits > 1 && splits * ctas <= 8 && tiles <= cluster_capacity(splits * ctas, sm_count);
+}
+long long tiles_of(long long M, long long N, int tile_n, int ctas) { return ((M + 128 * ctas - 1) / (128 * ctas)) * ((N + tile_n - 1) / tile_n); }
+
 // a divided k-loop keeps at least this many k-blocks per work item: 16 in the three-MMA pairs, whose k-blocks take longest, else 8
 constexpr int kMinSplitKBlocks = 8, kMinSplitKBlocksThree = 16;
 constexpr int kMaxSplits = 32;
@@ -509,13 +523,14 @@ constexpr int kMaxSplits = 32;
 // Estimates the time of each cut (in ns at 1.9 GHz) and takes the shortest.  Per k-block: measured on 1024 x 1024 x K, MMA-bound
 // at 256 columns (843 ns with three MMAs per k-step, 277 with one), near it at 192 and 128, bound by the operands' shared-memory
 // reads at 64 (340 ns) and by the latency around a stage in the one-MMA modes (165 ns).  256-column tiles have the best ratio of
-// tensor-core work to shared-memory, L2 and electric power, so a narrower tile has to win by 3 % after a charge: 10 % in the
-// one-MMA modes, which wait for operands, and for k-loops of 128 blocks and more, whose operands outgrow L2; 2 % otherwise.  It
+// tensor-core work to shared-memory, L2 and electric power, so a narrower tile has to win by 3 % after a charge: 2 %,
+// and 10 % for k-loops of 128 blocks and more, whose operands outgrow L2; 10 and 40 % in the one-MMA modes, which wait for
+// operands (1000 x 1000 x 8000: 128 columns 270 ns per k-block instead of 165).  It
 // does when there are fewer 256-column tiles than pairs, or when its last wave is fuller (4096 x 4096 x 1024 in 3xTF32: 3.5
 // waves of 256 columns 154 us, 6.9 waves of 128 columns 143 us).  192 columns serve the three-MMA modes only.  Fixed: launch,
 // set-up, pipeline fill, and 500 ns per 32 columns of epilogue that nothing overlaps.
 // Dividing the k-loop pays when the tiles occupy a fraction of the SMs and k is long; it costs a second launch and the
-// partial results' way through L2 (about 4 TB/s), and has to win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one
+// partial results' way through L2 (about 4 TB/s), or within a cluster two barriers and a round of distributed shared memory, and has to win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one
 // of 32 takes 11.1; 40 x 300 x 1200 unaligned 18.7 against 28.8).
 // fixed_splits > 0: the division is given (a row block of a larger product is divided as the whole is, so that it has the
 // same bits).
@@ -527,9 +542,9 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
   double best_cost = 0.0;
   bool have = false;
   const long long tiles_m = (M + 128 * ctas - 1) / (128 * ctas);
-  const int min_blocks = three && ctas == 2 ? kMinSplitKBlocksThree : kMinSplitKBlocks;
+  const int sm_count = units * ctas;
   for (int sp = 1; sp <= kMaxSplits; ++sp) {
-    if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * min_blocks)) continue;
+    if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * kMinSplitKBlocks)) continue;
     const long long per_item = (kblocks + sp - 1) / sp;
     if (sp > 1 && per_item * (sp - 1) >= kblocks) continue;  // the last item would be empty
     for (int bn : {256, 192, 128, 64}) {
@@ -539,11 +554,16 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
       const double per_kblock = convert ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0))
                                 : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0)
                                         : (bn == 256 ? 277.0 : 165.0);
-      const double charge = bn == 256 ? 1.0 : three && kblocks < 128 ? 1.02 : 1.1;
+      const double charge = bn == 256 ? 1.0 : three ? (kblocks < 128 ? 1.02 : 1.1) : (kblocks < 128 ? 1.1 : 1.4);
       const long long tiles = tiles_m * ((N + bn - 1) / bn);
-      const long long waves = (tiles * sp + units - 1) / units;
+      const bool in_cluster = split_in_cluster(tiles, sp, ctas, sm_count);
+      if (!fixed_splits && sp > 1 && !in_cluster && three && ctas == 2 && kblocks < static_cast<long long>(sp) * kMinSplitKBlocksThree) continue;
+      const long long waves = in_cluster ? 1 : (tiles * sp + units - 1) / units;
       double c = waves * per_item * per_kblock * charge + 5500.0 + 500.0 * (bn / 32) + 800.0 * (waves - 1);
-      if (sp > 1) c += 2500.0 + (sp + 1.0) * M * N * 4.0 / 4000.0;
+      if (in_cluster)  // the barriers, and 2 ns per quad of a block's share
+        c += 1500.0 + 2.0 * (M < 128 ? M : 128) * (bn / 4) / sp;
+      else if (sp > 1)
+        c += 2500.0 + (sp + 1.0) * M * N * 4.0 / 4000.0;
       if (!have || c < (sp == best.splits ? 0.97 : best.splits == 1 ? 0.92 : 0.97) * best_cost) {
         best.tile_n = bn;
         best.splits = sp;
@@ -563,6 +583,13 @@ struct OperandMaps {
 // The parameters and output maps a GEMM kernel is launched with: *kp is *gp with the epilogue as it is, or, when the k-loop is
 // divided, with one that stores plain partial sums to `part` ([splits][part_rows][roundup(N, 4)] floats).
 int output_maps(GemmParams* gp, GemmParams* kp, float* part, const CUtensorMap& filler, CUtensorMap* map_d, CUtensorMap* map_c) {
+  if (gp->cluster_splits > 1) {  // nothing but the finished result leaves the chip
+    gp->part_rows = gp->tma_epilogue = 0;
+    gp->epoch_ctr = nullptr;
+    *map_d = *map_c = filler;
+    *kp = *gp;
+    return SB200_OK;
+  }
   if (gp->splits == 1) {
     gp->part_rows = 0;
     epilogue_maps(gp, filler, map_d, map_c);
@@ -584,11 +611,11 @@ int output_maps(GemmParams* gp, GemmParams* kp, float* part, const CUtensorMap& 
 
 // The launch that adds up the partial sums of a divided k-loop (none when it was not divided).
 int launch_reduce(int sm_count, cudaStream_t st, const GemmParams& gp, const float* part) {
-  if (gp.splits == 1) return SB200_OK;
+  if (gp.splits == 1 || gp.cluster_splits > 1) return SB200_OK;
   const long long ld = round_up(gp.N, 4), quads = static_cast<long long>(gp.M) * (ld >> 2);
-  long long blocks = (quads + 255) / 256;
-  if (blocks > static_cast<long long>(sm_count) * 8) blocks = static_cast<long long>(sm_count) * 8;
-  CU_TRY(launch_pdl(gemm_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, st, 1, part, ld, gp.part_rows, gp.splits, gp));
+  long long blocks = (quads + REDUCE_THREADS - 1) / REDUCE_THREADS;
+  if (blocks > static_cast<long long>(sm_count) * 32) blocks = static_cast<long long>(sm_count) * 32;
+  CU_TRY(launch_pdl(gemm_reduce_kernel, dim3(static_cast<unsigned>(blocks)), dim3(REDUCE_THREADS), 0, st, 1, part, ld, gp.part_rows, gp.splits, gp));
   return launch_check("gemm_reduce_kernel");
 }
 
@@ -630,12 +657,13 @@ int launch_tiles(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   if (gp.splits < 1) gp.splits = 1;
   gp.split_k_blocks = (gp.num_k_blocks + gp.splits - 1) / gp.splits;
   const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
-  const long long used = items < units ? items : units;
+  gp.cluster_splits = split_in_cluster(items / gp.splits, gp.splits, CTAS, sm_count) ? gp.splits : 1;
+  const long long used = items < units || gp.cluster_splits > 1 ? items : units;
   const dim3 grid(static_cast<unsigned>(CTAS * used)), block(Cfg::kThreads);
   CUtensorMap map_d, map_c;
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
-  CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_c, kp));
+  CU_TRY(launch_pdl(kernel, grid, block, Cfg::kSmemBytes, st, CTAS * gp.cluster_splits, m.a_hi, m.b_hi, m.a_lo, m.b_lo, m.a_x, m.b_x, map_d, map_c, kp));
   if (int rc = launch_check("gemm_pair_kernel")) return rc;
   return launch_reduce(sm_count, st, gp, part);
 }
@@ -656,12 +684,13 @@ int launch_convert(int dev_index, int sm_count, cudaStream_t st, const ConvOpera
   if (gp.splits < 1) gp.splits = 1;
   gp.split_k_blocks = (gp.num_k_blocks + gp.splits - 1) / gp.splits;
   const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
-  const dim3 grid(static_cast<unsigned>(items < sm_count ? items : sm_count));
+  gp.cluster_splits = split_in_cluster(items / gp.splits, gp.splits, 1, sm_count) ? gp.splits : 1;
+  const dim3 grid(static_cast<unsigned>(items < sm_count || gp.cluster_splits > 1 ? items : sm_count));
   CUtensorMap map_d, map_c;
   memset(&map_d, 0, sizeof map_d);
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, map_d, &map_d, &map_c)) return rc;
-  CU_TRY(launch_pdl(kernel, grid, dim3(CONV_THREADS), Cfg::kSmemBytes, st, 1, o, map_d, map_c, kp));
+  CU_TRY(launch_pdl(kernel, grid, dim3(CONV_THREADS), Cfg::kSmemBytes, st, gp.cluster_splits, o, map_d, map_c, kp));
   if (int rc = launch_check("gemm_convert_kernel")) return rc;
   return launch_reduce(sm_count, st, gp, part);
 }
@@ -674,8 +703,9 @@ int launch_convert_for(int bn, bool vec, int dev_index, int sm_count, cudaStream
   return vec ? launch_convert<MODE, 128, true>(dev_index, sm_count, st, o, gp, part) : launch_convert<MODE, 128, false>(dev_index, sm_count, st, o, gp, part);
 }
 
-size_t partial_bytes(long long M, long long N, int splits) {
-  return splits > 1 ? static_cast<size_t>(round_up(M, 32)) * round_up(N, 4) * 4 * splits : 0;
+size_t partial_bytes(long long M, long long N, const TileShape& shape, int ctas, int sm_count) {
+  const int splits = shape.splits;
+  return splits > 1 && !split_in_cluster(tiles_of(M, N, shape.tile_n, ctas), splits, ctas, sm_count) ? static_cast<size_t>(round_up(M, 32)) * round_up(N, 4) * 4 * splits : 0;
 }
 
 template <int MODE, int SRC>
@@ -788,7 +818,7 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
     const size_t parts = round_up(K * route_b_pitch(N, addressable) * 4, 1024) + round_up(panel_rows_a * kp * 4, 1024);
     r.operand_bytes = addressable ? parts : std::max<size_t>((three ? 2 : 1) * parts, gemm_workspace_need(mode, panel_rows_a, N, K));
   }
-  r.workspace = r.operand_bytes + partial_bytes(M, N, r.splits);
+  r.workspace = r.operand_bytes + partial_bytes(M, N, shape, r.ctas, sm_count);
   return r;
 }
 
@@ -983,7 +1013,7 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
   const int tile_n = shape.tile_n;
   const size_t need = round_up(gemm_f16_workspace_need(M, N, K, THREE), 1024);
   std::unique_lock<std::mutex> scratch_lock(d.scratch_mu);
-  int rc = ensure_workspace(d, need + partial_bytes(M, N, shape.splits));
+  int rc = ensure_workspace(d, need + partial_bytes(M, N, shape, ctas, d.sm_count));
   if (rc) return rc;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
@@ -2514,7 +2544,7 @@ int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64
     const bool three = mode == SB200_MODE_3XF16;
     int ctas;
     const TileShape shape = f16_shape(M, N, K, three, kSms, &ctas);
-    *bytes = gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape.splits);
+    *bytes = gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, kSms);
     return SB200_OK;
   }
   // upper bound: which route runs depends on the operands' addresses
@@ -2542,7 +2572,8 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
     snprintf(fb, sizeof fb, "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
              ctas == 1 ? "single" : "pair", 128 * ctas, shape.tile_n, stages_of(three, shape.tile_n, ctas), tiles,
              (tiles * shape.splits + units - 1) / units, shape.splits,
-             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape.splits), shape.splits > 1 ? 5 : 4);
+             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count),
+             4 + (shape.splits > 1 && !split_in_cluster(tiles, shape.splits, ctas, sm_count) ? 1 : 0));
     return copy_out(fb, out, outlen);
   }
   if (mode == SB200_MODE_3XMIXED) {
@@ -2563,7 +2594,8 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   // "panels" for operands TMA cannot address also when they are copied or converted on their way (converted: launches=1, no
   // scratch for operands); the passes over A and B are counted apart although one launch makes both
   const bool apart = r.src == SRC_PANELS || (r.src == SRC_DIRECT && !addressable);
-  const int launches = (apart ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + (r.splits > 1 ? 1 : 0);
+  const int launches = (apart ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) +
+                       (r.splits > 1 && !split_in_cluster(r.tiles, r.splits, r.ctas, sm_count) ? 1 : 0);
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
            r.splits, r.workspace, launches);

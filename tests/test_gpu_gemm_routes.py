@@ -95,3 +95,37 @@ def test_192_column_tiles_match_the_256_column_ones(backend, device):
         L.load().sb200_set_gemm_tile_n(0)
         for x in (A, B, D):
             x.free()
+
+
+# (mode, M, N, K, aligned, splits): the blocks or pairs of one cluster share a k-loop; one row, rows and columns that end within
+# a block's share, shares of unequal length, a last block with a shorter k-loop, two to eight items
+CLUSTERS = [(L.MODE_TF32, 1, 8, 1024, True, 4), (L.MODE_TF32, 64, 256, 1028, True, 4), (L.MODE_TF32, 65, 132, 1000, True, 4),
+            (L.MODE_3XTF32, 17, 33, 1025, False, 4), (L.MODE_3XTF32, 128, 64, 2080, False, 8), (L.MODE_3XTF32, 257, 191, 2049, True, 4),
+            (L.MODE_3XTF32, 581, 118, 819, True, 3), (L.MODE_3XTF32, 71, 1411, 1414, True, 4), (L.MODE_TF32, 236, 3528, 4165, True, 4),
+            (L.MODE_3XF16, 36, 3162, 1876, True, 2), (L.MODE_F16, 842, 98, 2240, True, 4)]
+
+
+@pytest.mark.parametrize("mode,M,N,K,aligned,splits", CLUSTERS)
+def test_k_loops_divided_within_a_cluster(backend, device, mode, M, N, K, aligned, splits):
+    text = describe(mode, M, N, K, int(aligned))
+    assert f"splits={splits} " in text
+    a, b, c = O.fill(M * K, 63, 1), O.fill(K * N, 63, 2), O.fill(M * N, 63, 3)
+    bias = O.fill(N, 63, 4, kind=1)
+    off = 0 if aligned else 1
+    pad = lambda x, cols: np.ascontiguousarray(np.pad(x.reshape(-1, cols), ((0, 0), (0, -cols % 4)))).ravel() if aligned else x   # noqa: E731
+    A, B = dev_from(backend, device, pad(a, K), offset=off), dev_from(backend, device, pad(b, N), offset=off)
+    lda, ldb = (K + -K % 4, N + -N % 4) if aligned else (K, N)
+    Cm, Bi, D = dev_from(backend, device, c), dev_from(backend, device, bias), Dev(backend, device, M * N)
+    try:
+        first = None
+        for _ in range(3):
+            D.clear()
+            gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=N, ldd=N)
+            got = D.download()
+            first = got.copy() if first is None else first
+            assert np.array_equal(got.view(np.uint32), first.view(np.uint32))     # the order of the sums is fixed
+        ref = O.gemm(a, b, M, N, K, 1.5, 0.5, c, bias, 1)
+        assert O.gemm_rel_error(got.reshape(M, N), ref) <= tol(mode, K) * 1.5 * math.sqrt(2), text
+    finally:
+        for x in (A, B, Cm, Bi, D):
+            x.free()
