@@ -748,6 +748,122 @@ __global__ void __launch_bounds__(256) prep_b_f16_kernel(const float* B, long lo
   }
 }
 
+// Both operands in one launch, for K up to F16_ONE_MAX_K: the blocks [0, blocks_b) prepare B, a cluster of eight per strip of 32
+// columns.  Each block reads its run of rows_per_block (a multiple of 64) rows of the strip once into shared memory, the
+// cluster agrees on the columns' largest magnitudes through distributed shared memory, and each block scales, splits and writes
+// its run, as prep_b_f16_kernel does.  The other blocks take A's rows.  Bound by HBM: A and B are read once, where the two
+// launches above read B twice, one behind the other.  The shared memory, which A's blocks of the launch hold too, sets the limit of K:
+// 64 KiB a block at 4096, three blocks an SM.  Whole operator, three-term and one-term mode: 1024^3 22.5 -> 17.9 and 19.6 -> 14.7 us,
+// 2048^3 65.4 -> 60.2 and 44.2 -> 40.0, 64 x 4096 x 4096 68.7 -> 55.7 and 55.6 -> 42.5, 64^3 12.1 -> 9.7.
+constexpr int F16_ONE_MAX_K = 4096, F16_ONE_BLOCKS = 8, F16_ONE_COLS = 32, F16_ONE_PITCH = 33;
+struct F16WholeB {
+  const float* src;
+  long long ld;
+  __half *hi, *lo;
+  float* inv_scale;
+  int rows, cols, rowsp, rows_per_block, vec_ok;  // K, N, K rounded up to 64
+};
+__device__ __forceinline__ void prep_b_f16_strip(const F16WholeB& j, unsigned int block, float* tile, unsigned int* smem) {
+  const int tid = threadIdx.x, rank = static_cast<int>(cluster_ctarank());
+  const int n0 = static_cast<int>(block / F16_ONE_BLOCKS) * F16_ONE_COLS;
+  const int k0 = rank * j.rows_per_block, rows = max(0, min(j.rowsp - k0, j.rows_per_block));  // a multiple of 64
+  unsigned int* warp_max = smem;        // [8 warps][32 columns]
+  unsigned int* block_max = smem + 256; // [32], read by the cluster
+  unsigned int* all_max = smem + 288;   // [8 blocks][32]
+  if (j.vec_ok) {
+    const int n = (tid & 7) * 4;
+    unsigned int m[4] = {0, 0, 0, 0};
+#pragma unroll 1
+    for (int r = tid >> 3; r < rows; r += 128) {
+      float4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        x[u] = r + 32 * u < rows && k0 + r + 32 * u < j.rows ? load_quad(j.src + static_cast<long long>(k0 + r + 32 * u) * j.ld, n0 + n, j.cols, 1)
+                                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (r + 32 * u >= rows) break;
+        float* dst = tile + (r + 32 * u) * F16_ONE_PITCH + n;
+        dst[0] = x[u].x;
+        dst[1] = x[u].y;
+        dst[2] = x[u].z;
+        dst[3] = x[u].w;
+        m[0] = max(m[0], abs_bits(x[u].x));
+        m[1] = max(m[1], abs_bits(x[u].y));
+        m[2] = max(m[2], abs_bits(x[u].z));
+        m[3] = max(m[3], abs_bits(x[u].w));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      m[i] = max(m[i], __shfl_xor_sync(0xffffffffu, m[i], 8));
+      m[i] = max(m[i], __shfl_xor_sync(0xffffffffu, m[i], 16));
+      if ((tid & 31) < 8) warp_max[(tid >> 5) * 32 + n + i] = m[i];
+    }
+  } else {
+    const int n = tid & 31;
+    unsigned int m = 0;
+#pragma unroll 1
+    for (int r = tid >> 5; r < rows; r += 64) {  // eight rows of 64
+      float x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        x[u] = k0 + r + 8 * u < j.rows && n0 + n < j.cols ? j.src[static_cast<long long>(k0 + r + 8 * u) * j.ld + n0 + n] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        tile[(r + 8 * u) * F16_ONE_PITCH + n] = x[u];
+        m = max(m, abs_bits(x[u]));
+      }
+    }
+    warp_max[tid] = m;
+  }
+  __syncthreads();
+  if (tid < 32) {
+    unsigned int m = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = max(m, warp_max[w * 32 + tid]);
+    block_max[tid] = m;
+  }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  all_max[tid] = ld_cluster_u32(map_to_cta(smem_u32(block_max + (tid & 31)), tid >> 5));
+  cluster_arrive();  // this block has read what it needs of the others
+  __syncthreads();
+  const int nl = tid >> 3, n = n0 + nl;
+  unsigned int m = 0;
+#pragma unroll
+  for (int b = 0; b < F16_ONE_BLOCKS; ++b) m = max(m, all_max[b * 32 + nl]);
+  const float s = f16_panel_scale(m);
+  if (n < j.cols) {
+    if (rank == 0 && (tid & 7) == 0) j.inv_scale[n] = 1.0f / s;
+    const int kq = (tid & 7) * 8;
+#pragma unroll 2
+    for (int r = kq; r < rows; r += 64) {
+      __align__(16) __half h[8];
+      __align__(16) __half l[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f16_split(tile[(r + i) * F16_ONE_PITCH + nl], s, h[i], l[i]);
+      const long long off = static_cast<long long>(n) * j.rowsp + k0 + r;
+      *reinterpret_cast<uint4*>(j.hi + off) = *reinterpret_cast<const uint4*>(h);
+      if (j.lo) *reinterpret_cast<uint4*>(j.lo + off) = *reinterpret_cast<const uint4*>(l);
+    }
+  }
+  __syncwarp();
+  cluster_wait();  // the others have read this block's maxima
+}
+template <int TPR>
+__global__ void __launch_bounds__(256, 4) prep_f16_one_kernel(const F16PrepA a, const F16WholeB b, int blocks_b) {
+  extern __shared__ float tile[];
+  __shared__ unsigned int smem[256 + 32 + 256];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  if (static_cast<int>(blockIdx.x) >= blocks_b)
+    prep_a_f16_rows<TPR, 4>(a, blockIdx.x - blocks_b, gridDim.x - blocks_b, smem);
+  else
+    prep_b_f16_strip(b, blockIdx.x, tile, smem);
+}
+
 // ------------------------------------------------------------------------
 // Operand preparation for the mixed mode (SB200_MODE_3XMIXED)
 // ------------------------------------------------------------------------

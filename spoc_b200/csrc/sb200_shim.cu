@@ -996,6 +996,13 @@ long long f16_scan_rows(long long N, long long K) {
   return rows < 32 ? 32 : rows;
 }
 
+// Whether one launch prepares both operands (prep_f16_one_kernel).  Above 32 KiB of shared memory a block (K = 2048) A's rows have too
+// few blocks an SM in flight, which shows when nearly all the work is A's: 8192 x 512 x 4000 in the one-term mode 97.6 us in one
+// launch and 92.2 in two, 512 x 8192 x 4000 104.9 and 122.0.
+bool f16_prepared_at_once(long long M, long long N, long long K) {
+  return K <= F16_ONE_MAX_K && N <= (1ll << 24) && (K <= F16_ONE_MAX_K / 2 || M <= 8 * N);
+}
+
 size_t gemm_f16_workspace_need(long long M, long long N, long long K, bool three) {
   const long long kp = round_up(K, 64), per = f16_scan_rows(N, K), runs = (K + per - 1) / per;
   return round_up(runs * N * 4, 1024) + round_up(N * 4, 1024) + round_up(M * 4, 1024) +
@@ -1055,20 +1062,39 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
     // threads per row of A: as few as hold a row in four quads each, which lets four blocks share an SM
     const int tpr = kp <= 512 ? 32 : kp <= 1024 ? 64 : kp <= 2048 ? 128 : 256;
     const int grid_a = grid_for(M, 256 / tpr, static_cast<long long>(d.sm_count) * 64);
-    const int grid_b = static_cast<int>(((N + 127) / 128) * runs);
-    const dim3 grid(static_cast<unsigned>(grid_a + grid_b));
-    auto first = tpr == 32   ? prep_f16_first_kernel<32, 4>
-                 : tpr == 64  ? prep_f16_first_kernel<64, 4>
-                 : tpr == 128 ? prep_f16_first_kernel<128, 4>
-                 : kp <= 4096 ? prep_f16_first_kernel<256, 4>
-                              : prep_f16_first_kernel<256, 8>;
-    CU_TRY(launch_pdl(first, grid, dim3(256), 0, st, 1, ja, jb, grid_b));
-    if ((rc = launch_check("prep_f16_first_kernel"))) return rc;
-    const int tiles = grid_for((kp >> 6) * ((N + 63) >> 6), 1, static_cast<long long>(d.sm_count) * 16);
-    CU_TRY(launch_pdl(prep_b_f16_kernel, dim3(static_cast<unsigned>(tiles)), dim3(256), 0, st, 1, B, ldb, b_hi, b_lo, col_scale,
-                      static_cast<const unsigned int*>(col_max), static_cast<int>(runs), static_cast<int>(K), static_cast<int>(N),
-                      static_cast<int>(kp), vec_b));
-    if ((rc = launch_check("prep_b_f16_kernel"))) return rc;
+    const long long strips = (N + F16_ONE_COLS - 1) / F16_ONE_COLS;
+    if (f16_prepared_at_once(M, N, K)) {
+      const int per_block = static_cast<int>(round_up((K + F16_ONE_BLOCKS - 1) / F16_ONE_BLOCKS, 64));
+      const F16WholeB whole{B, ldb, b_hi, b_lo, col_scale, static_cast<int>(K), static_cast<int>(N), static_cast<int>(kp), per_block, vec_b};
+      const int blocks_b = static_cast<int>(strips) * F16_ONE_BLOCKS;
+      const dim3 grid(static_cast<unsigned>(blocks_b + round_up(grid_a, F16_ONE_BLOCKS)));
+      auto one = tpr == 32 ? prep_f16_one_kernel<32> : tpr == 64 ? prep_f16_one_kernel<64> : tpr == 128 ? prep_f16_one_kernel<128> : prep_f16_one_kernel<256>;
+      const size_t smem = static_cast<size_t>(per_block) * F16_ONE_PITCH * 4;
+      static std::atomic<int> attr_set[kMaxDevices];
+      if (!attr_set[&d - g_dev].load()) {
+        constexpr int most = F16_ONE_MAX_K / F16_ONE_BLOCKS * F16_ONE_PITCH * 4;
+        for (auto k : {prep_f16_one_kernel<32>, prep_f16_one_kernel<64>, prep_f16_one_kernel<128>, prep_f16_one_kernel<256>})
+          CU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        attr_set[&d - g_dev].store(1);
+      }
+      CU_TRY(launch_pdl(one, grid, dim3(256), smem, st, F16_ONE_BLOCKS, ja, whole, blocks_b));
+      if ((rc = launch_check("prep_f16_one_kernel"))) return rc;
+    } else {
+      const int grid_b = static_cast<int>(((N + 127) / 128) * runs);
+      const dim3 grid(static_cast<unsigned>(grid_a + grid_b));
+      auto first = tpr == 32   ? prep_f16_first_kernel<32, 4>
+                   : tpr == 64  ? prep_f16_first_kernel<64, 4>
+                   : tpr == 128 ? prep_f16_first_kernel<128, 4>
+                   : kp <= 4096 ? prep_f16_first_kernel<256, 4>
+                                : prep_f16_first_kernel<256, 8>;
+      CU_TRY(launch_pdl(first, grid, dim3(256), 0, st, 1, ja, jb, grid_b));
+      if ((rc = launch_check("prep_f16_first_kernel"))) return rc;
+      const int tiles = grid_for((kp >> 6) * ((N + 63) >> 6), 1, static_cast<long long>(d.sm_count) * 16);
+      CU_TRY(launch_pdl(prep_b_f16_kernel, dim3(static_cast<unsigned>(tiles)), dim3(256), 0, st, 1, B, ldb, b_hi, b_lo, col_scale,
+                        static_cast<const unsigned int*>(col_max), static_cast<int>(runs), static_cast<int>(K), static_cast<int>(N),
+                        static_cast<int>(kp), vec_b));
+      if ((rc = launch_check("prep_b_f16_kernel"))) return rc;
+    }
   }
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
   if ((rc = encode_map_f16(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
@@ -2573,7 +2599,7 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
              ctas == 1 ? "single" : "pair", 128 * ctas, shape.tile_n, stages_of(three, shape.tile_n, ctas), tiles,
              (tiles * shape.splits + units - 1) / units, shape.splits,
              gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count),
-             4 + (shape.splits > 1 && !split_in_cluster(tiles, shape.splits, ctas, sm_count) ? 1 : 0));
+             4 + (shape.splits > 1 && !split_in_cluster(tiles, shape.splits, ctas, sm_count) ? 1 : 0) - (f16_prepared_at_once(M, N, K) ? 2 : 1));
     return copy_out(fb, out, outlen);
   }
   if (mode == SB200_MODE_3XMIXED) {

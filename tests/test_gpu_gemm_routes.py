@@ -129,3 +129,26 @@ def test_k_loops_divided_within_a_cluster(backend, device, mode, M, N, K, aligne
     finally:
         for x in (A, B, Cm, Bi, D):
             x.free()
+
+
+# the edges of a block's 64 rows, of the eight blocks' runs, of the 32-column strips, and of the range of K
+@pytest.mark.parametrize("mode", [L.MODE_3XF16, L.MODE_F16])
+@pytest.mark.parametrize("M,N,K", [(5, 1, 1), (40, 31, 64), (33, 36, 65), (64, 64, 513), (70, 97, 1000), (9, 32, 4095), (20, 100, 4096), (20, 100, 4097)])
+@pytest.mark.parametrize("aligned", [True, False], ids=["aligned", "unaligned"])
+def test_column_maxima_of_the_fp16_panels_are_found_wherever_they_lie(backend, device, mode, M, N, K, aligned):
+    """Every column of B has one element 2^30 times the others, in a row of its own: with a scale from any smaller maximum its fp16
+    part would be infinite."""
+    rng = np.random.default_rng(K)
+    lda, ldb = (((x + 3) // 4 * 4 if aligned else x + 1 - x % 2) for x in (K, N))
+    a, b = rng.uniform(-1, 1, (M, lda)).astype(np.float32), rng.uniform(-1, 1, (K, ldb)).astype(np.float32)
+    cols = np.arange(N)
+    b[(cols * 37 + K - 1) % K, cols] = np.ldexp(1.5, 30).astype(np.float32)
+    A, B, D = dev_from(backend, device, a.ravel()), dev_from(backend, device, b.ravel()), Dev(backend, device, M * N)
+    try:
+        gemm(backend, device, mode, M, N, K, A, B, D, lda=lda, ldb=ldb, ldd=N)
+        got = D.download().reshape(M, N)
+        ref = O.gemm(np.ascontiguousarray(a[:, :K]).ravel(), np.ascontiguousarray(b[:, :N]).ravel(), M, N, K)
+        assert O.gemm_rel_error(got, ref) <= tol(mode, K)
+    finally:
+        for x in (A, B, D):
+            x.free()
