@@ -175,7 +175,8 @@ struct ConvTile {
   }
 };
 
-template <int MODE, int BN, bool VEC>
+// IN_CLUSTER: a k-loop divided within a cluster; a form of its own, because what it adds took 0.3 to 0.6 us from the smallest products.
+template <int MODE, int BN, bool VEC, bool IN_CLUSTER>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
 gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c,
                     const GemmParams p) {
@@ -191,8 +192,8 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full_bar + 2 * STAGES + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // a k-loop divided within a cluster: item `split * num_tiles + tile` is this block's only one
-  const bool in_cluster = p.cluster_splits > 1;
+  // in_cluster: item `split * num_tiles + tile` is this block's only one
+  constexpr bool in_cluster = IN_CLUSTER;
   const int split_rank = in_cluster ? static_cast<int>(cluster_ctarank()) : 0;
 
   if (threadIdx.x == 0) {
@@ -269,7 +270,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
         const int row0 = m0 + quarter * 32, c0 = n0 + half * (BN / 2);
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2);
         if (c0 < p.N) {
-          if (in_cluster) {
+          if constexpr (in_cluster) {
             static_assert(ClusterPart<BN>::kBytes <= STAGES * Cfg::kStageBytes, "partial sums fit the ring");
             cluster_part_store<BN>(reinterpret_cast<float*>(smem), taddr, quarter * 32 + lane, half * (BN / 2), BN / 2);
           } else if (!p.tma_epilogue) {
@@ -290,7 +291,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       if (*abort_flag) ok = false;  // a wait ran out in some warp: all leave together
     }
     __syncwarp();
-    if (in_cluster) {
+    if constexpr (in_cluster) {
       cluster_arrive();
       cluster_wait();
       int tm, tn;
@@ -342,7 +343,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       }
     }
     __syncwarp();
-    if (in_cluster) {
+    if constexpr (in_cluster) {
       cluster_arrive();
       cluster_wait();
     }
@@ -350,7 +351,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
 
   tc_fence_before_sync();
   __syncthreads();
-  if (in_cluster) {  // no block retires while others read its partial sums
+  if constexpr (in_cluster) {  // no block retires while others read its partial sums
     cluster_arrive();
     cluster_wait();
   }

@@ -672,10 +672,10 @@ int launch_tiles(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
 template <int MODE, int BN, bool VEC>
 int launch_convert(int dev_index, int sm_count, cudaStream_t st, const ConvOperands& o, GemmParams gp, float* part) {
   using Cfg = ConvCfg<MODE, BN>;
-  auto kernel = gemm_convert_kernel<MODE, BN, VEC>;
   static std::atomic<int> attr_set[kMaxDevices];
   if (!attr_set[dev_index].load()) {
-    CU_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
+    for (auto k : {gemm_convert_kernel<MODE, BN, VEC, false>, gemm_convert_kernel<MODE, BN, VEC, true>})
+      CU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
     attr_set[dev_index].store(1);
   }
   gp.tiles_m = (gp.M + 127) / 128;
@@ -690,6 +690,7 @@ int launch_convert(int dev_index, int sm_count, cudaStream_t st, const ConvOpera
   memset(&map_d, 0, sizeof map_d);
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, map_d, &map_d, &map_c)) return rc;
+  auto kernel = gp.cluster_splits > 1 ? gemm_convert_kernel<MODE, BN, VEC, true> : gemm_convert_kernel<MODE, BN, VEC, false>;
   CU_TRY(launch_pdl(kernel, grid, dim3(CONV_THREADS), Cfg::kSmemBytes, st, gp.cluster_splits, o, map_d, map_c, kp));
   if (int rc = launch_check("gemm_convert_kernel")) return rc;
   return launch_reduce(sm_count, st, gp, part);
@@ -753,6 +754,9 @@ constexpr long long kSingleRows = 64;
 // Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands.
 constexpr double kConvertMacs = 16777216.0;              // 2^24
 constexpr double kConvertMacsUnaligned = 134217728.0;    // 2^27
+// In TF32 mode, where aligned operands need no preparation, it is the shorter way for k-loops of a few k-blocks only: no operand maps
+// to encode and fetch (64 x 64 x 128 with the epilogue 7.0 us by a pair, 6.5 so; it loses 0.5 us a k-block on the device).
+constexpr long long kConvertKOneTerm = 128;
 
 int stages_of(bool three, int bn, int ctas) {
   const long long stage = (three ? 2 : 1) * (16384ll + (bn / ctas) * 128ll);
@@ -800,7 +804,8 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   // would prepare panels weigh more than the pair kernel's faster tiles give (aligned: 256^3 is about even; unaligned: 512^3).
   const double macs = static_cast<double>(M) * N * K;
   const bool convert = variant == 0 && tile_n_setting() != 256 &&
-                       (addressable ? three && (M <= kSingleRows || macs < kConvertMacs) : M <= kSingleRows || macs < kConvertMacsUnaligned);
+                       (addressable ? (three ? M <= kSingleRows || macs < kConvertMacs : K <= kConvertKOneTerm && macs < kConvertMacs)
+                                    : M <= kSingleRows || macs < kConvertMacsUnaligned);
   // Read directly a pair wins from 65 rows on; from panels a block on its own serves up to 128 rows when a single block is asked for.
   r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
   const int units = units_of(r.ctas, sm_count);
