@@ -83,6 +83,9 @@ struct DeviceState {
   int cc_major = 0;
   void* workspace = nullptr;
   size_t workspace_bytes = 0;
+  // counts the calls that were given the scratch (ensure_workspace), so that a call in several launches can tell whether what
+  // the launch before left there is still there
+  unsigned long long ws_uses = 1;
   // the scratch is shared by every stream of the device: a call on another stream than the last user's waits for it
   cudaEvent_t ws_event = nullptr;
   cudaStream_t ws_last_stream = nullptr;
@@ -307,7 +310,9 @@ int run_map(DeviceState& d, cudaStream_t st, int op, uint64_t out0, uint64_t out
 // -------------------------------------------------------------- GEMM host
 inline long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
+// Gives the calling launch (which holds scratch_mu) a scratch of at least `bytes`; growing it loses its contents.
 int ensure_workspace(DeviceState& d, size_t bytes) {
+  ++d.ws_uses;
   if (bytes <= d.workspace_bytes) return SB200_OK;
   if (d.workspace) {
     CU_TRY(cudaDeviceSynchronize());
@@ -858,9 +863,11 @@ int launch_prep_panels(int sm_count, cudaStream_t st, const float* A, long long 
 template <int MODE>
 int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, long long K, const float* A,
                      long long lda, const float* B, long long ldb, const GemmParams& gp_in, long long panel_rows_a = 0,
-                     bool b_panels_ready = false) {
+                     unsigned long long* b_prepared = nullptr) {
   // panel_rows_a: rows the A panels are laid out for (>= M); callers that run several row blocks
-  // against one prepared B pass the largest block so that the B panels keep their place.
+  // against one B pass the largest block so that the B panels keep their place.
+  // b_prepared: 0 before such a caller's first block; afterwards the use of the scratch that left B's parts there.  They are
+  // prepared again when another launch has been given the scratch since, or when this block needs a larger one.
   if (panel_rows_a < M) panel_rows_a = M;
   const bool addressable_a = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0,
              addressable_b = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (ldb & 3) == 0, addressable = addressable_a && addressable_b;
@@ -874,10 +881,11 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   // Calls that use the device's scratch are ordered across streams: two streams would otherwise write their
   // operand panels into the same memory at once.  Not while the stream is being captured into a graph (an
   // event of the capture cannot order work outside it): a captured sequence is ordered by its own stream.
-  bool track_scratch = false;
+  bool track_scratch = false, b_panels_ready = false;
   std::unique_lock<std::mutex> scratch_lock(d.scratch_mu, std::defer_lock);
   if (route.workspace) {
     scratch_lock.lock();
+    b_panels_ready = b_prepared && *b_prepared == d.ws_uses && route.workspace <= d.workspace_bytes;
     rc = ensure_workspace(d, route.workspace);
     if (rc) return rc;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -973,6 +981,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   if (track_scratch && rc == SB200_OK) {
     rc = scratch_release(d, st);
   }
+  if (b_prepared) *b_prepared = route.workspace && route.src != SRC_CONVERT ? d.ws_uses : 0;
   return rc;
 }
 
@@ -3038,6 +3047,7 @@ extern "C" int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int6
     if (rem > 0) blocks.emplace_back(r, rem);
   }
   const int nblocks = static_cast<int>(blocks.size());
+  unsigned long long b_prepared = 0;
 
   // Pageable host operands (what a Bigarray is): asynchronous copies from pageable memory are neither
   // asynchronous nor fast, so such a call moves its operands with the staged copier instead — several host
@@ -3114,10 +3124,9 @@ extern "C" int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int6
         rc = launch_gemm_mix(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp);
       } else if (mode == SB200_MODE_3XTF32 || mode == SB200_MODE_3XMIXED) {
         // a block the mixed mode leaves to 3xTF32 finds the scratch holding fp16 panels: B's low parts are made anew
-        rc = launch_gemm_mode<3>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows,
-                                 mode == SB200_MODE_3XTF32 && i > 0);
+        rc = launch_gemm_mode<3>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows, &b_prepared);
       } else {
-        rc = launch_gemm_mode<1>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows, i > 0);
+        rc = launch_gemm_mode<1>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows, &b_prepared);
       }
       if (rc) return finish(rc, "");
       if ((e = static_cast<int>(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming)))) return finish(e, "event");
@@ -3202,10 +3211,9 @@ extern "C" int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int6
     } else if (mode == SB200_MODE_3XMIXED && gemm_mix_applies(rows, N, K, operands_addressable(dA + r0 * K, K, dB, N))) {
       rc = launch_gemm_mix(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp);
     } else if (mode == SB200_MODE_3XTF32 || mode == SB200_MODE_3XMIXED) {
-      rc = launch_gemm_mode<3>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows,
-                               mode == SB200_MODE_3XTF32 && i > 0);
+      rc = launch_gemm_mode<3>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows, &b_prepared);
     } else {
-      rc = launch_gemm_mode<1>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows, i > 0);
+      rc = launch_gemm_mode<1>(*d, d->pipe_compute, rows, N, K, dA + r0 * K, K, dB, N, gp, block_rows, &b_prepared);
     }
     if (rc == SB200_OK) PIPE_TRY(cudaEventRecord(ev_done[i], d->pipe_compute));
     // outbound stream: the finished block of D

@@ -3,6 +3,9 @@ converted in registers, 192-column tiles, divided k-loops and their reduction â€
 epilogue, for operands TMA can and cannot address, against the oracle at the bounds of the numeric modes."""
 import ctypes as C
 import math
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -152,3 +155,39 @@ def test_column_maxima_of_the_fp16_panels_are_found_wherever_they_lie(backend, d
     finally:
         for x in (A, B, D):
             x.free()
+
+
+GROWING_SCRATCH = """
+import ctypes as C
+import numpy as np
+from spoc_b200 import Backend, _lib as L
+from tests import oracle_lib as O
+from tests.gpu_util import Dev, dev_from, gemm
+from tests.test_gpu_gemm import tol
+
+M, N, K, mode = 455, 1149, 6946, L.MODE_TF32
+backend = Backend()
+backend.Device.init()
+device, lib = backend.Device.get(0), L.load()
+a, b = O.fill(M * K, 71, 1), O.fill(K * N, 71, 2)
+# the scratch as large as the first block (256 rows, its k-loop divided within clusters) needs it, and no room behind it to grow into
+A, B, D = dev_from(backend, device, a[:256 * K]), dev_from(backend, device, b), Dev(backend, device, 256 * N)
+assert lib.sb200_set_gemm_tile_n(256) == 0
+gemm(backend, device, mode, 256, N, K, A, B, D)
+assert lib.sb200_set_gemm_tile_n(0) == 0
+fence = [Dev(backend, device, 1 << 20) for _ in range(16)]
+d = np.empty(M * N, np.float32)
+ptr = lambda x: x.ctypes.data_as(C.c_void_p)
+assert lib.sb200_gemm_f32_host(device.id, mode, M, N, K, ptr(a), K, ptr(b), N, ptr(d), N, 1.0, None, 0, 0.0, None, 0) == 0
+err = O.gemm_rel_error(d.reshape(M, N), O.gemm(a, b, M, N, K))
+assert err <= tol(mode, K), err
+"""
+
+
+def test_a_row_block_that_needs_more_scratch_still_finds_b():
+    """The second of this product's row blocks (199 rows) keeps the sums of its divided k-loop in global memory, so it needs more
+    scratch than the first, which left the copy of B there: growing the scratch loses the copy.  A process of its own: whatever
+    ran before it here has grown the scratch already."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", GROWING_SCRATCH], cwd=root, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
