@@ -90,7 +90,6 @@ struct DeviceState {
   cudaEvent_t ws_event = nullptr;
   cudaStream_t ws_last_stream = nullptr;
   bool ws_in_use = false;
-  bool ws_event_due = false;  // the last user was stream 0: its event is recorded when another stream needs it
   // held by a call from the moment it sizes the scratch until its launches are enqueued and its event recorded, so
   // that another host thread cannot free and regrow the scratch under launches that already point into it
   std::mutex scratch_mu;
@@ -325,29 +324,21 @@ int ensure_workspace(DeviceState& d, size_t bytes) {
   return SB200_OK;
 }
 
-// Order of the calls that use the scratch, across streams: `st` waits for the last user when that was another stream.
-// Stream 0 exists as long as the process does, so the event behind its launches is only recorded when another stream asks
-// for it; a stream of the caller's may be destroyed at any time and records its event at once.
+// Order of the calls that use the scratch, across streams: `st` waits for the last user when that was another stream.  Every
+// user records its event at once, stream 0 too: to record it when another stream asks is refused, and spoils the capture, while
+// a blocking stream is being captured into a graph.
 int scratch_acquire(DeviceState& d, cudaStream_t st) {
   std::lock_guard<std::mutex> lock(d.mu);
-  if (!d.ws_in_use || d.ws_last_stream == st) return SB200_OK;
-  if (d.ws_event_due) {
-    if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
-    CU_TRY(cudaEventRecord(d.ws_event, d.ws_last_stream));
-    d.ws_event_due = false;
-  }
-  CU_TRY(cudaStreamWaitEvent(st, d.ws_event, 0));
+  if (d.ws_in_use && d.ws_last_stream != st) CU_TRY(cudaStreamWaitEvent(st, d.ws_event, 0));
   return SB200_OK;
 }
 
 int scratch_release(DeviceState& d, cudaStream_t st) {
   std::lock_guard<std::mutex> lock(d.mu);
-  d.ws_last_stream = st;
-  d.ws_in_use = true;
-  d.ws_event_due = st == nullptr;
-  if (st == nullptr) return SB200_OK;
   if (!d.ws_event) CU_TRY(cudaEventCreateWithFlags(&d.ws_event, cudaEventDisableTiming));
   CU_TRY(cudaEventRecord(d.ws_event, st));
+  d.ws_last_stream = st;
+  d.ws_in_use = true;
   return SB200_OK;
 }
 

@@ -261,6 +261,39 @@ def test_gemm_and_map_calls_can_be_captured_in_a_cuda_graph(backend, device, mod
     assert lib.sb200_device_synchronize(device.id) == 0
 
 
+def test_calls_beside_the_capture_of_a_blocking_stream(backend, device):
+    """While a stream that synchronises with stream 0 is being captured, nothing may be recorded on stream 0.  A product on another
+    stream, behind one on stream 0 with the same scratch, is no part of the capture: it is accepted and leaves it valid."""
+    from cuda.bindings import runtime as rt
+    ok = rt.cudaError_t.cudaSuccess
+    lib = L.load()
+    S = 320
+    A, B, D = (Dev(backend, device, S * S) for _ in range(3))
+    other = backend.Stream.create(device)
+    assert lib.sb200_fill_f32(device.id, 0, A.ptr, S * S, 9, 1, 0, 1.0, 0) == 0
+    assert lib.sb200_fill_f32(device.id, 0, B.ptr, S * S, 9, 2, 0, 1.0, 0) == 0
+    for stream in (other.handle, 0):     # the last user of the scratch is stream 0
+        gemm(backend, device, L.MODE_3XTF32, S, S, S, A, B, D, stream=stream)
+    backend.Device.synchronize(device)
+    want = D.download()
+    D.clear()
+    backend.Device.synchronize(device)
+    for mode in (rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed, rt.cudaStreamCaptureMode.cudaStreamCaptureModeGlobal):
+        gemm(backend, device, L.MODE_3XTF32, S, S, S, A, B, D)
+        err, blocking = rt.cudaStreamCreate()
+        assert err == ok and rt.cudaStreamBeginCapture(blocking, mode)[0] == ok
+        rc = lib.sb200_gemm_f32(device.id, other.handle, L.MODE_3XTF32, S, S, S, A.ptr, S, B.ptr, S, D.ptr, S, 1.0, 0, 0, 0.0, 0, 0)
+        why = lib.sb200_last_error_string() if rc else b""
+        err, graph = rt.cudaStreamEndCapture(blocking)
+        assert rc == 0, why
+        assert err == ok and rt.cudaGraphDestroy(graph)[0] == ok and rt.cudaStreamDestroy(blocking)[0] == ok
+    backend.Device.synchronize(device)
+    assert np.array_equal(D.download().view(np.uint32), want.view(np.uint32))
+    backend.Stream.destroy(other)
+    for x in (A, B, D):
+        x.free()
+
+
 @pytest.mark.parametrize("seed", [1, 2, 3])
 def test_randomised_shapes_strides_tiles_and_epilogues(backend, device, seed):
     """Eighty seeded draws per seed of sizes around the tile edges, aligned and unaligned operands and strides (direct
