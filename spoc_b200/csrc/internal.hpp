@@ -12,17 +12,17 @@ inline bool valid_mode(int mode) {
          mode == SB200_MODE_3XMIXED;
 }
 
-// While one of these lives, the products its thread launches are row blocks of one of `rows` rows: a k-loop is then divided,
-// or not, as it would be for the whole, and the blocks have the bits of the whole.
-class RowBlocksOf {
+// While one of these lives, the products its thread launches are parts (rows, columns or both) of one of `rows` rows and `cols`
+// columns: a k-loop is then divided, or not, as it would be for the whole, and the parts have the bits of the whole.
+class PartsOf {
  public:
-  explicit RowBlocksOf(long long rows);
-  ~RowBlocksOf();
-  RowBlocksOf(const RowBlocksOf&) = delete;
-  RowBlocksOf& operator=(const RowBlocksOf&) = delete;
+  PartsOf(long long rows, long long cols);
+  ~PartsOf();
+  PartsOf(const PartsOf&) = delete;
+  PartsOf& operator=(const PartsOf&) = delete;
 
  private:
-  long long before_;
+  long long rows_before_, cols_before_;
 };
 
 }  // namespace sb200

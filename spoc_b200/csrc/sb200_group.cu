@@ -377,7 +377,7 @@ extern "C" int sb200_gemm_sharded(uint64_t group, int mode, int64_t M, int64_t N
   g->rep_b_bytes = b_count * 4;
   g->rep_bias_src = bias;
   // the row blocks
-  const sb200::RowBlocksOf whole(M);
+  const sb200::PartsOf whole(M, N);
   int64_t first[kMaxGroup], rows[kMaxGroup];
   for (int i = 0; i < n; ++i) split(M, n, i, &first[i], &rows[i]);
   for (int i = 0; i < n && !rc; ++i) {
@@ -484,7 +484,7 @@ void member_main(Group* g, int i, const HostCall* hc, int64_t first, int64_t row
   cudaError_t e = cudaSetDevice(dev);
   if (e != cudaSuccess) return fail_here(set_error(static_cast<int>(e), "cudaSetDevice(%d): %s", dev, cudaGetErrorString(e)));
   const HostCall& c = *hc;
-  const sb200::RowBlocksOf whole(c.M);
+  const sb200::PartsOf whole(c.M, c.N);
   const bool staged_a = sb200::staged_copy_enabled() && c.K > 0 && sb200::host_memory_is_pageable(c.A);
   const bool staged_c = sb200::staged_copy_enabled() && c.C && sb200::host_memory_is_pageable(c.C);
   const bool staged_d = sb200::staged_copy_enabled() && sb200::host_memory_is_pageable(c.D) && c.ldd == c.N;

@@ -528,8 +528,7 @@ constexpr int kMaxSplits = 32;
 // Dividing the k-loop pays when the tiles occupy a fraction of the SMs and k is long; it costs a second launch and the
 // partial results' way through L2 (about 4 TB/s), or within a cluster two barriers and a round of distributed shared memory, and has to win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one
 // of 32 takes 11.1; 40 x 300 x 1200 unaligned 18.7 against 28.8).
-// fixed_splits > 0: the division is given (a row block of a larger product is divided as the whole is, so that it has the
-// same bits).
+// fixed_splits > 0: the division is given (a part of a larger product is divided as the whole is, so that it has the same bits).
 // convert: gemm_convert_kernel's rates (see there) instead of the pair kernel's.
 TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
                        bool convert = false) {
@@ -760,20 +759,24 @@ int stages_of(bool three, int bn, int ctas) {
   return static_cast<int>(fit > 8 ? 8 : fit);
 }
 
-// Set by RowBlocksOf (the host-operand calls, the launches that upload by blocks, partial launches, device groups).
-thread_local long long t_whole_rows = 0;
+// Set by PartsOf (the host-operand calls, the launches that upload by blocks, partial launches, device groups).
+struct Whole {
+  long long rows = 0, cols = 0;
+};
+thread_local Whole t_whole;
+bool part_of_whole(long long M, long long N) { return t_whole.rows > M || t_whole.cols > N; }
 
 int units_of(int ctas, int sm_count) { return ctas == 1 ? sm_count : (sm_count / 2 > 0 ? sm_count / 2 : 1); }
 
 // The fp16 modes: panels always, so a block on its own up to 128 rows.
 TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_count, int* ctas) {
-  auto cut = [&](long long rows, int fixed, int* c) {
+  auto cut = [&](long long rows, long long cols, int fixed, int* c) {
     *c = rows <= GEMM_BM ? 1 : 2;
-    return choose_tiles(rows, N, round_up(K, 64) / 64, *c, units_of(*c, sm_count), three, true, fixed);
+    return choose_tiles(rows, cols, round_up(K, 64) / 64, *c, units_of(*c, sm_count), three, true, fixed);
   };
   int whole_ctas;
-  const int fixed_splits = t_whole_rows > M ? cut(t_whole_rows, 0, &whole_ctas).splits : 0;
-  return cut(M, fixed_splits, ctas);
+  const int fixed_splits = part_of_whole(M, N) ? cut(t_whole.rows, t_whole.cols, 0, &whole_ctas).splits : 0;
+  return cut(M, N, fixed_splits, ctas);
 }
 
 // Row length of the parts of B the direct kernel reads from the scratch.
@@ -781,11 +784,11 @@ long long route_b_pitch(long long N, bool addressable) { return round_up(N, addr
 
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
   int fixed_splits = 0;
-  if (t_whole_rows > M) {
-    const long long whole = t_whole_rows;
-    t_whole_rows = 0;
-    fixed_splits = route_gemm(mode, whole, N, K, addressable, sm_count, whole).splits;
-    t_whole_rows = whole;
+  if (part_of_whole(M, N)) {
+    const Whole whole = t_whole;
+    t_whole = Whole();
+    fixed_splits = route_gemm(mode, whole.rows, whole.cols, K, addressable, sm_count, whole.rows).splits;
+    t_whole = whole;
   }
   GemmRoute r;
   const int variant = gemm_variant_setting();
@@ -1685,6 +1688,7 @@ int launch_gemm_kernel(DeviceState& d, const KernelPlan& plan, const std::vector
   const uint64_t A = s[g.a].ptr, B = s[g.b].ptr, D = s[g.d].ptr, C = g.c >= 0 ? s[g.c].ptr : 0,
                  bias = g.bias >= 0 ? s[g.bias].ptr : 0;
   const int mode = current_mode();
+  const PartsOf whole(M, N);
   if (plan.kind == KIND_GEMM_TILED) {
     if (static_cast<long long>(block[0]) != g.tile || static_cast<long long>(block[1]) != g.tile)
       return fail(SB200_ERR_ARGS, "kernel '%s': block is %ux%u but the kernel's tiles are %dx%d", plan.name.c_str(), block[0],
@@ -1714,7 +1718,6 @@ int launch_gemm_kernel(DeviceState& d, const KernelPlan& plan, const std::vector
   }
   if (pipeline_uploads) return SB200_OK;  // partial launch: as above
   const long long full_rows = covered / N, rest = covered - full_rows * N;
-  const RowBlocksOf whole(M);
   rc = run_gemm(d, st, mode, full_rows, N, K, A, K, B, N, D, N, alpha, C, N, beta, bias, g.act);
   if (!rc && rest != 0) {
     const uint64_t off_a = static_cast<uint64_t>(full_rows) * K * 4, off_d = static_cast<uint64_t>(full_rows) * N * 4;
@@ -1732,7 +1735,7 @@ int launch_gemm_kernel(DeviceState& d, const KernelPlan& plan, const std::vector
 int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M, long long N, long long K, const Slot& a,
                          const Slot& b, const Slot* c, const Slot* bias, const Slot& dd, float alpha, float beta, int act, void* d_host) {
   std::lock_guard<std::mutex> host_call_lock(d.host_call_mu);  // the inbound stream is shared with the host-operand calls
-  const RowBlocksOf whole(M);
+  const PartsOf whole(M, N);
   int src = ensure_pipe_streams(d);
   if (src) return src;
   static const int nblocks = [] {  // row blocks per product (SAREK_B200_PIPE_BLOCKS, 2..64)
@@ -1859,8 +1862,14 @@ int gemm_upload_pipeline(DeviceState& d, cudaStream_t st, int mode, long long M,
 }  // namespace
 
 namespace sb200 {
-RowBlocksOf::RowBlocksOf(long long rows) : before_(t_whole_rows) { t_whole_rows = rows; }
-RowBlocksOf::~RowBlocksOf() { t_whole_rows = before_; }
+PartsOf::PartsOf(long long rows, long long cols) : rows_before_(t_whole.rows), cols_before_(t_whole.cols) {
+  t_whole.rows = rows;
+  t_whole.cols = cols;
+}
+PartsOf::~PartsOf() {
+  t_whole.rows = rows_before_;
+  t_whole.cols = cols_before_;
+}
 
 int set_error(int code, const char* fmt, ...) {
   char buf[1024];
@@ -2990,7 +2999,7 @@ extern "C" int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int6
   int rc = device_ready(dev, &d);
   if (rc) return rc;
   std::lock_guard<std::mutex> host_call_lock(d->host_call_mu);
-  const RowBlocksOf whole(M);
+  const PartsOf whole(M, N);
   if ((rc = ensure_pipe_streams(*d))) return rc;
   // device mirrors, packed: A[M x K], B[K x N], C[M x N] (if any), D[M x N], bias[N]
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };

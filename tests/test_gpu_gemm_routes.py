@@ -10,7 +10,7 @@ import sys
 import numpy as np
 import pytest
 
-from spoc_b200 import _lib as L
+from spoc_b200 import Vector, _lib as L, dims1d, dims2d, run_vectors, sarek_ir
 from tests import oracle_lib as O
 from tests.gpu_util import CANARY, Dev, dev_from, gemm
 from tests.test_gpu_gemm import tol
@@ -191,3 +191,40 @@ def test_a_row_block_that_needs_more_scratch_still_finds_b():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     res = subprocess.run([sys.executable, "-c", GROWING_SCRATCH], cwd=root, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stderr[-2000:]
+
+
+# (form, grid, block, m, n, k): launches that compute the first rows (and part of the next one), or the first rows and columns, of a
+# product whose k-loop is divided
+PARTIAL = [("naive", (37 * 4096 + 100, 1), 1, 64, 4096, 4096), ("naive", (5 * 300 + 7, 1), 1, 40, 300, 2000), ("tiled", (75, 3), 16, 64, 4096, 4096),
+           ("tiled", (2, 2), 16, 1024, 96, 3000)]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("form,grid,side,m,n,k", PARTIAL)
+def test_a_partial_launch_has_the_bits_of_the_whole(backend, device, mode, form, grid, side, m, n, k):
+    ir = (sarek_ir.matmul_tiled_ir if form == "tiled" else sarek_ir.matmul_naive_ir)()
+    assert "splits=1 " not in describe(mode, m, n, k, 1)
+    va, vb = Vector(backend, O.fill(m * k, 72, 1)), Vector(backend, O.fill(k * n, 72, 2))
+    scalars = [("int32", m), ("int32", n), ("int32", k)]
+    block = dims2d(side, side)
+    whole = dims2d((n + 15) // 16, (m + 15) // 16) if form == "tiled" else dims1d(m * n)
+    out = []
+    backend.set_mode(mode)
+    try:
+        for g in (whole, dims2d(*grid)):
+            vd = Vector.create(backend, m * n)
+            run_vectors(backend, device=device, ir=ir, args=[va, vb, vd] + scalars, block=block, grid=g)
+            out.append(vd.to_array().reshape(m, n).copy())
+            vd.free()
+    finally:
+        backend.set_mode(L.MODE_3XTF32)
+        va.free()
+        vb.free()
+    if form == "naive":
+        covered = grid[0]
+        assert np.array_equal(out[1].ravel()[:covered].view(np.uint32), out[0].ravel()[:covered].view(np.uint32))
+        assert not out[1].ravel()[covered:].any()
+    else:
+        rows, cols = min(m, grid[1] * side), min(n, grid[0] * side)
+        assert np.array_equal(out[1][:rows, :cols].view(np.uint32), out[0][:rows, :cols].view(np.uint32))
+        assert not out[1][rows:].any() and not out[1][:, cols:].any()
