@@ -530,8 +530,9 @@ constexpr int kMaxSplits = 32;
 // of 32 takes 11.1; 40 x 300 x 1200 unaligned 18.7 against 28.8).
 // fixed_splits > 0: the division is given (a part of a larger product is divided as the whole is, so that it has the same bits).
 // convert: gemm_convert_kernel's rates (see there) instead of the pair kernel's.
+// no_scratch: divisions within a cluster only, whose partial sums need no memory.
 TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
-                       bool convert = false) {
+                       bool convert = false, bool no_scratch = false) {
   TileShape best;
   const int forced = tile_n_setting();
   double best_cost = 0.0;
@@ -552,6 +553,7 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
       const double charge = bn == 256 ? 1.0 : three ? (kblocks < 128 ? 1.02 : 1.1) : (kblocks < 128 ? 1.1 : 1.4);
       const long long tiles = tiles_m * ((N + bn - 1) / bn);
       const bool in_cluster = split_in_cluster(tiles, sp, ctas, sm_count);
+      if (no_scratch && sp > 1 && !in_cluster) continue;
       if (!fixed_splits && sp > 1 && !in_cluster && three && ctas == 2 && kblocks < static_cast<long long>(sp) * kMinSplitKBlocksThree) continue;
       const long long waves = in_cluster ? 1 : (tiles * sp + units - 1) / units;
       double c = waves * per_item * per_kblock * charge + 5500.0 + 500.0 * (bn / 32) + 800.0 * (waves - 1);
@@ -808,7 +810,10 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   // Read directly a pair wins from 65 rows on; from panels a block on its own serves up to 128 rows when a single block is asked for.
   r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
   const int units = units_of(r.ctas, sm_count);
-  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, convert);
+  // TF32 mode on addressable operands uses no scratch at all: such calls run side by side on any streams, and a graph they were
+  // captured into stays good whatever other calls do to the scratch.  (A part always finds a cut: it has no more tiles than
+  // its whole, or up to twice as many single blocks, for which there is room for more than twice as many clusters.)
+  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, convert, !three && addressable);
   r.tile_n = shape.tile_n;
   r.splits = shape.splits;
   r.src = convert ? SRC_CONVERT : direct ? SRC_DIRECT : SRC_PANELS;

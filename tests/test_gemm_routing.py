@@ -1,5 +1,6 @@
 """How the library routes a product (kernel, tile, scratch, launches) — host logic, no GPU needed."""
 import ctypes as C
+import random
 
 import pytest
 
@@ -43,6 +44,20 @@ def test_operands_tma_cannot_address_go_through_panels():
     # at most 128 rows: the single-CTA kernel from panels, or the pair kernel when it can read the operands directly
     assert describe(L.MODE_TF32, 100, 300, 500, addressable=0)["kernel"] == "single panels"
     assert describe(L.MODE_TF32, 100, 300, 500, addressable=1)["kernel"] == "pair direct"
+
+
+def test_tf32_mode_reads_addressable_operands_without_scratch():
+    """Long k-loops over few tiles among them: their partial sums stay within a cluster, so that calls on different streams, and
+    graphs they were captured into, share nothing."""
+    rng = random.Random(5)
+    shapes = [(46, 1, 4640), (356, 329, 9218), (3420, 1398, 6654), (435, 1897, 8484), (128, 96, 16384), (1, 8, 16384)]
+    shapes += [tuple(int(2 ** rng.uniform(0, 14)) for _ in range(3)) for _ in range(3000)]
+    divided = 0
+    for shape in shapes:
+        d = describe(L.MODE_TF32, *shape)
+        assert d["workspace"] == "0" and d["launches"] == "1", (shape, d)
+        divided += d["splits"] != "1"
+    assert divided > 100
 
 
 def test_degenerate_and_bad_arguments():
