@@ -455,6 +455,11 @@ SB200_API int sb200_profile_gemm_read(int dev, uint64_t *calls, double *prep_ms,
  * returns SB200_ERR_TIMEOUT once, and the device stays usable.  No counterpart in the reference, whose
  * calls are synchronous and carry no device-side waits. */
 SB200_API int sb200_selftest_wait_timeout(int dev, uint32_t limit_ms);
+/* The decision by which the warps of a block leave a work loop together when another role gives up at any moment, also fault-free:
+ * `blocks` blocks (1..4096) of eight such warps go through at most max_items (1..100000) items each, and in block b a
+ * ninth warp gives up after b * step_ns (at most 10000) nanoseconds.  items (device memory, 8 * blocks int32) receives the
+ * number of items of every warp: the same for the warps of a block. */
+SB200_API int sb200_selftest_go_on(int dev, uint64_t items, int blocks, int max_items, uint32_t step_ns);
 
 /* number of kernels this library has launched on this thread's behalf since
  * load (monotonic; used by benchmarks to report launch counts) */

@@ -175,6 +175,36 @@ struct ConvTile {
   }
 };
 
+// The converting warps' barrier behind a work item, and one decision for all of them: whether to go on to the next.  The MMA issuer
+// is no part of the barrier and may give up at any time; if each warp read its flag behind the barrier, some could leave and the
+// others wait for them at the next barrier without end.
+__device__ __forceinline__ bool convert_go_on(bool ok, volatile int* abort_flag) {
+  return barrier_all(1, CONV_WARPS * 32, ok && *abort_flag == 0);
+}
+
+// Exercises that decision: the converting warps of each block go from item to item in different time, warp CONV_WARPS gives up
+// after block * step_ns, and every warp writes the number of its items (at most max_items).  All warps of a block write the same.
+__global__ void go_on_probe_kernel(int* items, int max_items, unsigned int step_ns) {
+  __shared__ int flag;
+  volatile int* abort_flag = &flag;
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) flag = 0;
+  __syncthreads();
+  if (warp == CONV_WARPS) {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < static_cast<uint64_t>(blockIdx.x) * step_ns) {
+    }
+    if ((threadIdx.x & 31) == 0) *abort_flag = 1;
+    return;
+  }
+  int n = 0;
+  for (bool ok = true; ok && n < max_items; ++n) {
+    for (int i = 0; i < ((warp * 5 + n) & 7); ++i) __nanosleep(20);
+    ok = convert_go_on(ok, abort_flag);
+  }
+  if ((threadIdx.x & 31) == 0) items[blockIdx.x * CONV_WARPS + warp] = n;
+}
+
 // IN_CLUSTER: a k-loop divided within a cluster; a form of its own, because what it adds took 0.3 to 0.6 us from the smallest products.
 template <int MODE, int BN, bool VEC, bool IN_CLUSTER>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
@@ -287,8 +317,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
         tc_fence_before_sync();
       }
       // every warp is through with the accumulator and the tiles before the next item's operands arrive
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (*abort_flag) ok = false;  // a wait ran out in some warp: all leave together
+      ok = convert_go_on(ok, abort_flag);
     }
     __syncwarp();
     if constexpr (in_cluster) {

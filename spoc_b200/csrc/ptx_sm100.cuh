@@ -71,6 +71,22 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
+// Barrier `id` of `threads` threads (whole warps) that tells all of them whether every one brought `ok`.
+__device__ __forceinline__ bool barrier_all(int id, int threads, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %3, 0;\n"
+      "barrier.cta.red.and.pred q, %1, %2, p;\n"
+      "selp.b32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(all)
+      : "r"(id), "r"(threads), "r"(static_cast<uint32_t>(ok))
+      : "memory");
+  return all != 0;
+}
+
 // True in exactly one lane of a converged warp, the same one every time.  The roles that a single thread plays (TMA
 // producer, MMA issuer) branch on this and not on `lane == 0`: the compiler then knows that one thread is active and keeps
 // descriptors and addresses in uniform registers, which tcgen05.mma and the bulk-tensor loads take them from.  With

@@ -2788,6 +2788,17 @@ int sb200_selftest_wait_timeout(int dev, uint32_t limit_ms) {
   return launch_check("wait_timeout_probe_kernel");
 }
 
+int sb200_selftest_go_on(int dev, uint64_t items, int blocks, int max_items, uint32_t step_ns) {
+  DeviceState* d;
+  int rc = device_ready(dev, &d);
+  if (rc) return rc;
+  if (!items || blocks < 1 || blocks > 4096 || max_items < 1 || max_items > 100000 || step_ns > 10000)
+    return fail(SB200_ERR_INVALID_VALUE, "blocks must be 1..4096, items 1..100000 and the step at most 10000 ns");
+  if ((rc = check_extent(*d, items, static_cast<uint64_t>(blocks) * CONV_WARPS * 4, "item counts"))) return rc;
+  go_on_probe_kernel<<<blocks, (CONV_WARPS + 1) * 32>>>(as_ptr<int>(items), max_items, step_ns);
+  return launch_check("go_on_probe_kernel");
+}
+
 int sb200_launch_count(uint64_t* count) {
   if (!count) return fail(SB200_ERR_INVALID_VALUE, "null count pointer");
   *count = g_launches.load();

@@ -678,6 +678,25 @@ def test_config_32768_cubed_epilogue_sampled(backend, device):
             backend.Memory.free(x)
 
 
+@pytest.mark.parametrize("blocks,max_items,step_ns", [(1, 5, 0), (600, 100000, 97), (148, 3, 50)])
+def test_warps_leave_a_work_loop_together_whenever_another_gives_up(backend, device, blocks, max_items, step_ns):
+    """The converting warps' decision to go on to the next work item, with the other role giving up between, before and after
+    their barriers: every warp of a block counts the same items, so none waits at a barrier the others have left behind."""
+    lib = L.load()
+    counts = np.zeros(blocks * 8, np.int32)
+    buf = backend.Memory.alloc(device, blocks * 8, np.float32)
+    try:
+        assert lib.sb200_selftest_go_on(device.id, buf.ptr, blocks, max_items, step_ns) == 0
+        assert lib.sb200_memcpy_dtoh(device.id, counts.ctypes.data, buf.ptr, counts.nbytes) == 0
+        per_warp = counts.reshape(blocks, 8)
+        assert np.array_equal(per_warp, np.repeat(per_warp[:, :1], 8, axis=1))
+        assert per_warp.min() >= 1 and per_warp.max() <= max_items
+        if step_ns == 97:
+            assert len(set(per_warp[:, 0])) > 8     # they gave up at many different items
+    finally:
+        backend.Memory.free(buf)
+
+
 def test_bounded_wait_gives_up_cleanly_and_the_device_stays_usable(backend, device):
     """Every device-side wait in the GEMM pipeline is bounded; when one runs out the kernel records it and returns.
     Exercised without any fault: a wait on a barrier nothing signals, limited to 20 ms."""
