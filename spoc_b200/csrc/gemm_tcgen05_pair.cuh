@@ -563,7 +563,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     __syncwarp();
   }
 
-  if (in_cluster) {
+  if (in_cluster && gate_open) {  // a closed gate leaves no partial sums
     cluster_arrive();
     cluster_wait();
     int tm, tn;
