@@ -377,7 +377,9 @@ SB200_API int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int64
                                   const float *A, int64_t lda, const float *B, int64_t ldb,
                                   float *D, int64_t ldd, float alpha, const float *C, int64_t ldc,
                                   float beta, const float *bias, int act);
-/* bytes of library-owned scratch sb200_gemm_f32 needs for these sizes */
+/* bytes of library-owned scratch sb200_gemm_f32 needs for these sizes on the current device (148 SMs when the library has not used
+ * it yet), at most: operands TMA cannot address take more than others.  The calls that cut a product into row blocks may
+ * need somewhat more, because a block may keep partial sums where the whole does not. */
 SB200_API int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64_t *bytes);
 /* how sb200_gemm_f32 would run these sizes on a device with sm_count SMs, as text:
  * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L"

@@ -2584,18 +2584,23 @@ int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64
     return fail(SB200_ERR_INVALID_VALUE, "unknown GEMM mode %d", mode);
   *bytes = 0;
   if (M == 0 || N == 0 || K == 0) return SB200_OK;
-  constexpr int kSms = 148;
+  // the cut of a product, and with it the room for partial sums, depends on the number of SMs
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess)
+    cudaGetLastError();
+  else if (dev >= 0 && dev < kMaxDevices && g_dev[dev].ready.load(std::memory_order_acquire))
+    sms = g_dev[dev].sm_count;
   if (mode == SB200_MODE_3XF16 || mode == SB200_MODE_F16) {
     const bool three = mode == SB200_MODE_3XF16;
     int ctas;
-    const TileShape shape = f16_shape(M, N, K, three, kSms, &ctas);
-    *bytes = gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, kSms);
+    const TileShape shape = f16_shape(M, N, K, three, sms, &ctas);
+    *bytes = round_up(gemm_f16_workspace_need(M, N, K, three), 1024) + partial_bytes(M, N, shape, ctas, sms);
     return SB200_OK;
   }
   // upper bound: which route runs depends on the operands' addresses
   const int plain = mode == SB200_MODE_TF32 ? SB200_MODE_TF32 : SB200_MODE_3XTF32;
   uint64_t most = mode == SB200_MODE_3XMIXED ? gemm_mix_workspace_need(M, N, K) : 0;
-  for (bool addressable : {false, true}) most = std::max<uint64_t>(most, route_gemm(plain, M, N, K, addressable, kSms, M).workspace);
+  for (bool addressable : {false, true}) most = std::max<uint64_t>(most, route_gemm(plain, M, N, K, addressable, sms, M).workspace);
   *bytes = most;
   return SB200_OK;
 }
