@@ -72,7 +72,6 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tile
 struct QuadColumns {  // what the rows of a column quad share
   float bias[4], scale[4];
 };
-template <bool VEC>
 __device__ __forceinline__ QuadColumns quad_columns(const GemmParams& p, int col) {
   QuadColumns q;
 #pragma unroll
@@ -165,7 +164,7 @@ __device__ __forceinline__ void cluster_part_finish(const GemmParams& p, const v
   const int begin = total * share / splits + tid, end = total * (share + 1) / splits;
   const int first_row = begin / QUADS, quad = begin - first_row * QUADS, col = n0 + quad * 4;
   if (col >= p.N) return;
-  const QuadColumns columns = quad_columns<VEC>(p, col);
+  const QuadColumns columns = quad_columns(p, col);
   const uint8_t* own = static_cast<const uint8_t*>(part) + quad * 16;
   constexpr int PITCH = ClusterPart<BN>::kPitch * 4;
   for (int at = begin, row = first_row; at < end; at += BATCH * THREADS, row += BATCH * STEP) {
@@ -610,7 +609,7 @@ __device__ __forceinline__ void reduce_quads(const float* part, long long ld, in
       for (int u = 0; u < AHEAD; ++u) v[u] = src[min(k + u, splits - 1) * step];
       if (k == 0) {
         c = quad_of_c<VEC>(p, row, col);
-        columns = quad_columns<VEC>(p, col);
+        columns = quad_columns(p, col);
         s = v[0];
       }
 #pragma unroll

@@ -104,20 +104,13 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // -------------------------------------------------------------------- TMA
-// 2-D tiled bulk-tensor load global -> this block's shared memory, completing
-// `bytes` on the mbarrier.  x is the innermost coordinate (elements) and must
-// make x * 4 a multiple of 16 bytes; callers pass multiples of 32.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar, int32_t x, int32_t y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
-// The same load carrying an L2 eviction policy (from l2_policy below).
+// 2-D tiled bulk-tensor load global -> this block's shared memory, completing its bytes on the mbarrier, with an L2 eviction
+// policy (from l2_policy below).  x is the innermost coordinate (elements) and must make x times the element size a multiple
+// of 16 bytes; callers pass multiples of 32.
 __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar, int32_t x, int32_t y,
                                                  uint64_t policy) {
   asm volatile(
@@ -246,16 +239,8 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// TMA load whose completion bytes are counted on an mbarrier of either block
-// of the pair (`bar` is a shared::cluster address); data lands in this block.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar_cluster_addr,
-                                                 int32_t x, int32_t y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
-      : "memory");
-}
-// The same load carrying an L2 eviction policy (from l2_policy below) for the lines it brings in.
+// TMA load whose completion bytes are counted on an mbarrier of either block of the pair (`bar` is a shared::cluster address), with
+// an L2 eviction policy (from l2_policy below) for the lines it brings in; data lands in this block.
 __device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar_cluster_addr,
                                                       int32_t x, int32_t y, uint64_t policy) {
   asm volatile(
