@@ -319,6 +319,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       // every warp is through with the accumulator and the tiles before the next item's operands arrive
       ok = convert_go_on(ok, abort_flag);
     }
+    if (!ok && elect_one()) wait_for_copies();  // tiles of C
     __syncwarp();
     if constexpr (in_cluster) {
       cluster_arrive();

@@ -416,13 +416,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
         for (int e = my_tiles * epochs_per_tile; e < most_tiles * epochs_per_tile; ++e)
           atomicAdd(p.epoch_ctr + (e % PAIR_EPOCH_RING), 1u);
       }
-      if (!ok) {
-        // Give loads that are still in flight a bounded chance to land before the block retires: a stage whose load was
-        // issued completes its full barrier regardless of the consumer.
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 2000000ull) {
-        }
-      }
+      if (!ok) wait_for_copies();  // operand tiles: a load that was issued completes regardless of its consumer
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -558,7 +552,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       }
     }
     __syncwarp();
-    if (elect_one()) bulk_wait_read<0>();  // the tiles must outlive the stores that read them
+    if (elect_one()) {
+      bulk_wait_read<0>();           // the tiles must outlive the stores that read them
+      if (!ok) wait_for_copies();  // tiles of C
+    }
     __syncwarp();
   }
 

@@ -71,6 +71,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
+// For a role that gives up: a bounded time in which copies still in flight land, so that none writes to the shared memory of a
+// block that has retired.
+__device__ __forceinline__ void wait_for_copies() {
+  const uint64_t t0 = global_timer_ns();
+  while (global_timer_ns() - t0 < 2000000ull) {
+  }
+}
+
 // Barrier `id` of `threads` threads (whole warps) that tells all of them whether every one brought `ok`.
 __device__ __forceinline__ bool barrier_all(int id, int threads, bool ok) {
   uint32_t all;
