@@ -382,9 +382,12 @@ SB200_API int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int64
  * need somewhat more, because a block may keep partial sums where the whole does not. */
 SB200_API int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64_t *bytes);
 /* how sb200_gemm_f32 would run these sizes on a device with sm_count SMs, as text:
- * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L"
- * (L: kernels' passes, the preparation of A and of B counted apart although they may share a launch).
- * addressable = operands 16-byte aligned with row strides that are multiples of 4 floats.  Needs no GPU. */
+ * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L operands=O kernels=N"
+ * (fp16 modes: "fp16-panels", mixed mode: "mixed" without splits, for the second word).  N is the number of kernels the call launches
+ * and O what becomes of A and B: direct (read where they lie, beside panels of their low parts in 3xTF32 mode), copied (row by row
+ * first, beside the same panels), converted (in registers on their way), panels (written in full) or mixed.  The second word says
+ * "panels" for every product of operands that are not addressable, and L counts their preparation as two passes, although one
+ * launch makes both.  addressable = operands 16-byte aligned with row strides that are multiples of 4 floats.  Needs no GPU. */
 SB200_API int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressable, int sm_count,
                                   char *out, int outlen);
 

@@ -2619,11 +2619,13 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
     const int units = units_of(ctas, sm_count);
     const long long tiles = ((M + 128 * ctas - 1) / (128 * ctas)) * ((N + shape.tile_n - 1) / shape.tile_n);
     char fb[256];
-    snprintf(fb, sizeof fb, "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
+    const int launches = (f16_prepared_at_once(M, N, K) ? 2 : 3) +
+                         (shape.splits > 1 && !split_in_cluster(tiles, shape.splits, ctas, sm_count) ? 1 : 0);
+    snprintf(fb, sizeof fb,
+             "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=panels kernels=%d",
              ctas == 1 ? "single" : "pair", 128 * ctas, shape.tile_n, stages_of(three, shape.tile_n, ctas), tiles,
              (tiles * shape.splits + units - 1) / units, shape.splits,
-             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count),
-             4 + (shape.splits > 1 && !split_in_cluster(tiles, shape.splits, ctas, sm_count) ? 1 : 0) - (f16_prepared_at_once(M, N, K) ? 2 : 1));
+             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count), launches, launches);
     return copy_out(fb, out, outlen);
   }
   if (mode == SB200_MODE_3XMIXED) {
@@ -2633,22 +2635,23 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
       const long long tiles = ((M + PAIR_BM - 1) / PAIR_BM) * ((N + tn - 1) / tn);
       const int stages = stages_of(true, tn, 2);
       char fb[256];
-      snprintf(fb, sizeof fb, "pair mixed tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu launches=7", PAIR_BM, tn, stages,
-               tiles, (tiles + clusters - 1) / clusters, gemm_mix_workspace_need(M, N, K));
+      snprintf(fb, sizeof fb, "pair mixed tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu launches=7 operands=mixed kernels=6",
+               PAIR_BM, tn, stages, tiles, (tiles + clusters - 1) / clusters, gemm_mix_workspace_need(M, N, K));
       return copy_out(fb, out, outlen);
     }
     mode = SB200_MODE_3XTF32;
   }
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
-  // "panels" for operands TMA cannot address also when they are copied or converted on their way (converted: launches=1, no
-  // scratch for operands); the passes over A and B are counted apart although one launch makes both
+  // the second word and `launches` speak of addressability and of passes; `operands` and `kernels` say what runs
   const bool apart = r.src == SRC_PANELS || (r.src == SRC_DIRECT && !addressable);
-  const int launches = (apart ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) +
-                       (r.splits > 1 && !split_in_cluster(r.tiles, r.splits, r.ctas, sm_count) ? 1 : 0);
-  snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d",
-           r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles, r.waves,
-           r.splits, r.workspace, launches);
+  const int reduction = r.splits > 1 && !split_in_cluster(r.tiles, r.splits, r.ctas, sm_count) ? 1 : 0;
+  const int launches = (apart ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + reduction;
+  const int kernels = (apart || (r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32) ? 2 : 1) + reduction;
+  const char* operands = r.src == SRC_CONVERT ? "converted" : r.src == SRC_PANELS ? "panels" : addressable ? "direct" : "copied";
+  snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=%s kernels=%d",
+           r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
+           r.waves, r.splits, r.workspace, launches, operands, kernels);
   return copy_out(buf, out, outlen);
 }
 

@@ -228,3 +228,31 @@ def test_a_partial_launch_has_the_bits_of_the_whole(backend, device, mode, form,
         rows, cols = min(m, grid[1] * side), min(n, grid[0] * side)
         assert np.array_equal(out[1][:rows, :cols].view(np.uint32), out[0][:rows, :cols].view(np.uint32))
         assert not out[1][rows:].any() and not out[1][:, cols:].any()
+
+
+# (mode, M, N, K, aligned, how the operands are read): converted, read in place, copied, panels in one launch and in two, with the
+# k-loop whole, divided within clusters and divided through global memory
+KERNELS = [(L.MODE_3XTF32, 64, 64, 64, True, "converted"), (L.MODE_3XTF32, 64, 8192, 8192, True, "converted"), (L.MODE_TF32, 65, 33, 100, False, "converted"),
+           (L.MODE_3XTF32, 512, 512, 512, True, "direct"), (L.MODE_TF32, 512, 512, 512, True, "direct"), (L.MODE_TF32, 128, 96, 4096, True, "direct"),
+           (L.MODE_3XTF32, 700, 900, 1000, False, "copied"), (L.MODE_TF32, 455, 1149, 6946, False, "copied"), (L.MODE_3XF16, 300, 200, 500, True, "panels"),
+           (L.MODE_F16, 300, 200, 5000, False, "panels"), (L.MODE_3XMIXED, 512, 512, 512, True, "mixed")]
+
+
+@pytest.mark.parametrize("mode,M,N,K,aligned,operands", KERNELS)
+def test_the_described_kernels_are_the_ones_launched(backend, device, mode, M, N, K, aligned, operands):
+    off = 0 if aligned else 1
+    A, B, D = Dev(backend, device, M * K, offset=off), Dev(backend, device, K * N, offset=off), Dev(backend, device, M * N)
+    lib = L.load()
+    lib.sb200_set_mixed_min_macs(1 << 20)
+    try:
+        out = C.create_string_buffer(256)
+        assert lib.sb200_gemm_describe(mode, M, N, K, int(aligned), device.sm_count, out, 256) == 0
+        text = out.value.decode()
+        before = backend.launch_count()
+        gemm(backend, device, mode, M, N, K, A, B, D)
+        assert f" operands={operands} " in text and text.endswith(f" kernels={backend.launch_count() - before}"), text
+        backend.Device.synchronize(device)
+    finally:
+        lib.sb200_set_mixed_min_macs(0)
+        for x in (A, B, D):
+            x.free()
