@@ -351,7 +351,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
     prep_ms = prof["prep_ms"] / max(prof["calls"], 1)
     achieved = flops_step / (main_ms * 1e-3) / 1e12
     roofline = {
-        "bound": "tensor", "kernel": "gemm_pair_kernel<3, true>", "achieved": achieved, "peak": tf32_peak, "unit": "TFLOP/s",
+        "bound": "tensor", "kernel": "gemm_pair_kernel<3, SRC_DIRECT, 256, 2>", "achieved": achieved, "peak": tf32_peak, "unit": "TFLOP/s",
         "frac": achieved / tf32_peak,
         # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this kernel at this size, taken from an
         # ncu capture of this same kernel and size (a profiler figure, not measured in this run)
@@ -376,7 +376,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
     main2 = prof2["main_ms"] / max(prof2["calls"], 1)
     tf32_mode = {
         "value": world * flops_step / (ms2 / s2 * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": ms2 / s2,
-        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<1, true> (operands read directly, no preparation)", "achieved": flops_step / (main2 * 1e-3) / 1e12,
+        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<1, SRC_DIRECT, 256, 2> (operands read directly, no preparation)", "achieved": flops_step / (main2 * 1e-3) / 1e12,
                      "peak": tf32_peak, "unit": "TFLOP/s", "frac": flops_step / (main2 * 1e-3) / 1e12 / tf32_peak,
                      "peak_source": roofline["peak_source"],
                      "frac_of_burst_peak": flops_step / (main2 * 1e-3) / 1e12 / burst_peak,
@@ -392,7 +392,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         "note": "SB200_MODE_3XF16: operands scaled by powers of two and split hi + lo in fp16, three kind::f16 MMAs per k-step; "
                 "parity bound 1e-5*sqrt(K) as for 3xTF32 (tests/test_gpu_gemm.py::test_f16_split_*); not the headline because its "
                 "accuracy depends on the dynamic range inside each matrix",
-        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<4, false> (fp16 panels)", "achieved": flops_step / (main_h * 1e-3) / 1e12,
+        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<4, SRC_PANELS, 256, 2> (fp16 panels)", "achieved": flops_step / (main_h * 1e-3) / 1e12,
                      "peak": f16_peak, "unit": "TFLOP/s", "frac": flops_step / (main_h * 1e-3) / 1e12 / f16_peak,
                      "mma_frac": 3.0 * flops_step / (main_h * 1e-3) / 1e12 / f16_peak,
                      "peak_source": f"{peaks['source']}: dense bf16/fp16 library GEMM, {'sustained' if sustained else 'burst'}",
@@ -403,7 +403,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         "value": world * flops_step / (ms_q / s5 * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": ms_q / s5,
         "note": "SB200_MODE_F16: one kind::f16 MMA per k-step on power-of-two-scaled fp16 panels; TF32 mode's 11 significant bits "
                 "and error bound (2e-3) at the fp16 tensor rate",
-        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<2, false> (fp16 panels)", "achieved": flops_step / (main_q * 1e-3) / 1e12,
+        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<2, SRC_PANELS, 256, 2> (fp16 panels)", "achieved": flops_step / (main_q * 1e-3) / 1e12,
                      "peak": f16_peak, "unit": "TFLOP/s", "frac": flops_step / (main_q * 1e-3) / 1e12 / f16_peak,
                      "peak_source": f16_split_mode["roofline"]["peak_source"], "kernel_ms": main_q,
                      "prep_ms": prof_q["prep_ms"] / max(prof_q["calls"], 1)}}
@@ -416,7 +416,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
                 "with one power-of-two scale per matrix, the accumulated cross terms rescaled inside the tensor core "
                 "(scale-input-d); the error of 3xTF32 for elements within 2^29 of their matrix's largest "
                 "(tests/test_gpu_gemm_mixed.py); kernel_ms covers the mixed kernel and the two gated 3xTF32 launches behind it",
-        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<5, true>", "achieved": flops_step / (main_x * 1e-3) / 1e12,
+        "roofline": {"bound": "tensor", "kernel": "gemm_pair_kernel<5, SRC_DIRECT, 256, 2>", "achieved": flops_step / (main_x * 1e-3) / 1e12,
                      "peak": tf32_peak, "unit": "TFLOP/s", "frac": flops_step / (main_x * 1e-3) / 1e12 / tf32_peak,
                      "mma_frac": 2.0 * flops_step / (main_x * 1e-3) / 1e12 / tf32_peak,
                      "peak_source": roofline["peak_source"], "kernel_ms": main_x,

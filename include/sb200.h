@@ -148,9 +148,10 @@ SB200_API int sb200_host_alloc(uint64_t bytes, void **ptr);
 SB200_API int sb200_host_free(void *ptr);
 /* Pin host memory the caller owns, in place (cudaHostRegister / cudaHostUnregister): later copies from or to it run at
  * the pinned rate (55 GB/s instead of the staged 37-50) and can overlap.  For the owner of a long-lived host array
- * — a Vector over a Bigarray (sarek/core/Vector_storage.ml:18-36), which the plugin registers on its second large
- * transfer and unregisters when the vector is freed.  The range must stay allocated until it is unregistered; both
- * calls are idempotent.  No counterpart in the reference, whose transfers are plain synchronous copies. */
+ * — a Vector over a Bigarray (sarek/core/Vector_storage.ml:18-36), which the plugins register on its second large
+ * transfer and unregister when the vector is freed.  The range must stay allocated until it is unregistered; both
+ * calls are idempotent.  A range that is not page-locked as a whole but shares pages with somebody's registration is
+ * not pinned, and the call says so with an error.  No counterpart in the reference, whose transfers are plain synchronous copies. */
 SB200_API int sb200_host_register(void *ptr, uint64_t bytes);
 SB200_API int sb200_host_unregister(void *ptr);
 
@@ -260,12 +261,14 @@ SB200_API int sb200_ir_fuse_pipeline_as(const char *const *kernels, int count, i
  * (benchmarks/bench_matrix_mul.ml:55-73, bench_matrix_mul_tiled.ml:55-94).
  * Operands that lie inside buffers from sb200_mem_alloc are checked against the end of their buffer
  * (SB200_ERR_BOUNDS, nothing is launched); memory from other allocators is taken at the caller's word.
- * Calls may be issued on any streams of the device: those that use the library's scratch (3xTF32 mode, or operands
- * TMA cannot address as they lie) are ordered against each other across streams by the library, the others run
- * concurrently.
+ * Calls may be issued on any streams of the device: those that use the library's scratch (workspace in
+ * sb200_gemm_describe: every mode but TF32, and operands TMA cannot address as they lie) are ordered against each other
+ * across streams by the library, the others run concurrently.
  * Once a first call with the same sizes has sized the library's scratch, a call enqueues nothing but kernel launches
- * (the GEMM launch carries the programmatic-stream-serialization attribute), so it can be captured into a CUDA graph
- * together with the map operators and replayed (tests/test_gpu_gemm.py). */
+ * (which carry the programmatic-stream-serialization attribute), so it can be captured into a CUDA graph
+ * together with the map operators and replayed (tests/test_gpu_gemm.py).  A graph of calls that use the scratch holds its
+ * address: capture it again when a larger call has grown the scratch since, and replay no two such graphs side by side.
+ * TF32 calls on addressable operands hold nothing. */
 SB200_API int sb200_gemm_f32(int dev, uint64_t stream, int mode,
                              int64_t M, int64_t N, int64_t K,
                              uint64_t A, int64_t lda, uint64_t B, int64_t ldb,
@@ -403,18 +406,17 @@ SB200_API int sb200_chain_triad_square_f32(int dev, uint64_t stream, uint64_t d,
  * (also read once from the environment variable SAREK_B200_MODE=3xtf32|tf32|3xf16|f16) */
 SB200_API int sb200_set_mode(int mode);
 SB200_API int sb200_get_mode(int *mode);
-/* which tensor-core kernel sb200_gemm_f32 launches: 0 = automatic (CTA pairs on
- * 256-row tiles when M > 128 or when the operands are 16-byte aligned with row
- * strides that are multiples of 4 floats, so that the kernel reads them directly;
- * else single-CTA 128x256 tiles fed from prepared panels), 1 = always
- * single-CTA tiles, 2 = always CTA pairs, 3 = CTA pairs fed from prepared
- * operand panels even where TF32 mode could read the caller's matrices
- * directly.  Also SAREK_B200_GEMM=single|pair|pair-panels.  All variants round
- * operands to TF32 the same way (nearest-even) and sum k ascending, so their
- * results agree to the last bit. */
+/* which tensor-core kernel sb200_gemm_f32 launches: 0 = automatic (CTA pairs on 256-row tiles; single CTAs on 128-row
+ * tiles for up to 64 rows, 128 in the fp16 modes; for few rows and for small products a kernel that converts the operands
+ * in registers; k-loops divided where tiles leave SMs idle), 1 = always single-CTA tiles fed from prepared panels, 2 =
+ * always CTA pairs, 3 = CTA pairs fed from prepared operand panels even where TF32 mode could read the caller's matrices
+ * directly.  Also SAREK_B200_GEMM=single|pair|pair-panels.  All variants round operands to TF32 the same way
+ * (nearest-even) and sum k ascending, so their results agree to the last bit unless the automatic choice divides the
+ * k-loop (splits in sb200_gemm_describe): its partial sums are then added in order of k. */
 SB200_API int sb200_set_gemm_variant(int variant);
-/* tile columns of the CTA-pair kernel: 0 = automatic (256, or 128 / 64 for problems with too few 256-column
- * tiles to occupy the SMs), else 64, 128 or 256.  Also SAREK_B200_TILE_N.  Results do not depend on it. */
+/* tile columns: 0 = automatic (256, or 192, 128 or 64 for problems with too few 256-column tiles to occupy the SMs or
+ * with a fuller last wave of narrower ones; 192 in the three-term modes), else 64, 128 or 256.  Also SAREK_B200_TILE_N.
+ * A forced width leaves every k-loop undivided; the width itself changes no result. */
 SB200_API int sb200_set_gemm_tile_n(int tile_n);
 /* The soft lockstep of the CTA-pair kernel: every 64 stages of the k-loop each pair counts itself into an epoch counter
  * in global memory and waits, 4 us at most and then regardless, for the other pairs of the launch, so that the pairs of a

@@ -205,7 +205,7 @@ __global__ void go_on_probe_kernel(int* items, int max_items, unsigned int step_
   if ((threadIdx.x & 31) == 0) items[blockIdx.x * CONV_WARPS + warp] = n;
 }
 
-// IN_CLUSTER: a k-loop divided within a cluster; a form of its own, because what it adds took 0.3 to 0.6 us from the smallest products.
+// IN_CLUSTER: a k-loop divided within a cluster; a form of its own, because what it adds cost the smallest products 0.3 to 0.6 us.
 template <int MODE, int BN, bool VEC, bool IN_CLUSTER>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
 gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c,

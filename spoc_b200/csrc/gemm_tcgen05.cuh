@@ -661,8 +661,9 @@ __device__ __forceinline__ void scan_b_f16(const F16ScanB& j, unsigned int block
 
 // First preparation launch of the fp16 modes: the column maxima of B by runs of rows (blocks [0, blocks_b), in front because they
 // take longest), and A's panels.  A block loads its rows, reduces and stores, so half of the blocks of an SM are loading at a
-// time: three to five of them keep the loads in flight that HBM needs (two: 3 TB/s at 8192^2).  (Two launches and a memset fewer than a pass each; the maxima need no atomics.  The column scan alone took 21 us of
-// the 50 a 2048^3 product's preparation took, on 64 blocks.)
+// time: three to five of them keep the loads in flight that HBM needs (two: 3 TB/s at 8192^2).  (Two launches and a memset fewer
+// than a pass each; the maxima need no atomics.  The column scan alone took 21 us of the 50 a 2048^3 product's preparation
+// took, on 64 blocks.)
 template <int TPR, int HOLD>
 __global__ void __launch_bounds__(256, HOLD == 4 ? 5 : 3) prep_f16_first_kernel(const F16PrepA a, const F16ScanB b, int blocks_b) {
   __shared__ unsigned int smem[8 * 128];
@@ -752,9 +753,10 @@ __global__ void __launch_bounds__(256) prep_b_f16_kernel(const float* B, long lo
 // columns.  Each block reads its run of rows_per_block (a multiple of 64) rows of the strip once into shared memory, the
 // cluster agrees on the columns' largest magnitudes through distributed shared memory, and each block scales, splits and writes
 // its run, as prep_b_f16_kernel does.  The other blocks take A's rows.  Bound by HBM: A and B are read once, where the two
-// launches above read B twice, one behind the other.  The shared memory, which A's blocks of the launch hold too, sets the limit of K:
-// 64 KiB a block at 4096, three blocks an SM.  Whole operator, three-term and one-term mode: 1024^3 22.5 -> 17.9 and 19.6 -> 14.7 us,
-// 2048^3 65.4 -> 60.2 and 44.2 -> 40.0, 64 x 4096 x 4096 68.7 -> 55.7 and 55.6 -> 42.5, 64^3 12.1 -> 9.7.
+// launches above read B twice, one behind the other.  The shared memory, which A's blocks of the launch hold too, sets the limit of
+// K: 64 KiB a block at 4096, three blocks an SM.  Whole operator without an epilogue, three-term and one-term mode: 1024^3 22.5 ->
+// 17.9 and 19.6 -> 14.7 us, 2048^3 65.4 -> 60.2 and 44.2 -> 40.0, 64 x 4096 x 4096 68.7 -> 55.7 and 55.6 -> 42.5, 64^3 12.1 -> 9.7.
+// The launch alone: 14.5 us for 2048^3 (10.2 for its bytes at the copy rate), 59 for 4096^3 (41).
 constexpr int F16_ONE_MAX_K = 4096, F16_ONE_BLOCKS = 8, F16_ONE_COLS = 32, F16_ONE_PITCH = 33;
 struct F16WholeB {
   const float* src;

@@ -131,8 +131,9 @@ __device__ __forceinline__ void add_to(float4& s, const float4& v) {
 // A k-loop divided among the blocks (pairs) of one cluster (p.cluster_splits > 1).  Each block leaves the partial sums of its
 // 128 rows and BN columns in its operand ring, which is idle once the accumulator is complete; behind a cluster barrier every
 // block adds up a share of the rows' quads from all of them, in order of k, and finishes it.  Bound by the peers' shared memory,
-// which delivers about 14 bytes a cycle and SM with the loads of several quads in flight (2 ns a quad).  Against partial results in
-// global memory and a second launch: 64 x 4096 x 4096 TF32 20.4 -> 17.5 us, 256 x 512 x 1024 3xTF32 15.2 -> 12.3 us, TF32 10.0 -> 8.0.
+// which delivers about 14 bytes a cycle and SM with the loads of several quads in flight (2 ns a quad).  Against partial results
+// in global memory and a second launch, without an epilogue and on operands in L2: 64 x 4096 x 4096 TF32 20.4 -> 17.5 us (with C,
+// bias and clamp, operands in HBM 19.9), 256 x 512 x 1024 3xTF32 15.2 -> 12.3 us, TF32 10.0 -> 8.0.
 template <int BN>
 struct ClusterPart {
   static constexpr int kPitch = BN + 4;  // floats per row: consecutive rows start four banks apart

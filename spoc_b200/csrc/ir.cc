@@ -976,10 +976,10 @@ std::string block_reduce_source(const KernelPlan& plan, const GenericMap& gm, co
   o << "  const int lane = threadIdx.x & 31;\n";
   o << "  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;\n";
   o << "  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;\n";
-  // a warp's segment: all of its elements are loaded before the first is used.  Of one
-  // input, whole segments take a path without bounds, whose 64-bit comparisons are a third of the instructions there (sum of
-  // 5e7: 35.3 -> 32.3 us, floor 30.6); with two inputs HBM is the bound and the bounds pace the streams (dot of 5e7: 61.4 us with
-  // them, 62.8 to 70 without, whatever the grid; floor 61.2).
+  // a warp's segment: all of its elements are loaded before the first is used.  Of one input, whole segments take a path without
+  // bounds, whose 64-bit comparisons are a third of the instructions there (sum of 5e7: 35.3 -> 32.3 us, floor 30.6); with two
+  // inputs HBM is the bound and the bounds pace the streams (dot of 5e7 on one GPU: 61.4 us with them, 62.8 to 70 without,
+  // whatever the grid; 62.3 and 64.5 with them on others; floor 61.2).
   auto segment = [&](bool whole) {
     for (size_t i = 0; i < ni; ++i) o << "      float a" << i << "[PER];\n";
     o << "#pragma unroll\n      for (int j = 0; j < PER; ++j) {\n        const long long g = seg * B + lane + 32 * j;\n";

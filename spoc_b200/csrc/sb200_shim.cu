@@ -419,7 +419,8 @@ void derive_params(GemmParams* gp) {
 }
 
 // Tensor maps of D and C for the epilogue that moves them by TMA; sets gp->tma_epilogue when it applies: 16-byte aligned
-// matrices and row strides, N a multiple of 4 (a store clips its columns at 16-byte granularity only), no replicas.  Otherwise the maps are left as `filler`.
+// matrices and row strides, N a multiple of 4 (a store clips its columns at 16-byte granularity only), no replicas.  Otherwise
+// the maps are left as `filler`.
 void epilogue_maps(GemmParams* gp, const CUtensorMap& filler, CUtensorMap* map_d, CUtensorMap* map_c) {
   *map_d = filler;
   *map_c = filler;
@@ -434,8 +435,8 @@ void epilogue_maps(GemmParams* gp, const CUtensorMap& filler, CUtensorMap* map_d
 // The epoch counters for one launch of the CTA-pair kernel, zeroed on `st` — or null when the lockstep is off: k-loops
 // below 128 stages (K < 4096: two epochs at most, nothing to hold together), SAREK_B200_LOCKSTEP=0, or no memory for the
 // rings.  Measured in the sustained loop at 8192^3: 245 against 221-227 TFLOP/s in alternating runs on one box, the SM
-// clock under the power cap 1400 against 1267-1305 MHz, because the pairs that stay together re-read less from DRAM.  Eight rings are handed out in turn so that launches in flight on several streams rarely share one
-// (sharing only blunts the hint).
+// clock under the power cap 1400 against 1267-1305 MHz, because the pairs that stay together re-read less from DRAM.  Eight rings
+// are handed out in turn so that launches in flight on several streams rarely share one (sharing only blunts the hint).
 std::atomic<int> g_lockstep{-2};  // -2 = not yet read from the environment; -1 by k-loop length, 0 off, 1 always
 
 unsigned int* next_epoch_ring(DeviceState& d, cudaStream_t st, long long stages_per_tile, bool by_default = true) {
@@ -525,12 +526,15 @@ constexpr int kMaxSplits = 32;
 // does when there are fewer 256-column tiles than pairs, or when its last wave is fuller (4096 x 4096 x 1024 in 3xTF32: 3.5
 // waves of 256 columns 154 us, 6.9 waves of 128 columns 143 us).  192 columns serve the three-MMA modes only.  Fixed: launch,
 // set-up, pipeline fill, and 500 ns per 32 columns of epilogue that nothing overlaps.
-// Dividing the k-loop pays when the tiles occupy a fraction of the SMs and k is long; it costs a second launch and the
-// partial results' way through L2 (about 4 TB/s), or within a cluster two barriers and a round of distributed shared memory, and has to win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one
-// of 32 takes 11.1; 40 x 300 x 1200 unaligned 18.7 against 28.8).
+// Dividing the k-loop pays when the tiles occupy a fraction of the SMs and k is long; it costs a second launch and the partial
+// results' way through L2 (about 4 TB/s), or within a cluster two barriers and a round of distributed shared memory, and has to
+// win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one of 32 takes 11.1; 40 x 300 x 1200
+// unaligned 18.7 against 28.8).
 // fixed_splits > 0: the division is given (a part of a larger product is divided as the whole is, so that it has the same bits).
-// convert: gemm_convert_kernel's rates (see there) instead of the pair kernel's.
-// no_scratch: divisions within a cluster only, whose partial sums need no memory.
+// convert: gemm_convert_kernel's rates instead of the pair kernel's: in 3xTF32 between those of quads and of single elements (1060
+// and 1430 ns at 128 columns, 790 and 1180 at 64), since one choice serves both.
+// no_scratch: divisions within a cluster only, whose partial sums need no memory (TF32, 64 x 512 x 16384 18.8 us so and 15.5 with
+// 29 items through memory, 666 x 8 x 9632 19.5 and 13.0, 128 x 96 x 16384 28.2 and 13.7; most shapes within 10 %).
 TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
                        bool convert = false, bool no_scratch = false) {
   TileShape best;
@@ -745,14 +749,20 @@ int gemm_variant_setting() {
   return variant;
 }
 
-// Products of at most this many rows are computed by blocks on their own: the second block of a pair would only see rows
-// past the end.
+// Products of at most this many rows are computed by blocks on their own (the fp16 modes: f16_shape): the second block of a pair
+// would only see rows past the end.  The reason holds up to 128 rows, and so does the gain: n = k = 4096 in TF32, 64 rows 18.9
+// us; 65 rows 27.3 by pairs and 18.5 by single blocks, 128 rows 27.1 and 18.9; in 3xTF32 62.6 and 44.5, 65.3 and 45.0 (1024 x 1024:
+// 9.4 and 7.9, 11.3 and 8.3; 14.0 both, 15.1 and 14.3).  The line is where the forms were first told apart.
 constexpr long long kSingleRows = 64;
-// Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands.
+// Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands.  Converted and
+// prepared by a launch in front, 3xTF32, us: addressable 100 x 64 x 100 7.6 and 8.8, 192^3 9.4 and 8.9, 256^3 11.3 and 9.8; unaligned
+// 128^3 9.0 and 8.7 (TF32 6.9 and 8.5), 256^3 13.9 and 10.3, 448^3 22.9 and 12.4, 576^3 17.5 and 14.5.  So both are even near
+// 2^22; the second line was drawn when unaligned operands still went through transposed panels (512^3 about even then).
 constexpr double kConvertMacs = 16777216.0;              // 2^24
 constexpr double kConvertMacsUnaligned = 134217728.0;    // 2^27
-// In TF32 mode, where aligned operands need no preparation, it is the shorter way for k-loops of a few k-blocks only: no operand maps
-// to encode and fetch (64 x 64 x 128 with the epilogue 7.0 us by a pair, 6.5 so; it loses 0.5 us a k-block on the device).
+// In TF32 mode, where aligned operands need no preparation, it is the shorter way for k-loops of a few k-blocks only: no operand
+// maps to encode and fetch, but 0.5 us more a k-block on the device.  Converted and by gemm_pair_kernel, us: 64 x 64 x 96 5.2 and 5.6,
+// x 128 5.4 and 5.6; 64 x 1024 x 96 5.3 and 5.6, x 128 6.1 and 5.6; 512 x 256 x 64 5.3 and 5.6, x 96 6.1 and 5.8.
 constexpr long long kConvertKOneTerm = 128;
 
 int stages_of(bool three, int bn, int ctas) {
@@ -801,13 +811,12 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   const bool direct = variant == 0 || (variant == 2 && addressable);
   const long long kp = round_up(K, GEMM_BK);
   // One launch that converts the operands on their way (gemm_convert_kernel): few rows in 3xTF32, where panels of B would
-  // triple the traffic, and any mode's few rows of matrices TMA cannot address; and products so small that the launches that
-  // would prepare panels weigh more than the pair kernel's faster tiles give (aligned: 256^3 is about even; unaligned: 512^3).
+  // triple the traffic, and any mode's few rows of matrices TMA cannot address; and products so small that the launch that
+  // would prepare operands weighs more than the pair kernel's faster tiles give (kConvertMacs).
   const double macs = static_cast<double>(M) * N * K;
   const bool convert = variant == 0 && tile_n_setting() != 256 &&
                        (addressable ? (three ? M <= kSingleRows || macs < kConvertMacs : K <= kConvertKOneTerm && macs < kConvertMacs)
                                     : M <= kSingleRows || macs < kConvertMacsUnaligned);
-  // Read directly a pair wins from 65 rows on; from panels a block on its own serves up to 128 rows when a single block is asked for.
   r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
   const int units = units_of(r.ctas, sm_count);
   // TF32 mode on addressable operands uses no scratch at all: such calls run side by side on any streams, and a graph they were
@@ -1009,9 +1018,10 @@ long long f16_scan_rows(long long N, long long K) {
   return rows < 32 ? 32 : rows;
 }
 
-// Whether one launch prepares both operands (prep_f16_one_kernel).  Above 32 KiB of shared memory a block (K = 2048) A's rows have too
-// few blocks an SM in flight, which shows when nearly all the work is A's: 8192 x 512 x 4000 in the one-term mode 97.6 us in one
-// launch and 92.2 in two, 512 x 8192 x 4000 104.9 and 122.0.
+// Whether one launch prepares both operands (prep_f16_one_kernel).  Above 32 KiB of shared memory a block (K = 2048) A's rows have
+// fewer blocks an SM in flight, which shows at most when nearly all the work is A's and K is near its limit.  One launch and two in
+// the one-term mode, us: 8192 x 512 at K = 2304 58.0 and 58.9, 3072 65.5 and 68.0, 4000 83.1 and 82.0 (3xF16 132.6 and 130.2);
+// 8192 x 1024 x 4000 106.7 and 111.0; 512 x 8192 x 4000 96.5 and 116.2; 8192 x 512 x 2048 46.4 and 51.4.
 bool f16_prepared_at_once(long long M, long long N, long long K) {
   return K <= F16_ONE_MAX_K && N <= (1ll << 24) && (K <= F16_ONE_MAX_K / 2 || M <= 8 * N);
 }

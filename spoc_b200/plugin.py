@@ -442,7 +442,7 @@ class Backend:
         return m.value
 
     def set_gemm_variant(self, variant: int) -> None:
-        """0 automatic, 1 single-CTA tiles, 2 CTA pairs."""
+        """0 automatic, 1 single-CTA tiles, 2 CTA pairs, 3 CTA pairs fed from prepared panels (sb200_set_gemm_variant)."""
         _check(L.load().sb200_set_gemm_variant(variant))
 
     def launch_count(self) -> int:
@@ -461,7 +461,9 @@ class Vector:
     PIN_MIN_BYTES = 16 << 20   # vectors at least this large are pinned in place on their second transfer
     # Smaller vectors are pinned once this many bytes of them have been moved: registering and releasing 0.25 to 12 MiB takes
     # 1.1 to 5.5 ms, as much as pinning saves in about that traffic (a pageable MiB takes 70-220 us up and 170 down, a pinned
-    # one 35 and 29).  Below PIN_LEAST_BYTES a pageable copy is as quick.
+    # one 35 and 29).  Below PIN_LEAST_BYTES a pageable copy is as quick.  Vectors that are given up soon after they were pinned
+    # lose: a 1024^3 product with all three moved every pass, fresh vectors to free(), takes 21.6 ms for 16 passes (15.6 without),
+    # 24.1 for 24 (22.3), and is ahead from 28 on, at 0.32 ms a pass instead of 0.80.
     PIN_TRAFFIC_BYTES = 64 << 20
     PIN_LEAST_BYTES = 256 << 10
 

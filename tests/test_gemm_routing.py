@@ -41,7 +41,7 @@ def test_operands_tma_cannot_address_go_through_panels():
     assert d["kernel"] == "pair panels" and d["launches"] == "3"
     kp = 1024
     assert int(d["workspace"]) == 2 * ((700 * kp * 4 + 1023) // 1024 * 1024 + (900 * kp * 4 + 1023) // 1024 * 1024)
-    # at most 128 rows: the single-CTA kernel from panels, or the pair kernel when it can read the operands directly
+    # at most 128 rows and a small product: converted in registers by single CTAs; a pair when it can read the operands directly
     assert describe(L.MODE_TF32, 100, 300, 500, addressable=0)["kernel"] == "single panels"
     assert describe(L.MODE_TF32, 100, 300, 500, addressable=1)["kernel"] == "pair direct"
 
