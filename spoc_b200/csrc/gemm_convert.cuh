@@ -200,6 +200,7 @@ __global__ void go_on_probe_kernel(int* items, int max_items, unsigned int step_
   int n = 0;
   for (bool ok = true; ok && n < max_items; ++n) {
     for (int i = 0; i < ((warp * 5 + n) & 7); ++i) __nanosleep(20);
+    __syncwarp();
     ok = convert_go_on(ok, abort_flag);
   }
   if ((threadIdx.x & 31) == 0) items[blockIdx.x * CONV_WARPS + warp] = n;
@@ -316,7 +317,9 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
         if (elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
         tc_fence_before_sync();
       }
+      if (item + item_step >= num_items) break;  // the block's last item: nothing follows but the barrier all threads share
       // every warp is through with the accumulator and the tiles before the next item's operands arrive
+      __syncwarp();
       ok = convert_go_on(ok, abort_flag);
     }
     if (!ok && elect_one()) wait_for_copies();  // tiles of C

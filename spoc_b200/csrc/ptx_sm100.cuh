@@ -79,14 +79,14 @@ __device__ __forceinline__ void wait_for_copies() {
   }
 }
 
-// Barrier `id` of `threads` threads (whole warps) that tells all of them whether every one brought `ok`.
+// Barrier `id` of `threads` threads (whole, converged warps) that tells all of them whether every one brought `ok`.
 __device__ __forceinline__ bool barrier_all(int id, int threads, bool ok) {
   uint32_t all;
   asm volatile(
       "{\n"
       ".reg .pred p, q;\n"
       "setp.ne.b32 p, %3, 0;\n"
-      "barrier.cta.red.and.pred q, %1, %2, p;\n"
+      "bar.red.and.pred q, %1, %2, p;\n"
       "selp.b32 %0, 1, 0, q;\n"
       "}\n"
       : "=r"(all)
