@@ -175,7 +175,7 @@ struct ConvTile {
   }
 };
 
-// The converting warps' barrier behind a work item, and one decision for all of them: whether to go on to the next.  The MMA issuer
+// The converting warps' barrier between two work items, and one decision for all of them: whether to go on to the next.  The MMA issuer
 // is no part of the barrier and may give up at any time; if each warp read its flag behind the barrier, some could leave and the
 // others wait for them at the next barrier without end.
 __device__ __forceinline__ bool convert_go_on(bool ok, volatile int* abort_flag) {
