@@ -360,8 +360,8 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
             if (MODE == 3) {
               const uint64_t da_lo = umma_desc_k_sw128(sa_lo + k * 32), db_lo = umma_desc_mn_sw128_32b(sb_lo + k * 1024, 4096);
               umma_tf32(tmem_base, da_lo, db_hi, idesc, accumulate);
-              umma_tf32(tmem_base, da_hi, db_lo, idesc, 1u);
-              umma_tf32(tmem_base, da_hi, db_hi, idesc, 1u);
+              umma_tf32<A_KEEP>(tmem_base, da_hi, db_lo, idesc, 1u);
+              umma_tf32<A_KEPT>(tmem_base, da_hi, db_hi, idesc, 1u);
             } else {
               umma_tf32(tmem_base, da_hi, db_hi, idesc, accumulate);
             }

@@ -492,8 +492,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                 const uint64_t da_lo = umma_desc_k_sw128(sa_lo + koff);
                 const uint64_t db_lo = DIRECT ? umma_desc_mn_sw128_32b(sb_lo + k * 1024, 4096) : umma_desc_k_sw128(sb_lo + koff);
                 umma_for<F16, CTAS>(tmem_d, da_lo, db_hi, idesc, accumulate);
-                umma_for<F16, CTAS>(tmem_d, da_hi, db_lo, idesc, 1u);
-                umma_for<F16, CTAS>(tmem_d, da_hi, db_hi, idesc, 1u);
+                umma_for<F16, CTAS, A_KEEP>(tmem_d, da_hi, db_lo, idesc, 1u);
+                umma_for<F16, CTAS, A_KEPT>(tmem_d, da_hi, db_hi, idesc, 1u);
               } else {
                 umma_for<F16, CTAS>(tmem_d, da_hi, db_hi, idesc, accumulate);
               }

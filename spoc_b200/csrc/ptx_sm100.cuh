@@ -159,16 +159,27 @@ __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// What an MMA does with the rows of A: read them (A_ONCE), read them and keep them in the collector beside the tensor core
+// (A_KEEP), or take those the MMA before it, which has the same A, kept there (A_KEPT).  The three-term modes read hi(A) once for
+// hi*lo and hi*hi so: 64 x 4096 x 4096 3xTF32, where the converting warps share shared memory with the MMAs, 42.0 -> 38.9 us; 1024^3
+// 19.88 -> 19.84, 2048^3 3xF16 with epilogue 63.3 -> 62.4, 8192^3 4450 -> 4410.
+enum { A_ONCE = 0, A_KEEP = 1, A_KEPT = 2 };
+#define SB200_UMMA_FORM(FORM)                                                                                           \
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma." FORM " [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d), \
+               "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                                                      \
+               : "memory");
+#define SB200_UMMA_BODY(FORM)                                                    \
+  if constexpr (A == A_KEEP) {                                                   \
+    SB200_UMMA_FORM(FORM ".collector::a::fill")                                  \
+  } else if constexpr (A == A_KEPT) {                                            \
+    SB200_UMMA_FORM(FORM ".collector::a::lastuse")                               \
+  } else {                                                                       \
+    SB200_UMMA_FORM(FORM)                                                        \
+  }
 // D[tmem] (+)= A[smem desc] * B[smem desc], TF32 inputs, fp32 accumulate.
+template <int A = A_ONCE>
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n"
-      "}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  SB200_UMMA_BODY("cta_group::1.kind::tf32")
 }
 // Arrive on the mbarrier once every tcgen05 operation issued so far by this
 // thread has completed.
@@ -293,29 +304,15 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // One MMA over both blocks: rows [0,128) of A and D belong to the leader, rows
 // [128,256) to its peer; each block's shared memory holds half of B's N rows.
-__device__ __forceinline__ void umma_tf32_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n"
-      "}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+template <int A = A_ONCE>
+__device__ __forceinline__ void umma_tf32_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  SB200_UMMA_BODY("cta_group::2.kind::tf32")
 }
 // The same MMA on half-precision (fp16) operands with fp32 accumulation: 256 x N x 16 per instruction,
 // twice the arithmetic of the TF32 form in the same number of operand bytes and cycles.
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+template <int A = A_ONCE>
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  SB200_UMMA_BODY("cta_group::2.kind::f16")
 }
 // The same instructions with scale-input-d: D = A*B + D * 2^-scale, scale in 0..15 (an immediate of the instruction,
 // hence the switch).  The accumulator is always an input here.
@@ -354,15 +351,9 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t leader) 
 }
 
 // One block on its own, half-precision operands.
+template <int A = A_ONCE>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  SB200_UMMA_BODY("cta_group::1.kind::f16")
 }
 
 // The same operations for a pair of blocks (CTAS = 2) or a block on its own (CTAS = 1).
@@ -382,12 +373,12 @@ template <int CTAS>
 __device__ __forceinline__ void umma_commit_for(uint32_t bar, uint32_t leader) {
   if constexpr (CTAS == 2) umma_commit_pair(bar, leader); else umma_commit(bar);
 }
-template <bool F16, int CTAS>
+template <bool F16, int CTAS, int A = A_ONCE>
 __device__ __forceinline__ void umma_for(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  if constexpr (F16 && CTAS == 2) umma_f16_pair(tmem_d, adesc, bdesc, idesc, accumulate);
-  else if constexpr (F16) umma_f16(tmem_d, adesc, bdesc, idesc, accumulate);
-  else if constexpr (CTAS == 2) umma_tf32_pair(tmem_d, adesc, bdesc, idesc, accumulate);
-  else umma_tf32(tmem_d, adesc, bdesc, idesc, accumulate);
+  if constexpr (F16 && CTAS == 2) umma_f16_pair<A>(tmem_d, adesc, bdesc, idesc, accumulate);
+  else if constexpr (F16) umma_f16<A>(tmem_d, adesc, bdesc, idesc, accumulate);
+  else if constexpr (CTAS == 2) umma_tf32_pair<A>(tmem_d, adesc, bdesc, idesc, accumulate);
+  else umma_tf32<A>(tmem_d, adesc, bdesc, idesc, accumulate);
 }
 template <int CTAS>
 __device__ __forceinline__ void tma_load_for(uint32_t dst_smem, const CUtensorMap* map, uint32_t bar, int32_t x, int32_t y, uint64_t policy) {
