@@ -16,7 +16,8 @@ LIB = os.path.join(HERE, "libsarek_b200.so")
 HOSTPATH = os.path.join(HERE, "_hostpath.so")   # CPython extension: the marshalling half of run_vectors
 
 SOURCES = ["sb200_shim.cu", "sb200_group.cu", "ir.cc", "fusion.cc", "map_jit.cc", "transfer.cc"]
-HEADERS = ["gemm_tcgen05.cuh", "gemm_tcgen05_pair.cuh", "gemm_convert.cuh", "map_fused.cuh", "ptx_sm100.cuh", "ir.hpp", "map_jit.hpp", "transfer.hpp", "internal.hpp",
+HEADERS = ["gemm_tcgen05.cuh", "gemm_tcgen05_pair.cuh", "gemm_convert.cuh", "gemm_split.cuh", "map_fused.cuh",
+           "ptx_sm100.cuh", "ir.hpp", "map_jit.hpp", "transfer.hpp", "internal.hpp",
            os.path.join("..", "..", "include", "sb200.h")]
 
 NVCC_FLAGS = [

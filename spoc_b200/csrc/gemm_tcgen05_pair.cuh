@@ -28,8 +28,9 @@ constexpr uint32_t PAIR_A_BYTES = 128 * GEMM_BK * 4;  // this block's A rows: 16
 //   SRC_DIRECT  the caller's row-major A and B through TFLOAT32 tensor maps (TMA rounds to TF32 on the way in); B arrives as
 //               [32 k][32 n] slabs (swizzle 128B with 32-byte atoms) and is consumed through an MN-major descriptor.  The low
 //               parts of 3xTF32 come from prepared panels: A [M x Kp], B row-major [K x Np] read as slabs like B itself.
-//   SRC_CONVERT not this kernel: gemm_convert_kernel loads the caller's matrices itself (gemm_convert.cuh).
-enum { SRC_PANELS = 0, SRC_DIRECT = 1, SRC_CONVERT = 2 };
+//   SRC_CONVERT, SRC_SPLIT  not this kernel: gemm_convert_kernel and gemm_split_kernel make the parts themselves (gemm_convert.cuh,
+//               gemm_split.cuh).
+enum { SRC_PANELS = 0, SRC_DIRECT = 1, SRC_CONVERT = 2, SRC_SPLIT = 3 };
 
 template <int MODE, int SRC, int BN, int CTAS>
 struct TileCfg {
@@ -157,7 +158,7 @@ template <int BN, int CTAS, int THREADS, bool VEC>
 __device__ __forceinline__ void cluster_part_finish(const GemmParams& p, const void* part, int share, int rank, int row0, int n0, int tid) {
   constexpr int QUADS = BN / 4;
   static_assert(THREADS % QUADS == 0, "a thread stays in its column quad");
-  constexpr int BATCH = 4, AHEAD = 4;    // quads, and partial sums of each, that a thread has in flight
+  constexpr int BATCH = THREADS > 256 ? 2 : 4, AHEAD = 4;  // quads, and partial sums of each, that a thread has in flight
   constexpr int STEP = THREADS / QUADS;  // rows between a thread's quads
   const int rows = min(128, p.M - row0);
   if (rows <= 0) return;
@@ -208,8 +209,10 @@ __device__ __forceinline__ void cluster_part_finish(const GemmParams& p, const v
     if (count >= BATCH) {
       batch(std::integral_constant<int, BATCH>());
     } else {
-      if (count & 2) batch(std::integral_constant<int, 2>());
-      if (count & 2) row += 2 * STEP;
+      if constexpr (BATCH > 2) {
+        if (count & 2) batch(std::integral_constant<int, 2>());
+        if (count & 2) row += 2 * STEP;
+      }
       if (count & 1) batch(std::integral_constant<int, 1>());
     }
   }

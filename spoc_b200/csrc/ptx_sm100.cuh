@@ -181,6 +181,30 @@ template <int A = A_ONCE>
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   SB200_UMMA_BODY("cta_group::1.kind::tf32")
 }
+// The same with A in tensor memory (row i of this block's rows in lane i, a 32-bit column per element of k).  CTAS = 2: each block's
+// tensor memory holds its own 128 rows, at the same columns.
+template <int CTAS>
+__device__ __forceinline__ void umma_tf32_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (CTAS == 2)
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+                 "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+                 : "memory");
+  else
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+                 "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+// 32 lanes x 16 consecutive columns, the other way: thread i writes columns [col, col+16) of lane (lane_base + i); tmem_st_wait()
+// returns when this thread's stores are done.
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Arrive on the mbarrier once every tcgen05 operation issued so far by this
 // thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -257,6 +281,12 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
 // arrive on an mbarrier that may live in the peer block (address from map_to_cta)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The same with what the arrival releases left at the scope of this block.  For signals about work that the tensor core reads from
+// this block's own shared and tensor memory: nothing of it has to become visible elsewhere, and the fence of the cluster form, which
+// waits for the whole chip, took 1400 cycles.
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load whose completion bytes are counted on an mbarrier of either block of the pair (`bar` is a shared::cluster address), with
 // an L2 eviction policy (from l2_policy below) for the lines it brings in; data lands in this block.

@@ -26,6 +26,7 @@
 
 #include "../../include/sb200.h"
 #include "gemm_convert.cuh"
+#include "gemm_split.cuh"
 #include "gemm_tcgen05.cuh"
 #include "gemm_tcgen05_pair.cuh"
 #include "internal.hpp"
@@ -497,6 +498,7 @@ int tile_n_setting() {
 // How a product is cut up: tile columns, and work items a tile's k-loop is divided into.
 struct TileShape {
   int tile_n = 256, splits = 1;
+  double cost = 0.0;  // estimated time, ns
 };
 
 // Clusters of `blocks` (at most 8) blocks that are resident at once when every block has an SM to itself.  A cluster lies within a
@@ -531,19 +533,23 @@ constexpr int kMaxSplits = 32;
 // win by 8 % (at 256 x 512 x 1024 four items of 8 k-blocks take 9.5 us in TF32 and one of 32 takes 11.1; 40 x 300 x 1200
 // unaligned 18.7 against 28.8).
 // fixed_splits > 0: the division is given (a part of a larger product is divided as the whole is, so that it has the same bits).
-// convert: gemm_convert_kernel's rates instead of the pair kernel's: in 3xTF32 between those of quads and of single elements (1060
+// src: SRC_CONVERT takes gemm_convert_kernel's rates instead of the pair kernel's: in 3xTF32 between those of quads and of single elements (1060
 // and 1430 ns at 128 columns, 790 and 1180 at 64), since one choice serves both.
 // no_scratch: divisions within a cluster only, whose partial sums need no memory (TF32, 64 x 512 x 16384 18.8 us so and 15.5 with
 // 29 items through memory, 666 x 8 x 9632 19.5 and 13.0, 128 x 96 x 16384 28.2 and 13.7; most shapes within 10 %).
+// SRC_SPLIT (gemm_split_kernel), measured on 1024 x 1024 x K and on 64 and 128 x 4096 x K: pairs 850, 645, 430 and 363 ns a k-block, blocks
+// on their own 540 and 375; a wave's epilogue overlaps nothing, so every wave has the fixed cost (4096 x 4096 x 512: 5.9 us a wave of
+// 128 columns, 8.7 of 256).  least_splits: no k-loop is divided into fewer, so that none is longer, and less exact, than in plain_route.
 TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
-                       bool convert = false, bool no_scratch = false) {
+                       int src = SRC_DIRECT, bool no_scratch = false, int least_splits = 1) {
   TileShape best;
   const int forced = tile_n_setting();
   double best_cost = 0.0;
+  const bool split_kernel = src == SRC_SPLIT;
   bool have = false;
   const long long tiles_m = (M + 128 * ctas - 1) / (128 * ctas);
   const int sm_count = units * ctas;
-  for (int sp = 1; sp <= kMaxSplits; ++sp) {
+  for (int sp = fixed_splits ? 1 : least_splits; sp <= kMaxSplits; ++sp) {
     if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * kMinSplitKBlocks)) continue;
     const long long per_item = (kblocks + sp - 1) / sp;
     if (sp > 1 && per_item * (sp - 1) >= kblocks) continue;  // the last item would be empty
@@ -551,30 +557,34 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
       if (ctas == 1 && bn > 128) continue;
       if (bn == 192 && (!three || forced)) continue;
       if (forced && bn != forced && !(ctas == 1 && forced == 256 && bn == 128)) continue;
-      const double per_kblock = convert ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0))
+      const double per_kblock = split_kernel ? (ctas == 1 ? (bn == 128 ? 540.0 : 375.0) : bn == 256 ? 850.0 : bn == 192 ? 645.0 : bn == 128 ? 430.0 : 363.0)
+                                : src == SRC_CONVERT ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0))
                                 : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0)
                                         : (bn == 256 ? 277.0 : 165.0);
-      const double charge = bn == 256 ? 1.0 : three ? (kblocks < 128 ? 1.02 : 1.1) : (kblocks < 128 ? 1.1 : 1.4);
+      const double charge = bn == 256 || (split_kernel && kblocks < 128) ? 1.0 : three ? (kblocks < 128 ? 1.02 : 1.1) : (kblocks < 128 ? 1.1 : 1.4);
       const long long tiles = tiles_m * ((N + bn - 1) / bn);
       const bool in_cluster = split_in_cluster(tiles, sp, ctas, sm_count);
       if (no_scratch && sp > 1 && !in_cluster) continue;
       if (!fixed_splits && sp > 1 && !in_cluster && three && ctas == 2 && kblocks < static_cast<long long>(sp) * kMinSplitKBlocksThree) continue;
       const long long waves = in_cluster ? 1 : (tiles * sp + units - 1) / units;
-      double c = waves * per_item * per_kblock * charge + 5500.0 + 500.0 * (bn / 32) + 800.0 * (waves - 1);
+      double c = split_kernel ? waves * (per_item * per_kblock * charge + (ctas == 1 ? 5000.0 : 5600.0) + 900.0 * (bn / 64))
+                              : waves * per_item * per_kblock * charge + 5500.0 + 500.0 * (bn / 32) + 800.0 * (waves - 1);
       if (in_cluster)  // the barriers, and 2 ns per quad of a block's share
         c += 1500.0 + 2.0 * (M < 128 ? M : 128) * (bn / 4) / sp;
       else if (sp > 1)
         c += 2500.0 + (sp + 1.0) * M * N * 4.0 / 4000.0;
-      if (!have || c < (sp == best.splits ? 0.97 : best.splits == 1 ? 0.92 : 0.97) * best_cost) {
+      if (!have || c < (sp == best.splits ? 0.97 : split_kernel ? 0.9 : best.splits == 1 ? 0.92 : 0.97) * best_cost) {
         best.tile_n = bn;
         best.splits = sp;
-        best_cost = c;
+        best.cost = best_cost = c;
         have = true;
       }
     }
   }
   return best;
 }
+
+int units_of(int ctas, int sm_count);
 
 // The operand maps of one launch; x: the mixed mode's third pair (else unused).
 struct OperandMaps {
@@ -705,6 +715,49 @@ int launch_convert_for(int bn, bool vec, int dev_index, int sm_count, cudaStream
   return vec ? launch_convert<MODE, 128, true>(dev_index, sm_count, st, o, gp, part) : launch_convert<MODE, 128, false>(dev_index, sm_count, st, o, gp, part);
 }
 
+// gemm_split_kernel, the same way.  m.a_hi and m.b_hi lie over the caller's matrices without rounding.
+template <int BN, int CTAS, int ROWS = 128>
+int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, int a_box_rows, GemmParams gp, float* part) {
+  using Cfg = SplitCfg<BN, CTAS, ROWS>;
+  static std::atomic<int> attr_set[kMaxDevices];
+  if (!attr_set[dev_index].load()) {
+    for (auto k : {gemm_split_kernel<BN, CTAS, ROWS, false>, gemm_split_kernel<BN, CTAS, ROWS, true>})
+      CU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
+    attr_set[dev_index].store(1);
+  }
+  const int units = units_of(CTAS, sm_count);
+  gp.tiles_m = (gp.M + 128 * CTAS - 1) / (128 * CTAS);
+  gp.tiles_n = static_cast<int>((static_cast<long long>(gp.N) + BN - 1) / BN);
+  gp.group_m = PAIR_GROUP_M;
+  if (gp.splits < 1) gp.splits = 1;
+  gp.split_k_blocks = (gp.num_k_blocks + gp.splits - 1) / gp.splits;
+  gp.epoch_ctr = nullptr;
+  const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
+  gp.cluster_splits = split_in_cluster(items / gp.splits, gp.splits, CTAS, sm_count) ? gp.splits : 1;
+  const dim3 grid(static_cast<unsigned>(CTAS * (items < units || gp.cluster_splits > 1 ? items : units)));
+  CUtensorMap map_d, map_c;
+  GemmParams kp;
+  if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
+  auto kernel = gp.cluster_splits > 1 ? gemm_split_kernel<BN, CTAS, ROWS, true> : gemm_split_kernel<BN, CTAS, ROWS, false>;
+  CU_TRY(launch_pdl(kernel, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, st, CTAS * gp.cluster_splits, m.a_hi, m.b_hi, map_d, map_c, a_box_rows, kp));
+  if (int rc = launch_check("gemm_split_kernel")) return rc;
+  return launch_reduce(sm_count, st, gp, part);
+}
+
+int launch_split_for(int bn, int ctas, int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, int a_box_rows, const GemmParams& gp,
+                     float* part) {
+  if (ctas == 1 && gp.M <= 64)
+    return bn == 64 ? launch_split<64, 1, 64>(dev_index, sm_count, st, m, a_box_rows, gp, part)
+                    : launch_split<128, 1, 64>(dev_index, sm_count, st, m, a_box_rows, gp, part);
+  if (ctas == 1)
+    return bn == 64 ? launch_split<64, 1>(dev_index, sm_count, st, m, a_box_rows, gp, part)
+                    : launch_split<128, 1>(dev_index, sm_count, st, m, a_box_rows, gp, part);
+  return bn == 64    ? launch_split<64, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part)
+         : bn == 128 ? launch_split<128, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part)
+         : bn == 192 ? launch_split<192, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part)
+                     : launch_split<256, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part);
+}
+
 size_t partial_bytes(long long M, long long N, const TileShape& shape, int ctas, int sm_count) {
   const int splits = shape.splits;
   return splits > 1 && !split_in_cluster(tiles_of(M, N, shape.tile_n, ctas), splits, ctas, sm_count) ? static_cast<size_t>(round_up(M, 32)) * round_up(N, 4) * 4 * splits : 0;
@@ -735,6 +788,7 @@ struct GemmRoute {
   int tile_n = 256, splits = 1;
   int stages = 0;
   long long tiles = 0, waves = 0;
+  double cost = 0.0;         // estimated time, ns
   size_t operand_bytes = 0;  // scratch of the operand panels
   size_t workspace = 0;      // bytes of library scratch, partial results included
 };
@@ -764,11 +818,26 @@ constexpr double kConvertMacsUnaligned = 134217728.0;    // 2^27
 // maps to encode and fetch, but 0.5 us more a k-block on the device.  Converted and by gemm_pair_kernel, us: 64 x 64 x 96 5.2 and 5.6,
 // x 128 5.4 and 5.6; 64 x 1024 x 96 5.3 and 5.6, x 128 6.1 and 5.6; 512 x 256 x 64 5.3 and 5.6, x 96 6.1 and 5.8.
 constexpr long long kConvertKOneTerm = 128;
+// gemm_split_kernel instead of gemm_pair_kernel behind a launch for the low parts, where the estimates say so.  It moves half the bytes
+// to the SMs, which the other pays with 10 % of its time beside the estimate (2048^3 88 -> 77 us, 4096^3 634 -> 565, 1024 x 1024 x 4096
+// 55 -> 42, 2048 x 2048 x 16384 650 -> 535); but its epilogues overlap nothing (8192 x 8192 x 512, 14 waves: 360 us, the other 290).
+// Not in several waves of long k-loops, whose pairs gemm_pair_kernel holds together (next_epoch_ring; 8192^3 4440 and 4360 us:
+// what lockstep saves in DRAM traffic on the largest products is not to be had here), nor in several waves of a divided one
+// (64 x 16384 x 16384: 625 and 532).  With two k-blocks or one the host's encoding of the operand maps costs what the device saves: 64^3 called
+// in a row 5.80 us and by gemm_convert_kernel 5.71, 32^3 6.6 and 6.5; 128^3 6.4 and 7.4.
+constexpr double kPlainCharge = 1.1;
+constexpr long long kSplitMaxKBlocks = 256;
 
 int stages_of(bool three, int bn, int ctas) {
   const long long stage = (three ? 2 : 1) * (16384ll + (bn / ctas) * 128ll);
   const long long fit = 192 * 1024 / stage;
   return static_cast<int>(fit > 8 ? 8 : fit);
+}
+
+int split_stages_of(int bn, int ctas, long long M) {
+  if (ctas == 1 && M <= 64) return bn == 64 ? SplitCfg<64, 1, 64>::kRaw : SplitCfg<128, 1, 64>::kRaw;
+  if (ctas == 1) return bn == 64 ? SplitCfg<64, 1, 128>::kRaw : SplitCfg<128, 1, 128>::kRaw;
+  return bn == 64 ? SplitCfg<64, 2, 128>::kRaw : bn == 128 ? SplitCfg<128, 2, 128>::kRaw : bn == 192 ? SplitCfg<192, 2, 128>::kRaw : SplitCfg<256, 2, 128>::kRaw;
 }
 
 // Set by PartsOf (the host-operand calls, the launches that upload by blocks, partial launches, device groups).
@@ -794,14 +863,8 @@ TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_co
 // Row length of the parts of B the direct kernel reads from the scratch.
 long long route_b_pitch(long long N, bool addressable) { return round_up(N, addressable ? 32 : 4); }
 
-GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
-  int fixed_splits = 0;
-  if (part_of_whole(M, N)) {
-    const Whole whole = t_whole;
-    t_whole = Whole();
-    fixed_splits = route_gemm(mode, whole.rows, whole.cols, K, addressable, sm_count, whole.rows).splits;
-    t_whole = whole;
-  }
+// Every route but that through gemm_split_kernel.
+GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a, int fixed_splits) {
   GemmRoute r;
   const int variant = gemm_variant_setting();
   const bool three = mode == SB200_MODE_3XTF32;
@@ -818,16 +881,17 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
                        (addressable ? (three ? M <= kSingleRows || macs < kConvertMacs : K <= kConvertKOneTerm && macs < kConvertMacs)
                                     : M <= kSingleRows || macs < kConvertMacsUnaligned);
   r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
+  r.src = convert ? SRC_CONVERT : direct ? SRC_DIRECT : SRC_PANELS;
   const int units = units_of(r.ctas, sm_count);
   // TF32 mode on addressable operands uses no scratch at all: such calls run side by side on any streams, and a graph they were
   // captured into stays good whatever other calls do to the scratch.  (A part always finds a cut: it has no more tiles than
   // its whole, or up to twice as many single blocks, for which there is room for more than twice as many clusters.)
-  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, convert, !three && addressable);
+  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, r.src, !three && addressable);
+  r.cost = shape.cost;
   r.tile_n = shape.tile_n;
   r.splits = shape.splits;
-  r.src = convert ? SRC_CONVERT : direct ? SRC_DIRECT : SRC_PANELS;
   r.stages = stages_of(three, r.tile_n, r.ctas);
-  r.tiles = ((M + 128 * r.ctas - 1) / (128 * r.ctas)) * ((N + r.tile_n - 1) / r.tile_n);
+  r.tiles = tiles_of(M, N, r.tile_n, r.ctas);
   r.waves = (r.tiles * r.splits + units - 1) / (units > 0 ? units : 1);
   if (panel_rows_a < M) panel_rows_a = M;
   if (r.src == SRC_PANELS) {
@@ -837,6 +901,37 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
     r.operand_bytes = addressable ? parts : std::max<size_t>((three ? 2 : 1) * parts, gemm_workspace_need(mode, panel_rows_a, N, K));
   }
   r.workspace = r.operand_bytes + partial_bytes(M, N, shape, r.ctas, sm_count);
+  return r;
+}
+
+GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
+  int fixed_splits = 0;
+  if (part_of_whole(M, N)) {
+    const Whole whole = t_whole;
+    t_whole = Whole();
+    fixed_splits = route_gemm(mode, whole.rows, whole.cols, K, addressable, sm_count, whole.rows).splits;
+    t_whole = whole;
+  }
+  GemmRoute r = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits);
+  if (mode != SB200_MODE_3XTF32 || !addressable || K <= 2 * GEMM_BK || gemm_variant_setting() != 0) return r;
+  const double macs = static_cast<double>(M) * N * K;
+  const long long kblocks = round_up(K, GEMM_BK) / GEMM_BK;
+  const int ctas = M <= 128 || macs < kConvertMacs ? 1 : 2, units = units_of(ctas, sm_count);
+  const TileShape shape = choose_tiles(M, N, kblocks, ctas, units, true, true, fixed_splits, SRC_SPLIT, false, r.splits);
+  const long long tiles = tiles_of(M, N, shape.tile_n, ctas), waves = (tiles * shape.splits + units - 1) / units;
+  const double prep = 1000.0 + 8.0 * (static_cast<double>(M) * K + static_cast<double>(K) * N) / 5000.0;  // ns: the launch for the low parts
+  const double plain = r.src == SRC_CONVERT ? r.cost : kPlainCharge * r.cost + prep;
+  if ((waves > 1 && (kblocks >= kSplitMaxKBlocks || shape.splits > 1)) || shape.cost >= plain) return r;
+  r.src = SRC_SPLIT;
+  r.ctas = ctas;
+  r.cost = shape.cost;
+  r.tile_n = shape.tile_n;
+  r.splits = shape.splits;
+  r.stages = split_stages_of(shape.tile_n, ctas, M);
+  r.tiles = tiles;
+  r.waves = waves;
+  r.operand_bytes = 0;
+  r.workspace = partial_bytes(M, N, shape, ctas, sm_count);
   return r;
 }
 
@@ -907,7 +1002,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     }
   }
   unsigned int* epoch_ring =
-      route.ctas == 2 && route.splits == 1 ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
+      route.ctas == 2 && route.splits == 1 && route.src != SRC_SPLIT ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
   const bool prof = g_profiling.load() != 0;
   DeviceState::ProfRec rec{nullptr, nullptr, nullptr};
   if (prof) {
@@ -917,8 +1012,15 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     CU_TRY(cudaEventRecord(rec.e0, st));
   }
   CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
+  int a_box_rows = GEMM_BM;
   if (route.src == SRC_CONVERT) {
     // no panels, no operand maps
+  } else if (route.src == SRC_SPLIT) {
+    a_box_rows = static_cast<int>(std::min<long long>(GEMM_BM, round_up(M, 8)));
+    if ((rc = encode_map_2d(&ma_hi, A, K, M, lda, GEMM_BK, a_box_rows, false))) return rc;
+    if ((rc = encode_map_2d(&mb_hi, B, N, K, ldb, 32, GEMM_BK, false, true))) return rc;
+    ma_lo = ma_hi;
+    mb_lo = mb_hi;
   } else if (direct) {
     // Workspace, B's parts first (their place does not depend on M): [B copy][B lo][A copy][A lo], each only when it is needed;
     // B's as K rows of np, A's as rows of kp.  The copies stand in for matrices TMA cannot address.
@@ -978,8 +1080,9 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     rc = launch_convert_for<MODE>(tile_n, addressable && (K & 3) == 0 && (N & 3) == 0, dev_index, d.sm_count, st, o, gp, part);
   } else {
     const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
-    rc = direct ? launch_tiles_for<MODE, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
-                : launch_tiles_for<MODE, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
+    rc = route.src == SRC_SPLIT ? launch_split_for(tile_n, route.ctas, dev_index, d.sm_count, st, maps, a_box_rows, gp, part)
+         : direct               ? launch_tiles_for<MODE, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
+                                : launch_tiles_for<MODE, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
   }
   if (prof) {
     CU_TRY(cudaEventRecord(rec.e2, st));
@@ -989,7 +1092,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   if (track_scratch && rc == SB200_OK) {
     rc = scratch_release(d, st);
   }
-  if (b_prepared) *b_prepared = route.workspace && route.src != SRC_CONVERT ? d.ws_uses : 0;
+  if (b_prepared) *b_prepared = route.operand_bytes ? d.ws_uses : 0;
   return rc;
 }
 
@@ -2656,9 +2759,9 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   // the second word and `launches` speak of addressability and of passes; `operands` and `kernels` say what runs
   const bool apart = r.src == SRC_PANELS || (r.src == SRC_DIRECT && !addressable);
   const int reduction = r.splits > 1 && !split_in_cluster(r.tiles, r.splits, r.ctas, sm_count) ? 1 : 0;
-  const int launches = (apart ? 3 : r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32 ? 2 : 1) + reduction;
+  const int launches = (apart ? 3 : r.ctas == 2 && mode == SB200_MODE_3XTF32 ? 2 : 1) + reduction;
   const int kernels = (apart || (r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32) ? 2 : 1) + reduction;
-  const char* operands = r.src == SRC_CONVERT ? "converted" : r.src == SRC_PANELS ? "panels" : addressable ? "direct" : "copied";
+  const char* operands = r.src == SRC_CONVERT || (r.src == SRC_SPLIT && r.ctas == 1) ? "converted" : r.src == SRC_PANELS ? "panels" : addressable ? "direct" : "copied";
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=%s kernels=%d",
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
            r.waves, r.splits, r.workspace, launches, operands, kernels);

@@ -256,3 +256,57 @@ def test_the_described_kernels_are_the_ones_launched(backend, device, mode, M, N
         lib.sb200_set_mixed_min_macs(0)
         for x in (A, B, D):
             x.free()
+
+
+# (M, N, K): rows and columns at the edges of 64- and 128-row blocks and of every tile width, pairs whose second block has no rows, k-loops
+# shorter than, as long as and one beyond the rings, k that ends within a k-block, more tiles than pairs
+SPLIT = [(1, 4, 65), (64, 64, 96), (63, 68, 100), (65, 64, 96), (128, 128, 256), (129, 60, 257), (257, 516, 288), (300, 1000, 300), (512, 64, 512),
+         (1536, 2044, 260), (2048, 2052, 68), (2304, 2304, 520)]
+
+
+@pytest.mark.parametrize("M,N,K", SPLIT)
+@pytest.mark.parametrize("epilogue", [False, True], ids=["plain", "epilogue"])
+def test_operands_split_on_chip_give_the_bits_of_the_panels(backend, device, M, N, K, epilogue):
+    lda, ldb, ldd = ((x + 3) // 4 * 4 + 4 for x in (K, N, N))
+    rng = np.random.default_rng(M + N + K)
+    a, b, c = (rng.uniform(-1, 1, (r, ld)).astype(np.float32) for r, ld in ((M, lda), (K, ldb), (M, ldd)))
+    a[0, 0], b[0, 0] = np.float32(2.0 ** -130), np.float32(2.0 ** 100)     # a subnormal element, and one that dwarfs the rest
+    a[M - 1, 1] = np.float32(3.4028234e38)                                # rounds to infinity: no low part may come of it
+    A, B, Cm, Bi = (dev_from(backend, device, x.ravel()) for x in (a, b, c, c[0, :N].copy()))
+    D = Dev(backend, device, M * ldd)
+    kw = dict(alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, ldc=ldd) if epilogue else {}
+    out = []
+    try:
+        text = describe(L.MODE_3XTF32, M, N, K, 1)
+        assert "splits=1 " in text and text.endswith("kernels=1")     # the k-loop is not divided; nothing is prepared
+        for variant in (3, 0):
+            backend.set_gemm_variant(variant)
+            D.clear()
+            gemm(backend, device, L.MODE_3XTF32, M, N, K, A, B, D, lda=lda, ldb=ldb, ldd=ldd, **kw)
+            out.append(D.download().reshape(M, ldd))
+        assert np.array_equal(out[0][:, :N].view(np.uint32), out[1][:, :N].view(np.uint32))
+        assert np.all(out[1][:, N:] == CANARY)
+    finally:
+        backend.set_gemm_variant(0)
+        for x in (A, B, Cm, Bi, D):
+            x.free()
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 4096, 4096), (128, 1024, 4096), (1024, 1024, 1024), (256, 2048, 4096), (2304, 2304, 520)])
+def test_operands_split_on_chip_give_the_same_bits_every_time(backend, device, M, N, K):
+    """Stages that are written again while a warp still reads them show here: operands in L2 and not, launches alone and in a row."""
+    A, B = (dev_from(backend, device, O.fill(n, 74, i)) for i, n in ((1, M * K), (2, K * N)))
+    D, other = Dev(backend, device, M * N), Dev(backend, device, 40 << 20)
+    try:
+        first = None
+        for i in range(12):
+            if i % 3 == 1:
+                other.clear()
+            for _ in range(1 + i % 2):
+                gemm(backend, device, L.MODE_3XTF32, M, N, K, A, B, D)
+            got = D.download().view(np.uint32)
+            first = got if first is None else first
+            assert np.array_equal(got, first)
+    finally:
+        for x in (A, B, D, other):
+            x.free()
