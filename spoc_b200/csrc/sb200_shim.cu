@@ -808,12 +808,16 @@ int gemm_variant_setting() {
 // us; 65 rows 27.3 by pairs and 18.5 by single blocks, 128 rows 27.1 and 18.9; in 3xTF32 62.6 and 44.5, 65.3 and 45.0 (1024 x 1024:
 // 9.4 and 7.9, 11.3 and 8.3; 14.0 both, 15.1 and 14.3).  The line is where the forms were first told apart.
 constexpr long long kSingleRows = 64;
-// Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands.  Converted and
-// prepared by a launch in front, 3xTF32, us: addressable 100 x 64 x 100 7.6 and 8.8, 192^3 9.4 and 8.9, 256^3 11.3 and 9.8; unaligned
-// 128^3 9.0 and 8.7 (TF32 6.9 and 8.5), 256^3 13.9 and 10.3, 448^3 22.9 and 12.4, 576^3 17.5 and 14.5.  So both are even near
-// 2^22; the second line was drawn when unaligned operands still went through transposed panels (512^3 about even then).
+// Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands (in 3xTF32 unless
+// gemm_split_kernel does it).  Converted and prepared by a launch in front, 3xTF32, us: addressable 100 x 64 x 100 7.6 and 8.8, 192^3 9.4 and
+// 8.9, 256^3 11.3 and 9.8.
 constexpr double kConvertMacs = 16777216.0;              // 2^24
 constexpr double kConvertMacsUnaligned = 134217728.0;    // 2^27
+// Of the unaligned products below that line and of more than kSingleRows rows, those from here on are copied by a launch in front all the
+// same, with k-loops no longer than the converting kernel would give them.  Converted and copied, us: 3xTF32 128^3 9.0 and 9.3, 191 x 193 x 195
+// 12.9 and 9.9, 255 x 257 x 259 15.2 and 10.5, 449^3 21.5 and 12.6; TF32 128^3 7.3 and 8.5, 255 x 257 x 259 11.3 and 9.1, 449^3 15.1 and 10.1.
+constexpr double kCopyMacsThree = 4194304.0;             // 2^22
+constexpr double kCopyMacs = 16777216.0;                 // 2^24
 // In TF32 mode, where aligned operands need no preparation, it is the shorter way for k-loops of a few k-blocks only: no operand
 // maps to encode and fetch, but 0.5 us more a k-block on the device.  Converted and by gemm_pair_kernel, us: 64 x 64 x 96 5.2 and 5.6,
 // x 128 5.4 and 5.6; 64 x 1024 x 96 5.3 and 5.6, x 128 6.1 and 5.6; 512 x 256 x 64 5.3 and 5.6, x 96 6.1 and 5.8.
@@ -863,8 +867,9 @@ TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_co
 // Row length of the parts of B the direct kernel reads from the scratch.
 long long route_b_pitch(long long N, bool addressable) { return round_up(N, addressable ? 32 : 4); }
 
-// Every route but that through gemm_split_kernel.
-GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a, int fixed_splits) {
+// Every route but that through gemm_split_kernel.  least_splits > 0: not through gemm_convert_kernel either, and no longer k-loops.
+GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a, int fixed_splits,
+                      int least_splits = 0) {
   GemmRoute r;
   const int variant = gemm_variant_setting();
   const bool three = mode == SB200_MODE_3XTF32;
@@ -877,7 +882,7 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
   // triple the traffic, and any mode's few rows of matrices TMA cannot address; and products so small that the launch that
   // would prepare operands weighs more than the pair kernel's faster tiles give (kConvertMacs).
   const double macs = static_cast<double>(M) * N * K;
-  const bool convert = variant == 0 && tile_n_setting() != 256 &&
+  const bool convert = variant == 0 && least_splits == 0 && tile_n_setting() != 256 &&
                        (addressable ? (three ? M <= kSingleRows || macs < kConvertMacs : K <= kConvertKOneTerm && macs < kConvertMacs)
                                     : M <= kSingleRows || macs < kConvertMacsUnaligned);
   r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
@@ -886,7 +891,8 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
   // TF32 mode on addressable operands uses no scratch at all: such calls run side by side on any streams, and a graph they were
   // captured into stays good whatever other calls do to the scratch.  (A part always finds a cut: it has no more tiles than
   // its whole, or up to twice as many single blocks, for which there is room for more than twice as many clusters.)
-  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, r.src, !three && addressable);
+  const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, r.src, !three && addressable,
+                                       least_splits > 0 ? least_splits : 1);
   r.cost = shape.cost;
   r.tile_n = shape.tile_n;
   r.splits = shape.splits;
@@ -913,15 +919,30 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
     t_whole = whole;
   }
   GemmRoute r = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits);
-  if (mode != SB200_MODE_3XTF32 || !addressable || K <= 2 * GEMM_BK || gemm_variant_setting() != 0) return r;
   const double macs = static_cast<double>(M) * N * K;
+  const bool three = mode == SB200_MODE_3XTF32;
+  if (r.src == SRC_CONVERT && !addressable && M > kSingleRows && macs >= (three ? kCopyMacsThree : kCopyMacs)) {
+    const GemmRoute copied = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits, r.splits);
+    if (copied.cost > 0.0) r = copied;  // 0: pairs cannot divide the k-loop so often
+  }
+  if (gemm_variant_setting() != 0) return r;
+  if (!three || K <= 2 * GEMM_BK) return r;
   const long long kblocks = round_up(K, GEMM_BK) / GEMM_BK;
   const int ctas = M <= 128 || macs < kConvertMacs ? 1 : 2, units = units_of(ctas, sm_count);
   const TileShape shape = choose_tiles(M, N, kblocks, ctas, units, true, true, fixed_splits, SRC_SPLIT, false, r.splits);
   const long long tiles = tiles_of(M, N, shape.tile_n, ctas), waves = (tiles * shape.splits + units - 1) / units;
-  const double prep = 1000.0 + 8.0 * (static_cast<double>(M) * K + static_cast<double>(K) * N) / 5000.0;  // ns: the launch for the low parts
-  const double plain = r.src == SRC_CONVERT ? r.cost : kPlainCharge * r.cost + prep;
-  if ((waves > 1 && (kblocks >= kSplitMaxKBlocks || shape.splits > 1)) || shape.cost >= plain) return r;
+  // ns: a launch in front that reads the operands and writes their low parts, copies of them, or both
+  auto prep = [&](int written) { return 1000.0 + 4.0 * (1 + written) * (static_cast<double>(M) * K + static_cast<double>(K) * N) / 5000.0; };
+  const double plain = r.src == SRC_CONVERT ? r.cost : kPlainCharge * r.cost + prep(addressable ? 1 : 2);
+  // a launch in front costs 2.5 us beside its bytes; where plain_route has one too, 64-column tiles over copies bring nothing
+  const double cost = shape.cost + (addressable ? 0.0 : prep(1) + (r.src == SRC_CONVERT ? 2500.0 : shape.tile_n == 64 ? 5000.0 : 0.0));
+  if ((waves > 1 && (kblocks >= kSplitMaxKBlocks || shape.splits > 1)) || shape.cost == 0.0 || cost >= plain) return r;
+  if (!addressable) {
+    const size_t copies = round_up(K * route_b_pitch(N, false) * 4, 1024) + round_up(std::max(panel_rows_a, M) * round_up(K, GEMM_BK) * 4, 1024);
+    r.operand_bytes = r.src == SRC_CONVERT ? copies : std::max(copies, r.operand_bytes);
+  } else {
+    r.operand_bytes = 0;
+  }
   r.src = SRC_SPLIT;
   r.ctas = ctas;
   r.cost = shape.cost;
@@ -930,8 +951,7 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   r.stages = split_stages_of(shape.tile_n, ctas, M);
   r.tiles = tiles;
   r.waves = waves;
-  r.operand_bytes = 0;
-  r.workspace = partial_bytes(M, N, shape, ctas, sm_count);
+  r.workspace = r.operand_bytes + partial_bytes(M, N, shape, ctas, sm_count);
   return r;
 }
 
@@ -942,8 +962,13 @@ int grid_for(long long work, long long per_block, long long cap) {
 
 int launch_prep_lo(int sm_count, cudaStream_t st, const PrepLoJob& a, const PrepLoJob& b, bool b_ready, const int* gate) {
   const long long cap = static_cast<long long>(sm_count) * 16;
-  const int grid_a = a.lo || a.copy ? grid_for(static_cast<long long>(a.rows) * (a.colsp >> 2), 256, cap) : 0;
-  const int grid_b = !b_ready && (b.lo || b.copy) ? grid_for(static_cast<long long>(b.rows) * (b.colsp >> 2), 256, cap) : 0;
+  auto blocks = [&](const PrepLoJob& j) {
+    if (!j.lo && !j.copy) return 0;
+    if (j.vec_ok) return grid_for(static_cast<long long>(j.rows) * (j.colsp >> 2), 256, cap);
+    constexpr int span = 128 * PREP_SHIFT;
+    return grid_for(static_cast<long long>(j.rows) * ((j.colsp + span - 1) / span), 8, cap);
+  };
+  const int grid_a = blocks(a), grid_b = b_ready ? 0 : blocks(b);
   if (grid_a + grid_b == 0) return SB200_OK;
   CU_TRY(launch_pdl(prep_lo_two_kernel, dim3(static_cast<unsigned>(grid_a + grid_b)), dim3(256), 0, st, 1, a, b, grid_a, gate));
   return launch_check("prep_lo_two_kernel");
@@ -1015,16 +1040,10 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   int a_box_rows = GEMM_BM;
   if (route.src == SRC_CONVERT) {
     // no panels, no operand maps
-  } else if (route.src == SRC_SPLIT) {
-    a_box_rows = static_cast<int>(std::min<long long>(GEMM_BM, round_up(M, 8)));
-    if ((rc = encode_map_2d(&ma_hi, A, K, M, lda, GEMM_BK, a_box_rows, false))) return rc;
-    if ((rc = encode_map_2d(&mb_hi, B, N, K, ldb, 32, GEMM_BK, false, true))) return rc;
-    ma_lo = ma_hi;
-    mb_lo = mb_hi;
-  } else if (direct) {
+  } else if (direct || route.src == SRC_SPLIT) {
     // Workspace, B's parts first (their place does not depend on M): [B copy][B lo][A copy][A lo], each only when it is needed;
     // B's as K rows of np, A's as rows of kp.  The copies stand in for matrices TMA cannot address.
-    const bool copy_a = !addressable_a, copy_b = !addressable_b;
+    const bool copy_a = !addressable_a, copy_b = !addressable_b, lows = MODE == 3 && direct;
     const long long np = route_b_pitch(N, addressable);
     const size_t b_part = round_up(K * np * 4, 1024), a_part = round_up(panel_rows_a * kp * 4, 1024);
     uint8_t* at = static_cast<uint8_t*>(d.workspace);
@@ -1034,18 +1053,20 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
       return q;
     };
     float* b_copy = take(copy_b, b_part);
-    float* b_lo = take(MODE == 3, b_part);
+    float* b_lo = take(lows, b_part);
     float* a_copy = take(copy_a, a_part);
-    float* a_lo = take(MODE == 3, a_part);
+    float* a_lo = take(lows, a_part);
     // one launch (B's are not made again for the row blocks after the first)
     const PrepLoJob ja{A, lda, a_lo, a_copy, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp), addressable_a ? 1 : 0};
     const PrepLoJob jb{B, ldb, b_lo, b_copy, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), addressable_b ? 1 : 0};
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, b_panels_ready, nullptr))) return rc;
-    if ((rc = encode_map_2d(&ma_hi, copy_a ? a_copy : A, K, M, copy_a ? kp : lda, GEMM_BK, GEMM_BM, true))) return rc;
-    if ((rc = encode_map_2d(&mb_hi, copy_b ? b_copy : B, N, K, copy_b ? np : ldb, 32, GEMM_BK, true, true))) return rc;
+    // the split kernel takes the elements as they are
+    if (!direct) a_box_rows = static_cast<int>(std::min<long long>(GEMM_BM, round_up(M, 8)));
+    if ((rc = encode_map_2d(&ma_hi, copy_a ? a_copy : A, K, M, copy_a ? kp : lda, GEMM_BK, a_box_rows, direct))) return rc;
+    if ((rc = encode_map_2d(&mb_hi, copy_b ? b_copy : B, N, K, copy_b ? np : ldb, 32, GEMM_BK, direct, true))) return rc;
     ma_lo = ma_hi;
     mb_lo = mb_hi;
-    if (MODE == 3) {
+    if (lows) {
       if ((rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
       if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     }
@@ -2757,11 +2778,11 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
   // the second word and `launches` speak of addressability and of passes; `operands` and `kernels` say what runs
-  const bool apart = r.src == SRC_PANELS || (r.src == SRC_DIRECT && !addressable);
+  const bool apart = r.src == SRC_PANELS || (r.src != SRC_CONVERT && !addressable);
   const int reduction = r.splits > 1 && !split_in_cluster(r.tiles, r.splits, r.ctas, sm_count) ? 1 : 0;
   const int launches = (apart ? 3 : r.ctas == 2 && mode == SB200_MODE_3XTF32 ? 2 : 1) + reduction;
   const int kernels = (apart || (r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32) ? 2 : 1) + reduction;
-  const char* operands = r.src == SRC_CONVERT || (r.src == SRC_SPLIT && r.ctas == 1) ? "converted" : r.src == SRC_PANELS ? "panels" : addressable ? "direct" : "copied";
+  const char* operands = r.src == SRC_CONVERT || (r.src == SRC_SPLIT && r.ctas == 1 && addressable) ? "converted" : r.src == SRC_PANELS ? "panels" : addressable ? "direct" : "copied";
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=%s kernels=%d",
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
            r.waves, r.splits, r.workspace, launches, operands, kernels);

@@ -310,3 +310,28 @@ def test_operands_split_on_chip_give_the_same_bits_every_time(backend, device, M
     finally:
         for x in (A, B, D, other):
             x.free()
+
+
+# copies of rows that start 1, 2 and 3 elements behind a 16-byte boundary and at all four in turn; row lengths at the edges of a warp's piece
+# (512 columns), of its lanes' quads and of the padding; a matrix of which only one operand needs the copy
+@pytest.mark.parametrize("mode", [L.MODE_3XTF32, L.MODE_TF32])
+@pytest.mark.parametrize("M,N,K,off,pad", [(600, 513, 259, 1, 1), (1030, 1021, 513, 2, 0), (260, 1021, 516, 3, 2), (1025, 1030, 511, 3, 4), (1100, 514, 260, 0, 3)])
+def test_copied_rows_give_the_bits_of_the_panels(backend, device, mode, M, N, K, off, pad):
+    lda, ldb = K + pad, N + pad
+    rng = np.random.default_rng(M + N + K)
+    A, B = (dev_from(backend, device, rng.uniform(-1, 1, n).astype(np.float32), offset=off) for n in ((M - 1) * lda + K, (K - 1) * ldb + N))
+    D, out = Dev(backend, device, M * N), []
+    try:
+        text = describe(mode, M, N, K, 0)
+        assert "operands=copied" in text and "splits=1 " in text
+        for variant in (3, 0):
+            backend.set_gemm_variant(variant)
+            D.clear()
+            gemm(backend, device, mode, M, N, K, A, B, D, lda=lda, ldb=ldb)
+            out.append(D.download())
+        assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
+    finally:
+        backend.set_gemm_variant(0)
+        for x in (A, B, D):
+            x.free()
+
