@@ -161,7 +161,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       for (unsigned int kb = (group + GROUPS - before % GROUPS) % GROUPS; kb < static_cast<unsigned int>(blocks); kb += GROUPS) {
         const unsigned int n = before + kb;
         const unsigned int rs = n % RAW, rp = (n / RAW) & 1u, ps = n % PARTS, pp = (n / PARTS) & 1u;
-        // the whole k-block into registers first: one latency of shared memory, and the raw stage is free again at once
+        // the whole k-block into registers first: one latency of shared memory
         bool landed = mbar_wait_bounded(smem_u32(&raw_full[rs]), rp, abort_flag);
         const uint8_t* raw = smem + rs * Cfg::kRawBytes;
         float a[GEMM_BK], b[PART_N / 4];
@@ -177,8 +177,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           ok = false;
           break;
         }
-        __syncwarp();  // every lane has its values: without this the compiler moved loads behind the arrival, where TMA may write again
-        if (lane == 0) mbar_arrive(smem_u32(&raw_empty[rs]));
         tc_fence_after_sync();
         if (rows_here) {
           const uint32_t ta = tmem_base + lanes + Cfg::kTmemA + ps * (2 * GEMM_BK);
@@ -207,7 +205,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         fence_async_shared();  // before the tensor core reads what was written here
         tc_fence_before_sync();
         __syncwarp();
+        // Not before the values have been used: handed back right after the loads, the stage was written again while some of them, which the
+        // compiler had moved behind the arrival of another lane, were still to come.
         if (lane == 0) {
+          mbar_arrive(smem_u32(&raw_empty[rs]));
           if (CTAS == 2)
             mbar_arrive_peer(map_to_cta(smem_u32(&part_full[ps]), leader));
           else
