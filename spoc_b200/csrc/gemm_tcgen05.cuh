@@ -437,63 +437,18 @@ struct PrepLoJob {
   int rows, cols, colsp, vec_ok;
 };
 
-__device__ __forceinline__ void prep_lo_store(const PrepLoJob& j, long long row, int k, const float4& x) {
-  if (j.copy) *reinterpret_cast<float4*>(j.copy + row * j.colsp + k) = x;
-  if (j.lo)
-    *reinterpret_cast<float4*>(j.lo + row * j.colsp + k) =
-        make_float4(tf32_lo(x.x, tf32_round(x.x)), tf32_lo(x.y, tf32_round(x.y)), tf32_lo(x.z, tf32_round(x.z)),
-                    tf32_lo(x.w, tf32_round(x.w)));
-}
-
 __device__ __forceinline__ void prep_lo_rows(const PrepLoJob& j, long long block, long long nblocks) {
   const long long quads_per_row = j.colsp >> 2;
   const long long total = static_cast<long long>(j.rows) * quads_per_row;
   for (long long q = block * blockDim.x + threadIdx.x; q < total; q += nblocks * blockDim.x) {
     const long long row = q / quads_per_row;
     const int k = static_cast<int>(q - row * quads_per_row) << 2;
-    prep_lo_store(j, row, k, load_quad(j.src + row * j.ld, k, j.cols, j.vec_ok));
-  }
-}
-
-// The same for rows that do not start on 16-byte boundaries: a warp takes PREP_SHIFT quads a lane of one row at a time, loads the
-// aligned quads that cover them and shifts them into place with its neighbour's.  Elements outside the row are not read.  One
-// 128-bit load instead of four 32-bit ones a quad.
-constexpr int PREP_SHIFT = 4;
-__device__ __forceinline__ void prep_lo_rows_shifted(const PrepLoJob& j, long long block, long long nblocks) {
-  constexpr int SPAN = 32 * 4 * PREP_SHIFT;  // columns of a warp's piece
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const int pieces = (j.colsp + SPAN - 1) / SPAN;
-  const long long total = static_cast<long long>(j.rows) * pieces;
-  for (long long w = block * warps + (threadIdx.x >> 5); w < total; w += nblocks * warps) {
-    const long long row = w / pieces;
-    const int k0 = static_cast<int>(w - row * pieces) * SPAN;
-    const float* src = j.src + row * j.ld;
-    const int shift = static_cast<int>((reinterpret_cast<uintptr_t>(src + k0) >> 2) & 3);  // elements before column k0 in its aligned quad
-    auto load = [&](int k) -> float4 {  // the aligned quad whose first element is column k (k < 0 or beyond the row: partly or not read)
-      if (k >= 0 && k + 3 < j.cols) return *reinterpret_cast<const float4*>(src + k);
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k >= 0 && k < j.cols) x.x = src[k];
-      if (k + 1 >= 0 && k + 1 < j.cols) x.y = src[k + 1];
-      if (k + 2 >= 0 && k + 2 < j.cols) x.z = src[k + 2];
-      if (k + 3 >= 0 && k + 3 < j.cols) x.w = src[k + 3];
-      return x;
-    };
-    float4 q[PREP_SHIFT + 1];
-#pragma unroll
-    for (int u = 0; u < PREP_SHIFT; ++u) q[u] = load(k0 - shift + (u * 32 + lane) * 4);
-    q[PREP_SHIFT] = shift && lane == 0 ? load(k0 - shift + SPAN) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int u = 0; u < PREP_SHIFT; ++u) {
-      float4 x = q[u];
-      if (shift) {  // the same for the whole warp
-        const float4 mine = lane == 0 ? q[u + 1] : q[u];  // what the lane below takes from here
-        const float nx = __shfl_sync(0xffffffffu, mine.x, lane + 1), ny = __shfl_sync(0xffffffffu, mine.y, lane + 1),
-                    nz = __shfl_sync(0xffffffffu, mine.z, lane + 1);
-        x = shift == 1 ? make_float4(x.y, x.z, x.w, nx) : shift == 2 ? make_float4(x.z, x.w, nx, ny) : make_float4(x.w, nx, ny, nz);
-      }
-      const int k = k0 + (u * 32 + lane) * 4;
-      if (k < j.colsp) prep_lo_store(j, row, k, x);
-    }
+    const float4 x = load_quad(j.src + row * j.ld, k, j.cols, j.vec_ok);
+    if (j.copy) *reinterpret_cast<float4*>(j.copy + row * j.colsp + k) = x;
+    if (j.lo)
+      *reinterpret_cast<float4*>(j.lo + row * j.colsp + k) =
+          make_float4(tf32_lo(x.x, tf32_round(x.x)), tf32_lo(x.y, tf32_round(x.y)), tf32_lo(x.z, tf32_round(x.z)),
+                      tf32_lo(x.w, tf32_round(x.w)));
   }
 }
 
@@ -502,13 +457,10 @@ __global__ void prep_lo_two_kernel(const PrepLoJob a, const PrepLoJob b, int blo
   grid_launch_dependents();  // the GEMM behind this launch may set itself up now; it waits before reading
   grid_dependency_wait();    // launched the same way, so behind the last user of the panels' memory
   if (gate && *gate != 0) return;
-  const bool first = static_cast<int>(blockIdx.x) < blocks_a;
-  const PrepLoJob& j = first ? a : b;
-  const long long block = first ? blockIdx.x : blockIdx.x - blocks_a, nblocks = first ? blocks_a : gridDim.x - blocks_a;
-  if (j.vec_ok)
-    prep_lo_rows(j, block, nblocks);
+  if (static_cast<int>(blockIdx.x) < blocks_a)
+    prep_lo_rows(a, blockIdx.x, blocks_a);
   else
-    prep_lo_rows_shifted(j, block, nblocks);
+    prep_lo_rows(b, blockIdx.x - blocks_a, gridDim.x - blocks_a);
 }
 
 // Panels for operands TMA cannot address, A and B in one launch (blocks [0, blocks_a) work on A).

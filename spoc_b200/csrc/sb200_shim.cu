@@ -803,10 +803,11 @@ int gemm_variant_setting() {
   return variant;
 }
 
-// Products of at most this many rows are computed by blocks on their own (the fp16 modes: f16_shape): the second block of a pair
-// would only see rows past the end.  The reason holds up to 128 rows, and so does the gain: n = k = 4096 in TF32, 64 rows 18.9
-// us; 65 rows 27.3 by pairs and 18.5 by single blocks, 128 rows 27.1 and 18.9; in 3xTF32 62.6 and 44.5, 65.3 and 45.0 (1024 x 1024:
-// 9.4 and 7.9, 11.3 and 8.3; 14.0 both, 15.1 and 14.3).  The line is where the forms were first told apart.
+// Products of at most this many rows are computed by blocks on their own (the fp16 modes: f16_shape; gemm_split_kernel: route_gemm): the
+// second block of a pair would only see rows past the end.  In TF32 mode up to 128 rows from matrices B of 2^20 elements on, where the
+// estimates agree (by pairs and by single blocks: n = k = 4096 65 rows 27.3 and 18.5 us, 128 rows 27.1 and 18.9; n = k = 1024 9.4 and
+// 7.9, 11.3 and 8.3).
+constexpr long long kSingleOperand = 1 << 20;
 constexpr long long kSingleRows = 64;
 // Multiply-adds below which gemm_convert_kernel does the whole product, for addressable and for unaligned operands (in 3xTF32 unless
 // gemm_split_kernel does it).  Converted and prepared by a launch in front, 3xTF32, us: addressable 100 x 64 x 100 7.6 and 8.8, 192^3 9.4 and
@@ -867,9 +868,10 @@ TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_co
 // Row length of the parts of B the direct kernel reads from the scratch.
 long long route_b_pitch(long long N, bool addressable) { return round_up(N, addressable ? 32 : 4); }
 
-// Every route but that through gemm_split_kernel.  least_splits > 0: not through gemm_convert_kernel either, and no longer k-loops.
+// Every route but that through gemm_split_kernel.  least_splits > 0: not through gemm_convert_kernel either, no longer k-loops, and
+// with single blocks where `single` says so.
 GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a, int fixed_splits,
-                      int least_splits = 0) {
+                      int least_splits = 0, bool single = false) {
   GemmRoute r;
   const int variant = gemm_variant_setting();
   const bool three = mode == SB200_MODE_3XTF32;
@@ -885,7 +887,7 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
   const bool convert = variant == 0 && least_splits == 0 && tile_n_setting() != 256 &&
                        (addressable ? (three ? M <= kSingleRows || macs < kConvertMacs : K <= kConvertKOneTerm && macs < kConvertMacs)
                                     : M <= kSingleRows || macs < kConvertMacsUnaligned);
-  r.ctas = convert || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
+  r.ctas = convert || single || variant == 1 || (variant == 0 && !three && M <= kSingleRows) ? 1 : 2;
   r.src = convert ? SRC_CONVERT : direct ? SRC_DIRECT : SRC_PANELS;
   const int units = units_of(r.ctas, sm_count);
   // TF32 mode on addressable operands uses no scratch at all: such calls run side by side on any streams, and a graph they were
@@ -926,6 +928,10 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
     if (copied.cost > 0.0) r = copied;  // 0: pairs cannot divide the k-loop so often
   }
   if (gemm_variant_setting() != 0) return r;
+  if (!three && r.src == SRC_DIRECT && M > kSingleRows && M <= GEMM_BM && N * K >= kSingleOperand) {
+    const GemmRoute alone = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits, r.splits, true);
+    if (alone.cost > 0.0 && alone.cost < r.cost) r = alone;
+  }
   if (!three || K <= 2 * GEMM_BK) return r;
   const long long kblocks = round_up(K, GEMM_BK) / GEMM_BK;
   const int ctas = M <= 128 || macs < kConvertMacs ? 1 : 2, units = units_of(ctas, sm_count);
@@ -934,8 +940,11 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   // ns: a launch in front that reads the operands and writes their low parts, copies of them, or both
   auto prep = [&](int written) { return 1000.0 + 4.0 * (1 + written) * (static_cast<double>(M) * K + static_cast<double>(K) * N) / 5000.0; };
   const double plain = r.src == SRC_CONVERT ? r.cost : kPlainCharge * r.cost + prep(addressable ? 1 : 2);
-  // a launch in front costs 2.5 us beside its bytes; where plain_route has one too, 64-column tiles over copies bring nothing
-  const double cost = shape.cost + (addressable ? 0.0 : prep(1) + (r.src == SRC_CONVERT ? 2500.0 : shape.tile_n == 64 ? 5000.0 : 0.0));
+  // Over copies (whose launch costs 2.5 us beside its bytes) instead of conversion in registers, and for few rows and divided k-loops:
+  // otherwise the ordinary epilogue of unaligned results, which overlaps nothing here, makes gemm_pair_kernel the faster one behind
+  // the same copies (1531 x 2047 x 1021 38 us and 44, 1001 x 1003 x 1005 22.6 and 24.2; but 300 x 3001 x 3003, divided, 66 and 61).
+  if (!addressable && r.src == SRC_DIRECT && M > GEMM_BM && r.splits == 1) return r;
+  const double cost = shape.cost + (addressable ? 0.0 : prep(1) + 2500.0);
   if ((waves > 1 && (kblocks >= kSplitMaxKBlocks || shape.splits > 1)) || shape.cost == 0.0 || cost >= plain) return r;
   if (!addressable) {
     const size_t copies = round_up(K * route_b_pitch(N, false) * 4, 1024) + round_up(std::max(panel_rows_a, M) * round_up(K, GEMM_BK) * 4, 1024);
@@ -962,13 +971,8 @@ int grid_for(long long work, long long per_block, long long cap) {
 
 int launch_prep_lo(int sm_count, cudaStream_t st, const PrepLoJob& a, const PrepLoJob& b, bool b_ready, const int* gate) {
   const long long cap = static_cast<long long>(sm_count) * 16;
-  auto blocks = [&](const PrepLoJob& j) {
-    if (!j.lo && !j.copy) return 0;
-    if (j.vec_ok) return grid_for(static_cast<long long>(j.rows) * (j.colsp >> 2), 256, cap);
-    constexpr int span = 128 * PREP_SHIFT;
-    return grid_for(static_cast<long long>(j.rows) * ((j.colsp + span - 1) / span), 8, cap);
-  };
-  const int grid_a = blocks(a), grid_b = b_ready ? 0 : blocks(b);
+  const int grid_a = a.lo || a.copy ? grid_for(static_cast<long long>(a.rows) * (a.colsp >> 2), 256, cap) : 0;
+  const int grid_b = !b_ready && (b.lo || b.copy) ? grid_for(static_cast<long long>(b.rows) * (b.colsp >> 2), 256, cap) : 0;
   if (grid_a + grid_b == 0) return SB200_OK;
   CU_TRY(launch_pdl(prep_lo_two_kernel, dim3(static_cast<unsigned>(grid_a + grid_b)), dim3(256), 0, st, 1, a, b, grid_a, gate));
   return launch_check("prep_lo_two_kernel");

@@ -292,7 +292,7 @@ def test_operands_split_on_chip_give_the_bits_of_the_panels(backend, device, M, 
             x.free()
 
 
-@pytest.mark.parametrize("M,N,K", [(64, 4096, 4096), (128, 1024, 4096), (1024, 1024, 1024), (256, 2048, 4096), (2304, 2304, 520)])
+@pytest.mark.parametrize("M,N,K", [(64, 4096, 4096), (64, 4096, 1024), (128, 4096, 4096), (128, 1024, 4096), (1024, 1024, 1024), (256, 2048, 4096), (2304, 2304, 520)])
 def test_operands_split_on_chip_give_the_same_bits_every_time(backend, device, M, N, K):
     """Stages that are written again while a warp still reads them show here: operands in L2 and not, launches alone and in a row."""
     A, B = (dev_from(backend, device, O.fill(n, 74, i)) for i, n in ((1, M * K), (2, K * N)))
@@ -335,3 +335,22 @@ def test_copied_rows_give_the_bits_of_the_panels(backend, device, mode, M, N, K,
         for x in (A, B, D):
             x.free()
 
+
+def test_tf32_up_to_128_rows_in_single_blocks_match_pairs(backend, device):
+    for M, N, K in ((65, 2048, 1028), (100, 1024, 1024), (128, 4096, 4096), (128, 96, 16384)):
+        A, B = (dev_from(backend, device, O.fill(n, 75, i)) for i, n in ((1, M * K), (2, K * N)))
+        D = Dev(backend, device, M * N)
+        try:
+            text = describe(L.MODE_TF32, M, N, K, 1)
+            assert text.startswith("single direct") and "workspace=0" in text
+            gemm(backend, device, L.MODE_TF32, M, N, K, A, B, D)
+            got = D.download()
+            backend.set_gemm_variant(2)
+            gemm(backend, device, L.MODE_TF32, M, N, K, A, B, D)
+            want = D.download()
+            # two float32 sums of the same rounded products in another order: 7e-9 of the result a term (the accumulator truncates)
+            assert np.linalg.norm(got - want) <= (1e-5 + 1e-8 * K) * np.linalg.norm(want)
+        finally:
+            backend.set_gemm_variant(0)
+            for x in (A, B, D):
+                x.free()
