@@ -12,7 +12,8 @@
 //
 // Bound: the tensor pipe from 192 columns on (645 and 850 ns per k-block with 192 and 256 columns), below that the latency of the
 // groups' way from shared memory through registers to tensor memory (pairs 430 and 363 ns with 128 and 64 columns, blocks on their own
-// 540 and 375).  Against the two launches: 64 x 4096 x 4096 45 -> 26 us, 1024^3 19.9 -> 18.1, 2048^3 88 -> 77, 4096^3 634 -> 565.
+// 540 and 375).  Against the two launches, and for few rows gemm_convert_kernel: 64 x 4096 x 4096 42.6 -> 30 us, 128 x 4096 x 4096 64.5 ->
+// 33, 1024^3 20.1 -> 16.9, 2048^3 85 -> 75, 4096^3 614 -> 568.
 #pragma once
 #include "gemm_tcgen05_pair.cuh"
 

@@ -824,8 +824,8 @@ constexpr double kCopyMacs = 16777216.0;                 // 2^24
 // x 128 5.4 and 5.6; 64 x 1024 x 96 5.3 and 5.6, x 128 6.1 and 5.6; 512 x 256 x 64 5.3 and 5.6, x 96 6.1 and 5.8.
 constexpr long long kConvertKOneTerm = 128;
 // gemm_split_kernel instead of gemm_pair_kernel behind a launch for the low parts, where the estimates say so.  It moves half the bytes
-// to the SMs, which the other pays with 10 % of its time beside the estimate (2048^3 88 -> 77 us, 4096^3 634 -> 565, 1024 x 1024 x 4096
-// 55 -> 42, 2048 x 2048 x 16384 650 -> 535); but its epilogues overlap nothing (8192 x 8192 x 512, 14 waves: 360 us, the other 290).
+// to the SMs, which the other pays with 10 % of its time beside the estimate (2048^3 85 -> 75 us, 4096^3 614 -> 568, 1024 x 1024 x 4096
+// 51 -> 38, 16384 x 2048 x 2048 572 -> 540); but its epilogues overlap nothing (8192 x 8192 x 512, 14 waves: 360 us, the other 290).
 // Not in several waves of long k-loops, whose pairs gemm_pair_kernel holds together (next_epoch_ring; 8192^3 4440 and 4360 us:
 // what lockstep saves in DRAM traffic on the largest products is not to be had here), nor in several waves of a divided one
 // (64 x 16384 x 16384: 625 and 532).  With two k-blocks or one the host's encoding of the operand maps costs what the device saves: 64^3 called
