@@ -12,7 +12,7 @@
 //
 // Bound: the tensor pipe from 192 columns on (645 and 850 ns per k-block with 192 and 256 columns), below that the latency of the
 // groups' way from shared memory through registers to tensor memory (pairs 430 and 363 ns with 128 and 64 columns, blocks on their own
-// 540 and 375).  Against the two launches, and for few rows gemm_convert_kernel: 64 x 4096 x 4096 42.6 -> 30 us, 128 x 4096 x 4096 64.5 ->
+// 540 and 375).  Against the two launches, and for few rows gemm_convert_kernel: 64 x 4096 x 4096 42.6 -> 24 us, 128 x 4096 x 4096 64.5 ->
 // 33, 1024^3 20.1 -> 16.9, 2048^3 85 -> 75, 4096^3 614 -> 568.
 #pragma once
 #include "gemm_tcgen05_pair.cuh"
@@ -36,7 +36,9 @@ struct SplitCfg {
   static constexpr uint32_t kABytes = ROWS * GEMM_BK * 4;
   static constexpr uint32_t kBBytes = kPartN * GEMM_BK * 4;
   static constexpr uint32_t kRawBytes = kABytes + kBBytes;            // a raw k-block
-  static constexpr int kParts = kPartN == 32 ? 6 : kPartN == 64 || ROWS == 64 ? 4 : 3;  // k-blocks held in parts
+  // K-blocks held in parts; the rest of shared memory holds raw ones, which a stream from HBM needs more of (64 x 4096 x 4096: four and three
+  // 30.3 us, three and five 23.8).
+  static constexpr int kParts = kPartN == 32 ? 6 : kPartN == 64 ? 4 : 3;
   static constexpr uint32_t kPartBytes = 2 * kBBytes;                 // hi(B), lo(B)
   static constexpr int kRawFit = (216 * 1024 - kParts * static_cast<int>(kPartBytes)) / static_cast<int>(kRawBytes);
   static constexpr int kRaw = kRawFit > 8 ? 8 : kRawFit;
