@@ -1017,7 +1017,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   std::unique_lock<std::mutex> scratch_lock(d.scratch_mu, std::defer_lock);
   if (route.workspace) {
     scratch_lock.lock();
-    b_panels_ready = b_prepared && *b_prepared == d.ws_uses && route.workspace <= d.workspace_bytes;
+    b_panels_ready = route.src != SRC_SPLIT && b_prepared && *b_prepared == d.ws_uses && route.workspace <= d.workspace_bytes;
     rc = ensure_workspace(d, route.workspace);
     if (rc) return rc;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1117,7 +1117,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   if (track_scratch && rc == SB200_OK) {
     rc = scratch_release(d, st);
   }
-  if (b_prepared) *b_prepared = route.operand_bytes ? d.ws_uses : 0;
+  // gemm_split_kernel's copies leave no low parts of B, and A's copy lies where those would
+  if (b_prepared) *b_prepared = route.operand_bytes && route.src != SRC_SPLIT ? d.ws_uses : 0;
   return rc;
 }
 

@@ -354,3 +354,14 @@ def test_tf32_up_to_128_rows_in_single_blocks_match_pairs(backend, device):
             backend.set_gemm_variant(0)
             for x in (A, B, D):
                 x.free()
+
+
+@pytest.mark.parametrize("M,N,K", [(455, 1149, 6946), (600, 100, 3001), (700, 1001, 1003), (1100, 301, 2050), (390, 2001, 3003)])
+def test_row_blocks_of_unaligned_host_operands_by_different_kernels(backend, device, M, N, K):
+    """The blocks of one host-operand product may be split on chip over copies or read beside panels of low parts: what one leaves in the
+    scratch is no preparation for the other."""
+    a, b, d = O.fill(M * K, 76, 1), O.fill(K * N, 76, 2), np.empty(M * N, np.float32)
+    ptr = lambda x: x.ctypes.data_as(C.c_void_p)   # noqa: E731
+    lib = L.load()
+    assert lib.sb200_gemm_f32_host(device.id, L.MODE_3XTF32, M, N, K, ptr(a), K, ptr(b), N, ptr(d), N, 1.0, None, 0, 0.0, None, 0) == 0
+    assert O.gemm_rel_error(d.reshape(M, N), O.gemm(a, b, M, N, K)) <= tol(L.MODE_3XTF32, K)
