@@ -408,8 +408,8 @@ SB200_API int sb200_chain_triad_square_f32(int dev, uint64_t stream, uint64_t d,
 SB200_API int sb200_set_mode(int mode);
 SB200_API int sb200_get_mode(int *mode);
 /* which tensor-core kernel sb200_gemm_f32 launches: 0 = automatic (CTA pairs on 256-row tiles; single CTAs on 128-row
- * tiles for up to 64 rows, 128 in the fp16 modes; for few rows and for small products a kernel that converts the operands
- * in registers; k-loops divided where tiles leave SMs idle), 1 = always single-CTA tiles fed from prepared panels, 2 =
+ * tiles for up to 64 rows, 128 in the fp16 modes and against large matrices; 3xTF32 mostly a kernel that splits the operands on chip;
+ * for few unaligned rows and the smallest products one that converts them in registers; k-loops divided where tiles leave SMs idle), 1 = always single-CTA tiles fed from prepared panels, 2 =
  * always CTA pairs, 3 = CTA pairs fed from prepared operand panels even where TF32 mode could read the caller's matrices
  * directly.  Also SAREK_B200_GEMM=single|pair|pair-panels.  All variants round operands to TF32 the same way
  * (nearest-even) and sum k ascending, so their results agree to the last bit unless the automatic choice divides the
