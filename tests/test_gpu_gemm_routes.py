@@ -259,9 +259,10 @@ def test_the_described_kernels_are_the_ones_launched(backend, device, mode, M, N
 
 
 # (M, N, K): rows and columns at the edges of 64- and 128-row blocks and of every tile width, pairs whose second block has no rows, k-loops
-# shorter than, as long as and one beyond the rings, k that ends within a k-block, more tiles than pairs
+# shorter than, as long as and one beyond the rings, k that ends within a k-block, more tiles than pairs, the last two with the ordinary
+# epilogue, whose staging tiles lie where the loads of the next tile land
 SPLIT = [(1, 4, 65), (64, 64, 96), (63, 68, 100), (65, 64, 96), (128, 128, 256), (129, 60, 257), (257, 516, 288), (300, 1000, 300), (512, 64, 512),
-         (1536, 2044, 260), (2048, 2052, 68), (2304, 2304, 520)]
+         (1536, 2044, 260), (2048, 2052, 68), (2304, 2304, 520), (3000, 2001, 1000), (2305, 2303, 776)]
 
 
 @pytest.mark.parametrize("M,N,K", SPLIT)
