@@ -227,7 +227,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // compiler had moved behind the arrival of another lane, were still to come.
         if (lane == 0) {
           mbar_arrive(smem_u32(&raw_empty[rs]));
-          if (CTAS == 2)
+          if (CTAS == 2 && rank != 0)
             mbar_arrive_peer(map_to_cta(smem_u32(&part_full[ps]), leader));
           else
             mbar_arrive(smem_u32(&part_full[ps]));
@@ -335,7 +335,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           break;
         }
         for (int kb = 0; kb < blocks; ++kb) {
-          if (!mbar_wait_bounded(smem_u32(&part_full[stage]), phase, abort_flag)) {
+          const uint32_t full = smem_u32(&part_full[stage]);
+          if (!(CTAS == 2 ? mbar_wait_cluster(full, phase, abort_flag) : mbar_wait_bounded(full, phase, abort_flag))) {
             atomicCAS(p.status, 0, 0x3300 | stage);
             ok = false;
             break;

@@ -31,17 +31,30 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// CLUSTER: an observation at the scope of the cluster, without a fence of its own.
+template <bool CLUSTER = false>
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.b32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.b32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.b32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok;
 }
 
@@ -52,13 +65,14 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // The abort flag lives in shared memory so every role sees it quickly.
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s, far above any legitimate wait
 
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                                   uint64_t limit_ns = kWaitLimitNs) {
   // The clock is read for the first time after 64 attempts: reading %globaltimer after the first failed one put about
   // 100 ns into every wait that was not already over, and a k-loop waits once per stage.
   uint64_t t0 = 0;
   for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     if ((it & 63u) == 0u) {
       if (*abort_flag) return false;
       const uint64_t now = global_timer_ns();
@@ -69,6 +83,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
       }
     }
   }
+}
+
+// A wait for signals of mbar_arrive_peer: what they announce is ordered before what follows.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  const bool ok = mbar_wait_bounded<true>(bar, parity, abort_flag);
+  asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+  return ok;
 }
 
 // For a role that gives up: a bounded time in which copies still in flight land, so that none writes to the shared memory of a
@@ -282,11 +303,14 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same with what the arrival releases left at the scope of this block.  For signals about work that the tensor core reads from
-// this block's own shared and tensor memory: nothing of it has to become visible elsewhere, and the fence of the cluster form, which
-// waits for the whole chip, took 1400 cycles.
+// The same for signals about nothing but this block's own shared memory and tensor memory (which the other block's MMAs read): the release
+// is restricted to objects in shared::cta, and mbar_wait_cluster is its acquiring side.  Tensor memory is ordered by tcgen05.wait::st and
+// tcgen05.fence.  The unrestricted release waits for the whole chip, 1400 cycles: 1024^3 17.2 us so and 22.0 with it.
 __device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile(
+      "fence.release.sync_restrict::shared::cta.cluster;\n"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+      : "memory");
 }
 // TMA load whose completion bytes are counted on an mbarrier of either block of the pair (`bar` is a shared::cluster address), with
 // an L2 eviction policy (from l2_policy below) for the lines it brings in; data lands in this block.
