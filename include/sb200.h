@@ -394,6 +394,10 @@ SB200_API int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t
  * launch makes both.  addressable = operands 16-byte aligned with row strides that are multiples of 4 floats.  Needs no GPU. */
 SB200_API int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressable, int sm_count,
                                   char *out, int outlen);
+/* the same for M rows and N columns computed as a part of a product of whole_M rows and whole_N columns (a partial launch, a row block of
+ * the calls on host operands, a device's share): its k-loops are divided as the whole's, so that it has the whole's bits. */
+SB200_API int sb200_gemm_describe_part(int mode, int64_t M, int64_t N, int64_t K, int64_t whole_M, int64_t whole_N, int addressable,
+                                       int sm_count, char *out, int outlen);
 
 /* c = a + b  (benchmarks/bench_vector_add.ml:47-55) */
 SB200_API int sb200_vector_add_f32(int dev, uint64_t stream, uint64_t c, uint64_t a, uint64_t b, int64_t n);

@@ -891,8 +891,9 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
   r.src = convert ? SRC_CONVERT : direct ? SRC_DIRECT : SRC_PANELS;
   const int units = units_of(r.ctas, sm_count);
   // TF32 mode on addressable operands uses no scratch at all: such calls run side by side on any streams, and a graph they were
-  // captured into stays good whatever other calls do to the scratch.  (A part always finds a cut: it has no more tiles than
-  // its whole, or up to twice as many single blocks, for which there is room for more than twice as many clusters.)
+  // captured into stays good whatever other calls do to the scratch.  (A part of a product by pairs always finds a cut: it has no more
+  // tiles than its whole, or up to twice as many single blocks, for which there is room for more than twice as many clusters.  A part of
+  // one by single blocks finds it by single blocks: route_gemm.)
   const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, r.src, !three && addressable,
                                        least_splits > 0 ? least_splits : 1);
   r.cost = shape.cost;
@@ -914,10 +915,13 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
 
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
   int fixed_splits = 0;
+  bool whole_alone = false;  // a part of a product that runs by single blocks: pairs may have no room for its division
   if (part_of_whole(M, N)) {
     const Whole whole = t_whole;
     t_whole = Whole();
-    fixed_splits = route_gemm(mode, whole.rows, whole.cols, K, addressable, sm_count, whole.rows).splits;
+    const GemmRoute w = route_gemm(mode, whole.rows, whole.cols, K, addressable, sm_count, whole.rows);
+    fixed_splits = w.splits;
+    whole_alone = w.src == SRC_DIRECT && w.ctas == 1;
     t_whole = whole;
   }
   GemmRoute r = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits);
@@ -928,9 +932,9 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
     if (copied.cost > 0.0) r = copied;  // 0: pairs cannot divide the k-loop so often
   }
   if (gemm_variant_setting() != 0) return r;
-  if (!three && r.src == SRC_DIRECT && M > kSingleRows && M <= GEMM_BM && N * K >= kSingleOperand) {
-    const GemmRoute alone = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits, r.splits, true);
-    if (alone.cost > 0.0 && alone.cost < r.cost) r = alone;
+  if (!three && r.src == SRC_DIRECT && M > kSingleRows && M <= GEMM_BM && (whole_alone || N * K >= kSingleOperand)) {
+    const GemmRoute alone = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits, fixed_splits ? fixed_splits : r.splits, true);
+    if (alone.cost > 0.0 && (whole_alone || alone.cost < r.cost)) r = alone;
   }
   if (!three || K <= 2 * GEMM_BK) return r;
   const long long kblocks = round_up(K, GEMM_BK) / GEMM_BK;
@@ -2792,6 +2796,13 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
            r.waves, r.splits, r.workspace, launches, operands, kernels);
   return copy_out(buf, out, outlen);
+}
+
+int sb200_gemm_describe_part(int mode, int64_t M, int64_t N, int64_t K, int64_t whole_M, int64_t whole_N, int addressable, int sm_count,
+                             char* out, int outlen) {
+  if (whole_M < M || whole_N < N) return fail(SB200_ERR_INVALID_VALUE, "bad argument");
+  const sb200::PartsOf whole(whole_M, whole_N);
+  return sb200_gemm_describe(mode, M, N, K, addressable, sm_count, out, outlen);
 }
 
 int sb200_vector_add_f32(int dev, uint64_t stream, uint64_t c, uint64_t a, uint64_t b, int64_t n) {

@@ -60,6 +60,35 @@ def test_tf32_mode_reads_addressable_operands_without_scratch():
     assert divided > 100
 
 
+def describe_part(mode, part, whole, K, addressable):
+    out = C.create_string_buffer(256)
+    assert L.load().sb200_gemm_describe_part(mode, *part, K, *whole, addressable, SMS, out, 256) == 0
+    return dict(kv.split("=") for kv in out.value.decode().split()[2:])
+
+
+@pytest.mark.parametrize("addressable", [1, 0])
+@pytest.mark.parametrize("mode", [L.MODE_3XTF32, L.MODE_TF32, L.MODE_3XF16, L.MODE_F16])
+def test_a_part_has_the_division_of_its_whole(mode, addressable):
+    """Rows, columns or both of a product, as partial launches and row blocks compute them: a k-loop divided otherwise has other bits."""
+    rng = random.Random(9)
+    pairs = [((128, 4096), (100, 4096), 4096), ((128, 2048), (100, 2048), 4096), ((96, 1056), (96, 678), 1600), ((128, 4096), (65, 17), 4096),
+             ((64, 4096), (37, 4096), 4096), ((128, 96), (128, 1), 16384)]
+    while len(pairs) < 3000:
+        M, N, K = (int(2 ** rng.uniform(0, 13.5)) for _ in range(3))
+        if rng.random() < 0.3:
+            M = rng.randint(65, 128)
+        part = (rng.randint(1, M) if rng.random() < 0.7 else M, rng.randint(1, N) if rng.random() < 0.5 else N)
+        pairs.append(((M, N), part, K))
+    divided = 0
+    for whole, part, K in pairs:
+        w = describe(mode, *whole, K, addressable)
+        p = describe_part(mode, part, whole, K, addressable)
+        assert p["splits"] == w["splits"], (whole, part, K, w, p)
+        assert mode != L.MODE_TF32 or not addressable or p["workspace"] == "0"
+        divided += w["splits"] != "1"
+    assert divided > 300
+
+
 def test_degenerate_and_bad_arguments():
     out = C.create_string_buffer(64)
     lib = L.load()

@@ -196,7 +196,7 @@ def test_a_row_block_that_needs_more_scratch_still_finds_b():
 # (form, grid, block, m, n, k): launches that compute the first rows (and part of the next one), or the first rows and columns, of a
 # product whose k-loop is divided
 PARTIAL = [("naive", (37 * 4096 + 100, 1), 1, 64, 4096, 4096), ("naive", (5 * 300 + 7, 1), 1, 40, 300, 2000), ("tiled", (75, 3), 16, 64, 4096, 4096),
-           ("tiled", (2, 2), 16, 1024, 96, 3000)]
+           ("tiled", (2, 2), 16, 1024, 96, 3000), ("naive", (100 * 4096, 1), 1, 128, 4096, 4096), ("tiled", (11, 6), 16, 96, 1056, 4000)]
 
 
 @pytest.mark.parametrize("mode", MODES)
