@@ -814,9 +814,8 @@ constexpr long long kSingleRows = 64;
 // 8.9, 256^3 11.3 and 9.8.
 constexpr double kConvertMacs = 16777216.0;              // 2^24
 constexpr double kConvertMacsUnaligned = 134217728.0;    // 2^27
-// Of the unaligned products below that line and of more than kSingleRows rows, those from here on are copied by a launch in front all the
-// same, with k-loops no longer than the converting kernel would give them.  Converted and copied, us: 3xTF32 128^3 9.0 and 9.3, 191 x 193 x 195
-// 12.9 and 9.9, 255 x 257 x 259 15.2 and 10.5, 449^3 21.5 and 12.6; TF32 128^3 7.3 and 8.5, 255 x 257 x 259 11.3 and 9.1, 449^3 15.1 and 10.1.
+// Unaligned products below that line, of more than kSingleRows rows, may be copied by a launch in front all the same, from these many
+// multiply-adds on, with k-loops no longer than the converting kernel would give them (copies_cost says where).
 constexpr double kCopyMacsThree = 4194304.0;             // 2^22
 constexpr double kCopyMacs = 16777216.0;                 // 2^24
 // In TF32 mode, where aligned operands need no preparation, it is the shorter way for k-loops of a few k-blocks only: no operand
@@ -913,6 +912,15 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
   return r;
 }
 
+// What copying the operands costs a product that could be converted in registers, ns beside the estimate of the kernel over the copies.
+// Fitted to 470 shapes of 2^21.5 to 2^27 multiply-adds timed both ways: what pays for the copies is the shorter time per k-block, so short
+// k-loops are converted (3xTF32 97 x 8712 x 43 converted 7.8 us, copied 16.1; TF32 114 x 10433 x 96 11.9 and 20.4, 854 x 1182 x 27 5.6
+// and 9.9) and long ones copied (3xTF32 255 x 257 x 259 15.2 and 10.5, 449^3 21.5 and 12.6; TF32 449^3 15.1 and 10.1).  A pair whose second
+// block has no rows wins less.
+double copies_cost(bool three, int ctas, long long M, long long N, long long K) {
+  return (three ? 2500.0 : 5000.0) + (ctas == 2 && M <= GEMM_BM ? 2500.0 : 0.0) + (static_cast<double>(M) * K + static_cast<double>(K) * N) / 500.0;
+}
+
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
   int fixed_splits = 0;
   bool whole_alone = false;  // a part of a product that runs by single blocks: pairs may have no room for its division
@@ -929,7 +937,8 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   const bool three = mode == SB200_MODE_3XTF32;
   if (r.src == SRC_CONVERT && !addressable && M > kSingleRows && macs >= (three ? kCopyMacsThree : kCopyMacs)) {
     const GemmRoute copied = plain_route(mode, M, N, K, addressable, sm_count, panel_rows_a, fixed_splits, r.splits);
-    if (copied.cost > 0.0) r = copied;  // 0: pairs cannot divide the k-loop so often
+    // 0: pairs cannot divide the k-loop so often
+    if (copied.cost > 0.0 && copied.cost + copies_cost(three, copied.ctas, M, N, K) < r.cost) r = copied;
   }
   if (gemm_variant_setting() != 0) return r;
   if (!three && r.src == SRC_DIRECT && M > kSingleRows && M <= GEMM_BM && (whole_alone || N * K >= kSingleOperand)) {

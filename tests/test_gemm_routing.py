@@ -46,6 +46,17 @@ def test_operands_tma_cannot_address_go_through_panels():
     assert describe(L.MODE_TF32, 100, 300, 500, addressable=1)["kernel"] == "pair direct"
 
 
+def test_unaligned_operands_of_short_k_loops_are_converted():
+    """In registers on their way: a copy in front of a few k-blocks takes longer than it saves (up to twice the time)."""
+    for mode, shape in [(L.MODE_3XTF32, (97, 8712, 43)), (L.MODE_TF32, (114, 10433, 96)), (L.MODE_TF32, (854, 1182, 27)), (L.MODE_TF32, (77, 2794, 356)),
+                        (L.MODE_3XTF32, (343, 3112, 9)), (L.MODE_3XTF32, (69, 1908, 149))]:
+        d = describe(mode, *shape, addressable=0)
+        assert d["operands"] == "converted" and d["workspace"] == "0", (mode, shape, d)
+    for mode, shape in [(L.MODE_3XTF32, (255, 257, 259)), (L.MODE_3XTF32, (449, 449, 449)), (L.MODE_TF32, (449, 449, 449)), (L.MODE_3XTF32, (600, 513, 259)),
+                        (L.MODE_TF32, (600, 513, 259))]:
+        assert describe(mode, *shape, addressable=0)["operands"] == "copied", (mode, shape)
+
+
 def test_tf32_mode_reads_addressable_operands_without_scratch():
     """Long k-loops over few tiles among them: their partial sums stay within a cluster, so that calls on different streams, and
     graphs they were captured into, share nothing."""
