@@ -918,7 +918,7 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
 // and 9.9) and long ones copied (3xTF32 255 x 257 x 259 15.2 and 10.5, 449^3 21.5 and 12.6; TF32 449^3 15.1 and 10.1).  A pair whose second
 // block has no rows wins less.
 double copies_cost(bool three, int ctas, long long M, long long N, long long K) {
-  return (three ? 2500.0 : 5000.0) + (ctas == 2 && M <= GEMM_BM ? 2500.0 : 0.0) + (static_cast<double>(M) * K + static_cast<double>(K) * N) / 500.0;
+  return (three ? 2500.0 : 4500.0) + (ctas == 2 && M <= GEMM_BM ? 2500.0 : 0.0) + (static_cast<double>(M) * K + static_cast<double>(K) * N) / 500.0;
 }
 
 GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addressable, int sm_count, long long panel_rows_a) {
