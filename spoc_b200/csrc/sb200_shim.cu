@@ -831,6 +831,7 @@ constexpr long long kConvertKOneTerm = 128;
 // in a row 5.80 us and by gemm_convert_kernel 5.71, 32^3 6.6 and 6.5; 128^3 6.4 and 7.4.
 constexpr double kPlainCharge = 1.1;
 constexpr long long kSplitMaxKBlocks = 256;
+constexpr long long kNarrowRows = 768;
 
 int stages_of(bool three, int bn, int ctas) {
   const long long stage = (three ? 2 : 1) * (16384ll + (bn / ctas) * 128ll);
@@ -946,6 +947,9 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
     if (alone.cost > 0.0 && (whole_alone || alone.cost < r.cost)) r = alone;
   }
   if (!three || K <= 2 * GEMM_BK) return r;
+  // Many blocks against a B of a few columns, whose short rows they all load at once, wait for those loads: 3xTF32 14000 x 4 x 200 17.3 us,
+  // converted 10.2; 9000 x 4 x 100 10.3 and 7.7, 9000 x 8 x 100 9.0 and 7.7, 6000 x 8 x 100 even, 4000 x 16 x 100 6.7 and 7.6.
+  if (r.src == SRC_CONVERT && addressable && M > kNarrowRows * N) return r;
   const long long kblocks = round_up(K, GEMM_BK) / GEMM_BK;
   const int ctas = M <= 128 || macs < kConvertMacs ? 1 : 2, units = units_of(ctas, sm_count);
   const TileShape shape = choose_tiles(M, N, kblocks, ctas, units, true, true, fixed_splits, SRC_SPLIT, false, r.splits);

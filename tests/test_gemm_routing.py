@@ -57,6 +57,14 @@ def test_unaligned_operands_of_short_k_loops_are_converted():
         assert describe(mode, *shape, addressable=0)["operands"] == "copied", (mode, shape)
 
 
+def test_many_rows_against_a_few_columns_are_converted_in_eight_warps():
+    """gemm_convert_kernel's four stages of a 64-column tile, not the six of the splitting kernel, which waits for B's short rows."""
+    for shape in [(9000, 4, 100), (14000, 4, 200), (9000, 8, 100), (14000, 16, 72)]:
+        assert describe(L.MODE_3XTF32, *shape)["stages"] == "4", shape
+    for shape in [(4000, 16, 100), (6000, 16, 128), (9000, 32, 128)]:
+        assert describe(L.MODE_3XTF32, *shape)["stages"] != "4", shape
+
+
 def test_tf32_mode_reads_addressable_operands_without_scratch():
     """Long k-loops over few tiles among them: their partial sums stay within a cluster, so that calls on different streams, and
     graphs they were captured into, share nothing."""
