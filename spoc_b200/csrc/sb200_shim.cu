@@ -1020,9 +1020,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   if (panel_rows_a < M) panel_rows_a = M;
   const bool addressable_a = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0,
              addressable_b = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (ldb & 3) == 0, addressable = addressable_a && addressable_b;
-  const GemmRoute route = route_gemm(MODE == 3 ? SB200_MODE_3XTF32 : SB200_MODE_TF32, M, N, K, addressable, d.sm_count, panel_rows_a);
-  const bool direct = route.src == SRC_DIRECT;
-  const int tile_n = route.tile_n;
+  constexpr int mode = MODE == 3 ? SB200_MODE_3XTF32 : SB200_MODE_TF32;
+  GemmRoute route = route_gemm(mode, M, N, K, addressable, d.sm_count, panel_rows_a);
 
   const long long kp = round_up(K, GEMM_BK);
   const size_t a_bytes = round_up(panel_rows_a * kp * 4, 1024), b_bytes = round_up(N * kp * 4, 1024);
@@ -1034,19 +1033,35 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   std::unique_lock<std::mutex> scratch_lock(d.scratch_mu, std::defer_lock);
   if (route.workspace) {
     scratch_lock.lock();
-    b_panels_ready = route.src != SRC_SPLIT && b_prepared && *b_prepared == d.ws_uses && route.workspace <= d.workspace_bytes;
-    rc = ensure_workspace(d, route.workspace);
-    if (rc) return rc;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
       cudaGetLastError();
       cap = cudaStreamCaptureStatusActive;
     }
     track_scratch = cap == cudaStreamCaptureStatusNone;
+    b_panels_ready = route.src != SRC_SPLIT && b_prepared && *b_prepared == d.ws_uses && route.workspace <= d.workspace_bytes;
+    // A scratch that is too small and cannot grow (not while the stream is being captured, nor without memory) leaves a product that would
+    // be copied to the converting kernel, which needs none or less: with the same division, and so the same bits, before its own.
+    rc = track_scratch || route.workspace <= d.workspace_bytes ? ensure_workspace(d, route.workspace) : static_cast<int>(SB200_ERR_INVALID_VALUE);
+    for (int splits : {route.splits, 0}) {
+      if (rc == SB200_OK || (splits == 0 && part_of_whole(M, N))) break;
+      const GemmRoute converted = plain_route(mode, M, N, K, addressable, d.sm_count, panel_rows_a, splits);
+      if (converted.src != SRC_CONVERT || converted.workspace >= route.workspace) continue;
+      if (!track_scratch && converted.workspace > d.workspace_bytes) continue;
+      if ((rc = ensure_workspace(d, converted.workspace)) == SB200_OK) {
+        route = converted;
+        b_panels_ready = false;
+      }
+    }
+    if (rc) rc = ensure_workspace(d, route.workspace);
+    if (rc) return rc;
+    track_scratch = track_scratch && route.workspace;
     if (track_scratch) {
       if ((rc = scratch_acquire(d, st))) return rc;
     }
   }
+  const bool direct = route.src == SRC_DIRECT;
+  const int tile_n = route.tile_n;
   unsigned int* epoch_ring =
       route.ctas == 2 && route.splits == 1 && route.src != SRC_SPLIT ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
   const bool prof = g_profiling.load() != 0;

@@ -193,6 +193,56 @@ def test_a_row_block_that_needs_more_scratch_still_finds_b():
     assert res.returncode == 0, res.stderr[-2000:]
 
 
+CAPTURED_FIRST = """
+import numpy as np
+from cuda.bindings import runtime as rt
+from spoc_b200 import Backend, _lib as L
+from tests import oracle_lib as O
+from tests.gpu_util import Dev, dev_from
+from tests.test_gpu_gemm import tol
+
+ok = rt.cudaError_t.cudaSuccess
+backend = Backend()
+backend.Device.init()
+device, lib = backend.Device.get(0), L.load()
+err, stream = rt.cudaStreamCreateWithFlags(rt.cudaStreamNonBlocking)
+assert err == ok
+captured = []
+for mode in (L.MODE_TF32, L.MODE_3XTF32):
+    for m, n, k in ((130, 130, 120), (449, 449, 449), (300, 300, 301)):     # the first one in front of the captures: kernels are loaded
+        a, b = O.fill(m * k, 77, 1), O.fill(k * n, 77, 2)
+        A, B, D = dev_from(backend, device, a, offset=1), dev_from(backend, device, b, offset=1), Dev(backend, device, m * n)
+        args = (mode, m, n, k, A.ptr, k, B.ptr, n, D.ptr, n, 1.0, 0, 0, 0.0, 0, 0)
+        if k != 120:
+            assert rt.cudaStreamBeginCapture(stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)[0] == ok
+        rc = lib.sb200_gemm_f32(device.id, int(stream), *args)
+        assert rc == 0, lib.sb200_last_error_string()
+        if k != 120:
+            err, graph = rt.cudaStreamEndCapture(stream)
+            assert err == ok
+            err, run = rt.cudaGraphInstantiate(graph, 0)
+            assert err == ok and rt.cudaGraphLaunch(run, stream)[0] == ok
+        assert rt.cudaStreamSynchronize(stream)[0] == ok
+        got = D.download()
+        err = O.gemm_rel_error(got.reshape(m, n), O.gemm(a, b, m, n, k))
+        assert err <= tol(mode, k), err
+        captured.append((args, got, D, A, B))
+for args, got, D, *_ in captured:       # with a scratch, by copies
+    D.clear()
+    assert lib.sb200_gemm_f32(device.id, 0, *args) == 0
+    backend.Device.synchronize(device)
+    assert np.array_equal(D.download().view(np.uint32), got.view(np.uint32))
+"""
+
+
+def test_unaligned_products_can_be_captured_before_there_is_any_scratch():
+    """Copied where there is a scratch to copy into, converted in registers, with the same bits, where a capture keeps it from growing.  A
+    process of its own, in which nothing has sized the scratch."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", CAPTURED_FIRST], cwd=root, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+
+
 # (form, grid, block, m, n, k): launches that compute the first rows (and part of the next one), or the first rows and columns, of a
 # product whose k-loop is divided
 PARTIAL = [("naive", (37 * 4096 + 100, 1), 1, 64, 4096, 4096), ("naive", (5 * 300 + 7, 1), 1, 40, 300, 2000), ("tiled", (75, 3), 16, 64, 4096, 4096),
