@@ -387,9 +387,9 @@ SB200_API int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t
 /* how sb200_gemm_f32 would run these sizes on a device with sm_count SMs, as text:
  * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L operands=O kernels=N"
  * (fp16 modes: "fp16-panels", mixed mode: "mixed" without splits, for the second word).  N is the number of kernels the call launches
- * and O what becomes of A and B: direct (read where they lie by pairs, which in 3xTF32 mode split them on chip, or read panels of
- * their low parts beside), copied (row by row first, beside such panels), converted (by single blocks, in registers on their way), panels
- * (written in full) or mixed.  L counts the making of 3xTF32's low parts as a pass wherever it happens.  The second word says
+ * and O what becomes of A and B: direct (read where they lie; in 3xTF32 mode beside panels of their low parts, which a launch in front
+ * writes), split (3xTF32: read where they lie and split on chip), copied (row by row first, beside the same panels), copied+split (row by
+ * row first, the copies split on chip), converted (in registers on their way), panels (written in full) or mixed.  The second word says
  * "panels" for every product of operands that are not addressable, and L counts their preparation as two passes, although one
  * launch makes both.  addressable = operands 16-byte aligned with row strides that are multiples of 4 floats.  Needs no GPU. */
 SB200_API int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressable, int sm_count,

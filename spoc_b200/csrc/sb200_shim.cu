@@ -2815,11 +2815,14 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
   const GemmRoute r = route_gemm(mode, M, N, K, addressable != 0, sm_count, M);
   char buf[256];
   // the second word and `launches` speak of addressability and of passes; `operands` and `kernels` say what runs
-  const bool apart = r.src == SRC_PANELS || (r.src != SRC_CONVERT && !addressable);
+  const bool apart = r.src == SRC_PANELS || (r.src != SRC_CONVERT && !addressable), lows = r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32;
   const int reduction = r.splits > 1 && !split_in_cluster(r.tiles, r.splits, r.ctas, sm_count) ? 1 : 0;
-  const int launches = (apart ? 3 : r.ctas == 2 && mode == SB200_MODE_3XTF32 ? 2 : 1) + reduction;
-  const int kernels = (apart || (r.src == SRC_DIRECT && mode == SB200_MODE_3XTF32) ? 2 : 1) + reduction;
-  const char* operands = r.src == SRC_CONVERT || (r.src == SRC_SPLIT && r.ctas == 1 && addressable) ? "converted" : r.src == SRC_PANELS ? "panels" : addressable ? "direct" : "copied";
+  const int launches = (apart ? 3 : lows ? 2 : 1) + reduction, kernels = (apart || lows ? 2 : 1) + reduction;
+  const char* operands = r.src == SRC_CONVERT ? "converted"
+                         : r.src == SRC_SPLIT ? (addressable ? "split" : "copied+split")
+                         : r.src == SRC_PANELS ? "panels"
+                         : addressable         ? "direct"
+                                               : "copied";
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=%s kernels=%d",
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
            r.waves, r.splits, r.workspace, launches, operands, kernels);

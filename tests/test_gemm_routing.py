@@ -20,11 +20,13 @@ def test_benchmark_configurations_take_the_large_tile(mode):
     for shape in [(8192, 8192, 8192), (32768 // 8, 32768, 32768), (65536 // 8, 4096, 4096), (4096, 4096, 4096), (2048, 2048, 2048)]:
         d = describe(mode, *shape)
         assert d["kernel"] == "pair direct" and d["tile"] == "256x256", (shape, d)
-        assert d["launches"] == ("2" if mode == L.MODE_3XTF32 else "1")
+        # 3xTF32 reads the largest ones beside panels of low parts, which are a launch of their own, and splits the others on chip
+        assert (d["operands"], d["launches"], d["kernels"]) in ([("direct", "2", "2"), ("split", "1", "1")] if mode == L.MODE_3XTF32 else [("direct", "1", "1")])
     d = describe(L.MODE_TF32, 8192, 8192, 8192)
     assert d["stages"] == "6" and d["tiles"] == "1024" and d["waves"] == "14" and d["workspace"] == "0"
     d = describe(L.MODE_3XTF32, 8192, 8192, 8192)
     assert d["stages"] == "3" and d["workspace"] == str(2 * 8192 * 8192 * 4)     # the two low-part panels
+    assert d["operands"] == "direct" and describe(L.MODE_3XTF32, 4096, 4096, 4096)["operands"] == "split"
 
 
 def test_problems_with_few_tiles_take_narrower_tiles():
@@ -58,11 +60,11 @@ def test_unaligned_operands_of_short_k_loops_are_converted():
 
 
 def test_many_rows_against_a_few_columns_are_converted_in_eight_warps():
-    """gemm_convert_kernel's four stages of a 64-column tile, not the six of the splitting kernel, which waits for B's short rows."""
+    """And not by the splitting kernel, which waits for B's short rows."""
     for shape in [(9000, 4, 100), (14000, 4, 200), (9000, 8, 100), (14000, 16, 72)]:
-        assert describe(L.MODE_3XTF32, *shape)["stages"] == "4", shape
+        assert describe(L.MODE_3XTF32, *shape)["operands"] == "converted", shape
     for shape in [(4000, 16, 100), (6000, 16, 128), (9000, 32, 128)]:
-        assert describe(L.MODE_3XTF32, *shape)["stages"] != "4", shape
+        assert describe(L.MODE_3XTF32, *shape)["operands"] == "split", shape
 
 
 def test_tf32_mode_reads_addressable_operands_without_scratch():

@@ -280,10 +280,10 @@ def test_a_partial_launch_has_the_bits_of_the_whole(backend, device, mode, form,
         assert not out[1][rows:].any() and not out[1][:, cols:].any()
 
 
-# (mode, M, N, K, aligned, how the operands are read): converted, read in place, copied, panels in one launch and in two, with the
-# k-loop whole, divided within clusters and divided through global memory
-KERNELS = [(L.MODE_3XTF32, 64, 64, 64, True, "converted"), (L.MODE_3XTF32, 64, 8192, 8192, True, "converted"), (L.MODE_TF32, 65, 33, 100, False, "converted"),
-           (L.MODE_3XTF32, 512, 512, 512, True, "direct"), (L.MODE_TF32, 512, 512, 512, True, "direct"), (L.MODE_TF32, 128, 96, 4096, True, "direct"),
+# (mode, M, N, K, aligned, how the operands are read): converted, read in place, split on chip, copied, panels in one launch and in two, with
+# the k-loop whole, divided within clusters and divided through global memory
+KERNELS = [(L.MODE_3XTF32, 64, 64, 64, True, "converted"), (L.MODE_3XTF32, 64, 8192, 8192, True, "converted"), (L.MODE_3XTF32, 64, 4096, 4096, True, "split"), (L.MODE_TF32, 65, 33, 100, False, "converted"),
+           (L.MODE_3XTF32, 512, 512, 512, True, "split"), (L.MODE_3XTF32, 8192, 4096, 512, True, "direct"), (L.MODE_3XTF32, 128, 4095, 1025, False, "copied+split"), (L.MODE_TF32, 512, 512, 512, True, "direct"), (L.MODE_TF32, 128, 96, 4096, True, "direct"),
            (L.MODE_3XTF32, 700, 900, 1000, False, "copied"), (L.MODE_TF32, 455, 1149, 6946, False, "copied"), (L.MODE_3XF16, 300, 200, 500, True, "panels"),
            (L.MODE_F16, 300, 200, 5000, False, "panels"), (L.MODE_3XMIXED, 512, 512, 512, True, "mixed")]
 
@@ -329,7 +329,7 @@ def test_operands_split_on_chip_give_the_bits_of_the_panels(backend, device, M, 
     out = []
     try:
         text = describe(L.MODE_3XTF32, M, N, K, 1)
-        assert "splits=1 " in text and text.endswith("kernels=1")     # the k-loop is not divided; nothing is prepared
+        assert "splits=1 " in text and text.endswith("operands=split kernels=1")     # the k-loop is not divided; nothing is prepared
         for variant in (3, 0):
             backend.set_gemm_variant(variant)
             D.clear()
@@ -346,9 +346,11 @@ def test_operands_split_on_chip_give_the_bits_of_the_panels(backend, device, M, 
 @pytest.mark.parametrize("M,N,K", [(64, 4096, 4096), (64, 4096, 1024), (128, 4096, 4096), (128, 1024, 4096), (1024, 1024, 1024), (256, 2048, 4096), (2304, 2304, 520)])
 def test_operands_split_on_chip_give_the_same_bits_every_time(backend, device, M, N, K):
     """Stages that are written again while a warp still reads them show here: operands in L2 and not, launches alone and in a row."""
-    A, B = (dev_from(backend, device, O.fill(n, 74, i)) for i, n in ((1, M * K), (2, K * N)))
+    a, b = O.fill(M * K, 74, 1), O.fill(K * N, 74, 2)
+    A, B = dev_from(backend, device, a), dev_from(backend, device, b)
     D, other = Dev(backend, device, M * N), Dev(backend, device, 40 << 20)
     try:
+        assert " operands=split " in describe(L.MODE_3XTF32, M, N, K, 1)
         first = None
         for i in range(12):
             if i % 3 == 1:
@@ -358,13 +360,37 @@ def test_operands_split_on_chip_give_the_same_bits_every_time(backend, device, M
             got = D.download().view(np.uint32)
             first = got if first is None else first
             assert np.array_equal(got, first)
+        assert O.gemm_rel_error(first.view(np.float32).reshape(M, N), O.gemm(a, b, M, N, K)) <= tol(L.MODE_3XTF32, K)
     finally:
         for x in (A, B, D, other):
             x.free()
 
 
-# copies of rows that start 1, 2 and 3 elements behind a 16-byte boundary and at all four in turn; row lengths at the edges of a warp's piece
-# (512 columns), of its lanes' quads and of the padding; a matrix of which only one operand needs the copy
+# (M, N, K, offset, padding): the copies of unaligned operands split on chip, by single blocks of 64 and 128 rows and both tile widths
+@pytest.mark.parametrize("M,N,K,off,pad", [(52, 5537, 331, 1, 0), (63, 70, 290, 0, 1), (114, 9, 259, 3, 0), (103, 2181, 711, 2, 3), (121, 10213, 577, 1, 0),
+                                           (25, 9589, 439, 0, 2)])
+def test_copies_split_on_chip_give_the_bits_of_the_panels(backend, device, M, N, K, off, pad):
+    lda, ldb = K + pad, N + pad
+    rng = np.random.default_rng(M + N + K)
+    A, B = (dev_from(backend, device, rng.uniform(-1, 1, n).astype(np.float32), offset=off) for n in ((M - 1) * lda + K, (K - 1) * ldb + N))
+    D, out = Dev(backend, device, M * N), []
+    try:
+        text = describe(L.MODE_3XTF32, M, N, K, 0)
+        assert " operands=copied+split " in text and "splits=1 " in text
+        for variant in (3, 0):
+            backend.set_gemm_variant(variant)
+            D.clear()
+            gemm(backend, device, L.MODE_3XTF32, M, N, K, A, B, D, lda=lda, ldb=ldb)
+            out.append(D.download())
+        assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
+    finally:
+        backend.set_gemm_variant(0)
+        for x in (A, B, D):
+            x.free()
+
+
+# copies of rows that start 1, 2 and 3 elements behind a 16-byte boundary and at all four in turn; a thread copies a quad of a row: lengths
+# that end 0, 1, 2 and 3 elements into one; a matrix of which only one operand needs the copy
 @pytest.mark.parametrize("mode", [L.MODE_3XTF32, L.MODE_TF32])
 @pytest.mark.parametrize("M,N,K,off,pad", [(600, 513, 259, 1, 1), (1030, 1021, 513, 2, 0), (260, 1021, 516, 3, 2), (1025, 1030, 511, 3, 4), (1100, 514, 260, 0, 3)])
 def test_copied_rows_give_the_bits_of_the_panels(backend, device, mode, M, N, K, off, pad):
@@ -374,7 +400,7 @@ def test_copied_rows_give_the_bits_of_the_panels(backend, device, mode, M, N, K,
     D, out = Dev(backend, device, M * N), []
     try:
         text = describe(mode, M, N, K, 0)
-        assert "operands=copied" in text and "splits=1 " in text
+        assert " operands=copied " in text and "splits=1 " in text
         for variant in (3, 0):
             backend.set_gemm_variant(variant)
             D.clear()
