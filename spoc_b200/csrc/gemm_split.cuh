@@ -10,10 +10,10 @@
 //
 // Rows of A from M on are not split: an accumulator row depends on its own row of A only, and those rows are not stored.
 //
-// Bound: the tensor pipe from 192 columns on (645 and 850 ns per k-block with 192 and 256 columns), below that the latency of the
-// groups' way from shared memory through registers to tensor memory (pairs 430 and 363 ns with 128 and 64 columns, blocks on their own
-// 540 and 375).  Against the two launches, and for few rows gemm_convert_kernel: 64 x 4096 x 4096 42.6 -> 24 us, 128 x 4096 x 4096 64.5 ->
-// 33, 1024^3 20.1 -> 16.9, 2048^3 85 -> 75, 4096^3 614 -> 568.
+// Bound: the tensor pipe from 128 columns on (430, 645 and 850 ns per k-block of a pair with 128, 192 and 256 columns); with 64 columns, where the
+// pipe would take 200 ns, the latency of the groups' way from shared memory through registers to tensor memory (363).  Blocks on their
+// own: 540 and 375 ns.  Against the two launches, and for few rows gemm_convert_kernel, in turn on one B200: 64 x 4096 x 4096 40.6 -> 25.1 us,
+// 128 x 4096 x 4096 65.1 -> 28.7, 512^3 13.6 -> 11.9, 1024^3 20.4 -> 17.1, 2048^3 79.8 -> 73.3, 4096^3 541 -> 503.
 #pragma once
 #include "gemm_tcgen05_pair.cuh"
 
@@ -25,12 +25,12 @@ struct SplitCfg {
   static_assert(BN == 256 || BN == 192 || BN == 128 || BN == 64, "tile columns");
   static_assert(ROWS == 128 || (ROWS == 64 && CTAS == 1), "rows");
   static constexpr int kPartN = BN / CTAS;                            // columns of B this block loads and splits
-  // Groups of four warps that split.  A group needs 2000 cycles for a k-block, nearly all of it latency; four groups (96 registers a
-  // thread instead of 128) were slower than three: 1024^3 19.5 us and 17.7, two groups 20.9.
+  // Groups of four warps that split.  A group needs 2000 cycles for a k-block, nearly all of it latency.  Tiles of 64 columns with two, three
+  // and four groups: 1024^3 19.2, 17.1 and 19.2 us, 512^3 12.3, 11.3 and 12.9, 64 x 1024 x 1024 10.0, 9.2 and 9.3.
   static constexpr int kGroups = 3;
   // Tiles of 128 columns and more: the registers of the last warpgroup go to the splitting ones, launched with 128 a thread
-  // (512 x 128 = 65536; 384 x 152 + 128 x 40 = 63488).  64 x 4096 x 3072 undivided 63 -> 56 us; tiles of 64 columns need no more than
-  // 128 and were slower (1024^3 18.3 -> 19.5).
+  // (512 x 128 = 65536; 384 x 152 + 128 x 40 = 63488).  48 x 16384 x 4096 90.6 -> 83.6 us, 2304 x 2304 x 520 44.3 -> 43.2, 2048^3 69.6 -> 68.9,
+  // other sizes even; tiles of 64 columns need no more than 128.
   static constexpr bool kMoveRegs = BN > 64;
   static constexpr int kThreads = kGroups * 128 + (kMoveRegs ? 128 : 64);
   static constexpr uint32_t kABytes = ROWS * GEMM_BK * 4;

@@ -823,12 +823,12 @@ constexpr double kCopyMacs = 16777216.0;                 // 2^24
 // x 128 5.4 and 5.6; 64 x 1024 x 96 5.3 and 5.6, x 128 6.1 and 5.6; 512 x 256 x 64 5.3 and 5.6, x 96 6.1 and 5.8.
 constexpr long long kConvertKOneTerm = 128;
 // gemm_split_kernel instead of gemm_pair_kernel behind a launch for the low parts, where the estimates say so.  It moves half the bytes
-// to the SMs, which the other pays with 10 % of its time beside the estimate (2048^3 85 -> 75 us, 4096^3 614 -> 568, 1024 x 1024 x 4096
-// 51 -> 38, 16384 x 2048 x 2048 572 -> 540); but its epilogues overlap nothing (8192 x 8192 x 512, 14 waves: 360 us, the other 290).
-// Not in several waves of long k-loops, whose pairs gemm_pair_kernel holds together (next_epoch_ring; 8192^3 4440 and 4360 us:
-// what lockstep saves in DRAM traffic on the largest products is not to be had here), nor in several waves of a divided one
-// (64 x 16384 x 16384: 625 and 532).  With two k-blocks or one the host's encoding of the operand maps costs what the device saves: 64^3 called
-// in a row 5.80 us and by gemm_convert_kernel 5.71, 32^3 6.6 and 6.5; 128^3 6.4 and 7.4.
+// to the SMs, which the other pays with 10 % of its time beside the estimate (2048^3 80 -> 73 us, 4096^3 541 -> 503, 1024 x 1024 x 4096
+// 49 -> 37, 16384 x 2048 x 2048 508 -> 476); but its epilogues overlap nothing (8192 x 8192 x 512, 14 waves: 360 us, the other 290).
+// Not in several waves of a divided k-loop (64 x 16384 x 16384: 625 and 532), nor in several waves of k-loops of kSplitMaxKBlocks: that line was
+// drawn from one size, 8192^3 (4440 and 4360 us, the pairs of the other held together by next_epoch_ring).  Another B200 had it 4226 and
+// 4300 there, 990 and 1080 at 4096 x 4096 x 8192, 779 and 785 at 2304 x 2304 x 16384.  With two k-blocks or one the host's encoding of the operand
+// maps costs what the device saves: 64^3 called in a row 5.80 us and by gemm_convert_kernel 5.71, 32^3 6.6 and 6.5; 128^3 6.8 and 8.5.
 constexpr double kPlainCharge = 1.1;
 constexpr long long kSplitMaxKBlocks = 256;
 constexpr long long kNarrowRows = 768;
@@ -957,9 +957,9 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   // ns: a launch in front that reads the operands and writes their low parts, copies of them, or both
   auto prep = [&](int written) { return 1000.0 + 4.0 * (1 + written) * (static_cast<double>(M) * K + static_cast<double>(K) * N) / 5000.0; };
   const double plain = r.src == SRC_CONVERT ? r.cost : kPlainCharge * r.cost + prep(addressable ? 1 : 2);
-  // Over copies (whose launch costs 2.5 us beside its bytes) instead of conversion in registers, and for few rows and divided k-loops:
-  // otherwise the ordinary epilogue of unaligned results, which overlaps nothing here, makes gemm_pair_kernel the faster one behind
-  // the same copies (1531 x 2047 x 1021 38 us and 44, 1001 x 1003 x 1005 22.6 and 24.2; but 300 x 3001 x 3003, divided, 66 and 61).
+  // Over copies (whose launch costs 2.5 us beside its bytes) instead of conversion in registers, and for few rows and divided k-loops.
+  // Undivided ones of more rows are faster by gemm_pair_kernel behind the same copies (1531 x 2047 x 1021 38 us and 44, 1001 x 1003 x 1005 22.6
+  // and 24.2; why is not established, both run one wave there; but 300 x 3001 x 3003, divided, 64 and 58).
   if (!addressable && r.src == SRC_DIRECT && M > GEMM_BM && r.splits == 1) return r;
   const double cost = shape.cost + (addressable ? 0.0 : prep(1) + 2500.0);
   if ((waves > 1 && (kblocks >= kSplitMaxKBlocks || shape.splits > 1)) || shape.cost == 0.0 || cost >= plain) return r;
