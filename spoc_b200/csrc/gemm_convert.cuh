@@ -314,10 +314,10 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
             }
           }
         }
-        if (elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
         tc_fence_before_sync();
       }
       if (item + item_step >= num_items) break;  // the block's last item: nothing follows but the barrier all threads share
+      if (ok && elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
       // every warp is through with the accumulator and the tiles before the next item's operands arrive
       __syncwarp();
       ok = convert_go_on(ok, abort_flag);
@@ -385,12 +385,14 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   tc_fence_before_sync();
   __syncthreads();
   if constexpr (in_cluster) {  // no block retires while others read its partial sums
-    cluster_arrive();
+    cluster_arrive_relaxed();
     cluster_wait();
   }
   if (warp == CONV_WARPS) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, BN);
+  } else if (warp < CONV_WARPS && elect_one()) {
+    bulk_wait_read<0>();  // the epilogue's tiles outlive the stores that read them
   }
 }
 

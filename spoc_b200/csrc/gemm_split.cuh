@@ -144,9 +144,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tc_fence_before_sync();
   }
   __syncthreads();
+  // the blocks' barriers exist before any signal crosses between them; the producer's loads cross nothing
   if (CTAS == 2) {
-    cluster_arrive();
-    cluster_wait();
+    cluster_arrive_relaxed();
+    if (warp != GROUPS * 4) cluster_wait();
   }
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
@@ -259,13 +260,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             ok = false;
           }
         }
-        if (elect_one()) bulk_wait_read<0>();  // the tiles must outlive the stores that read them
       }
+      if (item + item_step >= num_items) break;  // nothing follows that would wait for the accumulator or the rings
+      if (elect_one()) bulk_wait_read<0>();  // the stores have read their tiles
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_u32(acc_empty));
-        if (CTAS == 2) mbar_arrive_cluster(map_to_cta(smem_u32(acc_empty), cta ^ 1u));
+        if (CTAS == 2) mbar_arrive_peer(map_to_cta(smem_u32(acc_empty), cta ^ 1u));
       }
     }
     if (!ok && elect_one()) wait_for_copies();  // tiles of C
@@ -295,7 +297,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
           const int blocks = item_blocks(item, kb0);
           const int m0 = tm * BM + static_cast<int>(rank) * 128, n0 = tn * BN + static_cast<int>(rank) * PART_N;
-          if (local > 0 && !mbar_wait_bounded(smem_u32(acc_empty), (local - 1) & 1, abort_flag)) {
+          if (local > 0 && !(CTAS == 2 ? mbar_wait_cluster(smem_u32(acc_empty), (local - 1) & 1, abort_flag)
+                                       : mbar_wait_bounded(smem_u32(acc_empty), (local - 1) & 1, abort_flag))) {
             atomicCAS(p.status, 0, 0x3200 | rank);
             ok = false;
             break;
@@ -321,6 +324,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
         if (!ok) wait_for_copies();
       }
+      __syncwarp();
+      if (CTAS == 2) cluster_wait();  // of the barrier in front
     } else if (warp == GROUPS * 4 + 1 && rank == 0 && elect_one()) {
       // ------------------------------------------------------- MMA issuer (leader block)
       constexpr uint32_t idesc = umma_idesc_tf32(BM, BN, true);
@@ -330,7 +335,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
         int kb0;
         const int blocks = item_blocks(item, kb0);
-        if (local > 0 && !mbar_wait_bounded(smem_u32(acc_empty), (local - 1) & 1, abort_flag)) {
+        if (local > 0 && !(CTAS == 2 ? mbar_wait_cluster(smem_u32(acc_empty), (local - 1) & 1, abort_flag)
+                                     : mbar_wait_bounded(smem_u32(acc_empty), (local - 1) & 1, abort_flag))) {
           atomicCAS(p.status, 0, 0x3210);
           break;
         }
@@ -367,16 +373,20 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       cluster_wait();
     }
   }
-  // no block retires, or frees tensor memory, while its peers signal its barriers, read its memory or write its accumulator
+  // No block retires, or frees tensor memory, while its peers signal its barriers, read its memory or write its accumulator.  The barrier
+  // orders no memory: what was read here is in registers.  Nor do the epilogue's last signals wait for anything: 1024^3 17.3 -> 16.1 us,
+  // 256^3 8.5 -> 7.5.
   tc_fence_before_sync();
   __syncthreads();
   if (CTAS == 2 || IN_CLUSTER) {
-    cluster_arrive();
+    cluster_arrive_relaxed();
     cluster_wait();
   }
   if (warp == GROUPS * 4 + 1) {
     tc_fence_after_sync();
     tmem_dealloc_for<CTAS>(tmem_base, GEMM_TMEM_COLS);
+  } else if (warp < EPI_WARPS && elect_one()) {
+    bulk_wait_read<0>();  // the epilogue's tiles outlive the stores that read them
   }
 }
 

@@ -279,6 +279,11 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
+// The same for a barrier that orders execution and nothing in memory (or what a fence in front of it has published, mbar_fence_init): the
+// release of the other waits until every store of the thread has reached L2.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -299,13 +304,10 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
   return v;
 }
-// arrive on an mbarrier that may live in the peer block (address from map_to_cta)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same for signals about nothing but this block's own shared memory and tensor memory (which the other block's MMAs read): the release
-// is restricted to objects in shared::cta, and mbar_wait_cluster is its acquiring side.  Tensor memory is ordered by tcgen05.wait::st and
-// tcgen05.fence.  The unrestricted release waits for the whole chip, 1400 cycles: 1024^3 17.2 us so and 22.0 with it.
+// Arrive on an mbarrier that may live in the peer block (address from map_to_cta), to signal about nothing but this block's own shared memory
+// and tensor memory (which the other block's MMAs read and write): the release is restricted to objects in shared::cta, and mbar_wait_cluster
+// is its acquiring side.  Tensor memory is ordered by tcgen05.wait and tcgen05.fence.  The unrestricted release waits for the whole
+// chip, 1400 cycles: 1024^3 17.2 us so and 22.0 with it in front of every k-block.
 __device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
   asm volatile(
       "fence.release.sync_restrict::shared::cta.cluster;\n"
