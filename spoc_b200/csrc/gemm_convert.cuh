@@ -227,17 +227,18 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   constexpr bool in_cluster = IN_CLUSTER;
   const int split_rank = in_cluster ? static_cast<int>(cluster_ctarank()) : 0;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), CONV_WARPS);
-      mbar_init(smem_u32(&empty_bar[s]), 1);
-    }
-    mbar_init(smem_u32(done_bar), 1);
-    for (int i = 0; i < 2 * CONV_WARPS; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
-    *abort_flag = 0;
+  if (warp == 0) {  // a lane a barrier: full, empty, done
+    constexpr int BARS = 2 * STAGES + 1;
+    static_assert(BARS <= 32, "a lane a barrier");
+    if (lane < BARS) mbar_init(smem_u32(&full_bar[lane]), lane < STAGES ? CONV_WARPS : 1);
+    if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
-    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
   }
+  if (warp == 1) {  // the barriers of the tiles of C
+    if (lane < 2 * CONV_WARPS) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + lane), 1);
+    mbar_fence_init();
+  }
+  if (threadIdx.x == 64 && p.tma_epilogue) tma_prefetch_desc(&map_d);
   if (warp == CONV_WARPS) {
     tmem_alloc(smem_u32(tmem_slot), BN);
     tmem_relinquish();
@@ -262,8 +263,8 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn;
-      pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
-      const int m0 = tm * 128, n0 = tn * BN, split = item / num_tiles;
+      item_tile_coords(item, p, num_tiles, tm, tn);
+      const int m0 = tm * 128, n0 = tn * BN, split = item_split(item, num_tiles);
       const int kb0 = split * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
       ConvTile<BN, VEC> t[CONV_AHEAD + 1];
 #pragma unroll
@@ -328,7 +329,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       cluster_arrive();
       cluster_wait();
       int tm, tn;
-      pair_tile_coords(first_item - split_rank * num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      item_tile_coords(first_item - split_rank * num_tiles, p, num_tiles, tm, tn);
       if (p.vec_epilogue)
         cluster_part_finish<BN, 1, CONV_WARPS * 32, true>(p, smem, split_rank, 0, tm * 128, tn * BN, threadIdx.x);
       else
@@ -343,7 +344,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       uint32_t phase = 0;
       bool ok = true;
       for (int item = first_item; item < num_items && ok; item += item_step) {
-        const int kb0 = (item / num_tiles) * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
+        const int kb0 = item_split(item, num_tiles) * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
         for (int kb = 0; kb < blocks; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), phase, abort_flag)) {
             atomicCAS(p.status, 0, 0x2300 | stage);

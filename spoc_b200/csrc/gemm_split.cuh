@@ -120,20 +120,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                                     : static_cast<int>(blockIdx.x) / CTAS;
   const int item_step = IN_CLUSTER ? 1 << 30 : static_cast<int>(gridDim.x) / CTAS;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < RAW; ++s) {
-      mbar_init(smem_u32(&raw_full[s]), 1);
-      mbar_init(smem_u32(&raw_empty[s]), 4);
-    }
-    for (int s = 0; s < PARTS; ++s) {
-      mbar_init(smem_u32(&part_full[s]), 4 * CTAS);
-      mbar_init(smem_u32(&part_empty[s]), 1);
-    }
-    mbar_init(smem_u32(acc_full), 1);
-    mbar_init(smem_u32(acc_empty), EPI_WARPS * CTAS);
-    for (int i = 0; i < 2 * EPI_WARPS; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
-    *abort_flag = 0;
+  if (warp == 0) {  // the lanes share the barriers: raw_full, raw_empty, part_full, part_empty, acc_full, acc_empty
+    constexpr int BARS = 2 * RAW + 2 * PARTS + 2;
+    for (int i = lane; i < BARS; i += 32)
+      mbar_init(smem_u32(raw_full + i), i < RAW ? 1 : i < 2 * RAW ? 4 : i < 2 * RAW + PARTS ? 4 * CTAS : i < BARS - 1 ? 1 : EPI_WARPS * CTAS);
+    if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
+  }
+  if (warp == 1) {  // the barriers of the tiles of C
+    if (lane < 2 * EPI_WARPS) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + lane), 1);
+    mbar_fence_init();
+  }
+  if (threadIdx.x == 64) {
     tma_prefetch_desc(&map_a);
     tma_prefetch_desc(&map_b);
     if (p.tma_epilogue) tma_prefetch_desc(&map_d);
@@ -155,7 +153,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   grid_dependency_wait();  // nothing above touched global memory
 
   auto item_blocks = [&](int item, int& kb0) {
-    kb0 = (item / num_tiles) * p.split_k_blocks;
+    kb0 = item_split(item, num_tiles) * p.split_k_blocks;
     return min(p.num_k_blocks - kb0, p.split_k_blocks);
   };
 
@@ -171,7 +169,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn, kb0;
-      pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      item_tile_coords(item, p, num_tiles, tm, tn);
       const int blocks = item_blocks(item, kb0);
       const int m0 = tm * BM + static_cast<int>(rank) * 128, n0 = tn * BN;
       const bool rows_here = quarter * 32 < ROWS && m0 + quarter * 32 < p.M;
@@ -255,7 +253,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           fence_async_shared();  // its ordinary stores to the tile before the loads of the next item, which land there
         } else {
           epilogue_tma_begin(p, &map_c, epi, lane, row0, c0);
-          if (!epilogue_tma<EPI_N>(p, &map_d, &map_c, taddr, epi, lane, row0, c0, (item / num_tiles) * p.part_rows, abort_flag)) {
+          if (!epilogue_tma<EPI_N>(p, &map_d, &map_c, taddr, epi, lane, row0, c0, item_split(item, num_tiles) * p.part_rows, abort_flag)) {
             if (lane == 0) atomicCAS(p.status, 0, 0x3500 | (rank << 4));
             ok = false;
           }
@@ -276,7 +274,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       cluster_arrive();
       cluster_wait();
       int tm, tn;
-      pair_tile_coords(first_item - split_rank * num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      item_tile_coords(first_item - split_rank * num_tiles, p, num_tiles, tm, tn);
       const int row0 = tm * BM + static_cast<int>(rank) * 128;
       if (p.vec_epilogue)
         cluster_part_finish<BN, CTAS, GROUPS * 128, true>(p, smem, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
@@ -294,7 +292,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         bool ok = true;
         for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
           int tm, tn, kb0;
-          pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+          item_tile_coords(item, p, num_tiles, tm, tn);
           const int blocks = item_blocks(item, kb0);
           const int m0 = tm * BM + static_cast<int>(rank) * 128, n0 = tn * BN + static_cast<int>(rank) * PART_N;
           if (local > 0 && !(CTAS == 2 ? mbar_wait_cluster(smem_u32(acc_empty), (local - 1) & 1, abort_flag)

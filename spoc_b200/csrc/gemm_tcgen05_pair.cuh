@@ -58,14 +58,26 @@ __device__ __forceinline__ void pair_soft_epoch(unsigned int* ctr, unsigned int 
   }
 }
 
-__device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tiles_n, int group_m, int& tm, int& tn) {
-  const int band_tiles = group_m * tiles_n;
-  const int band = tile / band_tiles;
-  const int within = tile - band * band_tiles;
-  const int first_m = band * group_m;
-  const int band_m = min(group_m, tiles_m - first_m);
-  tm = first_m + within % band_m;
+// Which part of a divided k-loop work item `item` is: item / num_tiles, without the division where it is 0.
+__device__ __forceinline__ int item_split(int item, int num_tiles) {
+  return item < num_tiles ? 0 : static_cast<int>(static_cast<unsigned int>(item) / static_cast<unsigned int>(num_tiles));
+}
+// The tile of work item `item`, in bands of group_m row tiles.  A division takes about 150 cycles, and every role of a block passes through
+// here before its first load: a product of one band, or whose k-loop is undivided, does with one.
+__device__ __forceinline__ void item_tile_coords(int item, const GemmParams& p, int num_tiles, int& tm, int& tn) {
+  const unsigned int tile = item - item_split(item, num_tiles) * num_tiles, tiles_m = p.tiles_m, group_m = p.group_m;
+  if (tiles_m <= group_m) {
+    tn = tile / tiles_m;
+    tm = tile - tn * tiles_m;
+    return;
+  }
+  const unsigned int band_tiles = group_m * p.tiles_n;
+  const unsigned int band = tile / band_tiles;
+  const unsigned int within = tile - band * band_tiles;
+  const unsigned int first_m = band * group_m;
+  const unsigned int band_m = min(group_m, tiles_m - first_m);
   tn = within / band_m;
+  tm = first_m + within - tn * band_m;
 }
 
 // Four columns of a row of D = act(alpha*sum + beta*C + bias): the operations of the other epilogues in the same order.  VEC: 128-bit
@@ -278,21 +290,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                                  : static_cast<int>(blockIdx.x) / CTAS;
   const int num_pairs = in_cluster ? 1 << 30 : static_cast<int>(gridDim.x) / CTAS;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&full_bar[s]), 1);
-      mbar_init(smem_u32(&empty_bar[s]), 1);
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(smem_u32(&tmem_full_bar[a]), 1);
-      mbar_init(smem_u32(&tmem_empty_bar[a]), 4 * CTAS);  // the epilogue warps of both blocks
-    }
-    for (int i = 0; i < 8; ++i) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + i), 1);
-    *abort_flag = 0;
+  if (warp == 0) {  // a lane a barrier: full and empty, tmem_full, tmem_empty (the epilogue warps of both blocks)
+    constexpr int BARS = 2 * STAGES + 4;
+    static_assert(BARS <= 32, "a lane a barrier");
+    if (lane < BARS) mbar_init(smem_u32(&bars[lane]), lane < 2 * STAGES + 2 ? 1 : 4 * CTAS);
+    if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
+  }
+  if (warp == 2) {  // the barriers of the tiles of C
+    if (lane < 8) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + lane), 1);
+    mbar_fence_init();
+  }
+  if (threadIdx.x == 96) {
     tma_prefetch_desc(&map_a_hi);
     tma_prefetch_desc(&map_b_hi);
-    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
     if (THREE || MIXED) {
       tma_prefetch_desc(&map_a_lo);
       tma_prefetch_desc(&map_b_lo);
@@ -301,6 +312,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       tma_prefetch_desc(&map_a_x);
       tma_prefetch_desc(&map_b_x);
     }
+    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
   }
   if (warp == 1) {
     tmem_alloc_for<CTAS>(smem_u32(tmem_slot), GEMM_TMEM_COLS);
@@ -332,7 +344,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   // stages of work item `item`: its k-blocks [k0, k0 + stages); in mixed mode (never divided) the cross stages, the rescale
   // stages, the main stages
   auto item_stages = [&](int item, int& k0) {
-    k0 = (item / num_tiles) * p.split_k_blocks;
+    k0 = item_split(item, num_tiles) * p.split_k_blocks;
     return MIXED ? 2 * p.num_k_blocks + mix_rescale : min(p.num_k_blocks - k0, p.split_k_blocks);
   };
 
@@ -350,7 +362,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       int my_tiles = 0;
       for (int item = pair_id; item < num_items && ok; item += num_pairs, ++my_tiles) {
         int tm, tn, k0;
-        pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+        item_tile_coords(item, p, num_tiles, tm, tn);
         const int stages = item_stages(item, k0);
         const int m0 = tm * BM + static_cast<int>(rank) * 128;     // this block's rows of A
         const int n0 = tn * BN + static_cast<int>(rank) * PART_N;  // this block's part of B's columns
@@ -523,7 +535,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       const int acc = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
       int tm, tn;
-      pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      item_tile_coords(item, p, num_tiles, tm, tn);
       const int row0 = tm * BM + static_cast<int>(rank) * 128 + quarter * 32;
       const int n0 = tn * BN;
       if (p.tma_epilogue) epilogue_tma_begin(p, &map_c, epi, lane, row0, n0);
@@ -542,7 +554,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
         cluster_part_store<BN>(reinterpret_cast<float*>(stage_base), taddr, quarter * 32 + lane, 0, BN);
       } else if (!p.tma_epilogue) {
         epilogue_rows<BN>(p, taddr, epi.buf, lane, row0, n0);
-      } else if (!epilogue_tma<BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, (item / num_tiles) * p.part_rows, abort_flag)) {
+      } else if (!epilogue_tma<BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, item_split(item, num_tiles) * p.part_rows, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, 0x1500 | (rank << 4) | acc);
         ok = false;
         break;
@@ -564,7 +576,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     cluster_arrive();
     cluster_wait();
     int tm, tn;
-    pair_tile_coords(pair_id - split_rank * num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+    item_tile_coords(pair_id - split_rank * num_tiles, p, num_tiles, tm, tn);
     const int row0 = tm * BM + static_cast<int>(rank) * 128;
     if (p.vec_epilogue)
       cluster_part_finish<BN, CTAS, Cfg::kThreads, true>(p, stage_base, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
