@@ -220,15 +220,16 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* done_bar = full_bar + 2 * STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full_bar + 2 * STAGES + 1);
+  uint64_t* recv = full_bar + 2 * STAGES + 1;  // in_cluster: the others' partial sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full_bar + 2 * STAGES + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // in_cluster: item `split * num_tiles + tile` is this block's only one
   constexpr bool in_cluster = IN_CLUSTER;
   const int split_rank = in_cluster ? static_cast<int>(cluster_ctarank()) : 0;
 
-  if (warp == 0) {  // a lane a barrier: full, empty, done
-    constexpr int BARS = 2 * STAGES + 1;
+  if (warp == 0) {  // a lane a barrier: full, empty, done, recv
+    constexpr int BARS = 2 * STAGES + 2;
     static_assert(BARS <= 32, "a lane a barrier");
     if (lane < BARS) mbar_init(smem_u32(&full_bar[lane]), lane < STAGES ? CONV_WARPS : 1);
     if (lane == 0) *abort_flag = 0;
@@ -260,7 +261,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     const int quarter = warp & 3, half = warp >> 2;
     int stage = 0, local = 0;
     uint32_t phase = 0;
-    bool ok = true;
+    bool ok = true, arrived = false;
     for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn;
       item_tile_coords(item, p, num_tiles, tm, tn);
@@ -299,12 +300,16 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
       }
       if (ok) {
         tc_fence_after_sync();
+        if constexpr (in_cluster) {
+          cluster_arrive_relaxed();  // the ring is idle
+          arrived = true;
+        }
         const int row0 = m0 + quarter * 32, c0 = n0 + half * (BN / 2);
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2);
         if (c0 < p.N) {
           if constexpr (in_cluster) {
-            static_assert(ClusterPart<BN>::kBytes <= STAGES * Cfg::kStageBytes, "partial sums fit the ring");
-            cluster_part_store<BN>(reinterpret_cast<float*>(smem), taddr, quarter * 32 + lane, half * (BN / 2), BN / 2);
+            static_assert(ClusterPart<BN>::bytes(1) <= STAGES * Cfg::kStageBytes, "partial sums and what arrives fit the ring");
+            cluster_part_store<BN>(smem, taddr, quarter * 32 + lane, half * (BN / 2), BN / 2);
           } else if (!p.tma_epilogue) {
             epilogue_rows<BN / 2>(p, taddr, epi.buf, lane, row0, c0);
           } else {
@@ -326,14 +331,17 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     if (!ok && elect_one()) wait_for_copies();  // tiles of C
     __syncwarp();
     if constexpr (in_cluster) {
-      cluster_arrive();
-      cluster_wait();
+      if (!arrived) cluster_arrive_relaxed();
       int tm, tn;
       item_tile_coords(first_item - split_rank * num_tiles, p, num_tiles, tm, tn);
-      if (p.vec_epilogue)
-        cluster_part_finish<BN, 1, CONV_WARPS * 32, true>(p, smem, split_rank, 0, tm * 128, tn * BN, threadIdx.x);
-      else
-        cluster_part_finish<BN, 1, CONV_WARPS * 32, false>(p, smem, split_rank, 0, tm * 128, tn * BN, threadIdx.x);
+      auto barrier = [](bool so_far) { return barrier_all(1, CONV_WARPS * 32, so_far); };
+      ok = p.vec_epilogue ? cluster_exchange<BN, 1, CONV_WARPS * 32, 0, true>(p, smem, recv, split_rank, 0, tm * 128, tn * BN, ok, abort_flag, barrier)
+                          : cluster_exchange<BN, 1, CONV_WARPS * 32, 0, false>(p, smem, recv, split_rank, 0, tm * 128, tn * BN, ok, abort_flag, barrier);
+      if (!ok) {
+        if (threadIdx.x == 0) atomicCAS(p.status, 0, 0x2600);
+        wait_for_copies();
+      }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------- MMA issuer
@@ -378,7 +386,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     }
     __syncwarp();
     if constexpr (in_cluster) {
-      cluster_arrive();
+      cluster_arrive_relaxed();
       cluster_wait();
     }
   }

@@ -43,12 +43,17 @@ struct SplitCfg {
   static constexpr int kRawFit = (216 * 1024 - kParts * static_cast<int>(kPartBytes)) / static_cast<int>(kRawBytes);
   static constexpr int kRaw = kRawFit > 8 ? 8 : kRawFit;
   static constexpr int kEpiGroups = 2;                                // groups that run the epilogue, each on a half of the columns
-  static constexpr uint32_t kCtrlBytes = 4096;
-  static constexpr uint32_t kSmemBytes = kRaw * kRawBytes + kParts * kPartBytes + kCtrlBytes + 1024;
+  static constexpr uint32_t kCtrlBytes = 2560;  // barriers, and from GEMM_CTRL_COLS on 256 bytes for each epilogue warp
+  static constexpr uint32_t kRingBytes = kRaw * kRawBytes + kParts * kPartBytes;
+  // a k-loop divided within a cluster: the partial sums and what arrives lie where the rings were
+  static constexpr uint32_t kClusterBytes = ClusterPart<BN>::bytes(CTAS);
+  __host__ __device__ static constexpr uint32_t area(bool in_cluster) { return in_cluster && kClusterBytes > kRingBytes ? kClusterBytes : kRingBytes; }
+  __host__ __device__ static constexpr uint32_t smem_bytes(bool in_cluster) { return area(in_cluster) + (in_cluster ? 1024 : kCtrlBytes) + 1024; }
+  static_assert(smem_bytes(true) <= 227 * 1024, "shared memory of a block");
   static constexpr uint32_t kTmemA = BN;                              // first tensor-memory column of A's parts
   static_assert(kTmemA + kParts * 2 * GEMM_BK <= 512, "the accumulator and A's parts fit tensor memory");
   static_assert(kRaw * kRawBytes >= kEpiGroups * 4 * GEMM_EPI_WARP_BYTES, "epilogue tiles fit the raw ring");
-  static_assert((2 * kRaw + 2 * kParts + 3) * 8 <= GEMM_CTRL_CBAR, "the barriers fit the control area");
+  static_assert((2 * kRaw + 2 * kParts + 4) * 8 <= GEMM_CTRL_CBAR, "the barriers fit the control area");
   // split_waits: what a group knows when it comes to a k-block.
   static_assert(kGroups <= kParts && kParts <= kRaw, "the part ring is as long as a turn of the groups, the raw ring as long as the part ring");
 };
@@ -101,14 +106,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* parts = smem + RAW * Cfg::kRawBytes;
-  uint8_t* ctrl = parts + PARTS * Cfg::kPartBytes;
+  uint8_t* ctrl = smem + Cfg::area(IN_CLUSTER);
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(ctrl);
   uint64_t* raw_empty = raw_full + RAW;
   uint64_t* part_full = raw_empty + RAW;     // used in the leader only
   uint64_t* part_empty = part_full + PARTS;  // one set per block
   uint64_t* acc_full = part_empty + PARTS;   // per block
   uint64_t* acc_empty = acc_full + 1;        // per block: both blocks' epilogues are through
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+  uint64_t* recv = acc_empty + 1;            // IN_CLUSTER: the others' partial sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(recv + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = CTAS == 2 || IN_CLUSTER ? cluster_ctarank() : 0u;
@@ -120,10 +126,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                                     : static_cast<int>(blockIdx.x) / CTAS;
   const int item_step = IN_CLUSTER ? 1 << 30 : static_cast<int>(gridDim.x) / CTAS;
 
-  if (warp == 0) {  // the lanes share the barriers: raw_full, raw_empty, part_full, part_empty, acc_full, acc_empty
-    constexpr int BARS = 2 * RAW + 2 * PARTS + 2;
+  if (warp == 0) {  // the lanes share the barriers: raw_full, raw_empty, part_full, part_empty, acc_full, acc_empty, recv
+    constexpr int BARS = 2 * RAW + 2 * PARTS + 3;
     for (int i = lane; i < BARS; i += 32)
-      mbar_init(smem_u32(raw_full + i), i < RAW ? 1 : i < 2 * RAW ? 4 : i < 2 * RAW + PARTS ? 4 * CTAS : i < BARS - 1 ? 1 : EPI_WARPS * CTAS);
+      mbar_init(smem_u32(raw_full + i), i < RAW ? 1 : i < 2 * RAW ? 4 : i < 2 * RAW + PARTS ? 4 * CTAS : i == BARS - 2 ? EPI_WARPS * CTAS : 1);
     if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
   }
@@ -166,7 +172,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     EpiWarp epi = epi_warp(smem, ctrl, warp);
     unsigned int before = 0;  // k-blocks of the items before
     int local = 0;
-    bool ok = true;
+    bool ok = true, arrived = false;
     for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn, kb0;
       item_tile_coords(item, p, num_tiles, tm, tn);
@@ -245,8 +251,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       // every tile of the item has been split and multiplied: the rings are idle until this epilogue hands them back
       const uint32_t taddr = tmem_base + lanes + group * EPI_N;
       if constexpr (IN_CLUSTER) {
-        static_assert(ClusterPart<BN>::kBytes <= RAW * Cfg::kRawBytes + PARTS * Cfg::kPartBytes, "partial sums fit the rings");
-        cluster_part_store<BN>(reinterpret_cast<float*>(smem), taddr, row, group * EPI_N, EPI_N);
+        cluster_arrive_relaxed();
+        cluster_part_store<BN>(smem, taddr, row, group * EPI_N, EPI_N);
+        arrived = true;
       } else if (c0 < p.N) {
         if (!p.tma_epilogue) {
           epilogue_rows<EPI_N>(p, taddr, epi.buf, lane, row0, c0);
@@ -271,15 +278,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     if (!ok && elect_one()) wait_for_copies();  // tiles of C
     __syncwarp();
     if constexpr (IN_CLUSTER) {
-      cluster_arrive();
-      cluster_wait();
+      if (!arrived) cluster_arrive_relaxed();
       int tm, tn;
       item_tile_coords(first_item - split_rank * num_tiles, p, num_tiles, tm, tn);
       const int row0 = tm * BM + static_cast<int>(rank) * 128;
-      if (p.vec_epilogue)
-        cluster_part_finish<BN, CTAS, GROUPS * 128, true>(p, smem, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
-      else
-        cluster_part_finish<BN, CTAS, GROUPS * 128, false>(p, smem, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
+      auto barrier = [](bool so_far) { return barrier_all(1, GROUPS * 128, so_far); };
+      ok = p.vec_epilogue ? cluster_exchange<BN, CTAS, GROUPS * 128, GROUPS * 4 - 1, true>(p, smem, recv, split_rank, rank, row0, tn * BN, ok, abort_flag, barrier)
+                          : cluster_exchange<BN, CTAS, GROUPS * 128, GROUPS * 4 - 1, false>(p, smem, recv, split_rank, rank, row0, tn * BN, ok, abort_flag, barrier);
+      if (!ok) {
+        if (threadIdx.x == 0) atomicCAS(p.status, 0, 0x3600 | rank);
+        wait_for_copies();
+      }
+      __syncwarp();
     }
   } else {
     if constexpr (Cfg::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
@@ -367,7 +377,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     __syncwarp();
     if constexpr (IN_CLUSTER) {
-      cluster_arrive();
+      cluster_arrive_relaxed();
       cluster_wait();
     }
   }

@@ -112,14 +112,22 @@ __device__ __forceinline__ void finish_quad(const GemmParams& p, long long row, 
                                             const QuadColumns& q) {
   float x[4] = {sum.x, sum.y, sum.z, sum.w};
   const float c[4] = {c4.x, c4.y, c4.z, c4.w};
-  const float rs = p.row_scale ? p.row_scale[row] : 1.0f;
+  if (p.row_scale) {
+    const float rs = p.row_scale[row];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    float y = __fmul_rn(p.alpha, (x[j] * rs) * q.scale[j]);
-    if (p.C) y = fmaf(p.beta, c[j], y);
-    y = __fadd_rn(y, q.bias[j]);
-    if (p.act == 1) y = (y > 0.0f) ? y : 0.0f;
-    x[j] = y;
+    for (int j = 0; j < 4; ++j) x[j] = (x[j] * rs) * q.scale[j];
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = __fmul_rn(p.alpha, x[j]);
+  if (p.C) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = fmaf(p.beta, c[j], x[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = __fadd_rn(x[j], q.bias[j]);
+  if (p.act == 1) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = (x[j] > 0.0f) ? x[j] : 0.0f;
   }
   const long long off = row * p.ldd + col;
   if (VEC) {
@@ -141,93 +149,193 @@ __device__ __forceinline__ void add_to(float4& s, const float4& v) {
   s.w += v.w;
 }
 
-// A k-loop divided among the blocks (pairs) of one cluster (p.cluster_splits > 1).  Each block leaves the partial sums of its
-// 128 rows and BN columns in its operand ring, which is idle once the accumulator is complete; behind a cluster barrier every
-// block adds up a share of the rows' quads from all of them, in order of k, and finishes it.  Bound by the peers' shared memory,
-// which delivers about 14 bytes a cycle and SM with the loads of several quads in flight (2 ns a quad).  Against partial results
-// in global memory and a second launch, without an epilogue and on operands in L2: 64 x 4096 x 4096 TF32 20.4 -> 17.5 us (with C,
-// bias and clamp, operands in HBM 19.9), 256 x 512 x 1024 3xTF32 15.2 -> 12.3 us, TF32 10.0 -> 8.0.
+// A k-loop divided among the blocks (pairs) of one cluster (p.cluster_splits > 1).  Each block leaves the partial sums of its 128 rows
+// and BN columns in its operand ring, which is idle once the accumulator is complete, and sends every other block the rows that one
+// finishes, with a bulk copy per block; what arrives is added up from the block's own shared memory, in order of k.  Block `share` of
+// `splits` finishes rows [rows * share / splits, rows * (share + 1) / splits).  In order: cluster_arrive_relaxed once the ring is idle,
+// cluster_part_store, and cluster_exchange: a barrier of the block, cluster_wait (all rings are idle), the copies, the wait for `recv`, and
+// the share of this block.
+// Bound by the way between the blocks, about 13 bytes a cycle and SM (32 KB 1600 to 2400 cycles), and by what runs once in a launch and
+// so comes from a cold instruction cache.  It replaced 128-bit loads from the peers' shared memory behind a cluster barrier with a release:
+// 512 x 512 x 2048 TF32 11.0 -> 9.2 us, 128 x 4096 x 4096 TF32 16.2 -> 15.8, 64 x 1024 x 1024 3xTF32 8.6 -> 8.3, 200 x 300 x 900 9.2 -> 8.6.
 template <int BN>
 struct ClusterPart {
-  static constexpr int kPitch = BN + 4;  // floats per row: consecutive rows start four banks apart
-  static constexpr uint32_t kBytes = 128 * kPitch * 4;
+  static constexpr uint32_t kRowBytes = BN * 4;  // quad q of row r lies at quad q ^ (r & 7): no bank conflicts with a lane a row
+  // the partial sums, and (splits - 1) * ceil(rows / splits) rows that arrive: at most 114 with seven blocks, 96 with four pairs
+  __host__ __device__ static constexpr uint32_t bytes(int ctas) { return (128 + (ctas == 2 ? 96 : 114)) * kRowBytes; }
 };
-// One warp's 32 rows (tensor-memory lanes from `row` of the block's 128) and `cols` columns from `col` on.
+// rows * share / splits, for at most 128 rows and eight splits: an integer division would take 150 cycles
+__device__ __forceinline__ int share_row(int rows, int share, int splits) {
+  return static_cast<int>(__fdividef(static_cast<float>(rows * share) + 0.5f, static_cast<float>(splits)));
+}
+
+// One warp's 32 rows (tensor-memory lanes from `row` of the block's 128) and `cols` columns from `col` on, for the copies to read.
 template <int BN>
-__device__ __forceinline__ void cluster_part_store(float* part, uint32_t taddr, int row, int col, int cols) {
+__device__ __forceinline__ void cluster_part_store(uint8_t* part, uint32_t taddr, int row, int col, int cols) {
 #pragma unroll 1
   for (int c = 0; c < cols; c += 32) {
     uint32_t r[32];
     tmem_ld_32x32b_x32(taddr + c, r);
     tmem_ld_wait_x32(r);
-    uint4* dst = reinterpret_cast<uint4*>(part + row * ClusterPart<BN>::kPitch + col + c);
+    uint8_t* dst = part + row * ClusterPart<BN>::kRowBytes + (col + c) * 4;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dst[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+    for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
   }
+  fence_async_shared();
 }
-// share: this block's split; rank: its rank in its pair; row0, n0: the first row and column of its part of the tile.
-template <int BN, int CTAS, int THREADS, bool VEC>
-__device__ __forceinline__ void cluster_part_finish(const GemmParams& p, const void* part, int share, int rank, int row0, int n0, int tid) {
-  constexpr int QUADS = BN / 4;
+// One warp, a lane a peer.  recv: the barrier of this block, at the same place in all, on which what arrives is counted.
+template <int BN, int CTAS>
+struct ClusterPush {
+  uint32_t dst, src, bytes, bar, expected;
+  // what is sent, and where to: before the others' rings are known to be idle
+  __device__ __forceinline__ void prepare(const uint8_t* part, uint64_t* recv, int rows, int share, int rank, int splits, int lane) {
+    constexpr uint32_t ROW = ClusterPart<BN>::kRowBytes;
+    const int slot_rows = share_row(rows + splits - 1, 1, splits);
+    const int to = share + 1 + lane < splits ? share + 1 + lane : share + 1 + lane - splits;  // of lane < splits - 1
+    const int first = share_row(rows, to, splits), slot = share < to ? share : share - 1;
+    bytes = lane < splits - 1 ? (share_row(rows, to + 1, splits) - first) * ROW : 0;
+    expected = (splits - 1) * (share_row(rows, share + 1, splits) - share_row(rows, share, splits)) * ROW;
+    src = smem_u32(part) + first * ROW;
+    dst = map_to_cta(smem_u32(part) + (128 + slot * slot_rows) * ROW, (bytes ? to : share) * CTAS + rank);
+    bar = map_to_cta(smem_u32(recv), (bytes ? to : share) * CTAS + rank);
+  }
+  __device__ __forceinline__ void send(uint64_t* recv, int lane) const {
+    if (lane == 0) mbar_arrive_expect_tx(smem_u32(recv), expected);
+    if (bytes) bulk_copy_to_cta(dst, src, bytes, bar);
+    __syncwarp();
+  }
+};
+// THREADS threads.  row0, n0: the first row and column of the block's part of the tile.  begin: what does not wait for the others.
+// The rows of a batch go through every operation together, so that what a launch has or has not (C, scales, a clamp, replicas) is asked
+// once a batch: asked for every quad it was 120 instructions a quad and 3100 of the 7500 cycles behind the k-loop (64 rows of 128 columns).
+template <int BN, int THREADS, bool VEC>
+struct ClusterFinish {
+  static constexpr int QUADS = BN / 4, STEP = THREADS / QUADS;
+  static constexpr int BATCH = STEP % 2 == 0 ? 4 : 8;  // rows a thread has in flight
   static_assert(THREADS % QUADS == 0, "a thread stays in its column quad");
-  constexpr int BATCH = THREADS > 256 ? 2 : 4, AHEAD = 4;  // quads, and partial sums of each, that a thread has in flight
-  constexpr int STEP = THREADS / QUADS;  // rows between a thread's quads
-  const int rows = min(128, p.M - row0);
-  if (rows <= 0) return;
-  const int total = rows * QUADS, splits = p.cluster_splits;
-  const int begin = total * share / splits + tid, end = total * (share + 1) / splits;
-  const int first_row = begin / QUADS, quad = begin - first_row * QUADS, col = n0 + quad * 4;
-  if (col >= p.N) return;
-  const QuadColumns columns = quad_columns(p, col);
-  const uint8_t* own = static_cast<const uint8_t*>(part) + quad * 16;
-  constexpr int PITCH = ClusterPart<BN>::kPitch * 4;
-  for (int at = begin, row = first_row; at < end; at += BATCH * THREADS, row += BATCH * STEP) {
-    const int count = (end - at + THREADS - 1) / THREADS;  // quads left to this thread
-    auto batch = [&](auto whole) {
-      constexpr int N = decltype(whole)::value;
-      float4 s[N], c[N];
+  static_assert(BATCH * STEP % 8 == 0, "the swizzle of a thread's rows is the same in every batch");
+  static constexpr uint32_t ROW = ClusterPart<BN>::kRowBytes;
+  int first, row, left, col;  // left: rows of this thread
+  uint32_t slot_bytes;
+  QuadColumns columns;
+  float4 c[BATCH];
+
+  __device__ __forceinline__ void load_c(const GemmParams& p, int row0, int from, int have) {
 #pragma unroll
-      for (int u = 0; u < N; ++u) c[u] = quad_of_c<VEC>(p, row0 + row + u * STEP, col);
-#pragma unroll 1
-      for (int k0 = 0; k0 < splits; k0 += AHEAD) {
-        float4 v[AHEAD][N];
+    for (int u = 0; u < BATCH; ++u)
+      if (u < have) c[u] = quad_of_c<VEC>(p, row0 + first + from + u * STEP, col);
+  }
+  __device__ __forceinline__ void begin(const GemmParams& p, int share, int rows, int row0, int n0, int tid) {
+    const int splits = p.cluster_splits;
+    row = tid / QUADS;
+    col = n0 + tid % QUADS * 4;
+    first = share_row(rows, share, splits);
+    const int count = share_row(rows, share + 1, splits) - first;
+    left = col < p.N && row < count ? (count - row + STEP - 1) / STEP : 0;
+    slot_bytes = share_row(rows + splits - 1, 1, splits) * ROW;
+    columns = quad_columns(p, col);
+    if (p.C) load_c(p, row0, row, left);
+  }
+  __device__ __forceinline__ void run(const GemmParams& p, const uint8_t* part, int share, int row0, int tid) {
+    uint32_t at[BATCH];  // of the batch's rows, from the first row of the share on
 #pragma unroll
-        for (int j = 0; j < AHEAD; ++j) {
-          if (k0 + j >= splits) break;
-          if (k0 + j == share) {
+    for (int u = 0; u < BATCH; ++u) at[u] = (row + u * STEP) * ROW + ((tid % QUADS ^ ((first + row + u * STEP) & 7)) << 4);
+    float* dp = p.D + static_cast<long long>(row0 + first + row) * p.ldd + col;
+    for (; left > 0; left -= BATCH, row += BATCH * STEP) {
+      float x[BATCH][4];
+      const uint8_t* theirs = part + 128 * ROW;
+      for (int k = 0; k < p.cluster_splits; ++k) {
+        const uint8_t* from = k == share ? part + first * ROW : theirs;
+        theirs += k == share ? 0 : slot_bytes;
 #pragma unroll
-            for (int u = 0; u < N; ++u) v[j][u] = *reinterpret_cast<const float4*>(own + (row + u * STEP) * PITCH);
+        for (int u = 0; u < BATCH; ++u) {
+          if (u >= left) break;
+          const float4 v = *reinterpret_cast<const float4*>(from + at[u]);
+          if (k == 0) {
+            *reinterpret_cast<float4*>(x[u]) = v;
           } else {
-            const uint32_t peer = map_to_cta(smem_u32(own), (k0 + j) * CTAS + rank) + row * PITCH;
-#pragma unroll
-            for (int u = 0; u < N; ++u) v[j][u] = ld_cluster_v4(peer + u * STEP * PITCH);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < AHEAD; ++j) {
-          if (k0 + j >= splits) break;
-#pragma unroll
-          for (int u = 0; u < N; ++u) {
-            if (k0 + j == 0)
-              s[u] = v[j][u];
-            else
-              add_to(s[u], v[j][u]);
+            x[u][0] += v.x;
+            x[u][1] += v.y;
+            x[u][2] += v.z;
+            x[u][3] += v.w;
           }
         }
       }
+      if (p.row_scale) {
 #pragma unroll
-      for (int u = 0; u < N; ++u) finish_quad<VEC>(p, row0 + row + u * STEP, col, s[u], c[u], columns);
-    };
-    if (count >= BATCH) {
-      batch(std::integral_constant<int, BATCH>());
-    } else {
-      if constexpr (BATCH > 2) {
-        if (count & 2) batch(std::integral_constant<int, 2>());
-        if (count & 2) row += 2 * STEP;
+        for (int u = 0; u < BATCH; ++u) {
+          const float rs = u < left ? p.row_scale[row0 + first + row + u * STEP] : 1.0f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[u][j] = (x[u][j] * rs) * columns.scale[j];
+        }
       }
-      if (count & 1) batch(std::integral_constant<int, 1>());
+#pragma unroll
+      for (int u = 0; u < BATCH; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[u][j] = __fmul_rn(p.alpha, x[u][j]);
+      if (p.C) {
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+          x[u][0] = fmaf(p.beta, c[u].x, x[u][0]);
+          x[u][1] = fmaf(p.beta, c[u].y, x[u][1]);
+          x[u][2] = fmaf(p.beta, c[u].z, x[u][2]);
+          x[u][3] = fmaf(p.beta, c[u].w, x[u][3]);
+        }
+        load_c(p, row0, row + BATCH * STEP, left - BATCH);
+      }
+#pragma unroll
+      for (int u = 0; u < BATCH; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[u][j] = __fadd_rn(x[u][j], columns.bias[j]);
+      if (p.act == 1) {
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[u][j] = (x[u][j] > 0.0f) ? x[u][j] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < BATCH; ++u) {
+        if (u >= left) break;
+        if (VEC) {
+          *reinterpret_cast<float4*>(dp + u * STEP * p.ldd) = *reinterpret_cast<const float4*>(x[u]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (col + j < p.N) dp[u * STEP * p.ldd + j] = x[u][j];
+        }
+      }
+      if (p.n_replicas) {
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+          if (u >= left) break;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (col + j < p.N) store_replicas(p, dp + u * STEP * p.ldd + j - p.D, x[u][j]);
+        }
+      }
+      dp += BATCH * STEP * p.ldd;
+#pragma unroll
+      for (int u = 0; u < BATCH; ++u) at[u] += BATCH * STEP * ROW;
     }
   }
+};
+// A block's part in the exchange behind cluster_part_store: all THREADS threads, `ok` whether all went well so far; false when the others'
+// sums did not arrive in time.  SENDER: the warp that sends.
+template <int BN, int CTAS, int THREADS, int SENDER, bool VEC, class Barrier>
+__device__ __forceinline__ bool cluster_exchange(const GemmParams& p, const uint8_t* part, uint64_t* recv, int share, int rank, int row0, int n0, bool ok,
+                                                 volatile int* abort_flag, Barrier&& barrier) {
+  const int rows = max(0, min(128, p.M - row0)), lane = threadIdx.x & 31;
+  ClusterPush<BN, CTAS> push;
+  if (threadIdx.x / 32 == SENDER) push.prepare(part, recv, rows, share, rank, p.cluster_splits, lane);
+  ok = barrier(ok);
+  cluster_wait();
+  if (!ok) return false;
+  if (threadIdx.x / 32 == SENDER) push.send(recv, lane);
+  ClusterFinish<BN, THREADS, VEC> finish;
+  finish.begin(p, share, rows, row0, n0, threadIdx.x);
+  if (!mbar_wait_bounded(smem_u32(recv), 0, abort_flag)) return false;
+  finish.run(p, part, share, row0, threadIdx.x);
+  return true;
 }
 
 // MODE 1: TF32, one MMA per k-step.  MODE 3: 3xTF32, lo*hi + hi*lo + hi*hi per k-step into one accumulator (the lo*lo term,
@@ -275,9 +383,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   uint64_t* empty_bar = bars + STAGES;               // one set per block
   uint64_t* tmem_full_bar = bars + 2 * STAGES;       // one set per block
   uint64_t* tmem_empty_bar = bars + 2 * STAGES + 2;  // used in the leader only
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint64_t* recv = bars + 2 * STAGES + 4;            // in_cluster: the others' partial sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  static_assert((2 * STAGES + 5) * 8 <= GEMM_CTRL_CBAR, "the barriers fit the control area");
+  static_assert((2 * STAGES + 6) * 8 <= GEMM_CTRL_CBAR, "the barriers fit the control area");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -290,10 +399,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                                  : static_cast<int>(blockIdx.x) / CTAS;
   const int num_pairs = in_cluster ? 1 << 30 : static_cast<int>(gridDim.x) / CTAS;
 
-  if (warp == 0) {  // a lane a barrier: full and empty, tmem_full, tmem_empty (the epilogue warps of both blocks)
-    constexpr int BARS = 2 * STAGES + 4;
+  if (warp == 0) {  // a lane a barrier: full and empty, tmem_full, tmem_empty (the epilogue warps of both blocks), recv
+    constexpr int BARS = 2 * STAGES + 5;
     static_assert(BARS <= 32, "a lane a barrier");
-    if (lane < BARS) mbar_init(smem_u32(&bars[lane]), lane < 2 * STAGES + 2 ? 1 : 4 * CTAS);
+    if (lane < BARS) mbar_init(smem_u32(&bars[lane]), lane / 2 == STAGES + 1 ? 4 * CTAS : 1);
     if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
   }
@@ -348,12 +457,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     return MIXED ? 2 * p.num_k_blocks + mix_rescale : min(p.num_k_blocks - k0, p.split_k_blocks);
   };
 
+  bool ok = true, arrived = false;
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = true;
       const uint64_t pol_a = l2_policy(p.l2_policy & 3), pol_b = l2_policy((p.l2_policy >> 2) & 3);
       const bool lockstep = p.epoch_ctr != nullptr && rank == 0;
       const int epoch_stages = p.epoch_stages > 0 ? p.epoch_stages : 64;
@@ -442,7 +551,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       int stage = 0;
       uint32_t phase = 0;
       int local_tile = 0;
-      bool ok = true;
       for (int item = pair_id; item < num_items && ok; item += num_pairs, ++local_tile) {
         const int acc = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
@@ -530,7 +638,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
     const int quarter = warp & 3;  // tensor-memory lanes [32*quarter, 32*quarter+32)
     EpiWarp epi = epi_warp(epi_base, ctrl, warp - 2);
     int local_tile = 0;
-    bool ok = true;
     for (int item = pair_id; item < num_items && ok; item += num_pairs, ++local_tile) {
       const int acc = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
@@ -550,8 +657,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * 256;
       if (in_cluster) {
-        static_assert(ClusterPart<BN>::kBytes <= STAGES * Cfg::kStageBytes, "partial sums fit the ring");
-        cluster_part_store<BN>(reinterpret_cast<float*>(stage_base), taddr, quarter * 32 + lane, 0, BN);
+        static_assert(ClusterPart<BN>::bytes(CTAS) <= STAGES * Cfg::kStageBytes + GEMM_EPI_BUF_BYTES, "partial sums and what arrives fit the rings");
+        cluster_arrive_relaxed();
+        cluster_part_store<BN>(stage_base, taddr, quarter * 32 + lane, 0, BN);
+        arrived = true;
+        break;
       } else if (!p.tma_epilogue) {
         epilogue_rows<BN>(p, taddr, epi.buf, lane, row0, n0);
       } else if (!epilogue_tma<BN>(p, &map_d, &map_c, taddr, epi, lane, row0, n0, item_split(item, num_tiles) * p.part_rows, abort_flag)) {
@@ -573,15 +683,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   }
 
   if (in_cluster && gate_open) {  // a closed gate leaves no partial sums
-    cluster_arrive();
-    cluster_wait();
+    if (!arrived) cluster_arrive_relaxed();
     int tm, tn;
     item_tile_coords(pair_id - split_rank * num_tiles, p, num_tiles, tm, tn);
     const int row0 = tm * BM + static_cast<int>(rank) * 128;
-    if (p.vec_epilogue)
-      cluster_part_finish<BN, CTAS, Cfg::kThreads, true>(p, stage_base, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
-    else
-      cluster_part_finish<BN, CTAS, Cfg::kThreads, false>(p, stage_base, split_rank, static_cast<int>(rank), row0, tn * BN, threadIdx.x);
+    auto barrier = [](bool so_far) { return __syncthreads_and(so_far) != 0; };
+    ok = p.vec_epilogue ? cluster_exchange<BN, CTAS, Cfg::kThreads, 0, true>(p, stage_base, recv, split_rank, rank, row0, tn * BN, ok, abort_flag, barrier)
+                        : cluster_exchange<BN, CTAS, Cfg::kThreads, 0, false>(p, stage_base, recv, split_rank, rank, row0, tn * BN, ok, abort_flag, barrier);
+    if (!ok) {
+      if (threadIdx.x == 0) atomicCAS(p.status, 0, 0x1600 | rank);
+      wait_for_copies();
+    }
+    __syncwarp();
   }
 
   // Neither block may retire, or free tensor memory, while its peer can still signal its barriers, read its shared memory or

@@ -304,6 +304,13 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
   return v;
 }
+// Untiled bulk copy from this block's shared memory to that of a block of the cluster (addresses from map_to_cta), completing its bytes on
+// a barrier there.  Addresses and size are multiples of 16 bytes.
+__device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst_cluster_addr, uint32_t src_smem, uint32_t bytes, uint32_t bar_cluster_addr) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_cluster_addr),
+               "r"(src_smem), "r"(bytes), "r"(bar_cluster_addr)
+               : "memory");
+}
 // Arrive on an mbarrier that may live in the peer block (address from map_to_cta), to signal about nothing but this block's own shared memory
 // and tensor memory (which the other block's MMAs read and write): the release is restricted to objects in shared::cta, and mbar_wait_cluster
 // is its acquiring side.  Tensor memory is ordered by tcgen05.wait and tcgen05.fence.  The unrestricted release waits for the whole

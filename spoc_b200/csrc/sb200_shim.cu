@@ -721,8 +721,8 @@ int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   using Cfg = SplitCfg<BN, CTAS, ROWS>;
   static std::atomic<int> attr_set[kMaxDevices];
   if (!attr_set[dev_index].load()) {
-    for (auto k : {gemm_split_kernel<BN, CTAS, ROWS, false>, gemm_split_kernel<BN, CTAS, ROWS, true>})
-      CU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::kSmemBytes)));
+    CU_TRY(cudaFuncSetAttribute(gemm_split_kernel<BN, CTAS, ROWS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::smem_bytes(false))));
+    CU_TRY(cudaFuncSetAttribute(gemm_split_kernel<BN, CTAS, ROWS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Cfg::smem_bytes(true))));
     attr_set[dev_index].store(1);
   }
   const int units = units_of(CTAS, sm_count);
@@ -739,7 +739,7 @@ int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
   auto kernel = gp.cluster_splits > 1 ? gemm_split_kernel<BN, CTAS, ROWS, true> : gemm_split_kernel<BN, CTAS, ROWS, false>;
-  CU_TRY(launch_pdl(kernel, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, st, CTAS * gp.cluster_splits, m.a_hi, m.b_hi, map_d, map_c, a_box_rows, kp));
+  CU_TRY(launch_pdl(kernel, grid, dim3(Cfg::kThreads), Cfg::smem_bytes(gp.cluster_splits > 1), st, CTAS * gp.cluster_splits, m.a_hi, m.b_hi, map_d, map_c, a_box_rows, kp));
   if (int rc = launch_check("gemm_split_kernel")) return rc;
   return launch_reduce(sm_count, st, gp, part);
 }
