@@ -540,15 +540,32 @@ constexpr int kMaxSplits = 32;
 // SRC_SPLIT (gemm_split_kernel), measured on 1024 x 1024 x K and on 64 and 128 x 4096 x K: pairs 850, 645, 430 and 363 ns a k-block, blocks
 // on their own 540 and 375; a wave's epilogue overlaps nothing, so every wave has the fixed cost (4096 x 4096 x 512: 5.9 us a wave of
 // 128 columns, 8.7 of 256).  least_splits: no k-loop is divided into fewer, so that none is longer, and less exact, than in plain_route.
+// spread: a product that this leaves undivided, or divides through memory, is divided within clusters where the time that its k-loop saves
+// is more than the exchange takes, measured: 300 ns and what arrives at a block at 25 bytes a ns (3xTF32 and TF32 of 512^3 10.0 -> 8.4 and
+// 7.3 -> 6.9 us, 768^3 3xTF32 13.2 -> 12.1, 1024^3 16.1 -> 15.8, 512 x 1024 x 1024 15.7 -> 11.2 and 10.1 -> 8.8, 1024 x 1024 x 2048 TF32 16.1 -> 13.7),
+// by 5 % at least.  Of these estimates the fixed part is 1.6 us too long, which matters where what is fixed differs.  k-loops of fewer than 20
+// k-blocks: from 2^26 multiply-adds on, so that smaller ones keep the bits of the undivided kernels and of the allocation-free
+// entry (which costs 128 x 512 x 512 its 10.9 us instead of 8.5).
 TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
-                       int src = SRC_DIRECT, bool no_scratch = false, int least_splits = 1) {
+                       int src = SRC_DIRECT, bool no_scratch = false, int least_splits = 1, bool spread = false) {
   TileShape best;
+  constexpr double kFixedTooLong = 1600.0, kExchange = 300.0, kExchangeRate = 25.0;
   const int forced = tile_n_setting();
   double best_cost = 0.0;
   const bool split_kernel = src == SRC_SPLIT;
   bool have = false;
   const long long tiles_m = (M + 128 * ctas - 1) / (128 * ctas);
   const int sm_count = units * ctas;
+  auto loop_ns = [&](int bn, long long per_item) {
+    const double per_kblock = split_kernel ? (ctas == 1 ? (bn == 128 ? 540.0 : 375.0) : bn == 256 ? 850.0 : bn == 192 ? 645.0 : bn == 128 ? 430.0 : 363.0)
+                              : src == SRC_CONVERT ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0))
+                              : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0)
+                                      : (bn == 256 ? 277.0 : 165.0);
+    const double charge = bn == 256 || (split_kernel && kblocks < 128) ? 1.0 : three ? (kblocks < 128 ? 1.02 : 1.1) : (kblocks < 128 ? 1.1 : 1.4);
+    return per_item * per_kblock * charge;
+  };
+  auto fixed_ns = [&](int bn) { return split_kernel ? (ctas == 1 ? 5000.0 : 5600.0) + 900.0 * (bn / 64) : 5500.0 + 500.0 * (bn / 32); };
+  bool best_in_cluster = false;
   for (int sp = fixed_splits ? 1 : least_splits; sp <= kMaxSplits; ++sp) {
     if (fixed_splits ? sp != fixed_splits : sp > 1 && (!may_split || forced || kblocks < static_cast<long long>(sp) * kMinSplitKBlocks)) continue;
     const long long per_item = (kblocks + sp - 1) / sp;
@@ -557,18 +574,12 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
       if (ctas == 1 && bn > 128) continue;
       if (bn == 192 && (!three || forced)) continue;
       if (forced && bn != forced && !(ctas == 1 && forced == 256 && bn == 128)) continue;
-      const double per_kblock = split_kernel ? (ctas == 1 ? (bn == 128 ? 540.0 : 375.0) : bn == 256 ? 850.0 : bn == 192 ? 645.0 : bn == 128 ? 430.0 : 363.0)
-                                : src == SRC_CONVERT ? (three ? (bn == 128 ? 1200.0 : 950.0) : (bn == 128 ? 900.0 : 710.0))
-                                : three ? (bn == 256 ? 843.0 : bn == 192 ? 640.0 : bn == 128 ? 430.0 : 340.0)
-                                        : (bn == 256 ? 277.0 : 165.0);
-      const double charge = bn == 256 || (split_kernel && kblocks < 128) ? 1.0 : three ? (kblocks < 128 ? 1.02 : 1.1) : (kblocks < 128 ? 1.1 : 1.4);
       const long long tiles = tiles_m * ((N + bn - 1) / bn);
       const bool in_cluster = split_in_cluster(tiles, sp, ctas, sm_count);
       if (no_scratch && sp > 1 && !in_cluster) continue;
       if (!fixed_splits && sp > 1 && !in_cluster && three && ctas == 2 && kblocks < static_cast<long long>(sp) * kMinSplitKBlocksThree) continue;
       const long long waves = in_cluster ? 1 : (tiles * sp + units - 1) / units;
-      double c = split_kernel ? waves * (per_item * per_kblock * charge + (ctas == 1 ? 5000.0 : 5600.0) + 900.0 * (bn / 64))
-                              : waves * per_item * per_kblock * charge + 5500.0 + 500.0 * (bn / 32) + 800.0 * (waves - 1);
+      double c = split_kernel ? waves * (loop_ns(bn, per_item) + fixed_ns(bn)) : waves * loop_ns(bn, per_item) + fixed_ns(bn) + 800.0 * (waves - 1);
       if (in_cluster)  // the barriers, and 2 ns per quad of a block's share
         c += 1500.0 + 2.0 * (M < 128 ? M : 128) * (bn / 4) / sp;
       else if (sp > 1)
@@ -577,7 +588,25 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
         best.tile_n = bn;
         best.splits = sp;
         best.cost = best_cost = c;
+        best_in_cluster = in_cluster;
         have = true;
+      }
+    }
+  }
+  if (!spread || !have || best_in_cluster || fixed_splits || !may_split || forced) return best;
+  const TileShape first = best;
+  for (int sp = least_splits > 2 ? least_splits : 2; sp * ctas <= 8 && kblocks >= static_cast<long long>(sp) * kMinSplitKBlocks; ++sp) {
+    const long long per_item = (kblocks + sp - 1) / sp;
+    if (per_item * (sp - 1) >= kblocks) continue;
+    if (kblocks < 20 && static_cast<double>(M) * N * kblocks * GEMM_BK < 67108864.0) continue;  // 2^26
+    for (int bn : {256, 192, 128, 64}) {
+      if ((ctas == 1 && bn > 128) || (bn == 192 && !three) || !split_in_cluster(tiles_m * ((N + bn - 1) / bn), sp, ctas, sm_count)) continue;
+      const double arrives = (M < 128 ? M : 128) * (bn * 4.0) * (sp - 1) / sp;
+      const double c = loop_ns(bn, per_item) + fixed_ns(bn) + kExchange + arrives / kExchangeRate;
+      if (c - kFixedTooLong < 0.95 * (first.cost - kFixedTooLong) && c < best.cost) {
+        best.tile_n = bn;
+        best.splits = sp;
+        best.cost = c;
       }
     }
   }
@@ -858,7 +887,7 @@ int units_of(int ctas, int sm_count) { return ctas == 1 ? sm_count : (sm_count /
 TileShape f16_shape(long long M, long long N, long long K, bool three, int sm_count, int* ctas) {
   auto cut = [&](long long rows, long long cols, int fixed, int* c) {
     *c = rows <= GEMM_BM ? 1 : 2;
-    return choose_tiles(rows, cols, round_up(K, 64) / 64, *c, units_of(*c, sm_count), three, true, fixed);
+    return choose_tiles(rows, cols, round_up(K, 64) / 64, *c, units_of(*c, sm_count), three, true, fixed, SRC_DIRECT, false, 1, true);
   };
   int whole_ctas;
   const int fixed_splits = part_of_whole(M, N) ? cut(t_whole.rows, t_whole.cols, 0, &whole_ctas).splits : 0;
@@ -895,7 +924,7 @@ GemmRoute plain_route(int mode, long long M, long long N, long long K, bool addr
   // tiles than its whole, or up to twice as many single blocks, for which there is room for more than twice as many clusters.  A part of
   // one by single blocks finds it by single blocks: route_gemm.)
   const TileShape shape = choose_tiles(M, N, kp / GEMM_BK, r.ctas, units, three, variant == 0, fixed_splits, r.src, !three && addressable,
-                                       least_splits > 0 ? least_splits : 1);
+                                       least_splits > 0 ? least_splits : 1, !three && addressable);
   r.cost = shape.cost;
   r.tile_n = shape.tile_n;
   r.splits = shape.splits;
@@ -952,7 +981,7 @@ GemmRoute route_gemm(int mode, long long M, long long N, long long K, bool addre
   if (r.src == SRC_CONVERT && addressable && M > kNarrowRows * N) return r;
   const long long kblocks = round_up(K, GEMM_BK) / GEMM_BK;
   const int ctas = M <= 128 || macs < kConvertMacs ? 1 : 2, units = units_of(ctas, sm_count);
-  const TileShape shape = choose_tiles(M, N, kblocks, ctas, units, true, true, fixed_splits, SRC_SPLIT, false, r.splits);
+  const TileShape shape = choose_tiles(M, N, kblocks, ctas, units, true, true, fixed_splits, SRC_SPLIT, false, r.splits, addressable);
   const long long tiles = tiles_of(M, N, shape.tile_n, ctas), waves = (tiles * shape.splits + units - 1) / units;
   // ns: a launch in front that reads the operands and writes their low parts, copies of them, or both
   auto prep = [&](int written) { return 1000.0 + 4.0 * (1 + written) * (static_cast<double>(M) * K + static_cast<double>(K) * N) / 5000.0; };
