@@ -92,13 +92,13 @@ __device__ __forceinline__ void tf32_split(const float* x, uint32_t* hi, uint32_
   }
 }
 
-// map_a, map_b: the caller's matrices without rounding, boxes of 32 x a_box_rows (as many as there are rows of A, at most ROWS) and
-// of 32 x 32.  IN_CLUSTER: a k-loop divided within a cluster, as in gemm_pair_kernel.
+// map_a, map_b: the caller's matrices without rounding, boxes of 32 x ROWS and of 32 x 32; map_a_tail: of 32 x p.a_tail_rows, for the last,
+// partial ROWS rows.  Rows past the end, and slabs of B past the last column, are not loaded (gemm_pair_kernel says what they cost).  IN_CLUSTER: a k-loop divided within a cluster, as in gemm_pair_kernel.
 template <int BN, int CTAS, int ROWS, bool IN_CLUSTER>
 __global__ void __launch_bounds__(SplitCfg<BN, CTAS, ROWS>::kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_c, const int a_box_rows,
-                  const GemmParams p) {
+                  const __grid_constant__ CUtensorMap map_a_tail, const __grid_constant__ CUtensorMap map_d,
+                  const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   using Cfg = SplitCfg<BN, CTAS, ROWS>;
   constexpr int RAW = Cfg::kRaw, PARTS = Cfg::kParts, GROUPS = Cfg::kGroups, PART_N = Cfg::kPartN;
   constexpr uint32_t B_BYTES = Cfg::kBBytes;
@@ -118,7 +118,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = CTAS == 2 || IN_CLUSTER ? cluster_ctarank() : 0u;
-  const uint32_t rank = cta & (CTAS - 1u), leader = cta - rank;
+  const uint32_t rank = blockIdx.x & (CTAS - 1u), leader = cta - rank;  // uniform to the compiler, as in gemm_pair_kernel
   const int num_tiles = p.tiles_m * p.tiles_n, num_items = num_tiles * p.splits;
   // IN_CLUSTER: item `split * num_tiles + tile` is this pair's only one
   const int split_rank = IN_CLUSTER ? static_cast<int>(cta) / CTAS : 0;
@@ -140,6 +140,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (threadIdx.x == 64) {
     tma_prefetch_desc(&map_a);
     tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(&map_a_tail);
     if (p.tma_epilogue) tma_prefetch_desc(&map_d);
   }
   if (warp == GROUPS * 4 + 1) {
@@ -311,6 +312,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             ok = false;
             break;
           }
+          const bool whole_rows = m0 + ROWS <= p.M;
+          const int rows = whole_rows ? ROWS : m0 < p.M ? p.a_tail_rows : 0;
+          const int slabs = max(0, min(PART_N / 32, (p.N - n0 + 31) >> 5));
           for (int kb = kb0; kb < kb0 + blocks; ++kb) {
             if (!mbar_wait_bounded(smem_u32(&raw_empty[stage]), phase ^ 1u, abort_flag)) {
               atomicCAS(p.status, 0, 0x3000 | (rank << 4) | stage);
@@ -319,11 +323,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             const uint32_t bar = smem_u32(&raw_full[stage]);
             uint8_t* dst = smem + stage * Cfg::kRawBytes;
-            mbar_arrive_expect_tx(bar, a_box_rows * 128 + B_BYTES);
-            tma_load_2d_hint(smem_u32(dst), &map_a, bar, kb * GEMM_BK, m0, pol_a);
+            mbar_arrive_expect_tx(bar, rows * 128 + slabs * 4096);
+            if (whole_rows)
+              tma_load_2d_hint(smem_u32(dst), &map_a, bar, kb * GEMM_BK, m0, pol_a);
+            else if (rows)
+              tma_load_2d_hint(smem_u32(dst), &map_a_tail, bar, kb * GEMM_BK, m0, pol_a);
 #pragma unroll
             for (int sl = 0; sl < PART_N / 32; ++sl)
-              tma_load_2d_hint(smem_u32(dst + Cfg::kABytes + sl * 4096), &map_b, bar, n0 + 32 * sl, kb * GEMM_BK, pol_b);
+              if (sl < slabs) tma_load_2d_hint(smem_u32(dst + Cfg::kABytes + sl * 4096), &map_b, bar, n0 + 32 * sl, kb * GEMM_BK, pol_b);
             if (++stage == RAW) {
               stage = 0;
               phase ^= 1u;

@@ -51,6 +51,9 @@ struct GemmParams {
   int act;      // 0 none, 1 relu
   int* status;  // device word, set non-zero when a bounded wait expired
   int group_m;  // CTA-pair kernel: row tiles per rasterisation band
+  // Rows of the boxes that the last, partial 128 rows of A are loaded with (a multiple of 8; gemm_pair_kernel but for the mixed mode, and
+  // gemm_split_kernel): rows past the end are not asked for.
+  int a_tail_rows;
   // Gathered result: when n_replicas > 0 every output element is also stored to the same position of
   // these further copies of D (this GPU's own or peers' memory mapped into this process), so that a
   // row-sharded product leaves the whole matrix on every GPU without a separate all-gather.

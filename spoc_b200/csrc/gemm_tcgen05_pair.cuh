@@ -342,6 +342,10 @@ __device__ __forceinline__ bool cluster_exchange(const GemmParams& p, const uint
 // 2^-22 relative, is dropped).  MODE 4: the same three-term split on fp16 panels (kind::f16): a 128-byte operand row holds 64
 // halves instead of 32 floats, so a k-block spans 64 k and a k-step 16, in the same bytes, descriptors and cycles as the TF32
 // forms.  MODE 2: fp16 panels, one MMA.
+// map_a_x, map_b_x, but for the mixed mode: the high and low parts of A once more, for the last, partial 128 rows, with boxes of p.a_tail_rows.
+// TMA takes 3 ns for a row past the end when a few blocks ask for such rows and 15 ns when all do, so that few rows went slower than 128 (TF32
+// x 6144 x 1024: 10 rows 53 us, with their own boxes 9; 64 x 4096 x 4096 with epilogue 17.0 -> 13.3).  The accumulator's rows that nothing was
+// loaded for come of whatever the ring held, and are not stored.
 // MODE 5 (mixed; always SRC_DIRECT): map_a_hi / map_b_hi are TFLOAT32 maps over the caller's matrices, map_a_lo / map_b_lo lie
 // over the fp16 panels of the high parts and map_a_x / map_b_x over those of the low parts (all K-major, [rows x Kp], Kp a
 // multiple of 64).  A tile is computed in three runs of stages, every stage the same bytes: K/64 cross stages (the four fp16
@@ -392,7 +396,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
   const int lane = threadIdx.x & 31;
   const bool in_cluster = MODE != 5 && p.cluster_splits > 1;
   const uint32_t cta = CTAS == 2 || in_cluster ? cluster_ctarank() : 0u;
-  const uint32_t rank = cta & (CTAS - 1u), leader = cta - rank;  // rank 0 = leader of its pair
+  // Rank 0 is the leader of its pair.  From the block's index and not from its rank in the cluster, which is the same: so the compiler sees that
+  // what depends on it is the same in all threads, and keeps descriptors in uniform registers behind branches on it.
+  const uint32_t rank = blockIdx.x & (CTAS - 1u), leader = cta - rank;
   // in_cluster: item `split * num_tiles + tile` is this pair's only one
   const int split_rank = in_cluster ? static_cast<int>(cta) / CTAS : 0;
   const int pair_id = in_cluster ? static_cast<int>(blockIdx.x) / (CTAS * p.cluster_splits) + split_rank * p.tiles_m * p.tiles_n
@@ -417,10 +423,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       tma_prefetch_desc(&map_a_lo);
       tma_prefetch_desc(&map_b_lo);
     }
-    if (MIXED) {
-      tma_prefetch_desc(&map_a_x);
-      tma_prefetch_desc(&map_b_x);
-    }
+    tma_prefetch_desc(&map_a_x);
+    if (THREE || MIXED) tma_prefetch_desc(&map_b_x);
     if (p.tma_epilogue) tma_prefetch_desc(&map_d);
   }
   if (warp == 1) {
@@ -475,6 +479,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
         const int stages = item_stages(item, k0);
         const int m0 = tm * BM + static_cast<int>(rank) * 128;     // this block's rows of A
         const int n0 = tn * BN + static_cast<int>(rank) * PART_N;  // this block's part of B's columns
+        // the map of these rows is chosen here, so that the loads are the same straight line for every tile: behind branches on what lies
+        // past the end each took 100 cycles more (8192^3 TF32 1370 -> 1600 us)
+        auto rows_of_a = [&](int m) { return MIXED || m + 128 <= p.M ? 128 : p.a_tail_rows; };
+        const CUtensorMap* const pa_hi = rows_of_a(m0) == 128 ? &map_a_hi : &map_a_x;
+        const CUtensorMap* const pa_lo = rows_of_a(m0) == 128 ? &map_a_lo : &map_b_x;
+        int stage_bytes = 0;  // of both blocks
+        for (int r = 0; r < CTAS; ++r) stage_bytes += Cfg::kOperands * (rows_of_a(tm * BM + r * 128) * 128 + static_cast<int>(B_BYTES));
         for (int it = 0; it < stages; ++it) {
           const int kb = MIXED ? (it < p.num_k_blocks + mix_rescale ? it : it - p.num_k_blocks - mix_rescale) : k0 + it;
           if (lockstep && (it % epoch_stages) == 0)
@@ -486,7 +497,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
             break;
           }
           // the leader arms its barrier with the bytes of both blocks
-          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), CTAS * Cfg::kStageBytes);
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), stage_bytes);
           const uint32_t bar = CTAS == 2 ? map_to_cta(smem_u32(&full_bar[stage]), leader) : smem_u32(&full_bar[stage]);
           uint8_t* sp = stage_base + stage * Cfg::kStageBytes;
           auto load = [&](uint8_t* dst, const CUtensorMap& map, int x, int y, uint64_t pol) {
@@ -501,32 +512,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
               load(sp + 2 * PAIR_A_BYTES + B_BYTES, map_b_x, kb * 64, n0, pol_b);
             } else {
               // main stage: two consecutive k-blocks of 32 of the caller's A and B
-#pragma unroll
+  #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 uint8_t* hp = sp + h * (PAIR_A_BYTES + B_BYTES);
                 load(hp, map_a_hi, kb * 64 + 32 * h, m0, pol_a);
-#pragma unroll
+  #pragma unroll
                 for (int sl = 0; sl < SLABS; ++sl) load(hp + PAIR_A_BYTES + sl * 4096, map_b_hi, n0 + 32 * sl, kb * 64 + 32 * h, pol_b);
               }
             }
           } else {
-            load(sp, map_a_hi, kb * BK_ELEMS, m0, pol_a);
-            if (DIRECT) {
-              // B is K x N row-major: x = column, y = k; slabs of 32 columns cover this block's part
-#pragma unroll
-              for (int sl = 0; sl < SLABS; ++sl) load(sp + PAIR_A_BYTES + sl * 4096, map_b_hi, n0 + 32 * sl, kb * BK_ELEMS, pol_b);
-            } else {
-              load(sp + PAIR_A_BYTES, map_b_hi, kb * BK_ELEMS, n0, pol_b);
-            }
-            if (THREE) {
-              uint8_t* lp = sp + PAIR_A_BYTES + B_BYTES;
-              load(lp, map_a_lo, kb * BK_ELEMS, m0, pol_a);
+            auto load_b = [&](uint8_t* dst, const CUtensorMap& map) {
               if (DIRECT) {
+                // B is K x N row-major: x = column, y = k; slabs of 32 columns cover this block's part
 #pragma unroll
-                for (int sl = 0; sl < SLABS; ++sl) load(lp + PAIR_A_BYTES + sl * 4096, map_b_lo, n0 + 32 * sl, kb * BK_ELEMS, pol_b);
+                for (int sl = 0; sl < SLABS; ++sl) load(dst + sl * 4096, map, n0 + 32 * sl, kb * BK_ELEMS, pol_b);
               } else {
-                load(lp + PAIR_A_BYTES, map_b_lo, kb * BK_ELEMS, n0, pol_b);
+                load(dst, map, kb * BK_ELEMS, n0, pol_b);
               }
+            };
+            load(sp, *pa_hi, kb * BK_ELEMS, m0, pol_a);
+            load_b(sp + PAIR_A_BYTES, map_b_hi);
+            if (THREE) {
+              load(sp + PAIR_A_BYTES + B_BYTES, *pa_lo, kb * BK_ELEMS, m0, pol_a);
+              load_b(sp + 2 * PAIR_A_BYTES + B_BYTES, map_b_lo);
             }
           }
           if (++stage == STAGES) {

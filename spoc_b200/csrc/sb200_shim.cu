@@ -398,6 +398,13 @@ int l2_policy_setting() {
   return v;
 }
 
+// Rows of the boxes of the last, partial 128 rows of A (or of 64, all there are, for gemm_split_kernel's blocks of so few).  Beside whole rows they
+// take a map more, 0.3 us of the host's time, which small products have not got (5334 x 20 x 264 TF32 6.1 us, with it 6.6).
+int a_tail_rows(long long M, long long N, long long kblocks) {
+  if (M > GEMM_BM && static_cast<double>(M) * N * kblocks * GEMM_BK < 67108864.0) return GEMM_BM;  // 2^26 multiply-adds
+  return static_cast<int>(round_up((M - 1) % GEMM_BM + 1, 8));
+}
+
 // Fields of GemmParams that follow from the others: whether the epilogue may move 128-bit vectors, and the
 // eviction policies.
 int env_int(const char* name, int fallback, int lo, int hi) {
@@ -417,6 +424,7 @@ void derive_params(GemmParams* gp) {
   for (int r = 0; r < gp->n_replicas; ++r) vec = vec && al16(gp->replicas[r]);
   gp->vec_epilogue = vec ? 1 : 0;
   gp->l2_policy = l2_policy_setting();
+  gp->a_tail_rows = a_tail_rows(gp->M, gp->N, gp->num_k_blocks);
 }
 
 // Tensor maps of D and C for the epilogue that moves them by TMA; sets gp->tma_epilogue when it applies: 16-byte aligned
@@ -615,7 +623,7 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
 
 int units_of(int ctas, int sm_count);
 
-// The operand maps of one launch; x: the mixed mode's third pair (else unused).
+// The operand maps of one launch; x: the mixed mode's third pair, else the maps of A (hi, lo) for its last rows.
 struct OperandMaps {
   CUtensorMap a_hi, b_hi, a_lo, b_lo, a_x, b_x;
 };
@@ -746,7 +754,7 @@ int launch_convert_for(int bn, bool vec, int dev_index, int sm_count, cudaStream
 
 // gemm_split_kernel, the same way.  m.a_hi and m.b_hi lie over the caller's matrices without rounding.
 template <int BN, int CTAS, int ROWS = 128>
-int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, int a_box_rows, GemmParams gp, float* part) {
+int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, GemmParams gp, float* part) {
   using Cfg = SplitCfg<BN, CTAS, ROWS>;
   static std::atomic<int> attr_set[kMaxDevices];
   if (!attr_set[dev_index].load()) {
@@ -768,23 +776,23 @@ int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
   auto kernel = gp.cluster_splits > 1 ? gemm_split_kernel<BN, CTAS, ROWS, true> : gemm_split_kernel<BN, CTAS, ROWS, false>;
-  CU_TRY(launch_pdl(kernel, grid, dim3(Cfg::kThreads), Cfg::smem_bytes(gp.cluster_splits > 1), st, CTAS * gp.cluster_splits, m.a_hi, m.b_hi, map_d, map_c, a_box_rows, kp));
+  CU_TRY(launch_pdl(kernel, grid, dim3(Cfg::kThreads), Cfg::smem_bytes(gp.cluster_splits > 1), st, CTAS * gp.cluster_splits, m.a_hi, m.b_hi, m.a_x, map_d, map_c, kp));
   if (int rc = launch_check("gemm_split_kernel")) return rc;
   return launch_reduce(sm_count, st, gp, part);
 }
 
-int launch_split_for(int bn, int ctas, int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, int a_box_rows, const GemmParams& gp,
+int launch_split_for(int bn, int ctas, int dev_index, int sm_count, cudaStream_t st, const OperandMaps& m, const GemmParams& gp,
                      float* part) {
   if (ctas == 1 && gp.M <= 64)
-    return bn == 64 ? launch_split<64, 1, 64>(dev_index, sm_count, st, m, a_box_rows, gp, part)
-                    : launch_split<128, 1, 64>(dev_index, sm_count, st, m, a_box_rows, gp, part);
+    return bn == 64 ? launch_split<64, 1, 64>(dev_index, sm_count, st, m, gp, part)
+                    : launch_split<128, 1, 64>(dev_index, sm_count, st, m, gp, part);
   if (ctas == 1)
-    return bn == 64 ? launch_split<64, 1>(dev_index, sm_count, st, m, a_box_rows, gp, part)
-                    : launch_split<128, 1>(dev_index, sm_count, st, m, a_box_rows, gp, part);
-  return bn == 64    ? launch_split<64, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part)
-         : bn == 128 ? launch_split<128, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part)
-         : bn == 192 ? launch_split<192, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part)
-                     : launch_split<256, 2>(dev_index, sm_count, st, m, a_box_rows, gp, part);
+    return bn == 64 ? launch_split<64, 1>(dev_index, sm_count, st, m, gp, part)
+                    : launch_split<128, 1>(dev_index, sm_count, st, m, gp, part);
+  return bn == 64    ? launch_split<64, 2>(dev_index, sm_count, st, m, gp, part)
+         : bn == 128 ? launch_split<128, 2>(dev_index, sm_count, st, m, gp, part)
+         : bn == 192 ? launch_split<192, 2>(dev_index, sm_count, st, m, gp, part)
+                     : launch_split<256, 2>(dev_index, sm_count, st, m, gp, part);
 }
 
 size_t partial_bytes(long long M, long long N, const TileShape& shape, int ctas, int sm_count) {
@@ -1101,8 +1109,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     CU_TRY(cudaEventCreate(&rec.e2));
     CU_TRY(cudaEventRecord(rec.e0, st));
   }
-  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
-  int a_box_rows = GEMM_BM;
+  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail;
+  const int tail = a_tail_rows(M, N, kp / GEMM_BK);
   if (route.src == SRC_CONVERT) {
     // no panels, no operand maps
   } else if (direct || route.src == SRC_SPLIT) {
@@ -1125,14 +1133,20 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     const PrepLoJob ja{A, lda, a_lo, a_copy, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp), addressable_a ? 1 : 0};
     const PrepLoJob jb{B, ldb, b_lo, b_copy, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), addressable_b ? 1 : 0};
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, b_panels_ready, nullptr))) return rc;
-    // the split kernel takes the elements as they are
-    if (!direct) a_box_rows = static_cast<int>(std::min<long long>(GEMM_BM, round_up(M, 8)));
-    if ((rc = encode_map_2d(&ma_hi, copy_a ? a_copy : A, K, M, copy_a ? kp : lda, GEMM_BK, a_box_rows, direct))) return rc;
+    // the split kernel takes the elements as they are, by up to 64 rows where that is all there are
+    auto map_a = [&](CUtensorMap* map, int rows) { return encode_map_2d(map, copy_a ? a_copy : A, K, M, copy_a ? kp : lda, GEMM_BK, rows, direct); };
+    if ((rc = map_a(&ma_hi_tail, tail))) return rc;
+    ma_hi = ma_hi_tail;  // where the whole rows' box is the same, or there are no whole rows (64, 128) and it is not used
+    const int whole = !direct && M <= 64 ? 64 : GEMM_BM;
+    if (M > whole && tail != whole && (rc = map_a(&ma_hi, whole))) return rc;
     if ((rc = encode_map_2d(&mb_hi, copy_b ? b_copy : B, N, K, copy_b ? np : ldb, 32, GEMM_BK, direct, true))) return rc;
     ma_lo = ma_hi;
     mb_lo = mb_hi;
+    ma_lo_tail = ma_hi_tail;
     if (lows) {
-      if ((rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
+      if ((rc = encode_map_2d(&ma_lo_tail, a_lo, kp, M, kp, GEMM_BK, tail, false))) return rc;
+      ma_lo = ma_lo_tail;
+      if (M > GEMM_BM && tail != GEMM_BM && (rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
       if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     }
   } else {
@@ -1144,11 +1158,13 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     float* a_hi = reinterpret_cast<float*>(ws + kOps * b_bytes);
     float* a_lo = MODE == 3 ? reinterpret_cast<float*>(ws + kOps * b_bytes + a_bytes) : a_hi;
     if ((rc = launch_prep_panels<MODE>(d.sm_count, st, A, lda, a_hi, a_lo, B, ldb, b_hi, b_lo, M, N, K, b_panels_ready))) return rc;
-    const int b_box_rows = tile_n / route.ctas;
+    const int b_box = tile_n / route.ctas;
     if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, b_box_rows))) return rc;
+    if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, b_box))) return rc;
     if ((rc = encode_panel_map(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, b_box_rows))) return rc;
+    if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, b_box))) return rc;
+    if ((rc = encode_panel_map(&ma_hi_tail, a_hi, kp, M, tail))) return rc;
+    if ((rc = encode_panel_map(&ma_lo_tail, a_lo, kp, M, tail))) return rc;
   }
 
   GemmParams gp = gp_in;
@@ -1165,8 +1181,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     const ConvOperands o{A, B, lda, ldb, static_cast<int>(K)};
     rc = launch_convert_for<MODE>(tile_n, addressable && (K & 3) == 0 && (N & 3) == 0, dev_index, d.sm_count, st, o, gp, part);
   } else {
-    const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
-    rc = route.src == SRC_SPLIT ? launch_split_for(tile_n, route.ctas, dev_index, d.sm_count, st, maps, a_box_rows, gp, part)
+    const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail};
+    rc = route.src == SRC_SPLIT ? launch_split_for(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
          : direct               ? launch_tiles_for<MODE, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
                                 : launch_tiles_for<MODE, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
   }
@@ -1309,14 +1325,21 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
       if ((rc = launch_check("prep_b_f16_kernel"))) return rc;
     }
   }
-  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
-  if ((rc = encode_map_f16(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_map_f16(&mb_hi, b_hi, kp, N, tile_n / ctas))) return rc;
+  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail;
+  const int tail = a_tail_rows(M, N, kp / 64), b_box = tile_n / ctas;
+  const bool whole = M > GEMM_BM && tail != GEMM_BM;  // whole 128 rows beside a partial last one
+  if ((rc = encode_map_f16(&ma_hi_tail, a_hi, kp, M, tail))) return rc;
+  ma_hi = ma_hi_tail;
+  if (whole && (rc = encode_map_f16(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
+  if ((rc = encode_map_f16(&mb_hi, b_hi, kp, N, b_box))) return rc;
   ma_lo = ma_hi;
+  ma_lo_tail = ma_hi_tail;
   mb_lo = mb_hi;
   if (THREE) {
-    if ((rc = encode_map_f16(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_map_f16(&mb_lo, b_lo, kp, N, tile_n / ctas))) return rc;
+    if ((rc = encode_map_f16(&ma_lo_tail, a_lo, kp, M, tail))) return rc;
+    ma_lo = ma_lo_tail;
+    if (whole && (rc = encode_map_f16(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
+    if ((rc = encode_map_f16(&mb_lo, b_lo, kp, N, b_box))) return rc;
   }
   GemmParams gp = gp_in;
   gp.num_k_blocks = static_cast<int>(kp / 64);
@@ -1329,7 +1352,7 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
   if (prof) CU_TRY(cudaEventRecord(rec.e1, st));
   const int dev_index = static_cast<int>(&d - g_dev);
   gp.splits = shape.splits;
-  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
+  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail};
   float* part = reinterpret_cast<float*>(ws + need);
   rc = launch_tiles_for<THREE ? 4 : 2, SRC_PANELS>(tile_n, ctas, dev_index, d.sm_count, st, maps, gp, part);
   if (prof) {
@@ -1449,13 +1472,15 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     const PrepLoJob ja{A, lda, pa_lo, nullptr, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp32), 1};
     const PrepLoJob jb{B, ldb, pb_lo, nullptr, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), 1};
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, false, gp.gate))) return rc;
-    CUtensorMap pma_lo, pmb_lo;
+    CUtensorMap pma_lo, pmb_lo, ma_tail, pma_lo_tail;
     if ((rc = encode_map_2d(&pma_lo, pa_lo, kp32, M, kp32, GEMM_BK, GEMM_BM, false))) return rc;
+    if ((rc = encode_map_2d(&ma_tail, A, K, M, lda, GEMM_BK, a_tail_rows(M, N, kp32 / GEMM_BK), true))) return rc;
+    if ((rc = encode_map_2d(&pma_lo_tail, pa_lo, kp32, M, kp32, GEMM_BK, a_tail_rows(M, N, kp32 / GEMM_BK), false))) return rc;
     if ((rc = encode_map_2d(&pmb_lo, pb_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     gp.num_k_blocks = static_cast<int>(kp32 / GEMM_BK);
     gp.gate_value = 0;
     gp.epoch_ctr = nullptr;  // the ring belongs to the launch in front
-    const OperandMaps plain{ma, mb, pma_lo, pmb_lo, pma_lo, pmb_lo};
+    const OperandMaps plain{ma, mb, pma_lo, pmb_lo, ma_tail, pma_lo_tail};
     rc = launch_tiles_for<3, SRC_DIRECT>(256, 2, dev_index, d.sm_count, st, plain, gp, nullptr);
   }
   if (prof) {
@@ -3120,15 +3145,18 @@ int launch_gemm_fixed_scratch(const NoAllocDevice& nd, int dev, cudaStream_t st,
   int rc = launch_prep_panels<MODE>(nd.sm_count, st, A, lda, a_hi, a_lo, B, ldb, b_hi, b_lo, M, N, K, false);
   if (rc) return rc;
   const int tile_n = choose_tiles(M, N, kp / GEMM_BK, 1, nd.sm_count, MODE == 3, false).tile_n;
-  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo;
+  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail;
+  const int tail = a_tail_rows(M, N, kp / GEMM_BK);
   if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
   if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, tile_n))) return rc;
   if ((rc = encode_panel_map(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
   if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, tile_n))) return rc;
+  if ((rc = encode_panel_map(&ma_hi_tail, a_hi, kp, M, tail))) return rc;
+  if ((rc = encode_panel_map(&ma_lo_tail, a_lo, kp, M, tail))) return rc;
   gp.num_k_blocks = static_cast<int>(kp / GEMM_BK);
   gp.status = nd.status;
   derive_params(&gp);
-  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_lo, mb_lo};
+  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail};
   return launch_tiles_for<MODE, SRC_PANELS>(tile_n, 1, dev, nd.sm_count, st, maps, gp, nullptr);
 }
 

@@ -1,0 +1,66 @@
+"""Rows past the end of A, which have boxes of their own, and k-loops that the second choice divides within clusters."""
+import ctypes as C
+import math
+
+import numpy as np
+import pytest
+
+from spoc_b200 import _lib as L
+from tests import oracle_lib as O
+from tests.gpu_util import CANARY, Dev, dev_from, gemm
+from tests.test_gpu_gemm import tol
+
+pytestmark = pytest.mark.gpu
+
+MODES = [L.MODE_3XTF32, L.MODE_TF32, L.MODE_3XF16, L.MODE_F16]
+
+
+def describe(mode, M, N, K, addressable):
+    out = C.create_string_buffer(256)
+    assert L.load().sb200_gemm_describe(mode, M, N, K, addressable, 148, out, 256) == 0
+    return out.value.decode()
+
+
+def check(backend, device, mode, M, N, K, lda, ldb, ldd, ldc):
+    rng = np.random.default_rng(M + N + K)
+    a, b, c = (rng.uniform(-1, 1, (r, ld)).astype(np.float32) for r, ld in ((M, lda), (K, ldb), (M, ldc)))
+    bias = rng.uniform(-0.1, 0.1, N).astype(np.float32)
+    A, B, Cm, Bi = (dev_from(backend, device, x.ravel()) for x in (a, b, c, bias))
+    D = Dev(backend, device, (M + 1) * ldd)
+    try:
+        gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=ldc, ldd=ldd)
+        got = D.download().reshape(M + 1, ldd)
+        ref = O.gemm(np.ascontiguousarray(a[:, :K]).ravel(), np.ascontiguousarray(b[:, :N]).ravel(), M, N, K, 1.5, 0.5,
+                     np.ascontiguousarray(c[:, :N]).ravel(), bias, 1)
+        # the clamp halves the reference's mean square, alpha scales the error: as in the other epilogue tests
+        assert O.gemm_rel_error(got[:M, :N], ref) <= tol(mode, K) * 1.5 * math.sqrt(2), describe(mode, M, N, K, 1)
+        assert np.all(got[:M, N:] == CANARY) and np.all(got[M] == CANARY)
+    finally:
+        for x in (A, B, Cm, Bi, D):
+            x.free()
+
+
+# One row, a multiple of 8 and one off it, whole 128 rows, and beside whole ones 1, 8, 9 and 127 more (from 2^26 multiply-adds on those
+# have boxes of their own; a pair's second block then has some of the rows, or none).
+TAILS = [(1, 132, 260), (7, 260, 132), (8, 64, 96), (9, 516, 516), (64, 132, 260), (65, 256, 300), (127, 132, 1028), (128, 64, 260), (129, 1028, 516),
+         (136, 2052, 260), (137, 1028, 516), (255, 516, 516), (257, 1028, 260), (393, 260, 700)]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("M,N,K", TAILS)
+def test_rows_past_the_end(backend, device, mode, M, N, K):
+    check(backend, device, mode, M, N, K, K, N, N, N)
+
+
+# (mode, M, N, K, splits): even and uneven shares of rows, rows and columns that end within a block's share, a last item that is shorter
+SPREAD = [(L.MODE_3XTF32, 512, 512, 512, 2), (L.MODE_3XTF32, 509, 516, 1028, 3), (L.MODE_3XTF32, 768, 768, 768, 3), (L.MODE_3XTF32, 1000, 1020, 1000, 2),
+          (L.MODE_TF32, 512, 512, 512, 2), (L.MODE_TF32, 1001, 1000, 2052, 2), (L.MODE_F16, 147, 56, 1700, 3), (L.MODE_3XF16, 300, 1020, 2052, 2)]
+
+
+@pytest.mark.parametrize("mode,M,N,K,splits", SPREAD)
+@pytest.mark.parametrize("ldd", ["quads", "single"])
+def test_k_loops_divided_by_the_second_choice(backend, device, mode, M, N, K, splits, ldd):
+    text = describe(mode, M, N, K, 1)
+    assert f"splits={splits} " in text, text
+    pad = 4 if ldd == "quads" else 1        # rows of the result on 16-byte boundaries, and not
+    check(backend, device, mode, M, N, K, K, N, N + pad, N + pad)
