@@ -311,10 +311,10 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
             static_assert(ClusterPart<BN>::bytes(1) <= STAGES * Cfg::kStageBytes, "partial sums and what arrives fit the ring");
             cluster_part_store<BN>(smem, taddr, quarter * 32 + lane, half * (BN / 2), BN / 2);
           } else if (!p.tma_epilogue) {
-            epilogue_rows<BN / 2>(p, taddr, epi.buf, lane, row0, c0);
+            epilogue_rows(p, taddr, epi.buf, lane, row0, c0, BN / 2);
           } else {
             epilogue_tma_begin(p, &map_c, epi, lane, row0, c0);
-            if (!epilogue_tma<BN / 2>(p, &map_d, &map_c, taddr, epi, lane, row0, c0, split * p.part_rows, abort_flag)) {
+            if (!epilogue_tma(p, &map_d, &map_c, taddr, epi, lane, row0, c0, BN / 2, split * p.part_rows, abort_flag)) {
               if (lane == 0) atomicCAS(p.status, 0, 0x2500);
               ok = false;
             }

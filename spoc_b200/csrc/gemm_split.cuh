@@ -257,11 +257,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         arrived = true;
       } else if (c0 < p.N) {
         if (!p.tma_epilogue) {
-          epilogue_rows<EPI_N>(p, taddr, epi.buf, lane, row0, c0);
+          epilogue_rows(p, taddr, epi.buf, lane, row0, c0, EPI_N);
           fence_async_shared();  // its ordinary stores to the tile before the loads of the next item, which land there
         } else {
           epilogue_tma_begin(p, &map_c, epi, lane, row0, c0);
-          if (!epilogue_tma<EPI_N>(p, &map_d, &map_c, taddr, epi, lane, row0, c0, item_split(item, num_tiles) * p.part_rows, abort_flag)) {
+          if (!epilogue_tma(p, &map_d, &map_c, taddr, epi, lane, row0, c0, EPI_N, item_split(item, num_tiles) * p.part_rows, abort_flag)) {
             if (lane == 0) atomicCAS(p.status, 0, 0x3500 | (rank << 4));
             ok = false;
           }

@@ -152,7 +152,7 @@ __device__ __forceinline__ void epilogue_tma_begin(const GemmParams& p, const CU
   __syncwarp();
 }
 
-// Epilogue of one warp for its 32 rows x BN columns of a finished accumulator, D (and C) moved by TMA: tensor memory ->
+// Epilogue of one warp for its 32 rows x `columns` columns of a finished accumulator, D (and C) moved by TMA: tensor memory ->
 // registers (lane = row), D = act(alpha*acc + beta*C + bias) there, -> a 32 x 32 tile in shared memory in the 128-byte
 // swizzle (no bank conflicts: eight lanes of a phase hit eight 16-byte columns) -> one bulk store per tile, two tiles in
 // turn.  Bound by issue latency of the one warp a scheduler has: a 32-column chunk takes about 300 instructions without
@@ -160,12 +160,11 @@ __device__ __forceinline__ void epilogue_tma_begin(const GemmParams& p, const CU
 // (6 us of 16 at 1024 x 1024 x 64 with 256-column tiles) whether it stored or not.
 // row_shift: added to the row that is stored to (partial results of a divided k-loop lie below one another).
 // Returns false when a wait for C ran out (warp-uniform).
-template <int BN>
 __device__ __forceinline__ bool epilogue_tma(const GemmParams& p, const CUtensorMap* map_d, const CUtensorMap* map_c, uint32_t taddr,
-                                             EpiWarp& e, int lane, int row0, int n0, int row_shift, volatile int* abort_flag) {
+                                             EpiWarp& e, int lane, int row0, int n0, int columns, int row_shift, volatile int* abort_flag) {
   if (row0 >= p.M) return true;
   const uint64_t pol = l2_policy((p.l2_policy >> 4) & 3);
-  const int chunks = min(BN / 32, (p.N - n0 + 31) >> 5);
+  const int chunks = min(columns >> 5, (p.N - n0 + 31) >> 5);
   const bool scaled = p.row_scale != nullptr;
   const float rs = scaled && row0 + lane < p.M ? p.row_scale[row0 + lane] : 1.0f;
 #pragma unroll 1
@@ -249,8 +248,8 @@ __device__ __forceinline__ bool epilogue_tma(const GemmParams& p, const CUtensor
 // floats of a row.  C and the bias of a chunk are loaded while the chunk before is stored: with the loads behind the staging a
 // chunk took 2 us, so that unaligned results cost TF32 products up to half of their time (4000 x 4000 x 1000: 117 us, with
 // aligned rows 61).
-template <int BN, bool FULL>
-__device__ __forceinline__ void epilogue_columns(const GemmParams& p, uint32_t taddr, float* tbuf, int lane, int row0, int n0, int rows) {
+template <bool FULL>
+__device__ __forceinline__ void epilogue_columns(const GemmParams& p, uint32_t taddr, float* tbuf, int lane, int row0, int n0, int columns, int rows) {
   const float rs = p.row_scale && lane < rows ? p.row_scale[row0 + lane] : 1.0f;
   const long long ldc = p.ldc, ldd = p.ldd;
   float cv[32], bias_v = 0.0f, cs = 1.0f;
@@ -271,7 +270,7 @@ __device__ __forceinline__ void epilogue_columns(const GemmParams& p, uint32_t t
   for (int rr = 0; rr < 32; ++rr) cv[rr] = 0.0f;
   load(n0 + lane);
 #pragma unroll 1
-  for (int chunk = 0; chunk < BN / 32; ++chunk) {
+  for (int chunk = 0; chunk < columns >> 5; ++chunk) {
     const int col = n0 + chunk * 32 + lane;
     if (n0 + chunk * 32 >= p.N) break;  // warp-uniform
     uint32_t v[32];
@@ -293,7 +292,7 @@ __device__ __forceinline__ void epilogue_columns(const GemmParams& p, uint32_t t
 #pragma unroll
       for (int rr = 0; rr < 32; ++rr) x[rr] = (x[rr] > 0.0f) ? x[rr] : 0.0f;
     }
-    if (chunk + 1 < BN / 32) load(col + 32);
+    if (chunk + 1 < columns >> 5) load(col + 32);
     if (col < p.N) {
       const long long off = static_cast<long long>(row0) * ldd + col;
       float* dp = p.D + off;
@@ -321,15 +320,14 @@ __device__ __forceinline__ void epilogue_columns(const GemmParams& p, uint32_t t
 // D = act(alpha*acc + beta*C + bias), and the same values to every replica of D.  `taddr` addresses the warp's 32
 // tensor-memory lanes at the accumulator's first column.  Every element goes through the same operations in the same
 // order on all paths, so they give the same bits.
-template <int BN>
-__device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t taddr, float* tbuf, int lane, int row0, int n0) {
+__device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t taddr, float* tbuf, int lane, int row0, int n0, int columns) {
   const int rows_here = min(32, p.M - row0);  // may be <= 0 for a ragged last tile
   if (p.vec_epilogue) {
     const int sub = lane >> 3;       // this lane's row within each group of four rows
     const int cq = (lane & 7) * 4;   // first column of this lane's quad within a 32-column chunk
     const uint64_t pol = l2_policy((p.l2_policy >> 4) & 3);
 #pragma unroll 1
-    for (int chunk = 0; chunk < BN / 32; ++chunk) {
+    for (int chunk = 0; chunk < columns >> 5; ++chunk) {
       if (n0 + chunk * 32 >= p.N) break;  // warp-uniform
       uint32_t v[32];
       tmem_ld_32x32b_x32(taddr + chunk * 32, v);
@@ -399,9 +397,9 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t tadd
   }
   // general path: any alignment, any N; full 32-row slabs without predicates
   if (rows_here >= 32)
-    epilogue_columns<BN, true>(p, taddr, tbuf, lane, row0, n0, 32);
+    epilogue_columns<true>(p, taddr, tbuf, lane, row0, n0, columns, 32);
   else
-    epilogue_columns<BN, false>(p, taddr, tbuf, lane, row0, n0, rows_here);
+    epilogue_columns<false>(p, taddr, tbuf, lane, row0, n0, columns, rows_here);
 }
 
 // ------------------------------------------------------------------------

@@ -707,7 +707,7 @@ int launch_tiles(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
   gp.cluster_splits = split_in_cluster(items / gp.splits, gp.splits, CTAS, sm_count) ? gp.splits : 1;
   const long long used = items < units || gp.cluster_splits > 1 ? items : units;
-  const dim3 grid(static_cast<unsigned>(CTAS * used)), block(Cfg::kThreads);
+  const dim3 grid(static_cast<unsigned>(CTAS * used)), block(gp.cluster_splits > 1 ? GEMM_THREADS : Cfg::kThreads);
   CUtensorMap map_d, map_c;
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
