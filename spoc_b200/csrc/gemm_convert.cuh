@@ -228,18 +228,30 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   constexpr bool in_cluster = IN_CLUSTER;
   const int split_rank = in_cluster ? static_cast<int>(cluster_ctarank()) : 0;
 
-  if (warp == 0) {  // a lane a barrier: full, empty, done, recv
-    constexpr int BARS = 2 * STAGES + 2;
-    static_assert(BARS <= 32, "a lane a barrier");
-    if (lane < BARS) mbar_init(smem_u32(&full_bar[lane]), lane < STAGES ? CONV_WARPS : 1);
-    if (lane == 0) *abort_flag = 0;
+  // Quads: a warp for the barriers, a lane each (64^3 5.7 -> 5.6 us).  Single elements: one thread, and below its own form of the coordinates and
+  // of the wait for the stores (with those of the quads 2 to 4 % longer: 9 x 1257 x 64 7.7 and 8.0 us, 7 x 5363 x 246 14.4 and 14.9; the difference is
+  // in what the compiler makes of the kernel, whose registers are all taken, and not in the set-up's time).
+  auto barrier_count = [](int i) { return i < STAGES ? CONV_WARPS : 1; };  // full, empty, done, recv
+  constexpr int BARS = 2 * STAGES + 2;
+  static_assert(BARS <= 32, "a lane a barrier");
+  uint64_t* c_bars = reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR);
+  if constexpr (VEC) {
+    if (warp == 0) {
+      if (lane < BARS) mbar_init(smem_u32(&full_bar[lane]), barrier_count(lane));
+      if (lane == 0) *abort_flag = 0;
+      mbar_fence_init();
+    } else if (warp == 1) {
+      if (lane < 2 * CONV_WARPS) mbar_init(smem_u32(c_bars + lane), 1);
+      mbar_fence_init();
+    }
+    if (threadIdx.x == 64 && p.tma_epilogue) tma_prefetch_desc(&map_d);
+  } else if (threadIdx.x == 0) {
+    for (int i = 0; i < BARS; ++i) mbar_init(smem_u32(&full_bar[i]), barrier_count(i));
+    for (int i = 0; i < 2 * CONV_WARPS; ++i) mbar_init(smem_u32(c_bars + i), 1);
+    *abort_flag = 0;
     mbar_fence_init();
+    if (p.tma_epilogue) tma_prefetch_desc(&map_d);
   }
-  if (warp == 1) {  // the barriers of the tiles of C
-    if (lane < 2 * CONV_WARPS) mbar_init(smem_u32(reinterpret_cast<uint64_t*>(ctrl + GEMM_CTRL_CBAR) + lane), 1);
-    mbar_fence_init();
-  }
-  if (threadIdx.x == 64 && p.tma_epilogue) tma_prefetch_desc(&map_d);
   if (warp == CONV_WARPS) {
     tmem_alloc(smem_u32(tmem_slot), BN);
     tmem_relinquish();
@@ -261,11 +273,14 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     const int quarter = warp & 3, half = warp >> 2;
     int stage = 0, local = 0;
     uint32_t phase = 0;
-    bool ok = true, arrived = false;
+    bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn;
-      item_tile_coords(item, p, num_tiles, tm, tn);
-      const int m0 = tm * 128, n0 = tn * BN, split = item_split(item, num_tiles);
+      if constexpr (VEC)
+        item_tile_coords(item, p, num_tiles, tm, tn);
+      else
+        pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
+      const int m0 = tm * 128, n0 = tn * BN, split = VEC ? item_split(item, num_tiles) : item / num_tiles;
       const int kb0 = split * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
       ConvTile<BN, VEC> t[CONV_AHEAD + 1];
 #pragma unroll
@@ -302,7 +317,6 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
         tc_fence_after_sync();
         if constexpr (in_cluster) {
           cluster_arrive_relaxed();  // the ring is idle
-          arrived = true;
         }
         const int row0 = m0 + quarter * 32, c0 = n0 + half * (BN / 2);
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2);
@@ -320,10 +334,11 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
             }
           }
         }
+        if (!VEC && elect_one()) bulk_wait_read<0>();  // (here for single elements: 2 % shorter than behind the closing barrier, as above)
         tc_fence_before_sync();
       }
       if (item + item_step >= num_items) break;  // the block's last item: nothing follows but the barrier all threads share
-      if (ok && elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
+      if (VEC && ok && elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
       // every warp is through with the accumulator and the tiles before the next item's operands arrive
       __syncwarp();
       ok = convert_go_on(ok, abort_flag);
@@ -331,7 +346,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     if (!ok && elect_one()) wait_for_copies();  // tiles of C
     __syncwarp();
     if constexpr (in_cluster) {
-      if (!arrived) cluster_arrive_relaxed();
+      if (!ok) cluster_arrive_relaxed();
       int tm, tn;
       item_tile_coords(first_item - split_rank * num_tiles, p, num_tiles, tm, tn);
       auto barrier = [](bool so_far) { return barrier_all(1, CONV_WARPS * 32, so_far); };
@@ -400,7 +415,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   if (warp == CONV_WARPS) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, BN);
-  } else if (warp < CONV_WARPS && elect_one()) {
+  } else if (VEC && warp < CONV_WARPS && elect_one()) {
     bulk_wait_read<0>();  // the epilogue's tiles outlive the stores that read them
   }
 }

@@ -63,6 +63,16 @@ __device__ __forceinline__ void pair_soft_epoch(unsigned int* ctr, unsigned int 
   }
 }
 
+// Tile coordinates for gemm_convert_kernel on single elements (item_tile_coords for all others).
+__device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tiles_n, int group_m, int& tm, int& tn) {
+  const int band_tiles = group_m * tiles_n;
+  const int band = tile / band_tiles;
+  const int within = tile - band * band_tiles;
+  const int first_m = band * group_m;
+  const int band_m = min(group_m, tiles_m - first_m);
+  tm = first_m + within % band_m;
+  tn = within / band_m;
+}
 // Which part of a divided k-loop work item `item` is: item / num_tiles, without the division where it is 0.
 __device__ __forceinline__ int item_split(int item, int num_tiles) {
   return item < num_tiles ? 0 : static_cast<int>(static_cast<unsigned int>(item) / static_cast<unsigned int>(num_tiles));
