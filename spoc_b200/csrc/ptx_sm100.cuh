@@ -293,12 +293,7 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-// 128-bit load from the shared memory of a block of the cluster (address from map_to_cta)
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
-  return v;
-}
+// 32-bit load from the shared memory of a block of the cluster (address from map_to_cta)
 __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t cluster_addr) {
   uint32_t v;
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
