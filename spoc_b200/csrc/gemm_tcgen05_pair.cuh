@@ -47,6 +47,11 @@ struct TileCfg {
   // Groups of four epilogue warps.  A half of 64 columns is not worth a second one, and blocks on their own nearly always divide their k-loop, whose
   // finish lost by the fewer registers a thread (64 x 4096 x 4096 TF32 13.1 and 13.4 us).
   static constexpr int kEpiGroups = BN >= 128 && CTAS == 2 ? 2 : 1;
+  // Arrivals that hand an accumulator back: the epilogue warps of both blocks, the second group's among them.  That group has nothing to do with
+  // a tile that is not the last, but waits for each accumulator in turn, and a wait on a barrier's parity takes the phase after the wanted one
+  // for one still to come: no accumulator may be completed again before all warps have seen it complete.  (Nobody waits for these
+  // arrivals where the k-loop is divided within a cluster, whose blocks have one tile and no second group.)
+  static constexpr int kHandBacks = 4 * kEpiGroups * CTAS;
   static constexpr int kThreads = GEMM_THREADS + (kEpiGroups - 1) * 128;  // (GEMM_THREADS where the k-loop is divided within a cluster)
 };
 
@@ -420,10 +425,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
                                  : static_cast<int>(blockIdx.x) / CTAS;
   const int num_pairs = in_cluster ? 1 << 30 : static_cast<int>(gridDim.x) / CTAS;
 
-  if (warp == 0) {  // a lane a barrier: full and empty, tmem_full, tmem_empty (the epilogue warps of both blocks), recv
+  if (warp == 0) {  // a lane a barrier: full and empty, tmem_full, tmem_empty, recv
     constexpr int BARS = 2 * STAGES + 5;
     static_assert(BARS <= 32, "a lane a barrier");
-    if (lane < BARS) mbar_init(smem_u32(&bars[lane]), lane / 2 == STAGES + 1 ? 4 * CTAS : 1);
+    if (lane < BARS) mbar_init(smem_u32(&bars[lane]), lane / 2 == STAGES + 1 ? Cfg::kHandBacks : 1);
     if (lane == 0) *abort_flag = 0;
     mbar_fence_init();
   }
@@ -684,7 +689,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
         ok = false;
         break;
       }
-      if (second && !last) continue;  // (each accumulator has been awaited: a wait on a parity must not miss a phase)
+      auto hand_back = [&] {
+        __syncwarp();
+        if (lane == 0) {
+          if (CTAS == 2)
+            mbar_arrive_peer(map_to_cta(smem_u32(&tmem_empty_bar[acc]), leader));
+          else
+            mbar_arrive(smem_u32(&tmem_empty_bar[acc]));
+        }
+      };
+      if (second && !last) {
+        hand_back();  // (kHandBacks)
+        continue;
+      }
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * 256 + first_col;
       if (in_cluster) {
@@ -706,13 +723,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       }
       if (last) break;  // nobody waits for this accumulator
       tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        if (CTAS == 2)
-          mbar_arrive_peer(map_to_cta(smem_u32(&tmem_empty_bar[acc]), leader));
-        else
-          mbar_arrive(smem_u32(&tmem_empty_bar[acc]));
-      }
+      hand_back();
     }
     __syncwarp();
     if (!ok && elect_one()) wait_for_copies();  // tiles of C
