@@ -385,8 +385,9 @@ SB200_API int sb200_gemm_f32_host(int dev, int mode, int64_t M, int64_t N, int64
  * need somewhat more, because a block may keep partial sums where the whole does not. */
 SB200_API int sb200_gemm_workspace_bytes(int mode, int64_t M, int64_t N, int64_t K, uint64_t *bytes);
 /* how sb200_gemm_f32 would run these sizes on a device with sm_count SMs, as text:
- * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES launches=L operands=O kernels=N"
- * (fp16 modes: "fp16-panels", mixed mode: "mixed" without splits, for the second word).  N is the number of kernels the call launches
+ * "pair|single direct|panels tile=RxC stages=S tiles=T waves=W splits=P workspace=BYTES a_tail=R launches=L operands=O kernels=N"
+ * (fp16 modes: "fp16-panels", mixed mode: "mixed" without splits, for the second word).  R is the height of the boxes that load the last,
+ * partial 128 rows of A (0: nothing is loaded by boxes; mixed mode: in the plain 3xTF32 launch behind it).  N is the number of kernels the call launches
  * and O what becomes of A and B: direct (read where they lie; in 3xTF32 mode beside panels of their low parts, which a launch in front
  * writes), split (3xTF32: read where they lie and split on chip), copied (row by row first, beside the same panels), copied+split (row by
  * row first, the copies split on chip), converted (in registers on their way), panels (written in full) or mixed.  The second word says

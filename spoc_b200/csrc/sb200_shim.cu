@@ -424,7 +424,6 @@ void derive_params(GemmParams* gp) {
   for (int r = 0; r < gp->n_replicas; ++r) vec = vec && al16(gp->replicas[r]);
   gp->vec_epilogue = vec ? 1 : 0;
   gp->l2_policy = l2_policy_setting();
-  gp->a_tail_rows = a_tail_rows(gp->M, gp->N, gp->num_k_blocks);
 }
 
 // Tensor maps of D and C for the epilogue that moves them by TMA; sets gp->tma_epilogue when it applies: 16-byte aligned
@@ -623,9 +622,21 @@ TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, in
 
 int units_of(int ctas, int sm_count);
 
-// The operand maps of one launch; x: the mixed mode's third pair, else the maps of A (hi, lo) for its last rows.
+// The operand maps of one launch; x: the mixed mode's third pair, else the maps of A (hi, lo) for its last rows, and the rows of their boxes:
+// the kernel is told the number the maps were made with, or its barriers would count bytes that never come.
 struct OperandMaps {
   CUtensorMap a_hi, b_hi, a_lo, b_lo, a_x, b_x;
+  int a_tail_rows = GEMM_BM;
+
+  // High or low parts of A with M rows, in boxes of `whole` rows and of a_tail_rows: one map where these are the same, or where there are no
+  // whole rows.  encode(map, rows).
+  template <class Encode>
+  int encode_a(bool low, long long M, int whole, Encode&& encode) {
+    CUtensorMap &rows = low ? a_lo : a_hi, &tail = low ? b_x : a_x;
+    if (int rc = encode(&tail, a_tail_rows)) return rc;
+    rows = tail;
+    return M > whole && a_tail_rows != whole ? encode(&rows, whole) : static_cast<int>(SB200_OK);
+  }
 };
 
 // The parameters and output maps a GEMM kernel is launched with: *kp is *gp with the epilogue as it is, or, when the k-loop is
@@ -708,6 +719,7 @@ int launch_tiles(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   gp.cluster_splits = split_in_cluster(items / gp.splits, gp.splits, CTAS, sm_count) ? gp.splits : 1;
   const long long used = items < units || gp.cluster_splits > 1 ? items : units;
   const dim3 grid(static_cast<unsigned>(CTAS * used)), block(gp.cluster_splits > 1 ? GEMM_THREADS : Cfg::kThreads);
+  gp.a_tail_rows = m.a_tail_rows;
   CUtensorMap map_d, map_c;
   GemmParams kp;
   if (int rc = output_maps(&gp, &kp, part, m.a_hi, &map_d, &map_c)) return rc;
@@ -769,6 +781,7 @@ int launch_split(int dev_index, int sm_count, cudaStream_t st, const OperandMaps
   if (gp.splits < 1) gp.splits = 1;
   gp.split_k_blocks = (gp.num_k_blocks + gp.splits - 1) / gp.splits;
   gp.epoch_ctr = nullptr;
+  gp.a_tail_rows = m.a_tail_rows;
   const long long items = static_cast<long long>(gp.tiles_m) * gp.tiles_n * gp.splits;
   gp.cluster_splits = split_in_cluster(items / gp.splits, gp.splits, CTAS, sm_count) ? gp.splits : 1;
   const dim3 grid(static_cast<unsigned>(CTAS * (items < units || gp.cluster_splits > 1 ? items : units)));
@@ -1046,6 +1059,15 @@ int launch_prep_panels(int sm_count, cudaStream_t st, const float* A, long long 
   return launch_check("prep_panels_kernel");
 }
 
+// The maps over those panels: boxes of `b_box` columns of B.
+int encode_panel_maps(OperandMaps* m, const float* a_hi, const float* a_lo, const float* b_hi, const float* b_lo, long long M, long long N, long long kp,
+                      int b_box) {
+  int rc = m->encode_a(false, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_panel_map(map, a_hi, kp, M, rows); });
+  if (!rc) rc = m->encode_a(true, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_panel_map(map, a_lo, kp, M, rows); });
+  if (!rc) rc = encode_panel_map(&m->b_hi, b_hi, kp, N, b_box);
+  return rc ? rc : encode_panel_map(&m->b_lo, b_lo, kp, N, b_box);
+}
+
 template <int MODE>
 int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, long long K, const float* A,
                      long long lda, const float* B, long long ldb, const GemmParams& gp_in, long long panel_rows_a = 0,
@@ -1109,8 +1131,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     CU_TRY(cudaEventCreate(&rec.e2));
     CU_TRY(cudaEventRecord(rec.e0, st));
   }
-  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail;
-  const int tail = a_tail_rows(M, N, kp / GEMM_BK);
+  OperandMaps maps;
+  maps.a_tail_rows = a_tail_rows(M, N, kp / GEMM_BK);
   if (route.src == SRC_CONVERT) {
     // no panels, no operand maps
   } else if (direct || route.src == SRC_SPLIT) {
@@ -1135,19 +1157,15 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, b_panels_ready, nullptr))) return rc;
     // the split kernel takes the elements as they are, by up to 64 rows where that is all there are
     auto map_a = [&](CUtensorMap* map, int rows) { return encode_map_2d(map, copy_a ? a_copy : A, K, M, copy_a ? kp : lda, GEMM_BK, rows, direct); };
-    if ((rc = map_a(&ma_hi_tail, tail))) return rc;
-    ma_hi = ma_hi_tail;  // where the whole rows' box is the same, or there are no whole rows (64, 128) and it is not used
-    const int whole = !direct && M <= 64 ? 64 : GEMM_BM;
-    if (M > whole && tail != whole && (rc = map_a(&ma_hi, whole))) return rc;
-    if ((rc = encode_map_2d(&mb_hi, copy_b ? b_copy : B, N, K, copy_b ? np : ldb, 32, GEMM_BK, direct, true))) return rc;
-    ma_lo = ma_hi;
-    mb_lo = mb_hi;
-    ma_lo_tail = ma_hi_tail;
+    auto map_a_lo = [&](CUtensorMap* map, int rows) { return encode_map_2d(map, a_lo, kp, M, kp, GEMM_BK, rows, false); };
+    if ((rc = maps.encode_a(false, M, !direct && M <= 64 ? 64 : GEMM_BM, map_a))) return rc;
+    if ((rc = encode_map_2d(&maps.b_hi, copy_b ? b_copy : B, N, K, copy_b ? np : ldb, 32, GEMM_BK, direct, true))) return rc;
+    maps.a_lo = maps.a_hi;
+    maps.b_lo = maps.b_hi;
+    maps.b_x = maps.a_x;
     if (lows) {
-      if ((rc = encode_map_2d(&ma_lo_tail, a_lo, kp, M, kp, GEMM_BK, tail, false))) return rc;
-      ma_lo = ma_lo_tail;
-      if (M > GEMM_BM && tail != GEMM_BM && (rc = encode_map_2d(&ma_lo, a_lo, kp, M, kp, GEMM_BK, GEMM_BM, false))) return rc;
-      if ((rc = encode_map_2d(&mb_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
+      if ((rc = maps.encode_a(true, M, GEMM_BM, map_a_lo))) return rc;
+      if ((rc = encode_map_2d(&maps.b_lo, b_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     }
   } else {
     // workspace layout: B panels first (their size does not depend on M), then the A panels
@@ -1159,12 +1177,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     float* a_lo = MODE == 3 ? reinterpret_cast<float*>(ws + kOps * b_bytes + a_bytes) : a_hi;
     if ((rc = launch_prep_panels<MODE>(d.sm_count, st, A, lda, a_hi, a_lo, B, ldb, b_hi, b_lo, M, N, K, b_panels_ready))) return rc;
     const int b_box = tile_n / route.ctas;
-    if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, b_box))) return rc;
-    if ((rc = encode_panel_map(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, b_box))) return rc;
-    if ((rc = encode_panel_map(&ma_hi_tail, a_hi, kp, M, tail))) return rc;
-    if ((rc = encode_panel_map(&ma_lo_tail, a_lo, kp, M, tail))) return rc;
+    if ((rc = encode_panel_maps(&maps, a_hi, a_lo, b_hi, b_lo, M, N, kp, b_box))) return rc;
   }
 
   GemmParams gp = gp_in;
@@ -1181,7 +1194,6 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     const ConvOperands o{A, B, lda, ldb, static_cast<int>(K)};
     rc = launch_convert_for<MODE>(tile_n, addressable && (K & 3) == 0 && (N & 3) == 0, dev_index, d.sm_count, st, o, gp, part);
   } else {
-    const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail};
     rc = route.src == SRC_SPLIT ? launch_split_for(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
          : direct               ? launch_tiles_for<MODE, SRC_DIRECT>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part)
                                 : launch_tiles_for<MODE, SRC_PANELS>(tile_n, route.ctas, dev_index, d.sm_count, st, maps, gp, part);
@@ -1325,21 +1337,17 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
       if ((rc = launch_check("prep_b_f16_kernel"))) return rc;
     }
   }
-  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail;
-  const int tail = a_tail_rows(M, N, kp / 64), b_box = tile_n / ctas;
-  const bool whole = M > GEMM_BM && tail != GEMM_BM;  // whole 128 rows beside a partial last one
-  if ((rc = encode_map_f16(&ma_hi_tail, a_hi, kp, M, tail))) return rc;
-  ma_hi = ma_hi_tail;
-  if (whole && (rc = encode_map_f16(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_map_f16(&mb_hi, b_hi, kp, N, b_box))) return rc;
-  ma_lo = ma_hi;
-  ma_lo_tail = ma_hi_tail;
-  mb_lo = mb_hi;
+  OperandMaps maps;
+  maps.a_tail_rows = a_tail_rows(M, N, kp / 64);
+  const int b_box = tile_n / ctas;
+  if ((rc = maps.encode_a(false, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_f16(map, a_hi, kp, M, rows); }))) return rc;
+  if ((rc = encode_map_f16(&maps.b_hi, b_hi, kp, N, b_box))) return rc;
+  maps.a_lo = maps.a_hi;
+  maps.b_x = maps.a_x;
+  maps.b_lo = maps.b_hi;
   if (THREE) {
-    if ((rc = encode_map_f16(&ma_lo_tail, a_lo, kp, M, tail))) return rc;
-    ma_lo = ma_lo_tail;
-    if (whole && (rc = encode_map_f16(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-    if ((rc = encode_map_f16(&mb_lo, b_lo, kp, N, b_box))) return rc;
+    if ((rc = maps.encode_a(true, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_f16(map, a_lo, kp, M, rows); }))) return rc;
+    if ((rc = encode_map_f16(&maps.b_lo, b_lo, kp, N, b_box))) return rc;
   }
   GemmParams gp = gp_in;
   gp.num_k_blocks = static_cast<int>(kp / 64);
@@ -1352,7 +1360,6 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
   if (prof) CU_TRY(cudaEventRecord(rec.e1, st));
   const int dev_index = static_cast<int>(&d - g_dev);
   gp.splits = shape.splits;
-  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail};
   float* part = reinterpret_cast<float*>(ws + need);
   rc = launch_tiles_for<THREE ? 4 : 2, SRC_PANELS>(tile_n, ctas, dev_index, d.sm_count, st, maps, gp, part);
   if (prof) {
@@ -1472,15 +1479,16 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     const PrepLoJob ja{A, lda, pa_lo, nullptr, static_cast<int>(M), static_cast<int>(K), static_cast<int>(kp32), 1};
     const PrepLoJob jb{B, ldb, pb_lo, nullptr, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), 1};
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, false, gp.gate))) return rc;
-    CUtensorMap pma_lo, pmb_lo, ma_tail, pma_lo_tail;
-    if ((rc = encode_map_2d(&pma_lo, pa_lo, kp32, M, kp32, GEMM_BK, GEMM_BM, false))) return rc;
-    if ((rc = encode_map_2d(&ma_tail, A, K, M, lda, GEMM_BK, a_tail_rows(M, N, kp32 / GEMM_BK), true))) return rc;
-    if ((rc = encode_map_2d(&pma_lo_tail, pa_lo, kp32, M, kp32, GEMM_BK, a_tail_rows(M, N, kp32 / GEMM_BK), false))) return rc;
-    if ((rc = encode_map_2d(&pmb_lo, pb_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
+    OperandMaps plain;
+    plain.a_tail_rows = a_tail_rows(M, N, kp32 / GEMM_BK);
+    plain.b_hi = mb;
+    if ((rc = plain.encode_a(false, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_2d(map, A, K, M, lda, GEMM_BK, rows, true); }))) return rc;
+    if ((rc = plain.encode_a(true, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_2d(map, pa_lo, kp32, M, kp32, GEMM_BK, rows, false); })))
+      return rc;
+    if ((rc = encode_map_2d(&plain.b_lo, pb_lo, N, K, np, 32, GEMM_BK, false, true))) return rc;
     gp.num_k_blocks = static_cast<int>(kp32 / GEMM_BK);
     gp.gate_value = 0;
     gp.epoch_ctr = nullptr;  // the ring belongs to the launch in front
-    const OperandMaps plain{ma, mb, pma_lo, pmb_lo, ma_tail, pma_lo_tail};
     rc = launch_tiles_for<3, SRC_DIRECT>(256, 2, dev_index, d.sm_count, st, plain, gp, nullptr);
   }
   if (prof) {
@@ -2847,10 +2855,10 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
     const int launches = (f16_prepared_at_once(M, N, K) ? 2 : 3) +
                          (shape.splits > 1 && !split_in_cluster(tiles, shape.splits, ctas, sm_count) ? 1 : 0);
     snprintf(fb, sizeof fb,
-             "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=panels kernels=%d",
+             "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu a_tail=%d launches=%d operands=panels kernels=%d",
              ctas == 1 ? "single" : "pair", 128 * ctas, shape.tile_n, stages_of(three, shape.tile_n, ctas), tiles,
              (tiles * shape.splits + units - 1) / units, shape.splits,
-             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count), launches, launches);
+             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count), a_tail_rows(M, N, kp / 64), launches, launches);
     return copy_out(fb, out, outlen);
   }
   if (mode == SB200_MODE_3XMIXED) {
@@ -2860,8 +2868,9 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
       const long long tiles = ((M + PAIR_BM - 1) / PAIR_BM) * ((N + tn - 1) / tn);
       const int stages = stages_of(true, tn, 2);
       char fb[256];
-      snprintf(fb, sizeof fb, "pair mixed tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu launches=7 operands=mixed kernels=6",
-               PAIR_BM, tn, stages, tiles, (tiles + clusters - 1) / clusters, gemm_mix_workspace_need(M, N, K));
+      snprintf(fb, sizeof fb, "pair mixed tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu a_tail=%d launches=7 operands=mixed kernels=6",
+               PAIR_BM, tn, stages, tiles, (tiles + clusters - 1) / clusters, gemm_mix_workspace_need(M, N, K),
+               a_tail_rows(M, N, round_up(K, GEMM_BK) / GEMM_BK));
       return copy_out(fb, out, outlen);
     }
     mode = SB200_MODE_3XTF32;
@@ -2877,9 +2886,9 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
                          : r.src == SRC_PANELS ? "panels"
                          : addressable         ? "direct"
                                                : "copied";
-  snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu launches=%d operands=%s kernels=%d",
+  snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu a_tail=%d launches=%d operands=%s kernels=%d",
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
-           r.waves, r.splits, r.workspace, launches, operands, kernels);
+           r.waves, r.splits, r.workspace, r.src == SRC_CONVERT ? 0 : a_tail_rows(M, N, round_up(K, GEMM_BK) / GEMM_BK), launches, operands, kernels);
   return copy_out(buf, out, outlen);
 }
 
@@ -3145,18 +3154,12 @@ int launch_gemm_fixed_scratch(const NoAllocDevice& nd, int dev, cudaStream_t st,
   int rc = launch_prep_panels<MODE>(nd.sm_count, st, A, lda, a_hi, a_lo, B, ldb, b_hi, b_lo, M, N, K, false);
   if (rc) return rc;
   const int tile_n = choose_tiles(M, N, kp / GEMM_BK, 1, nd.sm_count, MODE == 3, false).tile_n;
-  CUtensorMap ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail;
-  const int tail = a_tail_rows(M, N, kp / GEMM_BK);
-  if ((rc = encode_panel_map(&ma_hi, a_hi, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_panel_map(&mb_hi, b_hi, kp, N, tile_n))) return rc;
-  if ((rc = encode_panel_map(&ma_lo, a_lo, kp, M, GEMM_BM))) return rc;
-  if ((rc = encode_panel_map(&mb_lo, b_lo, kp, N, tile_n))) return rc;
-  if ((rc = encode_panel_map(&ma_hi_tail, a_hi, kp, M, tail))) return rc;
-  if ((rc = encode_panel_map(&ma_lo_tail, a_lo, kp, M, tail))) return rc;
+  OperandMaps maps;
+  maps.a_tail_rows = a_tail_rows(M, N, kp / GEMM_BK);
+  if ((rc = encode_panel_maps(&maps, a_hi, a_lo, b_hi, b_lo, M, N, kp, tile_n))) return rc;
   gp.num_k_blocks = static_cast<int>(kp / GEMM_BK);
   gp.status = nd.status;
   derive_params(&gp);
-  const OperandMaps maps{ma_hi, mb_hi, ma_lo, mb_lo, ma_hi_tail, ma_lo_tail};
   return launch_tiles_for<MODE, SRC_PANELS>(tile_n, 1, dev, nd.sm_count, st, maps, gp, nullptr);
 }
 

@@ -121,3 +121,16 @@ def test_degenerate_and_bad_arguments():
     assert lib.sb200_set_gemm_tile_n(128) == 0
     assert describe(L.MODE_TF32, 8192, 8192, 8192)["tile"] == "256x128"
     assert lib.sb200_set_gemm_tile_n(0) == 0
+
+
+@pytest.mark.parametrize("mode", [L.MODE_3XTF32, L.MODE_TF32, L.MODE_3XF16, L.MODE_F16, L.MODE_3XMIXED])
+def test_the_last_rows_of_a_have_boxes_of_their_own(mode):
+    """As high as there are rows, to the next multiple of 8; beside whole 128 rows only in larger products."""
+    assert L.load().sb200_set_mixed_min_macs(1 << 26) == 0
+    try:
+        for M, N, K, rows in [(7, 4096, 4096, 8), (64, 4096, 4096, 64), (100, 4096, 4096, 104), (128, 4096, 4096, 128), (129, 4096, 4096, 8),
+                              (257, 2064, 1024, 8), (1100, 2000, 640, 80), (2047, 2048, 2048, 128), (2048, 2048, 2048, 128), (137, 64, 260, 128)]:
+            d = describe(mode, M, N, K)
+            assert d["a_tail"] == (str(rows) if d["operands"] != "converted" else "0"), (M, N, K, d)
+    finally:
+        assert L.load().sb200_set_mixed_min_macs(0) == 0

@@ -64,3 +64,28 @@ def test_k_loops_divided_by_the_second_choice(backend, device, mode, M, N, K, sp
     assert f"splits={splits} " in text, text
     pad = 4 if ldd == "quads" else 1        # rows of the result on 16-byte boundaries, and not
     check(backend, device, mode, M, N, K, K, N, N + pad, N + pad)
+
+
+@pytest.mark.parametrize("M,N,K,tail", [(257, 1032, 260, 8), (1100, 1000, 300, 80), (1153, 1024, 64, 8), (511, 2052, 132, 128)])
+def test_rows_past_the_end_behind_the_mixed_mode(backend, device, M, N, K, tail):
+    """Operands the mixed mode declines go to a plain 3xTF32 launch behind it, which loads the last rows as other launches do."""
+    lib = L.load()
+    lib.sb200_set_mixed_min_macs(1 << 26)
+    a, b = O.fill(M * K, 65, 1), O.fill(K * N, 65, 2)
+    a, b = np.ldexp(a, 25), np.ldexp(b, 20)
+    A, B, D = dev_from(backend, device, a), dev_from(backend, device, b), Dev(backend, device, (M + 1) * N)
+    out = []
+    try:
+        text = describe(L.MODE_3XMIXED, M, N, K, 1)
+        assert f" a_tail={tail} " in text and " operands=mixed " in text and " splits=1 " in describe(L.MODE_3XTF32, M, N, K, 1)
+        for mode in (L.MODE_3XMIXED, L.MODE_3XTF32):
+            D.clear()
+            gemm(backend, device, mode, M, N, K, A, B, D)
+            out.append(D.download())
+        assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
+        assert np.all(out[0][M * N:] == CANARY)
+        assert O.gemm_rel_error(out[0][:M * N].reshape(M, N), O.gemm(a, b, M, N, K)) <= tol(L.MODE_3XTF32, K)
+    finally:
+        lib.sb200_set_mixed_min_macs(0)
+        for x in (A, B, D):
+            x.free()
