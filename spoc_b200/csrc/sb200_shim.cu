@@ -399,9 +399,11 @@ int l2_policy_setting() {
 }
 
 // Rows of the boxes of the last, partial 128 rows of A (or of 64, all there are, for gemm_split_kernel's blocks of so few).  Beside whole rows they
-// take a map more, 0.3 us of the host's time, which small products have not got (5334 x 20 x 264 TF32 6.1 us, with it 6.6).
-int a_tail_rows(long long M, long long N, long long kblocks) {
-  if (M > GEMM_BM && static_cast<double>(M) * N * kblocks * GEMM_BK < 67108864.0) return GEMM_BM;  // 2^26 multiply-adds
+// take a map more, 0.3 us of the host's time, which products below 2^26 multiply-adds have not got (5334 x 20 x 264 TF32 6.1 us, with it 6.6).  Up
+// to 2^27 most are even (60 products in the fp16 modes: 0.996 on average), those of few rows beside whole ones win (138 x 3472 x 256 f16 14.9 -> 12.0 us,
+// 135 x 4028 x 144 3xF16 16.0 -> 13.6).
+int a_tail_rows(long long M, long long N, long long K) {
+  if (M > GEMM_BM && static_cast<double>(M) * N * K < 67108864.0) return GEMM_BM;  // 2^26
   return static_cast<int>(round_up((M - 1) % GEMM_BM + 1, 8));
 }
 
@@ -1132,7 +1134,7 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
     CU_TRY(cudaEventRecord(rec.e0, st));
   }
   OperandMaps maps;
-  maps.a_tail_rows = a_tail_rows(M, N, kp / GEMM_BK);
+  maps.a_tail_rows = a_tail_rows(M, N, K);
   if (route.src == SRC_CONVERT) {
     // no panels, no operand maps
   } else if (direct || route.src == SRC_SPLIT) {
@@ -1338,7 +1340,7 @@ int launch_gemm_f16(DeviceState& d, cudaStream_t st, long long M, long long N, l
     }
   }
   OperandMaps maps;
-  maps.a_tail_rows = a_tail_rows(M, N, kp / 64);
+  maps.a_tail_rows = a_tail_rows(M, N, K);
   const int b_box = tile_n / ctas;
   if ((rc = maps.encode_a(false, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_f16(map, a_hi, kp, M, rows); }))) return rc;
   if ((rc = encode_map_f16(&maps.b_hi, b_hi, kp, N, b_box))) return rc;
@@ -1480,7 +1482,7 @@ int launch_gemm_mix(DeviceState& d, cudaStream_t st, long long M, long long N, l
     const PrepLoJob jb{B, ldb, pb_lo, nullptr, static_cast<int>(K), static_cast<int>(N), static_cast<int>(np), 1};
     if ((rc = launch_prep_lo(d.sm_count, st, ja, jb, false, gp.gate))) return rc;
     OperandMaps plain;
-    plain.a_tail_rows = a_tail_rows(M, N, kp32 / GEMM_BK);
+    plain.a_tail_rows = a_tail_rows(M, N, K);
     plain.b_hi = mb;
     if ((rc = plain.encode_a(false, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_2d(map, A, K, M, lda, GEMM_BK, rows, true); }))) return rc;
     if ((rc = plain.encode_a(true, M, GEMM_BM, [&](CUtensorMap* map, int rows) { return encode_map_2d(map, pa_lo, kp32, M, kp32, GEMM_BK, rows, false); })))
@@ -2858,7 +2860,7 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
              "%s fp16-panels tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu a_tail=%d launches=%d operands=panels kernels=%d",
              ctas == 1 ? "single" : "pair", 128 * ctas, shape.tile_n, stages_of(three, shape.tile_n, ctas), tiles,
              (tiles * shape.splits + units - 1) / units, shape.splits,
-             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count), a_tail_rows(M, N, kp / 64), launches, launches);
+             gemm_f16_workspace_need(M, N, K, three) + partial_bytes(M, N, shape, ctas, sm_count), a_tail_rows(M, N, K), launches, launches);
     return copy_out(fb, out, outlen);
   }
   if (mode == SB200_MODE_3XMIXED) {
@@ -2870,7 +2872,7 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
       char fb[256];
       snprintf(fb, sizeof fb, "pair mixed tile=%dx%d stages=%d tiles=%lld waves=%lld workspace=%zu a_tail=%d launches=7 operands=mixed kernels=6",
                PAIR_BM, tn, stages, tiles, (tiles + clusters - 1) / clusters, gemm_mix_workspace_need(M, N, K),
-               a_tail_rows(M, N, round_up(K, GEMM_BK) / GEMM_BK));
+               a_tail_rows(M, N, K));
       return copy_out(fb, out, outlen);
     }
     mode = SB200_MODE_3XTF32;
@@ -2888,7 +2890,7 @@ int sb200_gemm_describe(int mode, int64_t M, int64_t N, int64_t K, int addressab
                                                : "copied";
   snprintf(buf, sizeof buf, "%s %s tile=%dx%d stages=%d tiles=%lld waves=%lld splits=%d workspace=%zu a_tail=%d launches=%d operands=%s kernels=%d",
            r.ctas == 2 ? "pair" : "single", r.src != SRC_PANELS && addressable ? "direct" : "panels", 128 * r.ctas, r.tile_n, r.stages, r.tiles,
-           r.waves, r.splits, r.workspace, r.src == SRC_CONVERT ? 0 : a_tail_rows(M, N, round_up(K, GEMM_BK) / GEMM_BK), launches, operands, kernels);
+           r.waves, r.splits, r.workspace, r.src == SRC_CONVERT ? 0 : a_tail_rows(M, N, K), launches, operands, kernels);
   return copy_out(buf, out, outlen);
 }
 
@@ -3155,7 +3157,7 @@ int launch_gemm_fixed_scratch(const NoAllocDevice& nd, int dev, cudaStream_t st,
   if (rc) return rc;
   const int tile_n = choose_tiles(M, N, kp / GEMM_BK, 1, nd.sm_count, MODE == 3, false).tile_n;
   OperandMaps maps;
-  maps.a_tail_rows = a_tail_rows(M, N, kp / GEMM_BK);
+  maps.a_tail_rows = a_tail_rows(M, N, K);
   if ((rc = encode_panel_maps(&maps, a_hi, a_lo, b_hi, b_lo, M, N, kp, tile_n))) return rc;
   gp.num_k_blocks = static_cast<int>(kp / GEMM_BK);
   gp.status = nd.status;

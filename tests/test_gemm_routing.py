@@ -129,7 +129,8 @@ def test_the_last_rows_of_a_have_boxes_of_their_own(mode):
     assert L.load().sb200_set_mixed_min_macs(1 << 26) == 0
     try:
         for M, N, K, rows in [(7, 4096, 4096, 8), (64, 4096, 4096, 64), (100, 4096, 4096, 104), (128, 4096, 4096, 128), (129, 4096, 4096, 8),
-                              (257, 2064, 1024, 8), (1100, 2000, 640, 80), (2047, 2048, 2048, 128), (2048, 2048, 2048, 128), (137, 64, 260, 128)]:
+                              (257, 2064, 1024, 8), (1100, 2000, 640, 80), (2047, 2048, 2048, 128), (2048, 2048, 2048, 128), (137, 64, 260, 128),
+                              (138, 3472, 256, 16), (135, 4028, 144, 8), (137, 3000, 160, 128)]:     # 2^26.9, 2^26.2 and 2^25.97 multiply-adds
             d = describe(mode, M, N, K)
             assert d["a_tail"] == (str(rows) if d["operands"] != "converted" else "0"), (M, N, K, d)
     finally:

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from spoc_b200 import _lib as L
+from spoc_b200.plugin import _check
 from tests import oracle_lib as O
 from tests.gpu_util import CANARY, Dev, dev_from, gemm
 from tests.test_gpu_gemm import tol
@@ -21,14 +22,18 @@ def describe(mode, M, N, K, addressable):
     return out.value.decode()
 
 
-def check(backend, device, mode, M, N, K, lda, ldb, ldd, ldc):
+def check(backend, device, mode, M, N, K, lda, ldb, ldd, ldc, noalloc=False):
     rng = np.random.default_rng(M + N + K)
     a, b, c = (rng.uniform(-1, 1, (r, ld)).astype(np.float32) for r, ld in ((M, lda), (K, ldb), (M, ldc)))
     bias = rng.uniform(-0.1, 0.1, N).astype(np.float32)
     A, B, Cm, Bi = (dev_from(backend, device, x.ravel()) for x in (a, b, c, bias))
     D = Dev(backend, device, (M + 1) * ldd)
     try:
-        gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=ldc, ldd=ldd)
+        if noalloc:
+            args = (M, N, K, A.ptr, lda, B.ptr, ldb, D.ptr, ldd, 1.5, Cm.ptr, ldc, 0.5, Bi.ptr, L.ACT_RELU)
+            _check(L.load().sb200_gemm_f32_noalloc(device.id, 0, mode, *args))
+        else:
+            gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=ldc, ldd=ldd)
         got = D.download().reshape(M + 1, ldd)
         ref = O.gemm(np.ascontiguousarray(a[:, :K]).ravel(), np.ascontiguousarray(b[:, :N]).ravel(), M, N, K, 1.5, 0.5,
                      np.ascontiguousarray(c[:, :N]).ravel(), bias, 1)
@@ -40,8 +45,7 @@ def check(backend, device, mode, M, N, K, lda, ldb, ldd, ldc):
             x.free()
 
 
-# One row, a multiple of 8 and one off it, whole 128 rows, and beside whole ones 1, 8, 9 and 127 more (from 2^26 multiply-adds on those
-# have boxes of their own; a pair's second block then has some of the rows, or none).
+# One row, a multiple of 8 and one off it, whole 128 rows, and beside whole ones 1, 8, 9 and 127 more.
 TAILS = [(1, 132, 260), (7, 260, 132), (8, 64, 96), (9, 516, 516), (64, 132, 260), (65, 256, 300), (127, 132, 1028), (128, 64, 260), (129, 1028, 516),
          (136, 2052, 260), (137, 1028, 516), (255, 516, 516), (257, 1028, 260), (393, 260, 700)]
 
@@ -50,6 +54,23 @@ TAILS = [(1, 132, 260), (7, 260, 132), (8, 64, 96), (9, 516, 516), (64, 132, 260
 @pytest.mark.parametrize("M,N,K", TAILS)
 def test_rows_past_the_end(backend, device, mode, M, N, K):
     check(backend, device, mode, M, N, K, K, N, N, N)
+
+
+# Whole 128 rows and boxes of the others side by side, which takes 2^26 multiply-adds; a pair's second block has some of the rows, or none.
+BESIDE = [(138, 3472, 300, 16), (257, 1032, 260, 8), (393, 1028, 700, 16)]
+
+
+@pytest.mark.parametrize("operands", ["read in place", "copied", "allocation-free"])
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("M,N,K,tail", BESIDE)
+def test_rows_past_the_end_beside_whole_ones(backend, device, mode, M, N, K, tail, operands):
+    noalloc, pad = operands == "allocation-free", 1 if operands == "copied" else 0
+    if noalloc and mode not in (L.MODE_3XTF32, L.MODE_TF32):
+        pytest.skip("the allocation-free entry has the TF32 modes")
+    text = describe(mode, M, N, K, 1 - pad)
+    assert f" a_tail={tail} " in text, text
+    assert " splits=1 " in text or mode == L.MODE_3XTF32, text
+    check(backend, device, mode, M, N, K, K + pad, N + pad, N, N, noalloc)
 
 
 # (mode, M, N, K, splits): even and uneven shares of rows, rows and columns that end within a block's share, a last item that is shorter
