@@ -337,7 +337,7 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
         if (!VEC && elect_one()) bulk_wait_read<0>();  // (here for single elements: 2 % shorter than behind the closing barrier, as above)
         tc_fence_before_sync();
       }
-      if (item + item_step >= num_items) break;  // the block's last item: nothing follows but the barrier all threads share
+      if (in_cluster || item + item_step >= num_items) break;  // the block's last item: nothing follows but the barrier all threads share
       if (VEC && ok && elect_one()) bulk_wait_read<0>();  // the ring takes operands again once the stores have read their tiles
       // every warp is through with the accumulator and the tiles before the next item's operands arrive
       __syncwarp();

@@ -28,10 +28,13 @@ struct SplitCfg {
   // Groups of four warps that split.  A group needs 2000 cycles for a k-block, nearly all of it latency.  Tiles of 64 columns with two, three
   // and four groups: 1024^3 19.2, 17.1 and 19.2 us, 512^3 12.3, 11.3 and 12.9, 64 x 1024 x 1024 10.0, 9.2 and 9.3.
   static constexpr int kGroups = 3;
-  // Tiles of 128 columns and more: the registers of the last warpgroup go to the splitting ones, launched with 128 a thread
-  // (512 x 128 = 65536; 384 x 152 + 128 x 40 = 63488).  48 x 16384 x 4096 90.6 -> 83.6 us, 2304 x 2304 x 520 44.3 -> 43.2, 2048^3 69.6 -> 68.9,
-  // other sizes even; tiles of 64 columns need no more than 128.
+  // Tiles of 128 columns and more: registers of the last warpgroup go to the splitting ones, launched with 128 a thread.  48 x 16384 x 4096 90.6 ->
+  // 83.6 us, 2304 x 2304 x 520 44.3 -> 43.2, 2048^3 69.6 -> 68.9, other sizes even; tiles of 64 columns need no more than 128.  How many: with
+  // these no instance spills.  With 152 and 40 the divided ones of pairs did (300 bytes reloaded a thread; 1024^3 15.8 us and 15.2, 768^3 12.0 and
+  // 11.4, 5113 x 148 x 2772 29.9 and 29.2), and blocks on their own did a little.
   static constexpr bool kMoveRegs = BN > 64;
+  static constexpr int kRegsSplit = 144, kRegsRest = BN == 256 ? 64 : 56;
+  static_assert(kGroups * kRegsSplit + kRegsRest <= (kGroups + 1) * 128, "the warpgroups share what the block was launched with");
   static constexpr int kThreads = kGroups * 128 + (kMoveRegs ? 128 : 64);
   static constexpr uint32_t kABytes = ROWS * GEMM_BK * 4;
   static constexpr uint32_t kBBytes = kPartN * GEMM_BK * 4;
@@ -93,7 +96,8 @@ __device__ __forceinline__ void tf32_split(const float* x, uint32_t* hi, uint32_
 }
 
 // map_a, map_b: the caller's matrices without rounding, boxes of 32 x ROWS and of 32 x 32; map_a_tail: of 32 x p.a_tail_rows, for the last,
-// partial ROWS rows.  Rows past the end, and slabs of B past the last column, are not loaded (gemm_pair_kernel says what they cost).  IN_CLUSTER: a k-loop divided within a cluster, as in gemm_pair_kernel.
+// partial ROWS rows.  Rows past the end, and slabs of B past the last column, are not loaded (gemm_pair_kernel says what they cost).
+// IN_CLUSTER: a k-loop divided within a cluster, as in gemm_pair_kernel.
 template <int BN, int CTAS, int ROWS, bool IN_CLUSTER>
 __global__ void __launch_bounds__(SplitCfg<BN, CTAS, ROWS>::kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -166,7 +170,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   if (warp < GROUPS * 4) {
     // ----------------------------------------- split; then the epilogue
-    if constexpr (Cfg::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+    if constexpr (Cfg::kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsSplit));
     const int group = warp >> 2, quarter = warp & 3, tid = threadIdx.x & 127;
     const int row = quarter * 32 + lane;
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
@@ -240,7 +244,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
       }
       before += blocks;
-      if (group >= Cfg::kEpiGroups || !ok) continue;
+      if (group >= Cfg::kEpiGroups || !ok) {
+        if (IN_CLUSTER) break;  // its one item
+        continue;
+      }
       const int row0 = m0 + quarter * 32, c0 = n0 + group * EPI_N;
       const bool landed = mbar_wait_bounded(smem_u32(acc_full), local & 1, abort_flag);
       if (!__all_sync(0xffffffffu, landed)) {
@@ -267,7 +274,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           }
         }
       }
-      if (item + item_step >= num_items) break;  // nothing follows that would wait for the accumulator or the rings
+      if (IN_CLUSTER || item + item_step >= num_items) break;  // nothing follows that would wait for the accumulator or the rings
       if (elect_one()) bulk_wait_read<0>();  // the stores have read their tiles
       tc_fence_before_sync();
       __syncwarp();
@@ -293,7 +300,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       __syncwarp();
     }
   } else {
-    if constexpr (Cfg::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if constexpr (Cfg::kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsRest));
     if (warp == GROUPS * 4) {
       // ------------------------------------------------------ TMA producer
       if (elect_one()) {
