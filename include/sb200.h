@@ -289,7 +289,8 @@ SB200_API int sb200_gemm_f32(int dev, uint64_t stream, int mode,
  * device looks up the array's address and should come before any stream
  * capture.  Every call waits on `stream` until its kernels have finished and reads
  * a status word back with a synchronous copy: do not issue it on a stream that is
- * being captured.  Operand extents are checked as in sb200_gemm_f32. */
+ * being captured.  Operand extents are checked as in sb200_gemm_f32.  It divides no k-loop: the results are those of
+ * sb200_gemm_f32 to the last bit where that does not either (splits=1 in sb200_gemm_describe), and within its bounds elsewhere. */
 SB200_API int sb200_gemm_f32_noalloc(int dev, uint64_t stream, int mode,
                                      int64_t M, int64_t N, int64_t K,
                                      uint64_t A, int64_t lda, uint64_t B, int64_t ldb,

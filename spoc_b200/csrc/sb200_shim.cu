@@ -549,12 +549,15 @@ constexpr int kMaxSplits = 32;
 // SRC_SPLIT (gemm_split_kernel), measured on 1024 x 1024 x K and on 64 and 128 x 4096 x K: pairs 850, 645, 430 and 363 ns a k-block, blocks
 // on their own 540 and 375; a wave's epilogue overlaps nothing, so every wave has the fixed cost (4096 x 4096 x 512: 5.9 us a wave of
 // 128 columns, 8.7 of 256).  least_splits: no k-loop is divided into fewer, so that none is longer, and less exact, than in plain_route.
-// spread: a product that this leaves undivided, or divides through memory, is divided within clusters where the time that its k-loop saves
-// is more than the exchange takes, measured: 300 ns and what arrives at a block at 25 bytes a ns (3xTF32 and TF32 of 512^3 10.0 -> 8.4 and
-// 7.3 -> 6.9 us, 768^3 3xTF32 13.2 -> 12.1, 1024^3 16.1 -> 15.8, 512 x 1024 x 1024 15.7 -> 11.2 and 10.1 -> 8.8, 1024 x 1024 x 2048 TF32 16.1 -> 13.7),
-// by 5 % at least.  Of these estimates the fixed part is 1.6 us too long, which matters where what is fixed differs.  k-loops of fewer than 20
-// k-blocks: from 2^26 multiply-adds on, so that smaller ones keep the bits of the undivided kernels and of the allocation-free
-// entry (which costs 128 x 512 x 512 its 10.9 us instead of 8.5).
+// Within clusters this first choice prices the exchange as it was by 128-bit loads from the peers' shared memory (1500 ns and 2 ns a quad of a
+// block's share), against which its 8 % were fitted: what it takes in clusters keeps its cut, and with it its bits.
+// spread: a product that it leaves undivided, or divides through memory, is divided within clusters where the time that its k-loop saves
+// is more than the exchange takes as it is now: 300 ns and what arrives at a block at 25 bytes a ns (3xTF32 and TF32 of 512^3 10.0 -> 8.4 and
+// 7.3 -> 6.9 us, 768^3 3xTF32 13.2 -> 11.4, 1024^3 16.1 -> 15.2, 512 x 1024 x 1024 15.7 -> 11.2 and 10.1 -> 8.8, 1024 x 1024 x 2048 TF32 16.1 -> 13.7),
+// by 5 % at least.  Of these estimates the fixed part is 1.6 us too long, which matters where what is fixed differs.  Left undivided all the
+// same: k-loops of fewer than 20 k-blocks in products below 2^26 multiply-adds (2^27 in the fp16 modes, whose k-blocks of 64 count as 32 here).  It
+// keeps the bits of the smallest products what the allocation-free entry gives, which divides nothing (300 x 260 x 520), and costs time: with 16
+// to 19 k-blocks and divided in two, 3xTF32 took 0.80 of it on average, TF32 0.89, 3xF16 0.89 and f16 0.94 (80 products, 0.76 to 1.07).
 TileShape choose_tiles(long long M, long long N, long long kblocks, int ctas, int units, bool three, bool may_split, int fixed_splits = 0,
                        int src = SRC_DIRECT, bool no_scratch = false, int least_splits = 1, bool spread = false) {
   TileShape best;

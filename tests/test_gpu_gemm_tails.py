@@ -8,6 +8,7 @@ import pytest
 from spoc_b200 import _lib as L
 from spoc_b200.plugin import _check
 from tests import oracle_lib as O
+from tests import test_gpu_gemm_routes as routes
 from tests.gpu_util import CANARY, Dev, dev_from, gemm
 from tests.test_gpu_gemm import tol
 
@@ -35,6 +36,9 @@ def check(backend, device, mode, M, N, K, lda, ldb, ldd, ldc, noalloc=False):
         else:
             gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=ldc, ldd=ldd)
         got = D.download().reshape(M + 1, ldd)
+        if noalloc and " splits=1 " in describe(mode, M, N, K, 1):     # it divides no k-loop: where the other entry does not either, the same bits
+            gemm(backend, device, mode, M, N, K, A, B, D, alpha=1.5, C_=Cm, beta=0.5, bias=Bi, act=1, lda=lda, ldb=ldb, ldc=ldc, ldd=ldd)
+            assert np.array_equal(D.download().view(np.uint32), got.ravel().view(np.uint32))
         ref = O.gemm(np.ascontiguousarray(a[:, :K]).ravel(), np.ascontiguousarray(b[:, :N]).ravel(), M, N, K, 1.5, 0.5,
                      np.ascontiguousarray(c[:, :N]).ravel(), bias, 1)
         # the clamp halves the reference's mean square, alpha scales the error: as in the other epilogue tests
@@ -85,6 +89,17 @@ def test_k_loops_divided_by_the_second_choice(backend, device, mode, M, N, K, sp
     assert f"splits={splits} " in text, text
     pad = 4 if ldd == "quads" else 1        # rows of the result on 16-byte boundaries, and not
     check(backend, device, mode, M, N, K, K, N, N + pad, N + pad)
+
+
+# (mode, form, grid, block, M, N, K): parts of such products, by pairs and by blocks on their own, rows, columns and a last row that is cut short
+PARTS = [(mode, *part, 509, 516, 1028) for mode in MODES for part in (("tiled", (33, 7), 16), ("tiled", (20, 20), 16), ("naive", (70 * 516 + 100, 1), 1))]
+PARTS += [(L.MODE_3XTF32, "tiled", (64, 32), 16, 1024, 1024, 1024), (L.MODE_3XTF32, "tiled", (19, 48), 16, 768, 768, 768),
+          (L.MODE_TF32, "tiled", (63, 8), 16, 1001, 1000, 2052), (L.MODE_3XF16, "tiled", (63, 8), 16, 1001, 1000, 2052)]
+
+
+@pytest.mark.parametrize("mode,form,grid,side,M,N,K", PARTS)
+def test_a_part_has_the_bits_of_a_whole_divided_by_the_second_choice(backend, device, mode, form, grid, side, M, N, K):
+    routes.test_a_partial_launch_has_the_bits_of_the_whole(backend, device, mode, form, grid, side, M, N, K)
 
 
 @pytest.mark.parametrize("M,N,K,tail", [(257, 1032, 260, 8), (1100, 1000, 300, 80), (1153, 1024, 64, 8), (511, 2052, 132, 128)])

@@ -51,8 +51,8 @@ def test_noalloc_gemm_matches_regular_entry_point_twice_in_a_row(backend, device
     # first call: the larger K, so that the second call's shorter panels overlay stale data
     for (M, N, K, seed) in ((300, 260, 520, 11), (257, 515, 70, 12)):
         want, got, oracle = _both(backend, device, mode, M, N, K, seed)
-        # same kernels, same tile schedule: the two entry points agree to the last bit,
-        # which is tighter than the tolerance the other GEMM tests allow
+        # neither entry point divides these k-loops (splits=1 in sb200_gemm_describe): they agree to the last
+        # bit, which is tighter than the tolerance the other GEMM tests allow
         assert O.gemm_rel_error(got, want) <= bound
         assert np.array_equal(got, want)
         assert O.gemm_rel_error(got, oracle) <= bound
