@@ -228,9 +228,9 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
   constexpr bool in_cluster = IN_CLUSTER;
   const int split_rank = in_cluster ? static_cast<int>(cluster_ctarank()) : 0;
 
-  // Quads: a warp for the barriers, a lane each (64^3 5.7 -> 5.6 us).  Single elements: one thread, and below its own form of the coordinates and
-  // of the wait for the stores (with those of the quads 2 to 4 % longer: 9 x 1257 x 64 7.7 and 8.0 us, 7 x 5363 x 246 14.4 and 14.9; the difference is
-  // in what the compiler makes of the kernel, whose registers are all taken, and not in the set-up's time).
+  // Quads: a warp for the barriers, a lane each (64^3 5.7 -> 5.6 us).  Single elements: one thread, and below their own place of the wait for the
+  // stores (with those of the quads up to 4 % longer: 7 x 5363 x 246 14.3 and 14.7 us, 4731 x 18 x 148 11.1 and 11.6; the difference is in
+  // what the compiler makes of the kernel, whose registers are all taken, and not in the set-up's time).
   auto barrier_count = [](int i) { return i < STAGES ? CONV_WARPS : 1; };  // full, empty, done, recv
   constexpr int BARS = 2 * STAGES + 2;
   static_assert(BARS <= 32, "a lane a barrier");
@@ -276,11 +276,8 @@ gemm_convert_kernel(const ConvOperands o, const __grid_constant__ CUtensorMap ma
     bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step, ++local) {
       int tm, tn;
-      if constexpr (VEC)
-        item_tile_coords(item, p, num_tiles, tm, tn);
-      else
-        pair_tile_coords(item % num_tiles, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
-      const int m0 = tm * 128, n0 = tn * BN, split = VEC ? item_split(item, num_tiles) : item / num_tiles;
+      item_tile_coords(item, p, num_tiles, tm, tn);
+      const int m0 = tm * 128, n0 = tn * BN, split = item_split(item, num_tiles);
       const int kb0 = split * p.split_k_blocks, blocks = min(p.num_k_blocks - kb0, p.split_k_blocks);
       ConvTile<BN, VEC> t[CONV_AHEAD + 1];
 #pragma unroll

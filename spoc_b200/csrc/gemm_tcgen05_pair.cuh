@@ -68,16 +68,6 @@ __device__ __forceinline__ void pair_soft_epoch(unsigned int* ctr, unsigned int 
   }
 }
 
-// Tile coordinates for gemm_convert_kernel on single elements (item_tile_coords for all others).
-__device__ __forceinline__ void pair_tile_coords(int tile, int tiles_m, int tiles_n, int group_m, int& tm, int& tn) {
-  const int band_tiles = group_m * tiles_n;
-  const int band = tile / band_tiles;
-  const int within = tile - band * band_tiles;
-  const int first_m = band * group_m;
-  const int band_m = min(group_m, tiles_m - first_m);
-  tm = first_m + within % band_m;
-  tn = within / band_m;
-}
 // Which part of a divided k-loop work item `item` is: item / num_tiles, without the division where it is 0.
 __device__ __forceinline__ int item_split(int item, int num_tiles) {
   return item < num_tiles ? 0 : static_cast<int>(static_cast<unsigned int>(item) / static_cast<unsigned int>(num_tiles));
@@ -532,11 +522,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
               load(sp + 2 * PAIR_A_BYTES + B_BYTES, map_b_x, kb * 64, n0, pol_b);
             } else {
               // main stage: two consecutive k-blocks of 32 of the caller's A and B
-  #pragma unroll
+#pragma unroll
               for (int h = 0; h < 2; ++h) {
                 uint8_t* hp = sp + h * (PAIR_A_BYTES + B_BYTES);
                 load(hp, map_a_hi, kb * 64 + 32 * h, m0, pol_a);
-  #pragma unroll
+#pragma unroll
                 for (int sl = 0; sl < SLABS; ++sl) load(hp + PAIR_A_BYTES + sl * 4096, map_b_hi, n0 + 32 * sl, kb * 64 + 32 * h, pol_b);
               }
             }
