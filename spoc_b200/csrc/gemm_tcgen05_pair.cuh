@@ -715,7 +715,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_cons
       tc_fence_before_sync();
       hand_back();
     }
-    __syncwarp();
     if (!ok && elect_one()) wait_for_copies();  // tiles of C
     __syncwarp();
   }
