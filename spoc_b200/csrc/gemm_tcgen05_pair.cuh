@@ -12,7 +12,8 @@
 // accumulator rows and hand the accumulator back by arriving on the leader's `tmem_empty` barrier, while the MMA warp
 // already works on the next tile in the other accumulator.  On a block's last tile, behind which nothing is left to hide the epilogue,
 // warps 6-9 (of pairs' tiles of 128 columns and more) take the right half of the columns, with staging tiles in the operand ring, which is
-// idle then: 2048^3 TF32 27.4 -> 26.3 us, with C, bias and clamp 30.2 -> 27.6, 3xF16 59.1 -> 55.1, 1280^3 TF32 13.8 -> 13.4.
+// idle then.  Passes repeated on the same operands: 2048^3 TF32 27.4 -> 26.3 us, with C, bias and clamp 30.1 -> 27.6, 3xF16 with them 60.3 -> 57.0,
+// 1280^3 TF32 14.6 -> 14.2.
 // Every TMA load is issued by the block that consumes it (plain per-block loads).
 #pragma once
 #include <type_traits>
@@ -353,9 +354,9 @@ __device__ __forceinline__ bool cluster_exchange(const GemmParams& p, const uint
 // halves instead of 32 floats, so a k-block spans 64 k and a k-step 16, in the same bytes, descriptors and cycles as the TF32
 // forms.  MODE 2: fp16 panels, one MMA.
 // map_a_x, map_b_x, but for the mixed mode: the high and low parts of A once more, for the last, partial 128 rows, with boxes of p.a_tail_rows.
-// TMA takes 3 ns for a row past the end when a few blocks ask for such rows and 15 ns when all do, so that few rows went slower than 128 (TF32
-// x 6144 x 1024: 10 rows 53 us, with their own boxes 9; 64 x 4096 x 4096 with epilogue 17.0 -> 13.3).  The accumulator's rows that nothing was
-// loaded for come of whatever the ring held, and are not stored.
+// TMA takes 3 ns for a row past the end when a few blocks ask for such rows and 15 ns when all do, so that few rows went slower than 128.  Passes
+// repeated on the same operands: TF32 10 x 6144 x 1024 30.0 -> 9.0 us, 64 x 4096 x 4096 with epilogue 17.0 -> 13.1 (16.4 with operands that come
+// from HBM).  The accumulator's rows that nothing was loaded for come of whatever the ring held, and are not stored.
 // MODE 5 (mixed; always SRC_DIRECT): map_a_hi / map_b_hi are TFLOAT32 maps over the caller's matrices, map_a_lo / map_b_lo lie
 // over the fp16 panels of the high parts and map_a_x / map_b_x over those of the low parts (all K-major, [rows x Kp], Kp a
 // multiple of 64).  A tile is computed in three runs of stages, every stage the same bytes: K/64 cross stages (the four fp16

@@ -815,7 +815,8 @@ int launch_split_for(int bn, int ctas, int dev_index, int sm_count, cudaStream_t
 
 size_t partial_bytes(long long M, long long N, const TileShape& shape, int ctas, int sm_count) {
   const int splits = shape.splits;
-  return splits > 1 && !split_in_cluster(tiles_of(M, N, shape.tile_n, ctas), splits, ctas, sm_count) ? static_cast<size_t>(round_up(M, 32)) * round_up(N, 4) * 4 * splits : 0;
+  if (splits <= 1 || split_in_cluster(tiles_of(M, N, shape.tile_n, ctas), splits, ctas, sm_count)) return 0;
+  return static_cast<size_t>(round_up(M, 32)) * round_up(N, 4) * 4 * splits;
 }
 
 template <int MODE, int SRC>
@@ -1126,8 +1127,8 @@ int launch_gemm_mode(DeviceState& d, cudaStream_t st, long long M, long long N, 
   }
   const bool direct = route.src == SRC_DIRECT;
   const int tile_n = route.tile_n;
-  unsigned int* epoch_ring =
-      route.ctas == 2 && route.splits == 1 && route.src != SRC_SPLIT ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;  // zeroed ahead of the preparation launch
+  // zeroed ahead of the preparation launch
+  unsigned int* epoch_ring = route.ctas == 2 && route.splits == 1 && route.src != SRC_SPLIT ? next_epoch_ring(d, st, kp / GEMM_BK, MODE == 3) : nullptr;
   const bool prof = g_profiling.load() != 0;
   DeviceState::ProfRec rec{nullptr, nullptr, nullptr};
   if (prof) {
