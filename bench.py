@@ -36,7 +36,7 @@ M = N = K = 8192
 SEED = 20260101
 MAP_N = 1 << 28
 METRIC = "fp32_gemm_fused_epilogue_8192cubed"
-WORKLOAD = "gemm M=N=K=8192 fp32 in/out, D=max(0,1.5*A.B+0.5*C+bias[col]), seeded uniform inputs (BASELINE configs[2])"
+WORKLOAD = "gemm M=N=K=8192 fp32 in/out, D=max(0,1.5*A.B+0.5*C+bias[col]), seeded uniform inputs"
 NOMINAL_TF32_TFLOPS = 1100.0   # dense TF32 tensor peak of a B200, nominal
 NOMINAL_HBM_GBS = 8000.0
 
@@ -163,7 +163,7 @@ class ClockSampler:
 
 # --------------------------------------------------------------------------- reference arm
 def oracle_lib():
-    from tests import oracle_lib as O  # the checker doubles as the timed CPU baseline
+    from tests import oracle_lib as O  # the oracle doubles as the timed CPU baseline
     return O
 
 
@@ -658,7 +658,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
             mm_args += [RSA_Buffer(buf_of(t), t.numel()), RSA_Int32(t.numel())]
         mm_args += [RSA_Int32(S1)] * 3
         mm_src = sarek_ir.matmul_tiled_ir()
-        cfg1 = {"workload": "gemm M=N=K=1024 (BASELINE configs[0]) through the matrix_mul_tiled IR, block 16x16, grid 64x64"}
+        cfg1 = {"workload": "gemm M=N=K=1024 through the matrix_mul_tiled IR, block 16x16, grid 64x64"}
         for mode, label in ((L.MODE_3XTF32, "3xtf32"), (L.MODE_TF32, "tf32")):
             backend.set_mode(mode)
             mm = lambda: backend.run_source(source=mm_src, lang=lang, kernel_name="sarek_kern", block=dims2d(16, 16),
@@ -970,7 +970,7 @@ def oracle_parity(ctx, D_rows_fn, A, B, M_rows, N, K, row_ids, a_row_fn, c_row_f
 
 
 def gather_leg(ctx, S: int, steps: int, warmup: int) -> dict:
-    """Strong scaling of the large square GEMM with epilogue and a gathered result (BASELINE configs[4]): M = N = K = S,
+    """Strong scaling of the large square GEMM with epilogue and a gathered result: M = N = K = S,
     rows of A/C/D split over the ranks, B replicated by NCCL broadcast.  Two ways to leave the whole D on every GPU
     are timed: the GEMM followed by an NCCL all-gather of the row blocks, and the GEMM whose epilogue stores each
     tile into every GPU's copy (peer stores over NVLink).  The two forms alternate over three rounds so that a
@@ -1078,7 +1078,7 @@ def gather_leg(ctx, S: int, steps: int, warmup: int) -> dict:
     return {
         "metric": f"fp32_gemm_fused_epilogue_{S}cubed_gathered", "unit": "TFLOP/s", "n_gpus": world, "steps": steps,
         "scaling": "strong", "dtype": "tf32x3 (f32 in/out)",
-        "workload": f"gemm M=N=K={S} with epilogue (BASELINE configs[4]), rows of A/C/D split over the GPUs, whole D on every GPU",
+        "workload": f"gemm M=N=K={S} with epilogue, rows of A/C/D split over the GPUs, whole D on every GPU",
         "value": flops / (ms_fused * 1e-3) / 1e12, "ms_per_step": ms_fused,
         "gemm_then_nccl_all_gather": {"value": flops / (ms_nccl * 1e-3) / 1e12, "ms_per_step": ms_nccl, "rounds_ms": rounds["nccl"]},
         "gather_fused_in_epilogue": {"value": flops / (ms_fused * 1e-3) / 1e12, "ms_per_step": ms_fused, "rounds_ms": rounds["fused"],
@@ -1105,7 +1105,7 @@ def run_gather(args, rank: int, local_rank: int, world: int) -> None:
 
 
 def skinny_leg(ctx, steps: int, warmup: int) -> dict:
-    """Strong scaling of the skinny GEMM (BASELINE configs[3]): C = A.B with M = 65536, N = K = 4096, rows of A drawn
+    """Strong scaling of the skinny GEMM: C = A.B with M = 65536, N = K = 4096, rows of A drawn
     from N(0,1), B from N(0,1/sqrt(K)); rows of A and C split over the ranks, B broadcast from rank 0 (NCCL).  Timed
     with B already on every GPU and with the broadcast of B inside every timed step, in both modes, the two variants
     alternating over three rounds (median); sampled rows of every rank's block are checked against the CPU oracle."""
@@ -1167,7 +1167,7 @@ def skinny_leg(ctx, steps: int, warmup: int) -> dict:
     torch.cuda.empty_cache()
     return {"metric": "fp32_gemm_65536x4096x4096_row_sharded", "unit": "TFLOP/s", "n_gpus": world, "steps": steps,
             "scaling": "strong", "dtype": "tf32x3, tf32 and tf32 + 2 x f16 cross terms (f32 in/out)",
-            "workload": "gemm M=65536 N=K=4096 (BASELINE configs[3]), A ~ N(0,1), B ~ N(0,1/sqrt(K)), rows of A/C split over the "
+            "workload": "gemm M=65536 N=K=4096, A ~ N(0,1), B ~ N(0,1/sqrt(K)), rows of A/C split over the "
                         "GPUs, B broadcast from rank 0 (64 MiB, NCCL)",
             "value": out["3xtf32"]["b_resident"]["value"], "ms_per_step": out["3xtf32"]["b_resident"]["ms_per_step"],
             "modes": out, "parity_ok": parity_ok, "parity_worst_over_bound": parity_rel,

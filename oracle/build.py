@@ -2,7 +2,7 @@
 
 The reference is OCaml and cannot be compiled on this toolchain (no ocaml,
 dune or opam), so there is no oracle/_ref: the C restatement is the only
-checker.  Run as ``python oracle/build.py``.
+one.  Run as ``python oracle/build.py``.
 """
 from __future__ import annotations
 

@@ -2,7 +2,7 @@
  * native_oracle.c — CPU restatement of the Sarek *Native* backend's arithmetic
  * for the dense-GEMM and element-wise map kernels.
  *
- * THIS FILE IS TEST INFRASTRUCTURE.  It is the checker the CUDA path is
+ * THIS FILE IS TEST INFRASTRUCTURE.  It is the oracle the CUDA path is
  * compared against and the timed CPU baseline; it is never linked into, loaded
  * by or called from the product library.
  *

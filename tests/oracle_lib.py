@@ -1,6 +1,6 @@
 """ctypes access to the CPU oracle (oracle/native_oracle.c) for the tests.
 
-The oracle is the checker only: nothing under spoc_b200/ imports this.
+The oracle is for comparison only: nothing under spoc_b200/ imports this.
 """
 from __future__ import annotations
 
